@@ -91,10 +91,14 @@ struct DevState {
     uint64_t nbuckets = 0;
     uint32_t* pos = nullptr;
     uint64_t num_index = 0;
+    // shape of a table that holds every seed window of the resident target
+    // (built here at step 1), else 0
+    uint64_t table_full = 0;
     Packed qf[kMaxBuffers], qr[kMaxBuffers];
     uint32_t* qkeys[kMaxBuffers][2] = {};  // per-position seed keys (batched seeding)
     uint64_t qkeys_cap[kMaxBuffers][2] = {};  // bytes allocated for qkeys
     bool qkeys_ok[kMaxBuffers][2] = {};       // qkeys hold the keys of the resident query
+    uint64_t qkeys_shape[kMaxBuffers][2] = {};  // shape they were computed with (sa_shape_id)
     char* stage = nullptr;                 // text staging of uploads (grow-only)
     uint64_t stage_cap = 0;
     std::vector<Slot*> slots;
@@ -120,6 +124,7 @@ struct Slot {
     uint64_t graph_key = 0;
     uint64_t graph_kernels = 0;
     bool graph_off = false;  // capture failed once: launch directly
+    bool no_sweep = false;   // the call at hand runs without the sweep (its list was too small)
     uint32_t max_units = 64;  // units per batched pass (batched kinds)
 };
 
@@ -319,6 +324,7 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
     w.seed_cap = seed_cap;
     w.surv_cap = surv_cap;
     w.long_cap = long_cap;
+    w.list_cap = std::min<uint64_t>(surv_cap, env_u64("SA_LIST_CAP", ~0ull)) & ~31ull;
     const uint64_t nunits = batch ? std::max<uint64_t>(64, std::min<uint64_t>(units, SA_MAX_UNITS)) : 64;
     s->max_units = (uint32_t)nunits;
     std::vector<Part> parts = {
@@ -357,7 +363,6 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         {(void**)&w.bounds, batch ? 8 * nunits * SA_BATCH_ITERS : 0},
         {(void**)&w.unit_iters, batch ? 4 * nunits : 0},
     };
-    w.flags = nullptr;
     uint64_t total = 0;
     for (auto& p : parts) total += (p.bytes + 255) & ~255ull;
     cudaError_t e = cudaMalloc(&s->arena, total);
@@ -457,8 +462,13 @@ uint64_t max_hits_now() {
     return g.max_hits_override ? g.max_hits_override : g.max_hits_default;
 }
 
-// One SeedAndFilter call on a slot: seeds -> hits -> X-drop -> dedup -> host.
-// mode 0 = plain, 1 = repeat masker.
+// Whether a call on this device may chain hits of one diagonal: the resident
+// table holds every seed window of the resident target for the shape in use.
+bool chains_allowed(const DevState& d) {
+    const Global& g = G();
+    return d.table_full != 0 && d.table_full == sa_shape_id(g.params) && sa_chain_params(g.params, g.tuning);
+}
+
 // Device work of one plain (mode 0) or rm (mode 1) call once its seed words
 // are on the device: descriptor uploads from the slot's pinned buffers,
 // counters reset, lookup, extension, dedup and the counters' copy back.
@@ -474,10 +484,13 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     SA_CUDA_OK(cudaMemcpyAsync(w.units, s->h_units, sizeof(SaUnit), cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.scope_flags, s->h_scope_flags, 4 * SA_MAX_ITERS, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
-    sa_launch_lookup_seeds(w, d.index, (uint32_t)d.nbuckets, g.params, Gr, st);
+    const bool chain = chains_allowed(d) && !s->no_sweep;
+    sa_launch_lookup_seeds(w, d.index, (uint32_t)d.nbuckets, g.params, Gr, st, chain);
     sa_launch_hash_init(w, false, st);
     tm.mark(1);
     SaExtendArgs xa;
+    xa.chain = chain ? 1 : 0;
+    xa.sweep = s->no_sweep ? 0 : 1;
     xa.ref = d.ref.data;
     xa.ref_len = (uint32_t)d.ref.len;
     xa.pos_table = d.pos;
@@ -509,7 +522,7 @@ int run_chain(Slot* s, int mode, PhaseTimer& tm) {
     if (!graphs_enabled() || s->graph_off || tm.on) return launch_call_chain(s, mode, tm);
     Global& g = G();
     cudaStream_t st = s->stream;
-    const uint64_t key = (g_graph_gen.load() << 1) | (uint64_t)mode;
+    const uint64_t key = (g_graph_gen.load() << 2) | (uint64_t)(s->no_sweep ? 2 : 0) | (uint64_t)mode;
     if (!s->graph || s->graph_key != key) {
         if (s->graph) cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
@@ -562,17 +575,23 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     u[0].rm_lo = rm_lo;
     u[0].rm_hi = rm_hi;
     u[0].flags = mode == 1 ? (1u | (rev ? 2u : 0u)) : 0u;
+    u[0].j_lo = n ? (uint32_t)seeds[0] : 0u;
+    u[0].j_hi = n ? (uint32_t)seeds[n - 1] + 1u : 0u;
     for (int i = 0; i < SA_MAX_ITERS; ++i)
         s->h_scope_flags[i] = (rev ? 1u : 0u) | ((mode == 1 && g.rm_exclude_diag) ? 2u : 0u);
     PhaseTimer tm(s);
     tm.mark(0);
     SA_CUDA_OK(cudaMemcpyAsync(w.seeds, seeds, 8ull * n, cudaMemcpyHostToDevice, st));
-    if (!w.hash_clean) sa_launch_hash_clear(w, st);
-    w.hash_clean = false;  // until this call is seen to complete
-    SA_TRY(run_chain(s, mode, tm));
-    SA_CUDA_OK(cudaStreamSynchronize(st));
-    SaCounters c = *s->h_ctr;
-    sa_note_hash_state(w, c);
+    SaCounters c;
+    for (s->no_sweep = false;; s->no_sweep = true) {
+        if (!w.hash_clean) sa_launch_hash_clear(w, st);
+        w.hash_clean = false;  // until this call is seen to complete
+        SA_TRY(run_chain(s, mode, tm));
+        SA_CUDA_OK(cudaStreamSynchronize(st));
+        c = *s->h_ctr;
+        sa_note_hash_state(w, c);
+        if (c.list_count <= w.list_cap) break;
+    }
     std::memset(&t_stats, 0, sizeof t_stats);
     t_stats.num_seeds = n;
     t_stats.num_hits = c.num_hits;
@@ -662,6 +681,7 @@ int ensure_keys(DevState& d, uint32_t buffer, int rev) {
     sa_launch_query_keys(q.data, q.len, g.params, d.qkeys[buffer][rev], 0);
     SA_CUDA_OK(cudaDeviceSynchronize());
     d.qkeys_ok[buffer][rev] = true;
+    d.qkeys_shape[buffer][rev] = sa_shape_id(g.params);
     return SA_OK;
 }
 
@@ -693,7 +713,7 @@ struct BatchResult {
 // Runs units [u0, u1) in one device pass.  Returns SA_ERR_CAPACITY when the
 // survivors do not fit (the caller splits the range).
 int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t u0, uint32_t u1, bool want_out,
-                    BatchResult& res) {
+                    BatchResult& res, bool sweep = true) {
     Global& g = G();
     SaWork& w = s->w;
     cudaStream_t st = s->stream;
@@ -703,6 +723,7 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     std::vector<SaBatchUnit> bu(n);
     SaUnit* hu = s->h_units;
     uint64_t slots = 0;
+    bool chain = sweep && chains_allowed(d);
     for (uint32_t i = 0; i < n; ++i) {
         const SaResolvedUnit& u = units[u0 + i];
         bu[i].slot_begin = slots;
@@ -716,6 +737,9 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
         hu[i].q_len = u.q_len;
         hu[i].rm_lo = hu[i].rm_hi = 0;
         hu[i].flags = 0;
+        hu[i].j_lo = u.start;
+        hu[i].j_hi = u.end;
+        chain = chain && !u.seeds && u.shape == d.table_full;  // keys of every window of [start, end)
         slots += sa_unit_slots(u, S);
     }
     SaCallDesc* hd = s->h_desc;
@@ -745,6 +769,14 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     xa.xdrop = g.params.xdrop;
     xa.hspthresh = g.params.hspthresh;
     xa.noentropy = g.params.noentropy;
+    xa.chain = chain ? 1 : 0;
+    xa.sweep = sweep ? 1 : 0;
+    // so many seed slots that the hits may need several segments: read their number
+    if ((double)slots * ((double)d.num_index / (double)d.nbuckets + 1.0) > (double)w.list_cap) {
+        SA_CUDA_OK(cudaMemcpyAsync(s->h_ctr, w.ctr, sizeof(SaCounters), cudaMemcpyDeviceToHost, st));
+        SA_CUDA_OK(cudaStreamSynchronize(st));
+        xa.hits = s->h_ctr->num_hits;
+    }
     sa_launch_extend_lane(w, xa, g.params, g.tuning, d.num_sms, st);
     tm.mark(2);
     sa_launch_extend_warp(w, xa, g.params, g.tuning, d.num_sms, st);
@@ -757,6 +789,7 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     SaCounters c = *s->h_ctr;
     sa_note_hash_state(w, c);
     if (c.hash_overflow || c.error == 4) return SA_ERR_CAPACITY;
+    if (c.list_count > w.list_cap) return run_batch_group(d, s, units, u0, u1, want_out, res, false);
     if (c.error) return map_device_error(c.error);
     res.tot.num_hits += c.num_hits;
     res.tot.extended += c.extended;
@@ -1370,6 +1403,7 @@ int sa_generate_shape_pos(const char* shape) {
         return SA_ERR_ARG;
     }
     Global& g = G();
+    invalidate_graphs();
     set_shape_positions(g.params, pat);
     g.shape_set = true;
     return k;
@@ -1384,7 +1418,10 @@ int sa_send_ref_write_request(const char* seq, size_t start_addr, uint32_t len) 
         return SA_ERR_STATE;
     }
     if (!seq) return SA_ERR_ARG;
-    for (auto& d : g.devs) SA_TRY(upload_pack(d, seq + start_addr, len, d.ref, nullptr));
+    for (auto& d : g.devs) {
+        d.table_full = 0;  // a table of the target before
+        SA_TRY(upload_pack(d, seq + start_addr, len, d.ref, nullptr));
+    }
     g.last_ref_ptr = seq;
     g.last_ref_start = start_addr;
     g.last_ref_len = len;
@@ -1405,6 +1442,7 @@ int sa_clear_ref(void) {
         if (d.pos) cudaFree(d.pos);
         d.index = d.pos = nullptr;
         d.nbuckets = d.num_index = 0;
+        d.table_full = 0;
     }
     g.last_ref_ptr = nullptr;
     return SA_OK;
@@ -1494,8 +1532,10 @@ int sa_generate_seed_pos_table(const char* ref_str, size_t start_addr, uint32_t 
     const bool resident = ref_str == g.last_ref_ptr && start_addr == g.last_ref_start &&
                           ref_length == g.last_ref_len && g.last_ref_ptr;
     for (auto& d : g.devs) {
+        d.table_full = 0;
         if (resident && d.ref.data) {
             SA_TRY(build_table_on(d, d.ref, step));
+            if (step == 1) d.table_full = sa_shape_id(g.params);
         } else {
             if (!ref_str) return SA_ERR_ARG;
             Packed tmp;
@@ -1527,6 +1567,7 @@ int sa_send_seed_pos_table(const uint32_t* index_table, uint32_t index_table_siz
         }
     for (auto& d : g.devs) {
         SA_CUDA_OK(cudaSetDevice(d.dev));
+        d.table_full = 0;
         if (d.index) cudaFree(d.index);
         if (d.pos) cudaFree(d.pos);
         d.index = d.pos = nullptr;
@@ -1808,6 +1849,7 @@ int sa_seed_and_filter_batch(const sa_unit* units, uint32_t n_units, sa_segment*
         const Packed& q = rev ? d.qr[units[i].buffer] : d.qf[units[i].buffer];
         ru[i] = SaResolvedUnit{d.qkeys[units[i].buffer][rev], q.data, (uint32_t)q.len, units[i].start, units[i].end,
                                rev};
+        ru[i].shape = d.qkeys_shape[units[i].buffer][rev];
     }
     BatchResult res;
     std::vector<int64_t> map;

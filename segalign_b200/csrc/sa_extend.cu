@@ -30,7 +30,6 @@
 #include "sa_radix.cuh"
 
 #define SA_FULL 0xffffffffu
-#define SA_LANE_TABLES 256  // lane kernel: the 64-entry score table
 
 struct SaExtK {
     const uint32_t* ref;
@@ -49,6 +48,18 @@ struct SaExtK {
     uint32_t substeps;  // steps per lane-kernel iteration (at most)
     uint32_t switch_now;  // 1: a lane starts its left side in the step after its right side ends
     uint32_t windowed;    // 1: hits outside their unit's rm window are dropped from the tiles
+    // chains of hits on one diagonal (see there); chain = 0: every hit is scanned
+    uint32_t chain;
+    uint32_t gap;         // largest distance to the hit before
+    int32_t match, swing; // smallest match score, and that minus the lowest mismatch score
+    uint32_t mismatches;  // as many mismatches in a row cannot stop a scan
+    uint32_t shift[16];   // shape positions, the first one again in the unused places
+    uint4* list;          // hits the sweep leaves to the lane kernel: {rl, ql, scope, unit | SA_CHAIN_NEXT}
+    uint64_t list_cap;    // 0: no sweep
+    // scanned hits that others may follow [list_cap]: {rl, ql, unit, bases left of
+    // the hit}, position of the right end, stop words right and left
+    uint4* lead;
+    uint32_t *lead_right, *lead_stop_r, *lead_stop_l;
 };
 
 // Reverse the order of the 8 nibbles of a word.
@@ -204,6 +215,405 @@ __device__ __forceinline__ void sa_window_exact(const char* tblb, uint32_t lo, u
     }
 }
 
+// ---------------------------------------------------------------------------
+// Chains: hits of one diagonal that give the same HSP are scanned once.
+//
+// Let T be the running sum of substitution scores along a diagonal, and a hit
+// at p scan right from p and left from p.  Take hits p' < p of one diagonal.
+// If T(p) > T(y) for all y in [p', p) and the scan from p' does not stop before
+// p, the right scan from p' has its best at or after p; from p on both scans
+// see the same maxima, so they stop at the same base and end the HSP at the
+// same base.  Likewise on the left if some x <= p' has T(x) < T(y) for all y in
+// (x, p] and the scan from p does not stop before x.  Both hold: one HSP, one
+// score, the same stops.  A hit p is therefore dropped when its nearest
+// predecessor p' on the diagonal is at most `gap` bases back and the two
+// conditions hold on the 32 bases before p with every match scored `match`
+// (the smallest match score) and every mismatch at its lowest: such sums are
+// lower bounds, so what they show positive is positive (sa_chain_joined).  At
+// most `mismatches` of the 32 may differ: then no drop exceeds xdrop and no
+// scan stops among them.
+//
+// Which hits there are is read off the two sequences: the table holds every
+// window of the target, the call's seeds every window of [j_lo, j_hi)
+// (checked by the lookup; else ctr->chain_bad), so a hit ends at p exactly if
+// the shape's positions match in the seed_size bases before p (one transition
+// allowed when the call has them).  Whether p is dropped depends on those 32
+// bases and on fixed limits only (predecessors lie in p's block of
+// SA_CHAIN_BLOCK query positions, which bounds a chain's length, and in the
+// call's window), so the hit that starts a chain finds the dropped ones
+// that follow it by the same test (sa_chain_members) and counts their tiles and
+// survivors: the call's statistics stay those of every hit scanned.
+//
+// On the genome workload 13-16% of the hits are dropped, with them a third to
+// two fifths of all 32-base scan steps (they are the hits inside long HSPs);
+// on repeat-rich targets half the steps, in a self-alignment nine of ten.
+// ---------------------------------------------------------------------------
+#define SA_CHAIN_BLOCK 1024u
+#define SA_CHAIN_NEXT 0x80000000u  // unit bit: a hit follows on the diagonal within `gap` bases
+
+// Bit 4k of v (k = 0..7) -> bit 24 + k of the result (lower bits are left over).
+__device__ __forceinline__ uint32_t sa_nibble_bits(uint32_t v) {
+    return ((v | (v >> 3)) & 0x03030303u) * 0x01041040u;
+}
+
+__device__ __forceinline__ uint32_t sa_join_bits(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3) {
+    return __byte_perm(__byte_perm(b0, b1, 0x0073), __byte_perm(b2, b3, 0x0073), 0x5410);
+}
+
+// Match and transition bits of 8 bases, as sa_nibble_bits gives them.
+template <bool TRANS>
+__device__ __forceinline__ void sa_match_bits(uint32_t rw, uint32_t qw, uint32_t& m, uint32_t& t) {
+    const uint32_t d = rw ^ qw, d1 = d >> 1, d2 = d >> 2;
+    m = sa_nibble_bits(~(d | d1 | d2) & 0x11111111u);
+    t = TRANS ? sa_nibble_bits(d1 & ~d & ~d2 & 0x11111111u) : 0u;  // codes differ by 2: A-G, C-T
+}
+
+// Bit b = 1: a seed match starts at bit b + off of the 64-base masks
+// (m0, m1: matches; t0, t1: transitions).  off + shape position <= 32.
+template <bool TRANS>
+__device__ __forceinline__ uint32_t sa_seed_bits(const SaExtK& a, int kmer, uint32_t m0, uint32_t m1, uint32_t t0,
+                                                 uint32_t t1, uint32_t off) {
+    uint32_t all = ~0u, one = 0;
+    if (!TRANS) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) all &= __funnelshift_rc(m0, m1, off + a.shift[i]);
+        return all;
+    }
+    for (int i = 0; i < kmer; ++i) {
+        const uint32_t m = __funnelshift_rc(m0, m1, off + a.shift[i]), t = __funnelshift_rc(t0, t1, off + a.shift[i]);
+        one = (one & m) | (all & t);
+        all &= m;
+    }
+    return all | one;
+}
+
+// The two conditions on the 32 bases before p, predecessor `delta` bases back.
+// mis bit k: base p - 32 + k differs.  c(o) = match * o - swing * (mismatches
+// among the o bases before p) bounds T(p) - T(p - o) from below: c(o) > 0 for
+// 1 <= o <= delta, and a new maximum of c at some o >= delta.
+__device__ __forceinline__ bool sa_chain_joined(const SaExtK& a, uint32_t mis, uint32_t delta) {
+    uint32_t r = __brev(mis);  // bit i: base p - 1 - i
+    if ((uint32_t)__popc(r) > a.mismatches) return false;
+    const uint32_t before = r & ((1u << (delta - 1)) - 1u), upto = r & ((1u << delta) - 1u);
+    int near = max(0, a.match * (int)(delta - 1) - a.swing * __popc(before));  // max of c below delta
+    const int last = max(a.match * (int)delta - a.swing * __popc(upto), a.match * 32 - a.swing * __popc(r));
+    int c0 = a.match;  // c(i) = match * i + c0 - match before the k-th mismatch, c0 falling by swing each time
+    for (; r; r &= r - 1) {
+        const int i = __ffs(r) - 1;
+        const int c = a.match * i + c0 - a.match;  // before the mismatch at o = i + 1
+        if (i < (int)delta) {
+            near = max(near, c);
+            if (c + a.match - a.swing <= 0) return false;
+        } else if (c > near) {
+            return true;
+        }
+        c0 -= a.swing;
+    }
+    return last > near;
+}
+
+// One hit: 0 = scan it, 1 = dropped, SA_CHAIN_NEXT = scan it, and a hit follows
+// within `gap` bases.  r, q: the 6 words (48 bases) from 32 bases before p.
+template <bool TRANS>
+__device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, const SaUnit& U, uint32_t rl, uint32_t ql,
+                                                  const uint32_t* r, const uint32_t* q) {
+    const uint32_t S = a.seed_size, own = 32 - S, j = ql - S;
+    uint32_t back = min(min(a.gap, j & (SA_CHAIN_BLOCK - 1)), min(j - U.j_lo, rl - S - 1));  // position 0 is not in the table
+    uint32_t ahead = min(a.gap, U.j_hi - 1 - j);
+    if (U.flags & 1u) {
+        back = min(back, rl - U.rm_lo);
+        ahead = min(ahead, U.rm_hi - rl);
+    }
+    uint32_t m[6], t[6], any = 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        if (k < 4) any |= r[k] | q[k];
+        sa_match_bits<TRANS>(r[k], q[k], m[k], t[k]);
+    }
+    const uint32_t m0 = sa_join_bits(m[0], m[1], m[2], m[3]), m1 = __byte_perm(m[4], m[5], 0x0073) & 0xffffu;
+    const uint32_t t0 = TRANS ? sa_join_bits(t[0], t[1], t[2], t[3]) : 0u;
+    const uint32_t t1 = TRANS ? __byte_perm(t[4], t[5], 0x0073) & 0xffffu : 0u;
+    const uint32_t H = sa_seed_bits<TRANS>(a, kmer, m0, m1, t0, t1, 0);  // bit own: this hit
+    const uint32_t prev = (H & ((1u << own) - 1u)) >> (own - back) << (own - back);
+    if (prev && !(any & 0x44444444u) && sa_chain_joined(a, ~m0, own - (31 - __clz(prev)))) return 1;
+    return ((H >> own >> 1) & ((1u << ahead) - 1u)) ? SA_CHAIN_NEXT : 0u;
+}
+
+// ---------------------------------------------------------------------------
+// The sweep: 32 consecutive hits per warp, one per lane, all in step.  Each is
+// scored over the 32 bases right of it and the 64 left of it (the seed and as
+// many again).  A hit whose scans both stop there with a total below hspthresh
+// is done: it adds its tiles and leaves nothing else.  These are the chance
+// hits, four of five on the genome workload.  Dropped hits of chains are
+// done too.  The others go to `list`, which the lane kernel scans.
+//
+// Why apart from the lane kernel: a chance hit's work there was the hand-out,
+// two direction set-ups and the bookkeeping of an iteration, most of it run
+// for a few lanes of a warp; here it is straight-line code for all 32.  Both
+// directions come from one window of the forward sequence: four aligned
+// 16-byte loads of the target (a scattered load costs an L1 wavefront per
+// lane, whatever its width), and query words that consecutive hits share.
+//
+// Bound by instruction issue and, close behind, the L1 data pipe (96 table
+// lookups and the target loads' wavefronts per round).  On a 2.5 Mbp query against
+// the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in the
+// lane kernel 5.65 ms; sweep 2.33, lane kernel 1.40, chain walk 0.27: 3.97 ms
+// (4.79 with the sweep and no chains).  Lane phase of 24 Mbp: 55.0 -> 36.4 ms;
+// of a repeat-masker call, 0.80 -> 0.39 ms, and its warp kernel 0.78 -> 0.13.
+// ---------------------------------------------------------------------------
+// One 8-base window of a scan, from its first base on (REV: from base 7
+// down): running score S, best B, and whether a base of it stops the scan (the
+// windowed stop test of the fast form).
+template <bool REV>
+__device__ __forceinline__ void sa_sweep_window(const char* tblb, uint32_t rw, uint32_t qw, int xdrop, int& S, int& B,
+                                                int& at, bool& stop) {
+    uint32_t lo, hi;
+    sa_merge8(rw, qw, lo, hi);
+    int mn = INT_MAX;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const int S0 = S + sa_tbl(tblb, lo, hi, REV ? 7 - k : k);
+        S = S0 + sa_tbl(tblb, lo, hi, REV ? 6 - k : k + 1);
+        B = __vimax3_s32(B, S0, S);
+        mn = __vimin3_s32(mn, S0, S);
+    }
+    if (!stop) at = B;
+    stop = stop || B - mn > xdrop;
+}
+
+#define SA_SWEEP_BUF 128  // list records a warp gathers before it writes them
+
+template <bool TRANS>
+__global__ void __launch_bounds__(256, 4)
+sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P, uint64_t h_begin, uint64_t h_end) {
+    __shared__ int tbl[64];
+    __shared__ uint4 s_buf[8][SA_SWEEP_BUF];
+    if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
+    __syncthreads();
+    const char* tblb = reinterpret_cast<const char*>(tbl);
+    SaCounters* const ctr = a.ctr;
+    const uint64_t H = min((uint64_t)ctr->num_hits, h_end), nnz = ctr->nnz;
+    if (ctr->error || h_begin >= H) return;
+    const bool chains = a.chain && !ctr->chain_bad;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = sa_lanemask_lt();
+    const uint32_t warps = gridDim.x * 8, w = blockIdx.x * 8 + (threadIdx.x >> 5);
+    uint4* const buf = s_buf[threadIdx.x >> 5];
+    uint32_t nbuf = 0, tiles = 0, ext = 0;
+    auto write_out = [&]() {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)nbuf);
+        at = __shfl_sync(SA_FULL, at, 0);
+        __syncwarp();
+        for (uint32_t i = lane; i < nbuf; i += 32)
+            if (at + i < a.list_cap) a.list[at + i] = buf[i];
+        __syncwarp();
+        nbuf = 0;
+    };
+    const uint64_t first = h_begin / 32, rounds = (H + 31) / 32;  // h_begin is a multiple of 32
+    // rounds a warp takes in a row: its first seed is searched for once
+    const uint64_t run = min((rounds - first + warps - 1) / warps, (uint64_t)64);
+    for (uint64_t r0 = first + w * run; r0 < rounds; r0 += (uint64_t)warps * run) {
+        const uint64_t r1 = min(r0 + run, rounds);
+        uint64_t c = sa_warp_find_seed(a.cs.E, nnz, 32 * r0);
+        for (uint64_t r = r0; r < r1; ++r) {
+            const uint64_t t = 32 * r, h = t + lane;
+            // the hit's seed: c, and one more for each seed that starts by then
+            const uint64_t ahead = c + 1 + lane < nnz ? a.cs.E[c + 1 + lane] - t : ~0ull;
+            const uint32_t starts = __reduce_or_sync(SA_FULL, ahead < 32 ? 1u << (uint32_t)ahead : 0u);
+            bool left = false;
+            uint4 rec = make_uint4(0, 0, 0, 0);
+            if (h < H) {
+                const uint64_t k = c + __popc(starts & ((2u << lane) - 1u));
+                const uint32_t rl = __ldg(a.pos_table + a.cs.lo[k] + (uint32_t)(h - a.cs.E[k])) + a.seed_size;  // find_hits :192
+                const uint32_t ql = a.cs.qpos[k] + a.seed_size;                                               // find_hits :176
+                const uint32_t unit = a.cs.unit[k];
+                rec = make_uint4(rl, ql, a.cs.scope[k], unit);
+                const SaUnit U = a.units[unit];
+                // rm: hits outside [ref_start, ref_end] are never extended
+                // (repeat_masker_src/seed_filter.cu:237-243, 304-333)
+                bool live = !(U.flags & 1u) || (rl >= U.rm_lo && rl <= U.rm_hi);
+                // Coordinates past either sequence end (a caller-supplied table or
+                // seed beyond the sequences) are rejected, not read.
+                if (rl > a.ref_len || ql > U.q_len) {
+                    atomicCAS(&ctr->error, 0ull, 5ull);
+                    live = false;
+                }
+                if (live) {
+                    ++ext;
+                    // bases [rl - 64, rl + 32) of both sequences as 12 words
+                    const uint32_t* __restrict__ pq = U.q_packed + (ql >> 3) - 8;
+                    uint32_t rw[16], qw[13];
+#pragma unroll
+                    for (int i = 0; i < 13; ++i) qw[i] = __ldg(pq + i);
+                    const uint4* __restrict__ pr = reinterpret_cast<const uint4*>(a.ref) + (int)(rl >> 5) - 2;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint4 v = __ldg(pr + i);
+                        rw[4 * i] = v.x;
+                        rw[4 * i + 1] = v.y;
+                        rw[4 * i + 2] = v.z;
+                        rw[4 * i + 3] = v.w;
+                    }
+                    if (rl & 8u) {
+#pragma unroll
+                        for (int i = 0; i < 15; ++i) rw[i] = rw[i + 1];
+                    }
+                    if (rl & 16u) {
+#pragma unroll
+                        for (int i = 0; i < 13; ++i) rw[i] = rw[i + 2];
+                    }
+                    const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
+#pragma unroll
+                    for (int i = 0; i < 12; ++i) {
+                        rw[i] = __funnelshift_r(rw[i], rw[i + 1], sr);
+                        qw[i] = __funnelshift_r(qw[i], qw[i + 1], sq);
+                    }
+                    const uint32_t f = chains ? sa_chain_test<TRANS>(a, P.kmer_size, U, rl, ql, rw + 4, qw + 4) : 0u;
+                    if (f != 1) {
+                        int S = 0, B = 0, R = 0, Lb = 0;
+                        bool stop_r = false, stop_l = false;
+#pragma unroll
+                        for (int i = 8; i < 12; ++i) sa_sweep_window<false>(tblb, rw[i], qw[i], a.xdrop, S, B, R, stop_r);
+                        S = B = 0;
+#pragma unroll
+                        for (int i = 7; i >= 4; --i) sa_sweep_window<true>(tblb, rw[i], qw[i], a.xdrop, S, B, Lb, stop_l);
+                        const uint32_t tl = stop_l ? 2 : 3;
+#pragma unroll
+                        for (int i = 3; i >= 0; --i) sa_sweep_window<true>(tblb, rw[i], qw[i], a.xdrop, S, B, Lb, stop_l);
+                        // a window that reaches past an end scans it to the end: the lane kernel does that
+                        const bool inside = rl >= 64 && ql >= 64 && rl + 32 <= a.ref_len && ql + 32 <= U.q_len;
+                        left = f || !inside || !stop_r || !stop_l || (int)(float)(R + Lb) >= a.hspthresh;
+                        if (!left) tiles += tl;
+                        rec.w |= f;
+                    }
+                }
+            }
+            const uint32_t m = __ballot_sync(SA_FULL, left);
+            if (left) buf[nbuf + __popc(m & lt)] = rec;
+            nbuf += __popc(m);
+            if (nbuf > SA_SWEEP_BUF - 32) write_out();
+            c += __popc(starts) + (__any_sync(SA_FULL, ahead == 32) ? 1 : 0);
+        }
+    }
+    if (nbuf) write_out();
+    unsigned long long sum = tiles, e = ext;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        sum += __shfl_xor_sync(SA_FULL, sum, s);
+        e += __shfl_xor_sync(SA_FULL, e, s);
+    }
+    if (lane == 0 && e) {
+        atomicAdd(&ctr->base_steps, sum);
+        atomicAdd(&ctr->extended, e);
+    }
+}
+
+// Match, transition and non-ACGT bits of 32 bases.
+__device__ __forceinline__ void sa_masks32(const uint32_t* __restrict__ R, const uint32_t* __restrict__ Q, uint32_t rl,
+                                           uint32_t ql, int off, uint32_t& m, uint32_t& t, uint32_t& bad) {
+    uint32_t mm[4], tt[4], bb[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t rw = sa_load8(R, (int64_t)rl + off + 8 * k), qw = sa_load8(Q, (int64_t)ql + off + 8 * k);
+        sa_match_bits<true>(rw, qw, mm[k], tt[k]);
+        bb[k] = sa_nibble_bits(((rw | qw) >> 2) & 0x11111111u);
+    }
+    m = sa_join_bits(mm[0], mm[1], mm[2], mm[3]);
+    t = sa_join_bits(tt[0], tt[1], tt[2], tt[3]);
+    bad = sa_join_bits(bb[0], bb[1], bb[2], bb[3]);
+}
+
+// The dropped hits that follow the scanned hit (rl, ql) of `unit`: their number
+// and the tiles of their scans.  stop_r, stop_l: offsets at which the hit's
+// right and left scans stop; a hit d bases on stops at stop_r - d and
+// stop_l + d.
+struct SaChain {
+    unsigned long long tiles;
+    uint32_t n;
+};
+
+__device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaParams& P, uint32_t unit, uint32_t rl,
+                                                 uint32_t ql, uint32_t stop_r, uint32_t stop_l) {
+    const SaUnit U = a.units[unit];
+    unsigned long long tiles = 0;
+    const uint32_t S = a.seed_size, j = ql - S;
+    uint32_t ahead = U.j_hi - 1 - j;
+    if (U.flags & 1u) ahead = min(ahead, U.rm_hi - rl);
+    uint32_t n = 0, last = 0, m0, t0, b0;
+    sa_masks32(a.ref, U.q_packed, rl, ql, -32, m0, t0, b0);
+    for (uint32_t c = 0; c + 1 - last <= a.gap; c += 32) {
+        uint32_t m1, t1, b1;
+        sa_masks32(a.ref, U.q_packed, rl, ql, (int)c, m1, t1, b1);
+        if ((m0 & m1) == ~0u && !(b0 | b1) && last == c && c + 32 <= ahead &&
+            ((j + c) & (SA_CHAIN_BLOCK - 1)) + 32 < SA_CHAIN_BLOCK) {
+            // 64 matching bases: each of the next 32 positions ends a dropped hit.  Over
+            // 32 consecutive d, (stop_r - d) >> 5 sums to stop_r - c - 32 and (stop_l + d) >> 5 to stop_l + c + 1.
+            n += 32;
+            tiles += (unsigned long long)(stop_r - c - 32) + (stop_l + c + 1) + 64;
+            last = c + 32;
+        } else {
+            // bit i - 1: a match ends c + i bases on
+            uint32_t hits = P.transition ? sa_seed_bits<true>(a, P.kmer_size, m0, m1, t0, t1, 33 - S)
+                                         : sa_seed_bits<false>(a, P.kmer_size, m0, m1, t0, t1, 33 - S);
+            for (; hits; hits &= hits - 1) {
+                const uint32_t i = __ffs(hits), d = c + i, delta = d - last;
+                if (d > ahead || delta > a.gap || delta > ((j + d) & (SA_CHAIN_BLOCK - 1)) ||
+                    __funnelshift_rc(b0, b1, i) || !sa_chain_joined(a, ~__funnelshift_rc(m0, m1, i), delta))
+                    return {tiles, n};
+                ++n;
+                tiles += ((stop_r - d) >> 5) + ((stop_l + d) >> 5) + 2;
+                last = d;
+            }
+        }
+        m0 = m1;
+        t0 = t1;
+        b0 = b1;
+    }
+    return {tiles, n};
+}
+
+// Where a scan of the fast form stops, to the base: w = (step start / 8) << 16
+// | (best - score there), from the stopping step (sa_stop_word).  sr, sq: the
+// scan's first bases in R and Q; SH: log2 of the table's score scale.
+__device__ __forceinline__ uint32_t sa_stop_word(uint32_t o, int depth) {
+    return (min(o >> 3, 0xffffu) << 16) | (uint32_t)depth;
+}
+
+template <int SH>
+__device__ __forceinline__ uint32_t sa_stop_offset(const char* tblb, const uint32_t* __restrict__ R,
+                                                const uint32_t* __restrict__ Q, uint32_t sr, uint32_t sq,
+                                                uint32_t avail, int xdrop, uint32_t w) {
+    // a step that starts past the word's range: from the scan's start
+    uint32_t o = (w >> 16) == 0xffffu ? 0u : (w >> 16) * 8;
+    int S = (w >> 16) == 0xffffu ? 0 : -(int)(w & 0xffffu), best = 0;
+    while (true) {
+        const uint32_t rw = sa_load8(R, (int64_t)sr + o), qw = sa_load8(Q, (int64_t)sq + o);
+        uint32_t lo, hi;
+        sa_merge8(rw, qw, lo, hi);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (o + k >= avail) return avail;
+            S += (sa_tbl(tblb, lo, hi, k) + 1) >> SH;
+            best = max(best, S);
+            if (best - S > xdrop) return o + k;
+        }
+        o += 8;
+    }
+}
+
+// Shared memory of the lane kernel: score table, the 8 warps' rings of
+// candidate HSPs, per thread the stop words of its current hit, then per warp
+// `tile` hit records and the tile's E window (relative to the tile's first hit).
+struct SaLaneSmem {
+    int tbl[64];
+    uint4 em[8][64];       // {ref_start, query_start (before the rm flip), len, scope}
+    uint2 ex[8][64];       // {total, unit}
+    uint32_t stop[2][256];
+};
+
+static size_t sa_lane_smem(uint32_t tile) { return sizeof(SaLaneSmem) + 8 * (size_t)tile * (sizeof(uint4) + sizeof(uint32_t)); }
+
 // Keep test of `n` (<= 32) ring candidates from slot `head` on, one per lane:
 // entropy factor from the per-base match counts over the HSP when the total
 // is in the entropy range (src/seed_filter.cu:580-621), then insertion of the
@@ -251,14 +661,10 @@ __device__ __forceinline__ void sa_flush_candidates(const SaExtK& a, const uint4
     sa_hash_note_used(a.hset, &a.ctr->hash_used, claimed);
 }
 
-// Dynamic shared memory of the lane kernel for `tile` hits per warp tile.
-static size_t sa_lane_smem(uint32_t tile) {
-    return SA_LANE_TABLES + 8 * (size_t)tile * 16 + 8 * (size_t)(tile + 1) * 8 + 8 * 64 * 16 + 8 * 64 * 8;
-}
-
-template <int MIN_CTAS, int STEP, bool EXACT>
+// LIST: the hits come from the sweep's list; else from the compacted seeds.
+template <int MIN_CTAS, int STEP, bool EXACT, bool LIST>
 __global__ void __launch_bounds__(256, MIN_CTAS)
-sa_k_extend_lane(SaExtK a, SaParams P) {
+sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
     constexpr int NW = STEP / 8;                  // 8-base windows per step
     constexpr int SCALE = 2 * STEP;               // packed score scale (fast form)
     constexpr int SH = STEP == 8 ? 4 : STEP == 16 ? 5 : 6;  // log2(SCALE)
@@ -269,26 +675,24 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
     // tile E window, and a 64-entry ring of candidate HSPs awaiting the keep
     // test and insertion.
     extern __shared__ __align__(16) unsigned char sa_smem[];
+    SaLaneSmem& L = *reinterpret_cast<SaLaneSmem*>(sa_smem);
     const uint32_t TILE = a.tile_hits;
     // entry (q << 3) | r: target code r vs query code q.  Codes 0..3 use
     // entries 0..27 only, one per bank: lookups of A/C/G/T pairs never conflict.
-    int* tbl = reinterpret_cast<int*>(sa_smem);
+    int* const tbl = L.tbl;
     if (threadIdx.x < 64) {
         const int sc = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
         tbl[threadIdx.x] = EXACT ? sc : sc * SCALE - 1;
     }
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
-    if (a.ctr->error) return;
+    if (a.ctr->error || (LIST && a.ctr->list_count > a.list_cap)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t lt = sa_lanemask_lt();
-    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + SA_LANE_TABLES) + wid * TILE;
-    unsigned long long* const s_E =
-        reinterpret_cast<unsigned long long*>(sa_smem + SA_LANE_TABLES + 128 * (size_t)TILE) + wid * (TILE + 1);
-    unsigned char* const em_base = sa_smem + SA_LANE_TABLES + 128 * (size_t)TILE + 64 * (size_t)(TILE + 1);
-    uint4* const s_em = reinterpret_cast<uint4*>(em_base) + wid * 64;
-    uint2* const s_ex = reinterpret_cast<uint2*>(em_base + 8 * 64 * 16) + wid * 64;
-
+    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + sizeof(SaLaneSmem)) + wid * TILE;
+    uint32_t* const s_E = reinterpret_cast<uint32_t*>(sa_smem + sizeof(SaLaneSmem) + 128 * (size_t)TILE) + wid * TILE;
+    uint4* const s_em = L.em[wid];
+    uint2* const s_ex = L.ex[wid];
     // H, nnz, ref_len, seed_size and xdrop are read where used (registers
     // are the lane kernel's limit)
     const uint32_t* __restrict__ ref = a.ref;
@@ -350,28 +754,34 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                 unsigned long long t0 = 0;
                 if (lane == 0) t0 = atomicAdd(&a.ctr->hit_cursor, (unsigned long long)TILE);
                 t0 = __shfl_sync(SA_FULL, t0, 0);
-                const uint64_t H = a.ctr->num_hits, nnz = a.ctr->nnz;
+                const uint64_t H = LIST ? a.ctr->list_count : a.ctr->num_hits, nnz = a.ctr->nnz;
                 if (t0 >= H) {
                     exhausted = true;
                     tile_n = tile_pos = 0;
+                } else if (LIST) {
+                    tile_n = (uint32_t)min((unsigned long long)TILE, H - t0);
+                    tile_pos = 0;
+                    for (uint32_t i = lane; i < tile_n; i += 32) s_hits[i] = __ldcs(a.list + t0 + i);
+                    __syncwarp();
                 } else {
                     uint32_t n = (uint32_t)min((unsigned long long)TILE, H - t0);
                     const uint64_t c0 = sa_warp_find_seed(a.cs.E, nnz, t0);
                     const uint32_t nw = (uint32_t)min((uint64_t)n, nnz - c0);  // seeds of the window
-                    for (uint32_t i = lane; i <= nw; i += 32) s_E[i] = a.cs.E[c0 + i];  // E[nnz] == H
+                    const uint32_t skip0 = (uint32_t)(t0 - a.cs.E[c0]);  // hits of the first seed before the tile
+                    for (uint32_t i = lane; i < nw; i += 32)
+                        s_E[i] = i ? (uint32_t)min(a.cs.E[c0 + i] - t0, 0xffffffffull) : 0u;
                     __syncwarp();
                     // record of hit t0 + i: its seed by binary search in the E window
                     auto record = [&](uint32_t i) {
-                        const unsigned long long h = t0 + i;
-                        uint32_t lo = 0, hi = nw;  // last k in [0, nw) with E[c0+k] <= h
+                        uint32_t lo = 0, hi = nw;  // last k in [0, nw) with E[c0+k] <= t0 + i
                         while (hi - lo > 1) {
                             const uint32_t mid = (lo + hi) >> 1;
-                            if (s_E[mid] <= h) lo = mid;
+                            if (s_E[mid] <= i) lo = mid;
                             else hi = mid;
                         }
                         const uint64_t c = c0 + lo;
                         uint4 r;
-                        r.x = __ldg(a.pos_table + a.cs.lo[c] + (uint32_t)(h - s_E[lo])) + a.seed_size;  // find_hits :192
+                        r.x = __ldg(a.pos_table + a.cs.lo[c] + (lo ? i - s_E[lo] : i + skip0)) + a.seed_size;  // find_hits :192
                         r.y = a.cs.qpos[c] + a.seed_size;                                                 // find_hits :176
                         r.z = a.cs.scope[c];
                         r.w = a.cs.unit[c];
@@ -424,24 +834,19 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
         // ---- start of a direction: a fresh hit (right), or the left side of
         // the current hit after its right end ----
         if (fresh || setup) {
-            const SaUnit U = a.units[unit_id];
+            const SaUnit U = a.units[unit_id & ~SA_CHAIN_NEXT];
             if (fresh) {
-                // rm: hits outside [ref_start, ref_end] are never extended
-                // (repeat_masker_src/seed_filter.cu:237-243, 304-333).
-                bool skip = (U.flags & 1u) && !(rl >= U.rm_lo && rl <= U.rm_hi);
                 // Coordinates past either sequence end (a caller-supplied table or
                 // seed beyond the sequences) are rejected, not read.
                 if (rl > a.ref_len || ql > U.q_len) {
                     atomicCAS(&a.ctr->error, 0ull, 5ull);
-                    skip = true;
-                }
-                if (!skip) {
+                } else {
                     has = true;
                     nocap = false;
                     setup = true;
                     dir = 0;
                     tiles = 0;
-                    ++ext_acc;
+                    if (!LIST) ++ext_acc;  // else counted by the sweep
                 }
             }
             if (setup) {
@@ -478,6 +883,7 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                 pq += NW;
                 const bool edge = o + STEP > avail;
                 bool stop = false;
+                int depth = 0;
                 uint32_t lo, hi;
                 if (EXACT) {
                     bool alive = true;
@@ -502,7 +908,8 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                     // B - min > SCALE * xdrop + STEP  <=>  (B >> SH) - (min >> SH) > xdrop, because
                     // the low parts of B (0..STEP) and min (0..STEP-1) differ by less than SCALE
                     const uint32_t T = (uint32_t)a.xdrop * SCALE + STEP;
-                    int Pk = ((S - best) << SH) + STEP, B = STEP, at = 0;
+                    depth = best - S;
+                    int Pk = STEP - (depth << SH), B = STEP, at = 0;
                     if (!edge) {
     #pragma unroll
                         for (int j = 0; j < NW; ++j) {
@@ -528,6 +935,7 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                     // Steps start at multiples of STEP (8, 16 or 32), so the stop offset
                     // lies in 32-base tile o >> 5 whichever base of the step it is.
                     tiles += (o >> 5) + 1;
+                    if (LIST) L.stop[dir][threadIdx.x] = sa_stop_word(o, depth);
                     if (dir == 0) {
                         Rbest = best;
                         Rpos = best > 0 ? bpos : -1;  // -1 when no positive score
@@ -557,7 +965,7 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
             if (a.switch_now && sub + 1 < a.substeps && __any_sync(SA_FULL, setup)) {
                 if (setup) {
                     setup = false;
-                    const SaUnit U = a.units[unit_id];
+                    const SaUnit U = a.units[unit_id & ~SA_CHAIN_NEXT];
                     begin_dir(U.q_packed, U.q_len);
                     scanning = true;
                 }
@@ -598,7 +1006,7 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                 const uint32_t slot = (em_tail + __popc(em & lt)) & 63u;
                 // {ref_start, query_start (before the rm flip), len, scope}, {total, unit} (:606-608)
                 s_em[slot] = make_uint4(rl - (uint32_t)Lpos, ql - (uint32_t)Lpos, (uint32_t)(Rpos + Lpos), scope);
-                s_ex[slot] = make_uint2((uint32_t)total, unit_id);
+                s_ex[slot] = make_uint2((uint32_t)total, unit_id & ~SA_CHAIN_NEXT);
             }
             em_tail += __popc(em);
             // full batches of 32; at the end, whatever is left
@@ -607,6 +1015,23 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
                 __syncwarp();
                 sa_flush_candidates(a, s_em, s_ex, em_head, n);
                 em_head += n;
+            }
+        }
+        // ---- hits that may stand for the dropped ones after them ----
+        if (LIST) {
+            const bool leads = finished && (unit_id & SA_CHAIN_NEXT);
+            const uint32_t cm = __ballot_sync(SA_FULL, leads);
+            if (cm) {
+                const int leader = __ffs(cm) - 1;
+                unsigned long long at = 0;
+                if (lane == leader) at = atomicAdd(&a.ctr->chain_count, (unsigned long long)__popc(cm));
+                at = __shfl_sync(SA_FULL, at, leader) + __popc(cm & lt);
+                if (leads) {  // at most one per list record
+                    a.lead[at] = make_uint4(rl, ql, unit_id & ~SA_CHAIN_NEXT, (uint32_t)Lpos);
+                    a.lead_right[at] = (uint32_t)Rpos;
+                    a.lead_stop_r[at] = L.stop[0][threadIdx.x];
+                    a.lead_stop_l[at] = L.stop[1][threadIdx.x];
+                }
             }
         }
         if (done) break;
@@ -624,13 +1049,65 @@ sa_k_extend_lane(SaExtK a, SaParams P) {
     }
 }
 
+// Chains, second half: one thread per scanned hit that others may follow
+// counts the dropped ones after it.  They are survivors if its HSP was kept,
+// that is, if the set holds it (the lane kernel has filled the set).
+// SH: log2 of the lane kernel's score scale (sa_stop_offset's table).
+template <int SH>
+__global__ void __launch_bounds__(256)
+sa_k_chain_walk(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
+    __shared__ int tbl[64];
+    if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SH) - 1;
+    __syncthreads();
+    const SaCounters* __restrict__ ctr = a.ctr;
+    const unsigned long long n = ctr->chain_count;
+    if (ctr->error) return;
+    unsigned long long tiles = 0, kept = 0;
+    for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
+        const uint4 h = a.lead[i];
+        const SaUnit U = a.units[h.z];
+        const uint32_t rl = h.x, ql = h.y;
+        const char* tblb = reinterpret_cast<const char*>(tbl);
+        const uint32_t stop_r = sa_stop_offset<SH>(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql),
+                                                   a.xdrop, a.lead_stop_r[i]);
+        const uint32_t stop_l = sa_stop_offset<SH>(tblb, a.ref + sa_rev_words(a.ref_len), U.q_packed + sa_rev_words(U.q_len),
+                                                   a.ref_len - rl, U.q_len - ql, min(rl, ql), a.xdrop,
+                                                   a.lead_stop_l[i]);
+        const SaChain c = sa_chain_members(a, P, h.z, rl, ql, stop_r, stop_l);
+        if (!c.n) continue;
+        tiles += c.tiles;
+        const uint32_t len = a.lead_right[i] + h.w;
+        uint32_t qs = ql - h.w;
+        if (U.flags & 2u) qs = a.ref_len - 1 - (qs + len);
+        // chains are of calls and units with one MAX_HITS iteration: scope (unit << 4) | 0, unit 0 in a call
+        if (sa_hash_holds(a.hset, ctr->hash_mask, h.z << 4, rl - h.w, qs, len)) kept += c.n;
+    }
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        tiles += __shfl_xor_sync(SA_FULL, tiles, s);
+        kept += __shfl_xor_sync(SA_FULL, kept, s);
+    }
+    if ((threadIdx.x & 31) == 0 && tiles) {
+        atomicAdd(&a.ctr->base_steps, tiles);
+        if (kept) atomicAdd(&a.ctr->surv_count, kept);
+    }
+}
+
+// Between the segments of a large batch: the list and the queue start again
+// (an overflow stays to be seen).
+__global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
+    if (ctr->list_count <= list_cap) ctr->list_count = 0;
+    ctr->hit_cursor = 0;
+    ctr->chain_count = 0;
+}
+
 // ---------------------------------------------------------------------------
 // Phase B: one warp per long hit, 256 bases per step.
 // ---------------------------------------------------------------------------
 struct SaDirResult {
     int best;
     int pos;
-    uint32_t tiles;
+    uint32_t stop;  // offset at which the scan stops
 };
 
 __device__ __forceinline__ int sa_warp_incl_max(int v) {
@@ -740,7 +1217,7 @@ __device__ SaDirResult sa_warp_xdrop(const int* sub, const uint32_t* __restrict_
                 bpos = (int)ci + dir;
             }
             const uint32_t stop_idx = __shfl_sync(SA_FULL, loff + (uint32_t)stop_k, f);
-            res.tiles = (stop_idx >> 5) + 1;
+            res.stop = stop_idx;
             break;
         }
         cv = amax;
@@ -759,7 +1236,7 @@ __device__ SaDirResult sa_warp_xdrop(const int* sub, const uint32_t* __restrict_
 }
 
 __global__ void __launch_bounds__(256)
-sa_k_extend_warp(SaExtK a, SaParams P) {
+sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
     __shared__ int sub[64];
     if (threadIdx.x < 64) sub[threadIdx.x] = P.sub_mat[threadIdx.x];
     __syncthreads();
@@ -773,12 +1250,12 @@ sa_k_extend_warp(SaExtK a, SaParams P) {
         idx = __shfl_sync(SA_FULL, idx, 0);
         if (idx >= nlong) break;
         const SaLongHit L = a.long_q[idx];
-        const SaUnit U = a.units[L.unit];
+        const SaUnit U = a.units[L.unit & ~SA_CHAIN_NEXT];
         const uint32_t rl = L.ref_loc, ql = L.query_loc;
         const uint32_t avail_r = (rl < a.ref_len && ql < U.q_len) ? min(a.ref_len - rl, U.q_len - ql) : 0u;
         const SaDirResult R = sa_warp_xdrop(sub, a.ref, U.q_packed, rl, ql, avail_r, 0, a.xdrop);
         const SaDirResult Lr = sa_warp_xdrop(sub, a.ref, U.q_packed, rl, ql, min(rl, ql), 1, a.xdrop);
-        tiles_acc += R.tiles + Lr.tiles;
+        tiles_acc += (R.stop >> 5) + (Lr.stop >> 5) + 2;
         const int total = R.best + Lr.best;
         const int ext = R.pos + Lr.pos;
         int cnt[4] = {0, 0, 0, 0};
@@ -795,10 +1272,16 @@ sa_k_extend_warp(SaExtK a, SaParams P) {
                 for (int s = 16; s >= 1; s >>= 1) cnt[b] += __shfl_xor_sync(SA_FULL, cnt[b], s);
         }
         if (lane == 0) {
+            uint32_t stands_for = 1;
+            if (L.unit & SA_CHAIN_NEXT) {
+                const SaChain ch = sa_chain_members(a, P, L.unit & ~SA_CHAIN_NEXT, rl, ql, R.stop, Lr.stop);
+                stands_for += ch.n;
+                tiles_acc += ch.tiles;
+            }
             int keep, score;
             sa_keep_score(total, ext, cnt, eb, a.hspthresh, &keep, &score);
             if (keep) {
-                atomicAdd(&a.ctr->surv_count, 1ull);
+                atomicAdd(&a.ctr->surv_count, (unsigned long long)stands_for);
                 const uint32_t rs = rl - (uint32_t)Lr.pos;
                 uint32_t qs = ql - (uint32_t)Lr.pos;
                 const uint32_t len = (uint32_t)ext;
@@ -815,8 +1298,49 @@ sa_k_extend_warp(SaExtK a, SaParams P) {
     if (lane == 0) atomicAdd(&a.ctr->base_steps, tiles_acc);
 }
 
-static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaTuning& t) {
+// The fast scoring form holds when 7 * max(0, max_sub) <= xdrop (see the
+// phase A notes) and its packed scores stay inside 31 bits: a step starts at
+// >= -xdrop * SCALE and adds STEP scores of >= min_sub * SCALE - 1 (or
+// -(xdrop + 1) * SCALE - 1 past a sequence end).
+static bool sa_lane_fast_form(const SaParams& p, int step) {
+    long long mx = 0, mn = 0;
+    for (int i = 0; i < 64; ++i) {
+        mx = std::max<long long>(mx, p.sub_mat[i]);
+        mn = std::min<long long>(mn, p.sub_mat[i]);
+    }
+    const long long scale = 2ll * step, x = p.xdrop;
+    const long long low = std::min(mn, -(x + 1)) * scale - 1;
+    return x >= 0 && 7 * mx <= x && x * scale - low * step < (1ll << 31) && mx * scale * step < (1ll << 31);
+}
+
+// Scores for which sa_chain_joined's bounds hold: matches of A, C, G and T
+// score above 0, and the fast form (whose stop words chains need) is in use.
+bool sa_chain_params(const SaParams& p, const SaTuning& t) {
+    if (!sa_lane_fast_form(p, t.step_bases) || p.xdrop > 0xffff || p.seed_size > 31) return false;
+    for (int b = 0; b < 4; ++b)
+        if (p.sub_mat[9 * b] <= 0) return false;
+    return true;
+}
+
+static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaParams& p, const SaTuning& t) {
     SaExtK a;
+    int match = p.sub_mat[0], low = p.sub_mat[1];
+    for (int i = 0; i < 4; ++i)
+        for (int k = 0; k < 4; ++k) (i == k ? match : low) = std::min(i == k ? match : low, p.sub_mat[8 * i + k]);
+    a.chain = x.chain && sa_chain_params(p, t) ? 1u : 0u;
+    a.match = match;
+    a.swing = match - std::min(low, -1);
+    a.mismatches = (uint32_t)std::min(32, p.xdrop / -std::min(low, -1));
+    for (int i = 0; i < 16; ++i) a.shift[i] = (uint32_t)p.shape_pos[i < p.kmer_size ? i : 0];
+    // buffers of the dedup that are free until then
+    a.list = reinterpret_cast<uint4*>(w.out);
+    a.list_cap = x.sweep && sa_lane_fast_form(p, t.step_bases) ? w.list_cap : 0;
+    a.lead = reinterpret_cast<uint4*>(w.rec[0]);
+    a.lead_right = w.scope[0];
+    a.lead_stop_r = w.scope[1];
+    a.lead_stop_l = w.out_scope;
+    // the 48-base window of sa_chain_test holds the seeds of hits up to `gap` either way
+    a.gap = (uint32_t)std::max(0, std::min({13, p.seed_size - 1, 32 - p.seed_size}));
     a.ref = x.ref;
     a.ref_len = x.ref_len;
     a.pos_table = x.pos_table;
@@ -838,40 +1362,28 @@ static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaTuning& t) {
     return a;
 }
 
-// The fast scoring form holds when 7 * max(0, max_sub) <= xdrop (see the
-// phase A notes) and its packed scores stay inside 31 bits: a step starts at
-// >= -xdrop * SCALE and adds STEP scores of >= min_sub * SCALE - 1 (or
-// -(xdrop + 1) * SCALE - 1 past a sequence end).
-static bool sa_lane_fast_form(const SaParams& p, int step) {
-    long long mx = 0, mn = 0;
-    for (int i = 0; i < 64; ++i) {
-        mx = std::max<long long>(mx, p.sub_mat[i]);
-        mn = std::min<long long>(mn, p.sub_mat[i]);
-    }
-    const long long scale = 2ll * step, x = p.xdrop;
-    const long long low = std::min(mn, -(x + 1)) * scale - 1;
-    return x >= 0 && 7 * mx <= x && x * scale - low * step < (1ll << 31) && mx * scale * step < (1ll << 31);
+template <int C, int STEP, bool EXACT, bool LIST>
+static void sa_lane_launch(const SaExtK& a, const SaParams& p, int grid, size_t smem, cudaStream_t st) {
+    if (grid > 0) sa_k_extend_lane<C, STEP, EXACT, LIST><<<grid, 256, smem, st>>>(a, p);
+    else cudaFuncSetAttribute(sa_k_extend_lane<C, STEP, EXACT, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-template <int C, int STEP, bool EXACT>
-static void sa_lane_launch(const SaExtK& a, const SaParams& p, int grid, size_t smem, cudaStream_t st) {
-    if (grid > 0) sa_k_extend_lane<C, STEP, EXACT><<<grid, 256, smem, st>>>(a, p);
-    else cudaFuncSetAttribute(sa_k_extend_lane<C, STEP, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+enum SaLaneForm { kLaneFast, kLaneExact, kLaneList };
+
+template <int C, int STEP>
+static void sa_lane_dispatch_form(const SaExtK& a, const SaParams& p, SaLaneForm form, int grid, size_t smem,
+                                  cudaStream_t st) {
+    if (form == kLaneList) sa_lane_launch<C, STEP, false, true>(a, p, grid, smem, st);
+    else if (form == kLaneExact) sa_lane_launch<C, STEP, true, false>(a, p, grid, smem, st);
+    else sa_lane_launch<C, STEP, false, false>(a, p, grid, smem, st);
 }
 
 template <int C>
-static void sa_lane_dispatch(const SaExtK& a, const SaParams& p, int step, bool exact, int grid, size_t smem,
+static void sa_lane_dispatch(const SaExtK& a, const SaParams& p, int step, SaLaneForm form, int grid, size_t smem,
                              cudaStream_t st) {
-    if (step == 32) {
-        if (exact) sa_lane_launch<C, 32, true>(a, p, grid, smem, st);
-        else sa_lane_launch<C, 32, false>(a, p, grid, smem, st);
-    } else if (step == 16) {
-        if (exact) sa_lane_launch<C, 16, true>(a, p, grid, smem, st);
-        else sa_lane_launch<C, 16, false>(a, p, grid, smem, st);
-    } else {
-        if (exact) sa_lane_launch<C, 8, true>(a, p, grid, smem, st);
-        else sa_lane_launch<C, 8, false>(a, p, grid, smem, st);
-    }
+    if (step == 32) sa_lane_dispatch_form<C, 32>(a, p, form, grid, smem, st);
+    else if (step == 16) sa_lane_dispatch_form<C, 16>(a, p, form, grid, smem, st);
+    else sa_lane_dispatch_form<C, 8>(a, p, form, grid, smem, st);
 }
 
 // Allows every lane-kernel instance the largest tile's shared memory, once
@@ -887,10 +1399,10 @@ void sa_prepare_extend_lane(const SaParams& p, const SaTuning& t) {
     const size_t smem = sa_lane_smem(1024);
     SaExtK none{};
     for (int step : {8, 16, 32})
-        for (bool exact : {false, true}) {
-            sa_lane_dispatch<2>(none, p, step, exact, 0, smem, 0);
-            sa_lane_dispatch<3>(none, p, step, exact, 0, smem, 0);
-            sa_lane_dispatch<4>(none, p, step, exact, 0, smem, 0);
+        for (SaLaneForm form : {kLaneFast, kLaneExact, kLaneList}) {
+            sa_lane_dispatch<2>(none, p, step, form, 0, smem, 0);
+            sa_lane_dispatch<3>(none, p, step, form, 0, smem, 0);
+            sa_lane_dispatch<4>(none, p, step, form, 0, smem, 0);
         }
     done[dev] = true;
 }
@@ -899,18 +1411,40 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
                            cudaStream_t st, int grid_ctas) {
     sa_prepare_extend_lane(p, t);
     // Register budget follows the CTAs per SM: 4 -> <= 64 registers, 3 -> <= 85, 2 -> <= 128.
-    const SaExtK a = sa_ext_args(w, x, t);
+    const SaExtK a = sa_ext_args(w, x, p, t);
     const int grid = grid_ctas > 0 ? grid_ctas : num_sms * t.ext_ctas_per_sm;
     const size_t smem = sa_lane_smem(a.tile_hits);
-    const bool exact = !sa_lane_fast_form(p, t.step_bases);
-    if (t.ext_ctas_per_sm >= 4) sa_lane_dispatch<4>(a, p, t.step_bases, exact, grid, smem, st);
-    else if (t.ext_ctas_per_sm == 3) sa_lane_dispatch<3>(a, p, t.step_bases, exact, grid, smem, st);
-    else sa_lane_dispatch<2>(a, p, t.step_bases, exact, grid, smem, st);
-    sa_note_launch();
+    const SaLaneForm form = a.list_cap ? kLaneList : sa_lane_fast_form(p, t.step_bases) ? kLaneFast : kLaneExact;
+    // Segments of hits whose list is sure to fit in practice; one unless the
+    // caller knows of more hits (x.hits).  A list that overflows all the same is
+    // seen by the host (list_count), which runs the call again without the sweep.
+    const uint64_t seg = form == kLaneList ? 4 * a.list_cap & ~31ull : 0;
+    uint64_t h0 = 0;
+    do {
+        const uint64_t h1 = form == kLaneList && x.hits > h0 + seg ? h0 + seg : ~0ull;
+        if (form == kLaneList) {
+            if (h0) sa_k_next_segment<<<1, 1, 0, st>>>(w.ctr, a.list_cap);
+            const int g = num_sms * 4;
+            if (p.transition) sa_k_sweep<true><<<g, 256, 0, st>>>(a, p, h0, h1);
+            else sa_k_sweep<false><<<g, 256, 0, st>>>(a, p, h0, h1);
+            sa_note_launch();
+        }
+        if (t.ext_ctas_per_sm >= 4) sa_lane_dispatch<4>(a, p, t.step_bases, form, grid, smem, st);
+        else if (t.ext_ctas_per_sm == 3) sa_lane_dispatch<3>(a, p, t.step_bases, form, grid, smem, st);
+        else sa_lane_dispatch<2>(a, p, t.step_bases, form, grid, smem, st);
+        sa_note_launch();
+        if (form == kLaneList && a.chain) {
+            if (t.step_bases == 32) sa_k_chain_walk<6><<<num_sms * 4, 256, 0, st>>>(a, p);
+            else if (t.step_bases == 16) sa_k_chain_walk<5><<<num_sms * 4, 256, 0, st>>>(a, p);
+            else sa_k_chain_walk<4><<<num_sms * 4, 256, 0, st>>>(a, p);
+            sa_note_launch();
+        }
+        h0 = h1;
+    } while (h0 != ~0ull);
 }
 
 void sa_launch_extend_warp(SaWork& w, const SaExtendArgs& x, const SaParams& p, const SaTuning& t, int num_sms,
                            cudaStream_t st) {
-    sa_k_extend_warp<<<num_sms * 4, t.long_block, 0, st>>>(sa_ext_args(w, x, t), p);
+    sa_k_extend_warp<<<num_sms * 4, t.long_block, 0, st>>>(sa_ext_args(w, x, p, t), p);
     sa_note_launch();
 }

@@ -65,6 +65,7 @@ struct SaUnit {
     uint32_t q_len;
     uint32_t rm_lo, rm_hi;   // rm window on ref_loc, inclusive
     uint32_t flags;          // bit0 = rm mode, bit1 = rev (rm coordinate flip)
+    uint32_t j_lo, j_hi;     // seed positions [j_lo, j_hi) (chains of hits on one diagonal)
 };
 
 // Survivor record (segmentPair, src/graph.h:25-30) + dedup scope.
@@ -102,6 +103,10 @@ struct SaCounters {
     unsigned long long hash_overflow;  // inserts that found no free slot
     unsigned long long hash_used;      // slots claimed in the HSP set (entries of its used list)
     unsigned long long pad[3];         // device-side counts of the dedup stages
+    unsigned long long chain_bad;      // nonzero: the call's hits are not known to be every seed match of its windows
+    unsigned long long windows;        // plain call: valid seed windows in [j_lo, j_hi)
+    unsigned long long list_count;     // hits the sweep left to the lane kernel (past the list's capacity: the call is run again without it)
+    unsigned long long chain_count;    // scanned hits that others may follow
 };
 
 // Open-addressing set of distinct HSPs of one call: slot = 16-byte key
@@ -184,6 +189,22 @@ __device__ __forceinline__ bool sa_hash_contains(const SaHashSet& hs, unsigned l
         asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(s0), "=l"(s1) : "l"(hs.keys + 2 * h));
         if (s0 == k0 && s1 == k1) return true;
         if (s0 == ~0ull || s1 == ~0ull) return false;
+        h = (h + 1) & mask;
+    }
+    return false;
+}
+
+// Whether the set holds the key, after the kernel that fills it: the search
+// goes as far as an insertion would.
+__device__ __forceinline__ bool sa_hash_holds(const SaHashSet& hs, unsigned long long mask, uint32_t scope,
+                                              uint32_t rs, uint32_t qs, uint32_t len) {
+    const unsigned long long k0 = ((unsigned long long)scope << 32) | rs;
+    const unsigned long long k1 = ((unsigned long long)qs << 32) | len;
+    unsigned long long h = sa_hash_mix(k0, k1) & mask;
+    for (int probe = 0; probe < SA_HASH_MAX_PROBES; ++probe) {
+        const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(hs.keys + 2 * h);
+        if (s.x == k0 && s.y == k1) return true;
+        if (s.x == ~0ull && s.y == ~0ull) return false;
         h = (h + 1) & mask;
     }
     return false;
@@ -284,6 +305,55 @@ __device__ __forceinline__ void sa_count_matches8(uint32_t rw, uint32_t qw, uint
         t = t & (t >> 1) & (t >> 2) & (t >> 3) & 0x11111111u;
         c[b] += __popc(eq & t);
     }
+}
+
+// Bit k = 1: the window of seed_size (<= 32) bases that starts at base k of
+// word pw[0] (k in 0..7) is all uppercase ACGT (code bit 2 clear throughout).
+__device__ __forceinline__ uint32_t sa_nonacgt8(uint32_t w) {
+    uint32_t t = (w >> 2) & 0x11111111u;  // bit 4k = code bit 2 of base k
+    t = (t | (t >> 3)) & 0x03030303u;
+    t = (t | (t >> 6)) & 0x000f000fu;
+    return (t | (t >> 12)) & 0xffu;
+}
+
+__device__ __forceinline__ uint32_t sa_valid_windows8(const uint32_t* __restrict__ pw, uint32_t seed_size) {
+    const uint64_t bad = (uint64_t)(sa_nonacgt8(__ldg(pw)) | (sa_nonacgt8(__ldg(pw + 1)) << 8) |
+                                    (sa_nonacgt8(__ldg(pw + 2)) << 16) | (sa_nonacgt8(__ldg(pw + 3)) << 24)) |
+                         ((uint64_t)sa_nonacgt8(__ldg(pw + 4)) << 32);
+    const uint64_t wmask = (1ull << seed_size) - 1;
+    uint32_t ok = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ok |= ((bad >> k) & wmask) ? 0u : 1u << k;
+    return ok;
+}
+
+// Spaced-seed key of the window at base p (common/ntcoding.cpp:43-61), or
+// SA_INVALID_KEY: the window's 2-bit codes in two words, then the shape
+// positions' codes in order, first position most significant.
+__device__ __forceinline__ uint32_t sa_window_key(const uint32_t* __restrict__ packed, uint32_t p, const SaParams& P) {
+    const uint32_t* pw = packed + (p >> 3);
+    const uint32_t sh = (p & 7u) * 4u;
+    uint32_t a = __ldg(pw), bad = 0, code[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t b = __ldg(pw + i + 1);
+        uint32_t x = __funnelshift_r(a, b, sh);
+        a = b;
+        const int n = P.seed_size - 8 * i;  // bases of the window in this word
+        bad |= x & (n >= 8 ? 0x44444444u : n <= 0 ? 0u : 0x44444444u >> (32 - 4 * n));
+        x &= 0x33333333u;
+        x = (x | (x >> 2)) & 0x0f0f0f0fu;
+        x = (x | (x >> 4)) & 0x00ff00ffu;
+        code[i] = (x | (x >> 8)) & 0xffffu;
+    }
+    if (bad) return SA_INVALID_KEY;
+    const uint32_t lo = code[0] | (code[1] << 16), hi = code[2] | (code[3] << 16);
+    uint32_t key = 0;
+    for (int i = 0; i < P.kmer_size; ++i) {
+        const int sp = P.shape_pos[i];
+        key = (key << 2) | (((sp < 16 ? lo : hi) >> (2 * (sp & 15))) & 3u);
+    }
+    return key;
 }
 
 #define SA_CUDA_OK(expr)                                   \

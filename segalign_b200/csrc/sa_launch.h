@@ -42,7 +42,15 @@ struct SaResolvedUnit {
     uint32_t start, end;       // seed positions [start, end) (word indices with seeds)
     int32_t rev;
     const uint64_t* seeds = nullptr;  // explicit seed words (device), or null
+    uint64_t shape = 0;               // sa_shape_id of the keys
 };
+
+// Identifies a seed shape: care positions and span.
+inline uint64_t sa_shape_id(const SaParams& p) {
+    uint64_t m = (uint64_t)p.seed_size << 32;
+    for (int i = 0; i < p.kmer_size; ++i) m |= 1ull << p.shape_pos[i];
+    return m;
+}
 
 // Seed slots of a resolved unit: S per position, one per explicit word.
 inline uint64_t sa_unit_slots(const SaResolvedUnit& u, uint64_t S) {
@@ -93,7 +101,7 @@ struct SaWork {
     // survivors (ping-pong) and dedup output
     SaRec* rec[2];
     uint32_t* scope[2];
-    uint32_t* flags;        // [surv_cap]
+    uint64_t list_cap;      // hits the sweep may leave to the lane kernel (a list in `out`), 0: no sweep
     uint64_t surv_cap;
     SaHashSet hset;         // [2 * surv_cap] slots: distinct HSPs of the call; used list aliases rec[1]
     bool hash_clean;        // host: every slot of hset is empty (no full clear needed)
@@ -164,7 +172,7 @@ void sa_launch_sort_kv(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint3
 
 // ---- sa_lookup.cu ----
 void sa_launch_lookup_seeds(SaWork& w, const uint32_t* index, uint32_t nbuckets,
-                            const SaParams& p, int G, cudaStream_t st);
+                            const SaParams& p, int G, cudaStream_t st, bool chain = false);
 void sa_launch_lookup_batch(SaWork& w, const uint32_t* index, uint32_t nbuckets, uint32_t n_bunits,
                             const SaParams& p, int G, cudaStream_t st);
 
@@ -178,6 +186,11 @@ struct SaExtendArgs {
     // 1: units may restrict their hits to a target window (repeat-masker
     // calls); the lane kernel drops the others when it expands a tile
     int32_t windowed = 0;
+    // 1: the resident table holds every seed window of the target (sa_chain_params
+    // says whether the scores allow chains; the device checks the seeds)
+    int32_t chain = 0;
+    int32_t sweep = 0;   // 1: the sweep takes the hits first (if the scores allow the fast form)
+    uint64_t hits = 0;   // the call's hits, where the caller has read them
 };
 // Phase A (lane per hit) and phase B (warp per long hit); B must follow A.
 // grid: CTAs of the persistent launch (0: num_sms x ext_ctas_per_sm).
@@ -185,6 +198,9 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& a, const SaParams& p, 
                            int num_sms, cudaStream_t st, int grid = 0);
 void sa_launch_extend_warp(SaWork& w, const SaExtendArgs& a, const SaParams& p, const SaTuning& t,
                            int num_sms, cudaStream_t st);
+
+// Whether the parameters allow chains of hits (SaExtK's chain fields).
+bool sa_chain_params(const SaParams& p, const SaTuning& t);
 
 // ---- sa_sort.cu ----
 // Sizes the call's HSP set from its hit count (<= 2 * surv_cap slots) and empties it.

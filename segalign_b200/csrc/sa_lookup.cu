@@ -16,16 +16,59 @@
 #define SA_DERR_MAX_HITS 2       // one seed holds >= MAX_HITS hits (reference UB)
 #define SA_DERR_ITERS 3          // more MAX_HITS iterations than supported
 
+// With `chain`, also checks that the call's words are every seed word of the
+// query window [j_lo, j_hi), in seeder order (src/seeder.cpp:57-74): word i is
+// the one that its position and its place i % S in the position's group of S
+// words call for, positions increase, and there are as many of them as valid
+// windows (counted into ctr->windows, compared by sa_k_groups).  Only then may
+// the extension tell a call's hits from the sequences alone.  A word out of
+// place sets ctr->chain_bad; nothing else depends on the check.
 __global__ void __launch_bounds__(256)
 sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restrict__ desc,
                   const uint32_t* __restrict__ index, uint32_t nbuckets, uint32_t* __restrict__ s_lo,
                   uint32_t* __restrict__ s_cnt, unsigned long long* cta_a, unsigned long long* cta_b,
-                  SaCounters* ctr) {
+                  SaCounters* ctr, const SaUnit* __restrict__ units, SaParams P, int chain) {
     uint64_t a, b;
     sa_cta_range(desc->num_seeds, a, b);
     unsigned long long hits = 0, nz = 0;
+    const uint32_t S = P.transition ? 1u + (uint32_t)P.kmer_size : 1u;
+    SaUnit U{};
+    bool bad = false;
+    if (chain) {
+        U = units[0];
+        const uint64_t n = desc->num_seeds, span = U.j_hi > U.j_lo ? U.j_hi - U.j_lo : 0;
+        // few words over a wide window are no seeder's chunk, and counting its windows would cost more than the call
+        if (n % S || U.j_hi > U.q_len || span > (1u << 20) + 2 * n) {
+            bad = true;
+            chain = 0;
+        } else {
+            uint64_t ga, gb;  // words of 8 positions
+            sa_cta_range(span ? ((U.j_hi - 1) >> 3) - (U.j_lo >> 3) + 1 : 0, ga, gb);
+            unsigned long long windows = 0;
+            for (uint64_t g = (U.j_lo >> 3) + ga + threadIdx.x; g < (U.j_lo >> 3) + gb; g += 256) {
+                uint32_t ok = sa_valid_windows8(U.q_packed + g, (uint32_t)P.seed_size);
+                if (8 * g < U.j_lo) ok &= 0xffu << (U.j_lo - 8 * g);
+                if (8 * g + 8 > U.j_hi) ok &= 0xffu >> (8 * g + 8 - U.j_hi);
+                windows += __popc(ok & 0xffu);
+            }
+#pragma unroll
+            for (int s = 16; s >= 1; s >>= 1) windows += __shfl_xor_sync(0xffffffffu, windows, s);
+            if ((threadIdx.x & 31) == 0 && windows) atomicAdd(&ctr->windows, windows);
+        }
+    }
     for (uint64_t i = a + threadIdx.x; i < b; i += 256) {
-        uint32_t key = (uint32_t)(seeds[i] >> 32);
+        const uint64_t word = seeds[i];
+        uint32_t key = (uint32_t)(word >> 32);
+        if (chain) {
+            const uint32_t j = (uint32_t)word, v = (uint32_t)(i % S);
+            const uint32_t before = i ? (uint32_t)seeds[i - 1] : 0u;
+            bool ok = j >= U.j_lo && j < U.j_hi && (v ? before == j : (i == 0 || before < j));
+            if (ok) {
+                const uint32_t k0 = sa_window_key(U.q_packed, j, P);
+                ok = k0 != SA_INVALID_KEY && key == (v ? k0 ^ (2u << (2 * (v - 1))) : k0);
+            }
+            bad |= !ok;
+        }
         uint32_t lo = 0, cnt = 0;
         if (key < nbuckets) {
             uint32_t hi = __ldg(index + key);
@@ -39,6 +82,7 @@ sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restri
         hits += cnt;
         nz += cnt != 0;
     }
+    if (bad) ctr->chain_bad = 1;
     __shared__ unsigned long long ws[9];
     unsigned long long tot;
     sa_block_excl_sum<unsigned long long, 256>(hits, ws, &tot);
@@ -82,10 +126,12 @@ sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restric
 
 // MAX_HITS iterations (src/seed_filter.cu:686-697): num_iter = num_hits/MAX_HITS + 1;
 // limit[i] = lower_bound(P, lim) - 1, lim = P[limit[i]] + MAX_HITS, last limit = n-1.
+// Hits of different iterations are deduplicated apart, so chains need one.
 __global__ void sa_k_groups(const uint64_t* __restrict__ P, const SaCallDesc* desc, uint64_t* limits,
-                            SaCounters* ctr) {
+                            SaCounters* ctr, uint32_t words_per_window) {
     const uint64_t n = desc->num_seeds, MH = desc->max_hits, H = ctr->num_hits;
     uint64_t num_iter = MH ? H / MH + 1 : 1;
+    if (num_iter > 1 || ctr->windows * words_per_window != n) ctr->chain_bad = 1;
     if (num_iter > SA_MAX_ITERS) {
         atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_ITERS);
         num_iter = 1;
@@ -124,14 +170,15 @@ __global__ void sa_k_scope(SaSeedList cs, const uint64_t* __restrict__ limits, S
 }
 
 void sa_launch_lookup_seeds(SaWork& w, const uint32_t* index, uint32_t nbuckets, const SaParams& p, int G,
-                            cudaStream_t st) {
-    sa_k_lookup_count<<<G, 256, 0, st>>>(w.seeds, w.desc, index, nbuckets, w.s_lo, w.s_cnt, w.cta_a, w.cta_b, w.ctr);
+                            cudaStream_t st, bool chain) {
+    sa_k_lookup_count<<<G, 256, 0, st>>>(w.seeds, w.desc, index, nbuckets, w.s_lo, w.s_cnt, w.cta_a, w.cta_b, w.ctr,
+                                         w.units, p, chain ? 1 : 0);
     sa_note_launch();
     sa_k_scan_partials<<<1, 1024, 0, st>>>(w.cta_a, w.cta_b, G, &w.ctr->num_hits, &w.ctr->nnz);
     sa_note_launch();
     sa_k_lookup_emit<<<G, 256, 0, st>>>(w.seeds, w.desc, w.s_lo, w.s_cnt, w.s_P, w.cs, w.cta_a, w.cta_b, w.ctr);
     sa_note_launch();
-    sa_k_groups<<<1, 1, 0, st>>>(w.s_P, w.desc, w.limits, w.ctr);
+    sa_k_groups<<<1, 1, 0, st>>>(w.s_P, w.desc, w.limits, w.ctr, p.transition ? 1u + (uint32_t)p.kmer_size : 1u);
     sa_note_launch();
     sa_k_scope<<<148 * 4, 256, 0, st>>>(w.cs, w.limits, w.ctr);
     sa_note_launch();
@@ -332,6 +379,7 @@ __global__ void sa_k_bgroups(const SaCallDesc* __restrict__ desc, SaSeedList cs,
             it = 1;
         }
         unit_iters[u] = (uint32_t)it;
+        if (it > 1) ctr->chain_bad = 1;  // its hits are deduplicated per iteration
         unsigned long long* B = bounds + (uint64_t)u * SA_BATCH_ITERS;
         if (it > 1) {
             // compacted seeds of the unit: c with base <= E[c] < base + H

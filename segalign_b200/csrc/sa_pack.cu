@@ -329,13 +329,6 @@ void sa_launch_sort_kv(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint3
 // seed_size bits from each position.  Keys: for each shape position s in
 // increasing order (the shape's order, common/ntcoding.cpp:21-37), the word
 // of bases p0 + s .. p0 + s + 7 gives the next 2-bit code of all 8 keys at once.
-__device__ __forceinline__ uint32_t sa_nonacgt8(uint32_t w) {
-    uint32_t t = (w >> 2) & 0x11111111u;  // bit 4k = code bit 2 of base k
-    t = (t | (t >> 3)) & 0x03030303u;
-    t = (t | (t >> 6)) & 0x000f000fu;
-    return (t | (t >> 12)) & 0xffu;
-}
-
 __global__ void __launch_bounds__(256)
 sa_k_query_keys(const uint32_t* __restrict__ packed, uint64_t len, SaParams P, uint32_t* __restrict__ keys) {
     uint64_t smask = 0;  // bit s set: shape position s is a care position

@@ -279,6 +279,7 @@ void runner_loop(Server& sv) {
                     break;
                 }
                 units.push_back(SaResolvedUnit{r->keys[u.strand], r->packed[u.strand], r->len, u.j0, u.j1, u.strand});
+                units.back().shape = sa_shape_id(sv.view.params);
                 owner.emplace_back(r, r->next_unit);
                 slots += add;
                 ++r->next_unit;
