@@ -113,8 +113,6 @@ struct Slot {
     SaCounters* h_ctr = nullptr;
     SaCallDesc* h_desc = nullptr;
     SaUnit* h_units = nullptr;
-    uint32_t* h_scope_flags = nullptr;
-    uint32_t* h_scope_count = nullptr;
     SaRec* h_out = nullptr;
     uint64_t h_out_cap = 0;
     cudaEvent_t ev[6] = {};
@@ -293,8 +291,6 @@ void free_slot(Slot* s) {
     if (s->h_ctr) cudaFreeHost(s->h_ctr);
     if (s->h_desc) cudaFreeHost(s->h_desc);
     if (s->h_units) cudaFreeHost(s->h_units);
-    if (s->h_scope_flags) cudaFreeHost(s->h_scope_flags);
-    if (s->h_scope_count) cudaFreeHost(s->h_scope_count);
     if (s->h_out) cudaFreeHost(s->h_out);
     for (auto& e : s->ev)
         if (e) cudaEventDestroy(e);
@@ -349,11 +345,7 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         {(void**)&w.hset.score, 4 * 2 * surv_cap},
         {(void**)&w.out, sizeof(SaRec) * surv_cap},
         {(void**)&w.out_scope, 4 * surv_cap},
-        {(void**)&w.scope_count, 4 * SA_MAX_SCOPES},
-        {(void**)&w.scope_flags, 4 * SA_MAX_SCOPES},
-        {(void**)&w.sort_hist, 4 * 256 * SA_SORT_MAX_DIGITS},
-        {(void**)&w.sort_cta_hist, 4 * 256 * (uint64_t)SA_MAX_CTAS + 4 * 64},
-        {(void**)&w.sort_in_buf, 4 * (SA_SORT_MAX_DIGITS + 2)},
+        {(void**)&w.scope_count, batch ? 4 * nunits : 0},
         {(void**)&w.ctr, sizeof(SaCounters)},
         {(void**)&w.desc, sizeof(SaCallDesc)},
         {(void**)&w.units, sizeof(SaUnit) * nunits},
@@ -383,8 +375,6 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         cudaMallocHost(&s->h_ctr, sizeof(SaCounters)) != cudaSuccess ||
         cudaMallocHost(&s->h_desc, sizeof(SaCallDesc)) != cudaSuccess ||
         cudaMallocHost(&s->h_units, sizeof(SaUnit) * nunits) != cudaSuccess ||
-        cudaMallocHost(&s->h_scope_flags, 4 * SA_MAX_ITERS) != cudaSuccess ||
-        cudaMallocHost(&s->h_scope_count, 4 * SA_MAX_ITERS) != cudaSuccess ||
         cudaEventCreate(&s->ev[0]) != cudaSuccess || cudaEventCreate(&s->ev[1]) != cudaSuccess ||
         cudaEventCreate(&s->ev[2]) != cudaSuccess || cudaEventCreate(&s->ev[3]) != cudaSuccess ||
         cudaEventCreate(&s->ev[4]) != cudaSuccess || cudaEventCreate(&s->ev[5]) != cudaSuccess) {
@@ -471,7 +461,7 @@ bool chains_allowed(const DevState& d) {
 
 // Device work of one plain (mode 0) or rm (mode 1) call once its seed words
 // are on the device: descriptor uploads from the slot's pinned buffers,
-// counters reset, lookup, extension, dedup and the counters' copy back.
+// counters reset, lookup, extension and the counters' copy back.
 // Every size is read on the device, so one capture serves every call.
 int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     Global& g = G();
@@ -482,11 +472,10 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     const int Gr = cg.range_ctas;
     SA_CUDA_OK(cudaMemcpyAsync(w.desc, s->h_desc, sizeof(SaCallDesc), cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.units, s->h_units, sizeof(SaUnit), cudaMemcpyHostToDevice, st));
-    SA_CUDA_OK(cudaMemcpyAsync(w.scope_flags, s->h_scope_flags, 4 * SA_MAX_ITERS, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
     const bool chain = chains_allowed(d) && !s->no_sweep;
     sa_launch_lookup_seeds(w, d.index, (uint32_t)d.nbuckets, g.params, Gr, st, chain);
-    sa_launch_hash_init(w, false, st);
+    sa_launch_hash_init(w, st);
     tm.mark(1);
     SaExtendArgs xa;
     xa.chain = chain ? 1 : 0;
@@ -503,8 +492,6 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     tm.mark(2);
     sa_launch_extend_warp(w, xa, g.params, g.tuning, d.num_sms, st);
     tm.mark(3);
-    sa_launch_dedup(w, mode, 0, Gr, st);
-    tm.mark(4);
     SA_CUDA_OK(cudaGetLastError());
     SA_CUDA_OK(cudaMemcpyAsync(s->h_ctr, w.ctr, sizeof(SaCounters), cudaMemcpyDeviceToHost, st));
     return SA_OK;
@@ -577,8 +564,6 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     u[0].flags = mode == 1 ? (1u | (rev ? 2u : 0u)) : 0u;
     u[0].j_lo = n ? (uint32_t)seeds[0] : 0u;
     u[0].j_hi = n ? (uint32_t)seeds[n - 1] + 1u : 0u;
-    for (int i = 0; i < SA_MAX_ITERS; ++i)
-        s->h_scope_flags[i] = (rev ? 1u : 0u) | ((mode == 1 && g.rm_exclude_diag) ? 2u : 0u);
     PhaseTimer tm(s);
     tm.mark(0);
     SA_CUDA_OK(cudaMemcpyAsync(w.seeds, seeds, 8ull * n, cudaMemcpyHostToDevice, st));
@@ -589,7 +574,6 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
         SA_TRY(run_chain(s, mode, tm));
         SA_CUDA_OK(cudaStreamSynchronize(st));
         c = *s->h_ctr;
-        sa_note_hash_state(w, c);
         if (c.list_count <= w.list_cap) break;
     }
     std::memset(&t_stats, 0, sizeof t_stats);
@@ -598,13 +582,14 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     t_stats.hits_extended = c.extended;
     t_stats.seeds_with_hits = c.nnz;
     t_stats.survivors = c.surv_count;
-    t_stats.num_hsps = c.uniq_count;
     t_stats.long_hits = c.long_count;
     t_stats.tiles = c.base_steps;
     t_stats.num_iter = (uint32_t)c.num_iter;
     t_stats.batch_calls = 1;
-    if (c.error) return map_device_error(c.error);
-    const uint64_t nh = c.uniq_count;
+    if (const int e = sa_check_set(w, c)) return map_device_error(e);
+    // the set's HSPs in output order; an rm call's diagonal dedup leaves at most n
+    const uint64_t n_set = c.hash_used;
+    uint64_t nh = n_set;
     if (nh + 1 > s->h_out_cap) {
         if (s->h_out) cudaFreeHost(s->h_out);
         s->h_out = nullptr;
@@ -613,9 +598,21 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
         SA_CUDA_OK(cudaMallocHost(&s->h_out, cap * sizeof(SaRec)));
         s->h_out_cap = cap;
     }
-    if (nh) SA_CUDA_OK(cudaMemcpyAsync(s->h_out + 1, w.out, nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
+    int buf;
+    if (mode == 1) {
+        buf = sa_launch_sort_rm(w, n_set, g.rm_exclude_diag && !rev, st);
+        SA_CUDA_OK(cudaMemcpyAsync(&s->h_ctr->uniq_count, &w.ctr->uniq_count, 8, cudaMemcpyDeviceToHost, st));
+    } else {
+        buf = sa_launch_sort(w, n_set, st);
+    }
+    tm.mark(4);
+    SA_CUDA_OK(cudaGetLastError());
+    if (nh) SA_CUDA_OK(cudaMemcpyAsync(s->h_out + 1, w.rec[buf], nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
     tm.mark(5);
-    SA_CUDA_OK(cudaStreamSynchronize(st));
+    if (nh || mode == 1 || tm.on) SA_CUDA_OK(cudaStreamSynchronize(st));
+    w.hash_clean = true;  // the output emptied the slots the call had used
+    if (mode == 1) nh = s->h_ctr->uniq_count;
+    t_stats.num_hsps = nh;
     tm.collect(t_stats);
     // header (src/seed_filter.cu:756-759): len = total anchors, score = num_hits
     s->h_out[0].ref_start = 0;
@@ -754,12 +751,11 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     SA_CUDA_OK(cudaMemcpyAsync(w.bunits, bu.data(), sizeof(SaBatchUnit) * n, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.units, hu, sizeof(SaUnit) * n, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.desc, hd, sizeof(SaCallDesc), cudaMemcpyHostToDevice, st));
-    SA_CUDA_OK(cudaMemsetAsync(w.scope_flags, 0, 4 * n, st));
     SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
     sa_launch_lookup_batch(w, d.index, (uint32_t)d.nbuckets, n, g.params, Gr, st);
     if (!w.hash_clean) sa_launch_hash_clear(w, st);
     w.hash_clean = false;  // until this group is seen to complete
-    sa_launch_hash_init(w, false, st);
+    sa_launch_hash_init(w, st);
     tm.mark(1);
     SaExtendArgs xa;
     xa.ref = d.ref.data;
@@ -781,21 +777,25 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     tm.mark(2);
     sa_launch_extend_warp(w, xa, g.params, g.tuning, d.num_sms, st);
     tm.mark(3);
-    sa_launch_dedup(w, 0, 4, Gr, st);
-    tm.mark(4);
     SA_CUDA_OK(cudaGetLastError());
     SA_CUDA_OK(cudaMemcpyAsync(s->h_ctr, w.ctr, sizeof(SaCounters), cudaMemcpyDeviceToHost, st));
     SA_CUDA_OK(cudaStreamSynchronize(st));
     SaCounters c = *s->h_ctr;
-    sa_note_hash_state(w, c);
-    if (c.hash_overflow || c.error == 4) return SA_ERR_CAPACITY;
+    const int bad = sa_check_set(w, c);
+    if (bad == SA_DERR_SURV_OVERFLOW) return SA_ERR_CAPACITY;
     if (c.list_count > w.list_cap) return run_batch_group(d, s, units, u0, u1, want_out, res, false);
-    if (c.error) return map_device_error(c.error);
+    if (bad) return map_device_error(bad);
+    const uint64_t nh = c.hash_used;
+    const int buf = sa_launch_sort(w, nh, st);
+    const SaRec* const sorted = w.rec[buf];
+    sa_launch_unit_counts(w, buf, nh, n, st);
+    tm.mark(4);
+    SA_CUDA_OK(cudaGetLastError());
     res.tot.num_hits += c.num_hits;
     res.tot.extended += c.extended;
     res.tot.nnz += c.nnz;
     res.tot.surv_count += c.surv_count;
-    res.tot.uniq_count += c.uniq_count;
+    res.tot.uniq_count += nh;
     res.tot.long_count += c.long_count;
     res.tot.base_steps += c.base_steps;
     std::vector<unsigned long long> hb(n), he(n);
@@ -805,7 +805,6 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     SA_CUDA_OK(cudaMemcpyAsync(hb.data(), w.unit_hit_base, 8ull * n, cudaMemcpyDeviceToHost, st));
     SA_CUDA_OK(cudaMemcpyAsync(he.data(), w.unit_hit_end, 8ull * n, cudaMemcpyDeviceToHost, st));
     SA_CUDA_OK(cudaMemcpyAsync(cnt.data(), w.scope_count, 4ull * n, cudaMemcpyDeviceToHost, st));
-    const uint64_t nh = c.uniq_count;
     if (want_out && nh + 1 > s->h_out_cap) {
         SA_CUDA_OK(cudaStreamSynchronize(st));
         if (s->h_out) cudaFreeHost(s->h_out);
@@ -836,12 +835,12 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
             part_u[k + 1] = u;
             part_r[k + 1] = r;
             if (r > part_r[k])
-                SA_CUDA_OK(cudaMemcpyAsync(s->h_out + part_r[k], w.out + part_r[k], (r - part_r[k]) * sizeof(SaRec),
+                SA_CUDA_OK(cudaMemcpyAsync(s->h_out + part_r[k], sorted + part_r[k], (r - part_r[k]) * sizeof(SaRec),
                                            cudaMemcpyDeviceToHost, st));
             SA_CUDA_OK(cudaEventRecord(s->part_ev[k], st));
         }
     } else if (want_out && nh) {
-        SA_CUDA_OK(cudaMemcpyAsync(s->h_out, w.out, nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
+        SA_CUDA_OK(cudaMemcpyAsync(s->h_out, sorted, nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
     }
     tm.mark(5);
     for (uint32_t i = 0; i < n; ++i) res.hits[u0 + i] = he[i] - hb[i];
@@ -862,10 +861,12 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
             }
         }
         SA_CUDA_OK(cudaStreamSynchronize(st));
+        w.hash_clean = true;
         tm.collect(res.timing);
         return SA_OK;
     }
     SA_CUDA_OK(cudaStreamSynchronize(st));
+    w.hash_clean = true;  // the output emptied the slots the group had used
     tm.collect(res.timing);
     if (want_out && res.sink) return res.sink->put(u0, n, s->h_out, cnt.data(), res.hits.data() + u0);
     uint64_t at = 0;
@@ -1940,6 +1941,7 @@ int sa_resident_view(uint32_t buffer, SaResidentView* v) {
     v->max_seeds = g.max_seeds;
     v->max_hits = max_hits_now();
     v->wga_chunk = g.wga_chunk;
+    v->chain = chains_allowed(d);
     v->params = g.params;
     v->tuning = g.tuning;
     return SA_OK;

@@ -102,7 +102,6 @@ struct SaCounters {
     unsigned long long hash_mask;      // slots - 1 of this call's HSP hash set
     unsigned long long hash_overflow;  // inserts that found no free slot
     unsigned long long hash_used;      // slots claimed in the HSP set (entries of its used list)
-    unsigned long long pad[3];         // device-side counts of the dedup stages
     unsigned long long chain_bad;      // nonzero: the call's hits are not known to be every seed match of its windows
     unsigned long long windows;        // plain call: valid seed windows in [j_lo, j_hi)
     unsigned long long list_count;     // hits the sweep left to the lane kernel (past the list's capacity: the call is run again without it)

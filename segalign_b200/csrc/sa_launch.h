@@ -105,14 +105,9 @@ struct SaWork {
     uint64_t surv_cap;
     SaHashSet hset;         // [2 * surv_cap] slots: distinct HSPs of the call; used list aliases rec[1]
     bool hash_clean;        // host: every slot of hset is empty (no full clear needed)
-    SaRec* out;             // [surv_cap] deduplicated records (device)
+    SaRec* out;             // [surv_cap] the sweep's list
     uint32_t* out_scope;
-    uint32_t* scope_count;  // [SA_MAX_SCOPES]
-    uint32_t* scope_flags;  // [SA_MAX_SCOPES] bit0 = rev (rm diagonal exclusion)
-    // sort state
-    unsigned int* sort_hist;      // [SA_SORT_MAX_DIGITS * 256] global histograms
-    unsigned int* sort_cta_hist;  // [256 * SA_MAX_CTAS]
-    int* sort_in_buf;             // [SA_SORT_MAX_DIGITS + 1] input buffer per pass, final at [D]
+    uint32_t* scope_count;  // [SA_MAX_UNITS] records per batch unit
     // counters + descriptor
     SaCounters* ctr;
     SaCallDesc* desc;
@@ -128,9 +123,8 @@ struct SaWork {
 
 #define SA_MAX_CTAS 1024
 #define SA_MAX_ITERS 256
-#define SA_MAX_SCOPES 65536
 #define SA_MAX_UNITS 65536
-#define SA_SORT_MAX_DIGITS 20
+#define SA_DERR_SURV_OVERFLOW 4  // device error code: more HSPs than the workspace holds
 
 struct SaTuning {
     int lane_cap;        // bases per direction handled lane-per-hit before a hit moves to the long queue
@@ -203,19 +197,23 @@ void sa_launch_extend_warp(SaWork& w, const SaExtendArgs& a, const SaParams& p, 
 bool sa_chain_params(const SaParams& p, const SaTuning& t);
 
 // ---- sa_sort.cu ----
-// Sizes the call's HSP set from its hit count (<= 2 * surv_cap slots) and empties it.
-// Sizes the call's HSP set (device side, from the hit count); `full` also
-// empties every slot.  sa_launch_hash_clear only empties every slot.
-void sa_launch_hash_init(SaWork& w, bool full, cudaStream_t st);
+// Sizes the call's HSP set (device side, from the hit count); sa_launch_hash_clear
+// empties every slot.
+void sa_launch_hash_init(SaWork& w, cudaStream_t st);
 void sa_launch_hash_clear(SaWork& w, cudaStream_t st);
 // Kernel attributes of the lane kernel, set once per device outside stream capture.
 void sa_prepare_extend_lane(const SaParams& p, const SaTuning& t);
-// After the host has read a call's counters: whether the HSP set was left empty.
-void sa_note_hash_state(SaWork& w, const SaCounters& c);
-// mode 0 = plain dedup; 1 = rm (adds diagonal sort/unique and final sort).
-// scope_shift: records are counted per (scope >> scope_shift) and flags are
-// looked up the same way (0 for single calls, 4 for batches: scope = unit<<4 | iteration).
-void sa_launch_dedup(SaWork& w, int mode, int scope_shift, int G, cudaStream_t st);
+// Device error code of a call whose counters the host has read: its own, or
+// SA_DERR_SURV_OVERFLOW if its HSPs did not fit; 0 if the set can be put out.
+int sa_check_set(const SaWork& w, const SaCounters& c);
+// Puts out the n = hash_used HSPs of the set in output order and empties it:
+// records and scopes end in w.rec[i] and w.scope[i], i returned.  The rm form also
+// applies unique_copy(hspDiagEqual) (and drops the main diagonal with `exclude`);
+// the records left are counted in ctr->uniq_count.
+int sa_launch_sort(SaWork& w, uint64_t n, cudaStream_t st);
+int sa_launch_sort_rm(SaWork& w, uint64_t n, bool exclude, cudaStream_t st);
+// Records per unit of the n sorted records in buffer buf, into w.scope_count.
+void sa_launch_unit_counts(SaWork& w, int buf, uint64_t n, uint32_t units, cudaStream_t st);
 // ---- sa_pack.cu (batched seeding) ----
 void sa_launch_query_keys(const uint32_t* packed, uint64_t len, const SaParams& p, uint32_t* keys, cudaStream_t st);
 
@@ -235,6 +233,7 @@ struct SaResidentView {
     uint64_t max_seeds;
     uint64_t max_hits;
     uint32_t wga_chunk;           // InitializeProcessor's WGA_CHUNK
+    bool chain;                   // calls may chain hits of one diagonal (SaExtendArgs)
     SaParams params;
     SaTuning tuning;
 };

@@ -46,8 +46,6 @@ constexpr uint64_t kParts[] = {
     sizeof(SaRec) * kSurv, sizeof(SaRec) * kSurv, 4 * kSurv, 4 * kSurv,  // rec[2], scope[2]
     16 * 2 * kSurv, 4 * 2 * kSurv,                       // HSP set: keys, scores
     sizeof(SaRec) * kSurv, 4 * kSurv,                    // out, out_scope
-    4 * SA_MAX_SCOPES, 4 * SA_MAX_SCOPES,                // scope_count, scope_flags
-    4 * 256 * SA_SORT_MAX_DIGITS, 4 * 256 * (uint64_t)SA_MAX_CTAS + 4 * 64, 4 * (SA_SORT_MAX_DIGITS + 2),
     sizeof(SaCounters), sizeof(SaCallDesc), sizeof(SaUnit) * SA_NOALLOC_UNITS,
 };
 constexpr uint64_t total_bytes() {
@@ -114,16 +112,11 @@ void carve(void* base, SaWork& w) {
     take((void**)&w.hset.score);
     take((void**)&w.out);
     take((void**)&w.out_scope);
-    take((void**)&w.scope_count);
-    take((void**)&w.scope_flags);
-    take((void**)&w.sort_hist);
-    take((void**)&w.sort_cta_hist);
-    take((void**)&w.sort_in_buf);
     take((void**)&w.ctr);
     take((void**)&w.desc);
     take((void**)&w.units);
     w.seed_cap = kSeeds;
-    w.list_cap = 0;  // no sweep
+    w.list_cap = kSurv;
     w.surv_cap = kSurv;
     w.long_cap = SA_NOALLOC_LONG_CAP;
     // the HSP set's list of claimed slots lives in rec[1], free until the sort
@@ -175,20 +168,13 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
     SaUnit unit{};
     unit.q_packed = q;
     unit.q_len = v.q_len;
-    uint32_t flags[SA_MAX_ITERS];
-    for (int i = 0; i < SA_MAX_ITERS; ++i) flags[i] = rev ? 1u : 0u;
-    SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
+    unit.j_lo = num_seeds ? (uint32_t)seeds[0] : 0u;
+    unit.j_hi = num_seeds ? (uint32_t)seeds[num_seeds - 1] + 1u : 0u;
     SA_CUDA_OK(cudaMemcpyAsync(w.seeds, seeds, 8ull * num_seeds, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.desc, &desc, sizeof desc, cudaMemcpyHostToDevice, st));
     SA_CUDA_OK(cudaMemcpyAsync(w.units, &unit, sizeof unit, cudaMemcpyHostToDevice, st));
-    SA_CUDA_OK(cudaMemcpyAsync(w.scope_flags, flags, sizeof flags, cudaMemcpyHostToDevice, st));
     // the grids and lane-kernel settings of a plain call (sa_seed_and_filter)
     const SaCallGrids cg = sa_call_grids(v.tuning, v.num_sms, 0);
-    const int G = cg.range_ctas;
-    sa_launch_lookup_seeds(w, v.index, (uint32_t)v.nbuckets, v.params, G, st);
-    if (!w.hash_clean) sa_launch_hash_clear(w, st);
-    w.hash_clean = false;
-    sa_launch_hash_init(w, false, st);
     SaExtendArgs xa;
     xa.ref = v.ref;
     xa.ref_len = v.ref_len;
@@ -197,29 +183,42 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
     xa.xdrop = v.params.xdrop;
     xa.hspthresh = v.params.hspthresh;
     xa.noentropy = v.params.noentropy;
-    sa_launch_extend_lane(w, xa, v.params, cg.lane_tuning, v.num_sms, st, cg.lane_ctas);
-    sa_launch_extend_warp(w, xa, v.params, v.tuning, v.num_sms, st);
-    sa_launch_dedup(w, 0, 0, G, st);
-    SA_CUDA_OK(cudaGetLastError());
     SaCounters c;
-    SA_CUDA_OK(cudaMemcpyAsync(&c, w.ctr, sizeof c, cudaMemcpyDeviceToHost, st));
-    SA_CUDA_OK(cudaStreamSynchronize(st));
-    sa_note_hash_state(w, c);
-    g_hash_clean[v.dev] = w.hash_clean;
-    if (c.hash_overflow || c.error == 4) {
+    for (bool sweep = true;; sweep = false) {  // again without the sweep if its list was too small
+        xa.sweep = sweep ? 1 : 0;
+        xa.chain = sweep && v.chain ? 1 : 0;
+        SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
+        sa_launch_lookup_seeds(w, v.index, (uint32_t)v.nbuckets, v.params, cg.range_ctas, st, xa.chain != 0);
+        if (!w.hash_clean) sa_launch_hash_clear(w, st);
+        w.hash_clean = false;
+        sa_launch_hash_init(w, st);
+        sa_launch_extend_lane(w, xa, v.params, cg.lane_tuning, v.num_sms, st, cg.lane_ctas);
+        sa_launch_extend_warp(w, xa, v.params, v.tuning, v.num_sms, st);
+        SA_CUDA_OK(cudaGetLastError());
+        SA_CUDA_OK(cudaMemcpyAsync(&c, w.ctr, sizeof c, cudaMemcpyDeviceToHost, st));
+        SA_CUDA_OK(cudaStreamSynchronize(st));
+        if (c.list_count <= w.list_cap) break;
+    }
+    const int bad = sa_check_set(w, c);
+    if (bad == SA_DERR_SURV_OVERFLOW) {
         sa_set_error(SA_ERR_CAPACITY, "more than %u distinct HSPs (no-allocation limit)", SA_NOALLOC_MAX_SURVIVORS);
         return SA_ERR_CAPACITY;
     }
-    if (c.error) return sa_map_device_error(c.error);
-    const uint64_t nh = c.uniq_count;
+    if (bad) return sa_map_device_error(bad);
+    const uint64_t nh = c.hash_used;
+    const int buf = sa_launch_sort(w, nh, st);
+    SA_CUDA_OK(cudaGetLastError());
     *out_len = nh + 1;
-    if (nh + 1 > out_cap) {
+    const bool fits = nh + 1 <= out_cap;
+    if (nh && fits)
+        SA_CUDA_OK(cudaMemcpyAsync(out + 1, w.rec[buf], nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
+    SA_CUDA_OK(cudaStreamSynchronize(st));
+    g_hash_clean[v.dev] = true;  // the output emptied the slots the call had used
+    if (!fits) {
         sa_set_error(SA_ERR_CAPACITY, "output needs %llu records, buffer holds %llu", (unsigned long long)(nh + 1),
                      (unsigned long long)out_cap);
         return SA_ERR_CAPACITY;
     }
-    if (nh) SA_CUDA_OK(cudaMemcpyAsync(out + 1, w.out, nh * sizeof(SaRec), cudaMemcpyDeviceToHost, st));
-    SA_CUDA_OK(cudaStreamSynchronize(st));
     out[0].ref_start = 0;
     out[0].query_start = 0;
     out[0].len = (uint32_t)nh;
