@@ -244,12 +244,25 @@ __device__ __forceinline__ void sa_window_exact(const char* tblb, uint32_t lo, u
 // that follow it by the same test (sa_chain_members) and counts their tiles and
 // survivors: the call's statistics stay those of every hit scanned.
 //
+// The sweep (below) finishes hits that stop early with a low total; such a hit
+// counts no others.  As p' has p's total, and stops delta bases further right
+// and delta fewer left, p sees whether the sweep finishes p': not if p itself
+// has not stopped in the sweep's 32 bases right, nor if both of p's scans
+// have stopped there and the total is high (else p would be finished).  In the
+// remaining case, stopped right and not left, p is not dropped.  Near a
+// sequence end (sa_sweep_margin) no hit is.
+//
 // On the genome workload 13-16% of the hits are dropped, with them a third to
 // two fifths of all 32-base scan steps (they are the hits inside long HSPs);
 // on repeat-rich targets half the steps, in a self-alignment nine of ten.
 // ---------------------------------------------------------------------------
 #define SA_CHAIN_BLOCK 1024u
 #define SA_CHAIN_NEXT 0x80000000u  // unit bit: a hit follows on the diagonal within `gap` bases
+#define SA_CHAIN_DROP 0x40000000u  // unit bit, inside the sweep: what it saw of the hit allows dropping it
+#define SA_CHAIN_HIGH 0x40000000u  // unit bit, in `lead`: the hit's total is at least hspthresh
+#define SA_CHAIN_GAP 13u           // largest `gap`
+#define SA_SWEEP_RIGHT 32u         // bases the sweep scores right and left of a hit
+#define SA_SWEEP_LEFT 64u
 
 // Bit 4k of v (k = 0..7) -> bit 24 + k of the result (lower bits are left over).
 __device__ __forceinline__ uint32_t sa_nibble_bits(uint32_t v) {
@@ -312,11 +325,18 @@ __device__ __forceinline__ bool sa_chain_joined(const SaExtK& a, uint32_t mis, u
     return last > near;
 }
 
-// One hit: 0 = scan it, 1 = dropped, SA_CHAIN_NEXT = scan it, and a hit follows
-// within `gap` bases.  r, q: the 6 words (48 bases) from 32 bases before p.
+// Whether the sweep's windows of a hit and of those up to SA_CHAIN_GAP bases
+// either way lie inside both sequences.
+__device__ __forceinline__ bool sa_sweep_margin(const SaExtK& a, const SaUnit& U, uint32_t rl, uint32_t ql) {
+    return min(rl, ql) >= SA_SWEEP_LEFT + SA_CHAIN_GAP && (uint64_t)rl + SA_SWEEP_RIGHT + SA_CHAIN_GAP <= a.ref_len &&
+           (uint64_t)ql + SA_SWEEP_RIGHT + SA_CHAIN_GAP <= U.q_len;
+}
+
+// One hit the sweep has not finished: 0 = scan it, 1 = dropped, SA_CHAIN_NEXT =
+// scan it, and a hit follows within `gap` bases.
 template <bool TRANS>
 __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, const SaUnit& U, uint32_t rl, uint32_t ql,
-                                                  const uint32_t* r, const uint32_t* q) {
+                                                  bool may_drop) {
     const uint32_t S = a.seed_size, own = 32 - S, j = ql - S;
     uint32_t back = min(min(a.gap, j & (SA_CHAIN_BLOCK - 1)), min(j - U.j_lo, rl - S - 1));  // position 0 is not in the table
     uint32_t ahead = min(a.gap, U.j_hi - 1 - j);
@@ -324,18 +344,28 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
         back = min(back, rl - U.rm_lo);
         ahead = min(ahead, U.rm_hi - rl);
     }
-    uint32_t m[6], t[6], any = 0;
+    // 48 bases from p - 32
+    const uint32_t* __restrict__ pr = a.ref + (int)(rl >> 3) - 4;
+    const uint32_t* __restrict__ pq = U.q_packed + (int)(ql >> 3) - 4;
+    const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
+    uint32_t r[7], q[7], m[6], t[6], any = 0;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        r[k] = __ldg(pr + k);
+        q[k] = __ldg(pq + k);
+    }
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        if (k < 4) any |= r[k] | q[k];
-        sa_match_bits<TRANS>(r[k], q[k], m[k], t[k]);
+        const uint32_t rw = __funnelshift_r(r[k], r[k + 1], sr), qw = __funnelshift_r(q[k], q[k + 1], sq);
+        if (k < 4) any |= rw | qw;
+        sa_match_bits<TRANS>(rw, qw, m[k], t[k]);
     }
     const uint32_t m0 = sa_join_bits(m[0], m[1], m[2], m[3]), m1 = __byte_perm(m[4], m[5], 0x0073) & 0xffffu;
     const uint32_t t0 = TRANS ? sa_join_bits(t[0], t[1], t[2], t[3]) : 0u;
     const uint32_t t1 = TRANS ? __byte_perm(t[4], t[5], 0x0073) & 0xffffu : 0u;
     const uint32_t H = sa_seed_bits<TRANS>(a, kmer, m0, m1, t0, t1, 0);  // bit own: this hit
     const uint32_t prev = (H & ((1u << own) - 1u)) >> (own - back) << (own - back);
-    if (prev && !(any & 0x44444444u) && sa_chain_joined(a, ~m0, own - (31 - __clz(prev)))) return 1;
+    if (may_drop && prev && !(any & 0x44444444u) && sa_chain_joined(a, ~m0, own - (31 - __clz(prev)))) return 1;
     return ((H >> own >> 1) & ((1u << ahead) - 1u)) ? SA_CHAIN_NEXT : 0u;
 }
 
@@ -344,8 +374,9 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // scored over the 32 bases right of it and the 64 left of it (the seed and as
 // many again).  A hit whose scans both stop there with a total below hspthresh
 // is done: it adds its tiles and leaves nothing else.  These are the chance
-// hits, four of five on the genome workload.  Dropped hits of chains are
-// done too.  The others go to `list`, which the lane kernel scans.
+// hits, four of five on the genome workload.  The others gather in a buffer
+// per warp; full batches of them take the chain test, and those it does not
+// drop go to `list`, which the lane kernel scans.
 //
 // Why apart from the lane kernel: a chance hit's work there was the hand-out,
 // two direction set-ups and the bookkeeping of an iteration, most of it run
@@ -354,12 +385,14 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // 16-byte loads of the target (a scattered load costs an L1 wavefront per
 // lane, whatever its width), and query words that consecutive hits share.
 //
-// Bound by instruction issue and, close behind, the L1 data pipe (96 table
-// lookups and the target loads' wavefronts per round).  On a 2.5 Mbp query against
-// the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in the
-// lane kernel 5.65 ms; sweep 2.33, lane kernel 1.40, chain walk 0.27: 3.97 ms
-// (4.79 with the sweep and no chains).  Lane phase of 24 Mbp: 55.0 -> 36.4 ms;
-// of a repeat-masker call, 0.80 -> 0.39 ms, and its warp kernel 0.78 -> 0.13.
+// Bound by the L1 data pipe (83%: 96 table lookups and 128 wavefronts of target
+// loads in about 250 per round), with the ALU pipe and issue at 70%.  On a 2.5 Mbp query
+// against the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in
+// the lane kernel 5.65 ms; sweep 2.00, lane kernel 1.46, chain walk 0.33: 3.75 ms (4.79
+// with the sweep and no chains).  The chain test on all hits as they were
+// scored, with the rounds split evenly over the warps, made the sweep 2.33 ms.
+// Lane phase of 24 Mbp: 55.0 -> 34.5 ms; of a repeat-masker call, 0.80 -> 0.40 ms,
+// and its warp kernel 0.78 -> 0.14.
 // ---------------------------------------------------------------------------
 // One 8-base window of a scan, from its first base on (REV: from base 7
 // down): running score S, best B, and whether a base of it stops the scan (the
@@ -381,7 +414,7 @@ __device__ __forceinline__ void sa_sweep_window(const char* tblb, uint32_t rw, u
     stop = stop || B - mn > xdrop;
 }
 
-#define SA_SWEEP_BUF 128  // list records a warp gathers before it writes them
+#define SA_SWEEP_BUF 128  // unfinished hits a warp gathers
 
 template <bool TRANS>
 __global__ void __launch_bounds__(256, 4)
@@ -397,26 +430,56 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
     const bool chains = a.chain && !ctr->chain_bad;
     const int lane = threadIdx.x & 31;
     const uint32_t lt = sa_lanemask_lt();
-    const uint32_t warps = gridDim.x * 8, w = blockIdx.x * 8 + (threadIdx.x >> 5);
     uint4* const buf = s_buf[threadIdx.x >> 5];
     uint32_t nbuf = 0, tiles = 0, ext = 0;
+    // chain test of the buffered hits, 32 at a time; those left, moved to the
+    // buffer's front, go to the list
     auto write_out = [&]() {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)nbuf);
-        at = __shfl_sync(SA_FULL, at, 0);
         __syncwarp();
-        for (uint32_t i = lane; i < nbuf; i += 32)
+        uint32_t kept = nbuf;
+        if (chains) {
+            kept = 0;
+            for (uint32_t i0 = 0; i0 < nbuf; i0 += 32) {
+                const bool on = i0 + lane < nbuf;
+                uint4 v = make_uint4(0, 0, 0, 0);
+                uint32_t f = 1;
+                if (on) {
+                    v = buf[i0 + lane];
+                    const bool may_drop = v.w & SA_CHAIN_DROP;
+                    v.w &= ~SA_CHAIN_DROP;
+                    f = sa_chain_test<TRANS>(a, P.kmer_size, a.units[v.w], v.x, v.y, may_drop);
+                }
+                const uint32_t m = __ballot_sync(SA_FULL, f != 1);
+                if (f != 1) {
+                    v.w |= f;
+                    buf[kept + __popc(m & lt)] = v;
+                }
+                kept += __popc(m);
+                __syncwarp();
+            }
+        }
+        nbuf = 0;
+        if (!kept) return;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)kept);
+        at = __shfl_sync(SA_FULL, at, 0);
+        for (uint32_t i = lane; i < kept; i += 32)
             if (at + i < a.list_cap) a.list[at + i] = buf[i];
         __syncwarp();
-        nbuf = 0;
     };
-    const uint64_t first = h_begin / 32, rounds = (H + 31) / 32;  // h_begin is a multiple of 32
-    // rounds a warp takes in a row: its first seed is searched for once
-    const uint64_t run = min((rounds - first + warps - 1) / warps, (uint64_t)64);
-    for (uint64_t r0 = first + w * run; r0 < rounds; r0 += (uint64_t)warps * run) {
-        const uint64_t r1 = min(r0 + run, rounds);
-        uint64_t c = sa_warp_find_seed(a.cs.E, nnz, 32 * r0);
-        for (uint64_t r = r0; r < r1; ++r) {
+    const uint64_t first = h_begin / 32, rounds = (H + 31) / 32 - first;  // h_begin is a multiple of 32
+    // Runs of rounds are handed out by a counter (the warps' speeds differ with
+    // their hits); a run's first seed is searched for once.  32 rounds where
+    // there are enough for every warp to take eight runs.
+    const uint64_t run = max((uint64_t)1, min((uint64_t)32, rounds / ((uint64_t)gridDim.x * 64)));
+    while (true) {
+        unsigned long long k0 = 0;
+        if (lane == 0) k0 = atomicAdd(&ctr->sweep_cursor, 1ull);
+        const uint64_t r0 = (uint64_t)__shfl_sync(SA_FULL, k0, 0) * run;
+        if (r0 >= rounds) break;
+        const uint64_t r1 = first + min(r0 + run, rounds);
+        uint64_t c = sa_warp_find_seed(a.cs.E, nnz, 32 * (first + r0));
+        for (uint64_t r = first + r0; r < r1; ++r) {
             const uint64_t t = 32 * r, h = t + lane;
             // the hit's seed: c, and one more for each seed that starts by then
             const uint64_t ahead = c + 1 + lane < nnz ? a.cs.E[c + 1 + lane] - t : ~0ull;
@@ -442,7 +505,7 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                 if (live) {
                     ++ext;
                     // bases [rl - 64, rl + 32) of both sequences as 12 words
-                    const uint32_t* __restrict__ pq = U.q_packed + (ql >> 3) - 8;
+                    const uint32_t* __restrict__ pq = U.q_packed + (int)(ql >> 3) - 8;
                     uint32_t rw[16], qw[13];
 #pragma unroll
                     for (int i = 0; i < 13; ++i) qw[i] = __ldg(pq + i);
@@ -464,31 +527,29 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                         for (int i = 0; i < 13; ++i) rw[i] = rw[i + 2];
                     }
                     const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
+                    int S = 0, B = 0, R = 0, L = 0;
+                    bool stop_r = false, stop_l = false;
 #pragma unroll
-                    for (int i = 0; i < 12; ++i) {
-                        rw[i] = __funnelshift_r(rw[i], rw[i + 1], sr);
-                        qw[i] = __funnelshift_r(qw[i], qw[i + 1], sq);
+                    for (int i = 8; i < 12; ++i)
+                        sa_sweep_window<false>(tblb, __funnelshift_r(rw[i], rw[i + 1], sr),
+                                               __funnelshift_r(qw[i], qw[i + 1], sq), a.xdrop, S, B, R, stop_r);
+                    S = B = 0;
+                    uint32_t tl = 0;
+#pragma unroll
+                    for (int i = 7; i >= 0; --i) {
+                        sa_sweep_window<true>(tblb, __funnelshift_r(rw[i], rw[i + 1], sr),
+                                              __funnelshift_r(qw[i], qw[i + 1], sq), a.xdrop, S, B, L, stop_l);
+                        if (i == 4) tl = stop_l ? 2 : 3;  // tiles of both scans, if they stop
                     }
-                    const uint32_t f = chains ? sa_chain_test<TRANS>(a, P.kmer_size, U, rl, ql, rw + 4, qw + 4) : 0u;
-                    if (f != 1) {
-                        int S = 0, B = 0, R = 0, Lb = 0;
-                        bool stop_r = false, stop_l = false;
-#pragma unroll
-                        for (int i = 8; i < 12; ++i) sa_sweep_window<false>(tblb, rw[i], qw[i], a.xdrop, S, B, R, stop_r);
-                        S = B = 0;
-#pragma unroll
-                        for (int i = 7; i >= 4; --i) sa_sweep_window<true>(tblb, rw[i], qw[i], a.xdrop, S, B, Lb, stop_l);
-                        const uint32_t tl = stop_l ? 2 : 3;
-#pragma unroll
-                        for (int i = 3; i >= 0; --i) sa_sweep_window<true>(tblb, rw[i], qw[i], a.xdrop, S, B, Lb, stop_l);
-                        // a window that reaches past an end scans it to the end: the lane kernel does that
-                        const bool inside = rl >= 64 && ql >= 64 && rl + 32 <= a.ref_len && ql + 32 <= U.q_len;
-                        left = f || !inside || !stop_r || !stop_l || (int)(float)(R + Lb) >= a.hspthresh;
-                        if (!left) tiles += tl;
-                        rec.w |= f;
-                    }
+                    // a window that reaches past an end scans it to the end: the lane kernel does that
+                    const bool inside = min(rl, ql) >= SA_SWEEP_LEFT && (uint64_t)rl + SA_SWEEP_RIGHT <= a.ref_len &&
+                                        (uint64_t)ql + SA_SWEEP_RIGHT <= U.q_len;
+                    left = !inside || !stop_r || !stop_l || (int)(float)(R + L) >= a.hspthresh;
+                    if (!left) tiles += tl;
+                    if (!(stop_r && !stop_l) && sa_sweep_margin(a, U, rl, ql)) rec.w |= SA_CHAIN_DROP;
                 }
             }
+            if (!chains) rec.w &= ~SA_CHAIN_DROP;
             const uint32_t m = __ballot_sync(SA_FULL, left);
             if (left) buf[nbuf + __popc(m & lt)] = rec;
             nbuf += __popc(m);
@@ -524,8 +585,8 @@ __device__ __forceinline__ void sa_masks32(const uint32_t* __restrict__ R, const
     bad = sa_join_bits(bb[0], bb[1], bb[2], bb[3]);
 }
 
-// The dropped hits that follow the scanned hit (rl, ql) of `unit`: their number
-// and the tiles of their scans.  stop_r, stop_l: offsets at which the hit's
+// The dropped hits that follow the scanned hit (rl, ql) of `unit` (high: its
+// total is at least hspthresh): their number and the tiles of their scans.  stop_r, stop_l: offsets at which the hit's
 // right and left scans stop; a hit d bases on stops at stop_r - d and
 // stop_l + d.
 struct SaChain {
@@ -534,7 +595,7 @@ struct SaChain {
 };
 
 __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaParams& P, uint32_t unit, uint32_t rl,
-                                                 uint32_t ql, uint32_t stop_r, uint32_t stop_l) {
+                                                 uint32_t ql, uint32_t stop_r, uint32_t stop_l, bool high) {
     const SaUnit U = a.units[unit];
     unsigned long long tiles = 0;
     const uint32_t S = a.seed_size, j = ql - S;
@@ -545,8 +606,9 @@ __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaPar
     for (uint32_t c = 0; c + 1 - last <= a.gap; c += 32) {
         uint32_t m1, t1, b1;
         sa_masks32(a.ref, U.q_packed, rl, ql, (int)c, m1, t1, b1);
-        if ((m0 & m1) == ~0u && !(b0 | b1) && last == c && c + 32 <= ahead &&
-            ((j + c) & (SA_CHAIN_BLOCK - 1)) + 32 < SA_CHAIN_BLOCK) {
+        if ((m0 & m1) == ~0u && !(b0 | b1) && last == c && c + 32 <= ahead && stop_r >= c + 64 &&
+            ((j + c) & (SA_CHAIN_BLOCK - 1)) + 32 < SA_CHAIN_BLOCK && sa_sweep_margin(a, U, rl + c + 1, ql + c + 1) &&
+            sa_sweep_margin(a, U, rl + c + 32, ql + c + 32)) {
             // 64 matching bases: each of the next 32 positions ends a dropped hit.  Over
             // 32 consecutive d, (stop_r - d) >> 5 sums to stop_r - c - 32 and (stop_l + d) >> 5 to stop_l + c + 1.
             n += 32;
@@ -559,7 +621,8 @@ __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaPar
             for (; hits; hits &= hits - 1) {
                 const uint32_t i = __ffs(hits), d = c + i, delta = d - last;
                 if (d > ahead || delta > a.gap || delta > ((j + d) & (SA_CHAIN_BLOCK - 1)) ||
-                    __funnelshift_rc(b0, b1, i) || !sa_chain_joined(a, ~__funnelshift_rc(m0, m1, i), delta))
+                    (stop_r - d < SA_SWEEP_RIGHT && (!high || stop_l + d >= SA_SWEEP_LEFT)) ||
+                    !sa_sweep_margin(a, U, rl + d, ql + d) || __funnelshift_rc(b0, b1, i) || !sa_chain_joined(a, ~__funnelshift_rc(m0, m1, i), delta))
                     return {tiles, n};
                 ++n;
                 tiles += ((stop_r - d) >> 5) + ((stop_l + d) >> 5) + 2;
@@ -1027,7 +1090,8 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 if (lane == leader) at = atomicAdd(&a.ctr->chain_count, (unsigned long long)__popc(cm));
                 at = __shfl_sync(SA_FULL, at, leader) + __popc(cm & lt);
                 if (leads) {  // at most one per list record
-                    a.lead[at] = make_uint4(rl, ql, unit_id & ~SA_CHAIN_NEXT, (uint32_t)Lpos);
+                    const uint32_t high = (int)(float)total >= a.hspthresh ? SA_CHAIN_HIGH : 0u;
+                    a.lead[at] = make_uint4(rl, ql, (unit_id & ~SA_CHAIN_NEXT) | high, (uint32_t)Lpos);
                     a.lead_right[at] = (uint32_t)Rpos;
                     a.lead_stop_r[at] = L.stop[0][threadIdx.x];
                     a.lead_stop_l[at] = L.stop[1][threadIdx.x];
@@ -1065,7 +1129,8 @@ sa_k_chain_walk(const __grid_constant__ SaExtK a, const __grid_constant__ SaPara
     unsigned long long tiles = 0, kept = 0;
     for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
         const uint4 h = a.lead[i];
-        const SaUnit U = a.units[h.z];
+        const uint32_t unit = h.z & ~SA_CHAIN_HIGH;
+        const SaUnit U = a.units[unit];
         const uint32_t rl = h.x, ql = h.y;
         const char* tblb = reinterpret_cast<const char*>(tbl);
         const uint32_t stop_r = sa_stop_offset<SH>(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql),
@@ -1073,14 +1138,14 @@ sa_k_chain_walk(const __grid_constant__ SaExtK a, const __grid_constant__ SaPara
         const uint32_t stop_l = sa_stop_offset<SH>(tblb, a.ref + sa_rev_words(a.ref_len), U.q_packed + sa_rev_words(U.q_len),
                                                    a.ref_len - rl, U.q_len - ql, min(rl, ql), a.xdrop,
                                                    a.lead_stop_l[i]);
-        const SaChain c = sa_chain_members(a, P, h.z, rl, ql, stop_r, stop_l);
+        const SaChain c = sa_chain_members(a, P, unit, rl, ql, stop_r, stop_l, h.z & SA_CHAIN_HIGH);
         if (!c.n) continue;
         tiles += c.tiles;
         const uint32_t len = a.lead_right[i] + h.w;
         uint32_t qs = ql - h.w;
         if (U.flags & 2u) qs = a.ref_len - 1 - (qs + len);
         // chains are of calls and units with one MAX_HITS iteration: scope (unit << 4) | 0, unit 0 in a call
-        if (sa_hash_holds(a.hset, ctr->hash_mask, h.z << 4, rl - h.w, qs, len)) kept += c.n;
+        if ((h.z & SA_CHAIN_HIGH) && sa_hash_holds(a.hset, ctr->hash_mask, unit << 4, rl - h.w, qs, len)) kept += c.n;
     }
 #pragma unroll
     for (int s = 16; s >= 1; s >>= 1) {
@@ -1098,6 +1163,7 @@ sa_k_chain_walk(const __grid_constant__ SaExtK a, const __grid_constant__ SaPara
 __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
     if (ctr->list_count <= list_cap) ctr->list_count = 0;
     ctr->hit_cursor = 0;
+    ctr->sweep_cursor = 0;
     ctr->chain_count = 0;
 }
 
@@ -1274,7 +1340,8 @@ sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         if (lane == 0) {
             uint32_t stands_for = 1;
             if (L.unit & SA_CHAIN_NEXT) {
-                const SaChain ch = sa_chain_members(a, P, L.unit & ~SA_CHAIN_NEXT, rl, ql, R.stop, Lr.stop);
+                const SaChain ch = sa_chain_members(a, P, L.unit & ~SA_CHAIN_NEXT, rl, ql, R.stop, Lr.stop,
+                                                    (int)(float)total >= a.hspthresh);
                 stands_for += ch.n;
                 tiles_acc += ch.tiles;
             }
@@ -1340,7 +1407,7 @@ static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaParams& p, c
     a.lead_stop_r = w.scope[1];
     a.lead_stop_l = w.out_scope;
     // the 48-base window of sa_chain_test holds the seeds of hits up to `gap` either way
-    a.gap = (uint32_t)std::max(0, std::min({13, p.seed_size - 1, 32 - p.seed_size}));
+    a.gap = (uint32_t)std::max(0, std::min({(int)SA_CHAIN_GAP, p.seed_size - 1, 32 - p.seed_size}));
     a.ref = x.ref;
     a.ref_len = x.ref_len;
     a.pos_table = x.pos_table;

@@ -106,6 +106,7 @@ struct SaCounters {
     unsigned long long windows;        // plain call: valid seed windows in [j_lo, j_hi)
     unsigned long long list_count;     // hits the sweep left to the lane kernel (past the list's capacity: the call is run again without it)
     unsigned long long chain_count;    // scanned hits that others may follow
+    unsigned long long sweep_cursor;   // sweep work counter
 };
 
 // Open-addressing set of distinct HSPs of one call: slot = 16-byte key
