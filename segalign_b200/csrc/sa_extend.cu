@@ -54,7 +54,8 @@ struct SaExtK {
     int32_t match, swing; // smallest match score, and that minus the lowest mismatch score
     uint32_t mismatches;  // as many mismatches in a row cannot stop a scan
     uint32_t shift[16];   // shape positions, the first one again in the unused places
-    uint4* list;          // hits the sweep leaves to the lane kernel: {rl, ql, scope, unit | SA_CHAIN_NEXT}
+    uint4* list;          // hits the sweep leaves to the lane kernel, two words of 16 bytes each:
+                          // {rl, ql, scope, unit | SA_CHAIN_NEXT}, {SaSwept}
     uint64_t list_cap;    // 0: no sweep
     // scanned hits that others may follow [list_cap]: {rl, ql, unit, bases left of
     // the hit}, position of the right end, stop words right and left
@@ -394,24 +395,47 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // Lane phase of 24 Mbp: 55.0 -> 34.5 ms; of a repeat-masker call, 0.80 -> 0.40 ms,
 // and its warp kernel 0.78 -> 0.14.
 // ---------------------------------------------------------------------------
+// What the sweep leaves of a hit, for the lane kernel to go on from: per
+// direction the best score (low half) and best - score (high half) after the
+// direction's sweep, and in `rest` the offsets of the first bases reaching the
+// bests (a byte each) and these flags.  A direction that has stopped leaves its
+// result.
+#define SA_SWEPT_SEEN 0x10000u     // else nothing is scored yet: both directions start anew
+#define SA_SWEPT_STOP_R 0x20000u
+#define SA_SWEPT_STOP_L 0x40000u
+#define SA_SWEPT_TILE_2 0x80000u   // the left scan stopped in its second 32-base tile
+
 // One 8-base window of a scan, from its first base on (REV: from base 7
-// down): running score S, best B, and whether a base of it stops the scan (the
-// windowed stop test of the fast form).
+// down), in the lane kernel's packed form with SA_SWEEP_LEFT in place of STEP
+// (SCALE = 2 * SA_SWEEP_LEFT): P running score, B running best, `at` B at the
+// end of the windows up to and including the one that stops.
+#define SA_SWEEP_SH 7  // log2(SCALE)
 template <bool REV>
-__device__ __forceinline__ void sa_sweep_window(const char* tblb, uint32_t rw, uint32_t qw, int xdrop, int& S, int& B,
+__device__ __forceinline__ void sa_sweep_window(const char* tblb, uint32_t rw, uint32_t qw, uint32_t T, int& P, int& B,
                                                 int& at, bool& stop) {
     uint32_t lo, hi;
     sa_merge8(rw, qw, lo, hi);
     int mn = INT_MAX;
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
-        const int S0 = S + sa_tbl(tblb, lo, hi, REV ? 7 - k : k);
-        S = S0 + sa_tbl(tblb, lo, hi, REV ? 6 - k : k + 1);
-        B = __vimax3_s32(B, S0, S);
-        mn = __vimin3_s32(mn, S0, S);
+        const int P0 = P + sa_tbl(tblb, lo, hi, REV ? 7 - k : k);
+        P = P0 + sa_tbl(tblb, lo, hi, REV ? 6 - k : k + 1);
+        B = __vimax3_s32(B, P0, P);
+        mn = __vimin3_s32(mn, P0, P);
     }
     if (!stop) at = B;
-    stop = stop || B - mn > xdrop;
+    stop = stop || (uint32_t)(B - mn) > T;
+}
+
+// Best score, best - score and best's offset of a direction after its sweep.
+__device__ __forceinline__ uint32_t sa_swept_word(int P, int at) {
+    const int best = at >> SA_SWEEP_SH;
+    return (uint32_t)best | ((uint32_t)(best - (P >> SA_SWEEP_SH)) << 16);
+}
+
+__device__ __forceinline__ uint32_t sa_swept_pos(int at) {
+    const uint32_t low = at & ((1 << SA_SWEEP_SH) - 1);
+    return low == SA_SWEEP_LEFT ? 0u : SA_SWEEP_LEFT - 1 - low;
 }
 
 #define SA_SWEEP_BUF 128  // unfinished hits a warp gathers
@@ -420,8 +444,8 @@ template <bool TRANS>
 __global__ void __launch_bounds__(256, 4)
 sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P, uint64_t h_begin, uint64_t h_end) {
     __shared__ int tbl[64];
-    __shared__ uint4 s_buf[8][SA_SWEEP_BUF];
-    if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
+    __shared__ uint4 s_buf[8][SA_SWEEP_BUF], s_swept[8][SA_SWEEP_BUF];
+    if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SA_SWEEP_SH) - 1;
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
     SaCounters* const ctr = a.ctr;
@@ -431,7 +455,9 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
     const int lane = threadIdx.x & 31;
     const uint32_t lt = sa_lanemask_lt();
     uint4* const buf = s_buf[threadIdx.x >> 5];
+    uint4* const swept = s_swept[threadIdx.x >> 5];
     uint32_t nbuf = 0, tiles = 0, ext = 0;
+    const uint32_t T = (uint32_t)a.xdrop * (2 * SA_SWEEP_LEFT) + SA_SWEEP_LEFT;
     // chain test of the buffered hits, 32 at a time; those left, moved to the
     // buffer's front, go to the list
     auto write_out = [&]() {
@@ -441,10 +467,11 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
             kept = 0;
             for (uint32_t i0 = 0; i0 < nbuf; i0 += 32) {
                 const bool on = i0 + lane < nbuf;
-                uint4 v = make_uint4(0, 0, 0, 0);
+                uint4 v = make_uint4(0, 0, 0, 0), x = v;
                 uint32_t f = 1;
                 if (on) {
                     v = buf[i0 + lane];
+                    x = swept[i0 + lane];
                     const bool may_drop = v.w & SA_CHAIN_DROP;
                     v.w &= ~SA_CHAIN_DROP;
                     f = sa_chain_test<TRANS>(a, P.kmer_size, a.units[v.w], v.x, v.y, may_drop);
@@ -453,6 +480,7 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                 if (f != 1) {
                     v.w |= f;
                     buf[kept + __popc(m & lt)] = v;
+                    swept[kept + __popc(m & lt)] = x;
                 }
                 kept += __popc(m);
                 __syncwarp();
@@ -463,8 +491,8 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)kept);
         at = __shfl_sync(SA_FULL, at, 0);
-        for (uint32_t i = lane; i < kept; i += 32)
-            if (at + i < a.list_cap) a.list[at + i] = buf[i];
+        for (uint32_t i = lane; i < 2 * kept; i += 32)
+            if (at + (i >> 1) < a.list_cap) a.list[2 * at + i] = (i & 1) ? swept[i >> 1] : buf[i >> 1];
         __syncwarp();
     };
     const uint64_t first = h_begin / 32, rounds = (H + 31) / 32 - first;  // h_begin is a multiple of 32
@@ -485,7 +513,7 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
             const uint64_t ahead = c + 1 + lane < nnz ? a.cs.E[c + 1 + lane] - t : ~0ull;
             const uint32_t starts = __reduce_or_sync(SA_FULL, ahead < 32 ? 1u << (uint32_t)ahead : 0u);
             bool left = false;
-            uint4 rec = make_uint4(0, 0, 0, 0);
+            uint4 rec = make_uint4(0, 0, 0, 0), x = rec;
             if (h < H) {
                 const uint64_t k = c + __popc(starts & ((2u << lane) - 1u));
                 const uint32_t rl = __ldg(a.pos_table + a.cs.lo[k] + (uint32_t)(h - a.cs.E[k])) + a.seed_size;  // find_hits :192
@@ -527,31 +555,40 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                         for (int i = 0; i < 13; ++i) rw[i] = rw[i + 2];
                     }
                     const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
-                    int S = 0, B = 0, R = 0, L = 0;
+                    int p = SA_SWEEP_LEFT, B = SA_SWEEP_LEFT, at = 0;
                     bool stop_r = false, stop_l = false;
 #pragma unroll
                     for (int i = 8; i < 12; ++i)
                         sa_sweep_window<false>(tblb, __funnelshift_r(rw[i], rw[i + 1], sr),
-                                               __funnelshift_r(qw[i], qw[i + 1], sq), a.xdrop, S, B, R, stop_r);
-                    S = B = 0;
+                                               __funnelshift_r(qw[i], qw[i + 1], sq), T, p, B, at, stop_r);
+                    x.x = sa_swept_word(p, at);
+                    x.z = sa_swept_pos(at);
+                    const int best_r = at >> SA_SWEEP_SH;
+                    p = B = SA_SWEEP_LEFT;
                     uint32_t tl = 0;
 #pragma unroll
                     for (int i = 7; i >= 0; --i) {
                         sa_sweep_window<true>(tblb, __funnelshift_r(rw[i], rw[i + 1], sr),
-                                              __funnelshift_r(qw[i], qw[i + 1], sq), a.xdrop, S, B, L, stop_l);
+                                              __funnelshift_r(qw[i], qw[i + 1], sq), T, p, B, at, stop_l);
                         if (i == 4) tl = stop_l ? 2 : 3;  // tiles of both scans, if they stop
                     }
+                    x.y = sa_swept_word(p, at);
                     // a window that reaches past an end scans it to the end: the lane kernel does that
                     const bool inside = min(rl, ql) >= SA_SWEEP_LEFT && (uint64_t)rl + SA_SWEEP_RIGHT <= a.ref_len &&
                                         (uint64_t)ql + SA_SWEEP_RIGHT <= U.q_len;
-                    left = !inside || !stop_r || !stop_l || (int)(float)(R + L) >= a.hspthresh;
+                    left = !inside || !stop_r || !stop_l || (int)(float)(best_r + (at >> SA_SWEEP_SH)) >= a.hspthresh;
+                    x.z |= (sa_swept_pos(at) << 8) | (inside ? SA_SWEPT_SEEN : 0u) | (stop_r ? SA_SWEPT_STOP_R : 0u) |
+                           (stop_l ? SA_SWEPT_STOP_L : 0u) | (tl == 3 ? SA_SWEPT_TILE_2 : 0u);
                     if (!left) tiles += tl;
                     if (!(stop_r && !stop_l) && sa_sweep_margin(a, U, rl, ql)) rec.w |= SA_CHAIN_DROP;
                 }
             }
             if (!chains) rec.w &= ~SA_CHAIN_DROP;
             const uint32_t m = __ballot_sync(SA_FULL, left);
-            if (left) buf[nbuf + __popc(m & lt)] = rec;
+            if (left) {
+                buf[nbuf + __popc(m & lt)] = rec;
+                swept[nbuf + __popc(m & lt)] = x;
+            }
             nbuf += __popc(m);
             if (nbuf > SA_SWEEP_BUF - 32) write_out();
             c += __popc(starts) + (__any_sync(SA_FULL, ahead == 32) ? 1 : 0);
@@ -673,9 +710,16 @@ struct SaLaneSmem {
     uint4 em[8][64];       // {ref_start, query_start (before the rm flip), len, scope}
     uint2 ex[8][64];       // {total, unit}
     uint32_t stop[2][256];
+    uint32_t left[2][256]; // list hits: what the sweep left of the left direction
 };
 
-static size_t sa_lane_smem(uint32_t tile) { return sizeof(SaLaneSmem) + 8 * (size_t)tile * (sizeof(uint4) + sizeof(uint32_t)); }
+// A tile of the list holds half as many hits, of two 16-byte words each.
+__host__ __device__ __forceinline__ uint32_t sa_list_tile(uint32_t tile) { return tile / 2 < 32 ? 32 : tile / 2; }
+
+static size_t sa_lane_smem(uint32_t tile, bool list) {
+    return sizeof(SaLaneSmem) + 8 * (size_t)(list ? sa_list_tile(tile) * 2 * sizeof(uint4)
+                                                  : tile * (sizeof(uint4) + sizeof(uint32_t)));
+}
 
 // Keep test of `n` (<= 32) ring candidates from slot `head` on, one per lane:
 // entropy factor from the per-base match counts over the HSP when the total
@@ -739,7 +783,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     // test and insertion.
     extern __shared__ __align__(16) unsigned char sa_smem[];
     SaLaneSmem& L = *reinterpret_cast<SaLaneSmem*>(sa_smem);
-    const uint32_t TILE = a.tile_hits;
+    const uint32_t TILE = LIST ? sa_list_tile(a.tile_hits) : a.tile_hits;
     // entry (q << 3) | r: target code r vs query code q.  Codes 0..3 use
     // entries 0..27 only, one per bank: lookups of A/C/G/T pairs never conflict.
     int* const tbl = L.tbl;
@@ -752,7 +796,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     if (a.ctr->error || (LIST && a.ctr->list_count > a.list_cap)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t lt = sa_lanemask_lt();
-    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + sizeof(SaLaneSmem)) + wid * TILE;
+    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + sizeof(SaLaneSmem)) + wid * (LIST ? 2 * TILE : TILE);
     uint32_t* const s_E = reinterpret_cast<uint32_t*>(sa_smem + sizeof(SaLaneSmem) + 128 * (size_t)TILE) + wid * TILE;
     uint4* const s_em = L.em[wid];
     uint2* const s_ex = L.ex[wid];
@@ -783,14 +827,15 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     // Start of a direction of the current hit (dir 0: right of the hit; 1:
     // left, read rightwards in the reversed copies): offsets, bases
     // available, word shifts and the first NW + 1 words of both sequences.
-    auto begin_dir = [&](const uint32_t* __restrict__ qp, uint32_t qlen) {
+    // LIST: from where the sweep left off (w: its word, first: offset of best).
+    auto begin_dir = [&](const uint32_t* __restrict__ qp, uint32_t qlen, uint32_t from, uint32_t w, uint32_t first) {
         const uint32_t ref_len = a.ref_len;
         const uint32_t sr = dir ? ref_len - rl : rl, sq = dir ? qlen - ql : ql;
         avail = min(ref_len - sr, qlen - sq);
         sh_r = (sr & 7u) * 4u;
         sh_q = (sq & 7u) * 4u;
-        pr = (dir ? ref + sa_rev_words(ref_len) : ref) + (sr >> 3);
-        pq = (dir ? qp + sa_rev_words(qlen) : qp) + (sq >> 3);
+        pr = (dir ? ref + sa_rev_words(ref_len) : ref) + (sr >> 3) + (from >> 3);
+        pq = (dir ? qp + sa_rev_words(qlen) : qp) + (sq >> 3) + (from >> 3);
 #pragma unroll
         for (int j = 0; j <= NW; ++j) {
             w_r[j] = __ldg(pr + j);
@@ -798,16 +843,25 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         }
         pr += NW + 1;
         pq += NW + 1;
-        o = 0;
-        S = 0;
-        best = 0;
-        bpos = 0;
+        o = from;
+        best = (int)(w & 0xffffu);
+        S = best - (int)(w >> 16);
+        bpos = (int)first;
+    };
+    // The left direction of the current hit, as begin_dir takes it.
+    auto begin_left = [&](const uint32_t* __restrict__ qp, uint32_t qlen) {
+        if (!LIST) return begin_dir(qp, qlen, 0, 0, 0);
+        const uint32_t w = L.left[0][threadIdx.x], rest = L.left[1][threadIdx.x];
+        const bool anew = !(rest & SA_SWEPT_SEEN);
+        begin_dir(qp, qlen, anew ? 0u : SA_SWEEP_LEFT, anew ? 0u : w, anew ? 0u : (rest >> 8) & 0xffu);
     };
 
     while (true) {
         // ---- idle lanes take the next hits of the warp tile, in order ----
         const uint32_t idle = __ballot_sync(SA_FULL, !has);
         bool fresh = false;
+        bool finished = false, to_long = false;
+        uint4 swept = make_uint4(0, 0, 0, 0);
         if (idle && !(exhausted && tile_pos >= tile_n)) {
             if (tile_pos >= tile_n) {
                 // Take the next tile of hits and expand it: the hits of the
@@ -824,7 +878,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 } else if (LIST) {
                     tile_n = (uint32_t)min((unsigned long long)TILE, H - t0);
                     tile_pos = 0;
-                    for (uint32_t i = lane; i < tile_n; i += 32) s_hits[i] = __ldcs(a.list + t0 + i);
+                    for (uint32_t i = lane; i < 2 * tile_n; i += 32) s_hits[i] = __ldcs(a.list + 2 * t0 + i);
                     __syncwarp();
                 } else {
                     uint32_t n = (uint32_t)min((unsigned long long)TILE, H - t0);
@@ -883,7 +937,8 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 const uint32_t m = min((uint32_t)__popc(idle), tile_n - tile_pos);
                 const uint32_t rank = __popc(idle & lt);
                 if (!has && rank < m) {
-                    const uint4 r = s_hits[tile_pos + rank];
+                    const uint4 r = s_hits[(tile_pos + rank) * (LIST ? 2 : 1)];
+                    if (LIST) swept = s_hits[2 * (tile_pos + rank) + 1];
                     rl = r.x;
                     ql = r.y;
                     scope = r.z;
@@ -910,11 +965,32 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                     dir = 0;
                     tiles = 0;
                     if (!LIST) ++ext_acc;  // else counted by the sweep
+                    if (LIST) {
+                        if (!(swept.z & SA_SWEPT_SEEN)) swept.x = swept.z = 0;
+                        L.left[0][threadIdx.x] = swept.y;
+                        L.left[1][threadIdx.x] = swept.z;
+                        if (swept.z) {
+                            if (swept.z & SA_SWEPT_STOP_L) tiles = (swept.z & SA_SWEPT_TILE_2) ? 2 : 1;
+                            L.stop[0][threadIdx.x] = L.stop[1][threadIdx.x] = 0;  // stops the sweep saw: from the scan's start
+                            if (swept.z & SA_SWEPT_STOP_R) {
+                                ++tiles;
+                                Rbest = (int)(swept.x & 0xffffu);
+                                Rpos = Rbest > 0 ? (int)(swept.z & 0xffu) : -1;
+                                dir = 1;
+                                if (swept.z & SA_SWEPT_STOP_L) {  // a candidate as it is
+                                    setup = false;
+                                    finished = true;
+                                }
+                            }
+                        }
+                    }
                 }
             }
             if (setup) {
                 setup = false;
-                begin_dir(U.q_packed, U.q_len);
+                if (dir) begin_left(U.q_packed, U.q_len);
+                else begin_dir(U.q_packed, U.q_len, LIST && swept.z ? SA_SWEEP_RIGHT : 0u, LIST ? swept.x : 0u,
+                               LIST ? swept.z & 0xffu : 0u);
             }
         }
         const bool done = !__any_sync(SA_FULL, has) && exhausted && tile_pos >= tile_n;
@@ -922,8 +998,18 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         // ---- up to `substeps` STEP-base steps per busy lane: the lanes still
         // scanning go on while any lane of the warp does; a lane stops for
         // this iteration when its direction ends or it goes to the long queue ----
-        bool finished = false, to_long = false;
         int Lpos = 0, total = 0;
+        auto finish_hit = [&]() {
+            if (LIST && (L.left[1][threadIdx.x] & SA_SWEPT_STOP_L)) {  // the sweep saw the left scan stop
+                best = (int)(L.left[0][threadIdx.x] & 0xffffu);
+                bpos = (int)((L.left[1][threadIdx.x] >> 8) & 0xffu);
+            }
+            Lpos = best > 0 ? bpos + 1 : 0;  // left offsets are 1-based
+            total = Rbest + best;
+            tiles_acc += tiles;
+            has = false;
+        };
+        if (LIST && finished) finish_hit();
         bool scanning = has;
 #pragma unroll 1
         for (uint32_t sub = 0; sub < a.substeps; ++sub) {
@@ -1003,7 +1089,8 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                         Rbest = best;
                         Rpos = best > 0 ? bpos : -1;  // -1 when no positive score
                         dir = 1;
-                        setup = true;
+                        if (LIST && (L.left[1][threadIdx.x] & SA_SWEPT_STOP_L)) finished = true;
+                        else setup = true;
                     } else {
                         finished = true;
                     }
@@ -1015,12 +1102,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                         scanning = false;
                     }
                 }
-                if (finished) {
-                    Lpos = best > 0 ? bpos + 1 : 0;  // left offsets are 1-based
-                    total = Rbest + best;
-                    tiles_acc += tiles;
-                    has = false;
-                }
+                if (finished) finish_hit();
             }
             // switch_now: a lane whose right side ended in this step starts
             // its left side at once and scans in the iteration's remaining
@@ -1029,7 +1111,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 if (setup) {
                     setup = false;
                     const SaUnit U = a.units[unit_id & ~SA_CHAIN_NEXT];
-                    begin_dir(U.q_packed, U.q_len);
+                    begin_left(U.q_packed, U.q_len);
                     scanning = true;
                 }
             }
@@ -1380,10 +1462,19 @@ static bool sa_lane_fast_form(const SaParams& p, int step) {
     return x >= 0 && 7 * mx <= x && x * scale - low * step < (1ll << 31) && mx * scale * step < (1ll << 31);
 }
 
+// The sweep and the lane kernel after it use the fast form, and what passes
+// between them fits its 16-bit fields.
+static bool sa_sweep_params(const SaParams& p, const SaTuning& t) {
+    int mx = 0;
+    for (int i = 0; i < 64; ++i) mx = std::max(mx, p.sub_mat[i]);
+    return sa_lane_fast_form(p, t.step_bases) && sa_lane_fast_form(p, SA_SWEEP_LEFT) && p.xdrop <= 0xffff &&
+           mx <= 0xffff / (int)SA_SWEEP_LEFT;
+}
+
 // Scores for which sa_chain_joined's bounds hold: matches of A, C, G and T
-// score above 0, and the fast form (whose stop words chains need) is in use.
+// score above 0, and the sweep is in use.
 bool sa_chain_params(const SaParams& p, const SaTuning& t) {
-    if (!sa_lane_fast_form(p, t.step_bases) || p.xdrop > 0xffff || p.seed_size > 31) return false;
+    if (!sa_sweep_params(p, t) || p.seed_size > 31) return false;
     for (int b = 0; b < 4; ++b)
         if (p.sub_mat[9 * b] <= 0) return false;
     return true;
@@ -1401,7 +1492,7 @@ static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaParams& p, c
     for (int i = 0; i < 16; ++i) a.shift[i] = (uint32_t)p.shape_pos[i < p.kmer_size ? i : 0];
     // buffers of the dedup that are free until then
     a.list = reinterpret_cast<uint4*>(w.out);
-    a.list_cap = x.sweep && sa_lane_fast_form(p, t.step_bases) ? w.list_cap : 0;
+    a.list_cap = x.sweep && sa_sweep_params(p, t) ? w.list_cap : 0;
     a.lead = reinterpret_cast<uint4*>(w.rec[0]);
     a.lead_right = w.scope[0];
     a.lead_stop_r = w.scope[1];
@@ -1463,7 +1554,7 @@ void sa_prepare_extend_lane(const SaParams& p, const SaTuning& t) {
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
     if (dev < 0 || dev >= 64 || done[dev]) return;
-    const size_t smem = sa_lane_smem(1024);
+    const size_t smem = sa_lane_smem(1024, false);
     SaExtK none{};
     for (int step : {8, 16, 32})
         for (SaLaneForm form : {kLaneFast, kLaneExact, kLaneList}) {
@@ -1480,8 +1571,8 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
     // Register budget follows the CTAs per SM: 4 -> <= 64 registers, 3 -> <= 85, 2 -> <= 128.
     const SaExtK a = sa_ext_args(w, x, p, t);
     const int grid = grid_ctas > 0 ? grid_ctas : num_sms * t.ext_ctas_per_sm;
-    const size_t smem = sa_lane_smem(a.tile_hits);
     const SaLaneForm form = a.list_cap ? kLaneList : sa_lane_fast_form(p, t.step_bases) ? kLaneFast : kLaneExact;
+    const size_t smem = sa_lane_smem(a.tile_hits, form == kLaneList);
     // Segments of hits whose list is sure to fit in practice; one unless the
     // caller knows of more hits (x.hits).  A list that overflows all the same is
     // seen by the host (list_count), which runs the call again without the sweep.

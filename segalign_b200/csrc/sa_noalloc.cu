@@ -116,7 +116,7 @@ void carve(void* base, SaWork& w) {
     take((void**)&w.desc);
     take((void**)&w.units);
     w.seed_cap = kSeeds;
-    w.list_cap = kSurv;
+    w.list_cap = kSurv / 2;
     w.surv_cap = kSurv;
     w.long_cap = SA_NOALLOC_LONG_CAP;
     // the HSP set's list of claimed slots lives in rec[1], free until the sort
