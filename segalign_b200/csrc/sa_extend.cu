@@ -63,12 +63,6 @@ struct SaExtK {
     uint32_t *lead_right, *lead_stop_r, *lead_stop_l;
 };
 
-// Reverse the order of the 8 nibbles of a word.
-__device__ __forceinline__ uint32_t sa_rev_nibbles(uint32_t x) {
-    x = __byte_perm(x, 0, 0x0123);
-    return ((x >> 4) & 0x0f0f0f0fu) | ((x & 0x0f0f0f0fu) << 4);
-}
-
 // Largest compacted seed c in [0, nnz) with E[c] <= h (E strictly increasing,
 // E[0] == 0 <= h).  Warp-cooperative 32-ary search; all lanes get the result.
 __device__ __forceinline__ uint64_t sa_warp_find_seed(const uint64_t* __restrict__ E, uint64_t nnz, uint64_t h) {
@@ -768,6 +762,14 @@ __device__ __forceinline__ void sa_flush_candidates(const SaExtK& a, const uint4
     sa_hash_note_used(a.hset, &a.ctr->hash_used, claimed);
 }
 
+// A list this short leaves most lanes without a hit, and a long scan's lane
+// steps are the call's critical path: hits past SA_FEW_CAP bases go to the warp
+// kernel, whose warps would idle too (lane + warp kernel at caps of 8192 and 128,
+// ms: 11 long hits 0.083 and 0.049, 785 0.152 and 0.082, 12 K 0.455 and 0.209).
+// A call with more keeps the tuning's cap: a warp per hit of a few hundred bases
+// costs more than a lane (120 K long hits: 0.35 and 0.74 ms).
+#define SA_FEW_HITS 32768u
+#define SA_FEW_CAP 128u
 // LIST: the hits come from the sweep's list; else from the compacted seeds.
 template <int MIN_CTAS, int STEP, bool EXACT, bool LIST>
 __global__ void __launch_bounds__(256, MIN_CTAS)
@@ -796,6 +798,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     if (a.ctr->error || (LIST && a.ctr->list_count > a.list_cap)) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t lt = sa_lanemask_lt();
+    const uint32_t lane_cap = LIST && a.ctr->list_count <= SA_FEW_HITS ? min(a.lane_cap, SA_FEW_CAP) : a.lane_cap;
     uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + sizeof(SaLaneSmem)) + wid * (LIST ? 2 * TILE : TILE);
     uint32_t* const s_E = reinterpret_cast<uint32_t*>(sa_smem + sizeof(SaLaneSmem) + 128 * (size_t)TILE) + wid * TILE;
     uint4* const s_em = L.em[wid];
@@ -1097,7 +1100,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                     scanning = false;
                 } else {
                     o += STEP;
-                    if (o >= a.lane_cap && !nocap) {
+                    if (o >= lane_cap && !nocap) {
                         to_long = true;
                         scanning = false;
                     }
@@ -1250,11 +1253,14 @@ __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
 }
 
 // ---------------------------------------------------------------------------
-// Phase B: one warp per long hit, 256 bases per step.
+// Phase B: one warp per long hit, 256 bases per step, 8 per lane.
+//
+// Bound by the latency of a step: its loads are issued a step ahead, and the
+// warp's part of it is one scan of sums and one of maxima (10 shuffles).
 // ---------------------------------------------------------------------------
 struct SaDirResult {
     int best;
-    int pos;
+    int pos;        // offset of the first base reaching best (-1: best is 0)
     uint32_t stop;  // offset at which the scan stops
 };
 
@@ -1268,141 +1274,117 @@ __device__ __forceinline__ int sa_warp_incl_max(int v) {
     return v;
 }
 
-// (value, index) arg-max over the warp: larger value wins, ties go to the smaller index.
-__device__ __forceinline__ void sa_warp_argmax(int& v, uint32_t& idx) {
-    long long key = ((long long)v << 32) | (long long)(uint32_t)(~idx);
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        long long o = __shfl_xor_sync(SA_FULL, key, s);
-        key = o > key ? o : key;
-    }
-    v = (int)(key >> 32);
-    idx = ~(uint32_t)(key & 0xffffffffll);
-}
-
-__device__ SaDirResult sa_warp_xdrop(const int* sub, const uint32_t* __restrict__ ref, const uint32_t* __restrict__ qp,
-                                     uint32_t rl, uint32_t ql, uint32_t avail, int dir, int xdrop) {
+// Rightward scan from base sr of R and sq of Q; `avail` bases until either
+// ends.  A base past the end scores -(xdrop + 1), which stops the scan there.
+// tblb: plain scores.
+__device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restrict__ R, const uint32_t* __restrict__ Q,
+                                     uint32_t sr, uint32_t sq, uint32_t avail, int xdrop) {
     const int lane = threadIdx.x & 31;
-    int S_prev = 0, best = 0, bpos = dir ? 0 : -1;
-    uint32_t o = 0;
-    SaDirResult res;
+    const uint32_t* __restrict__ pr = R + (sr >> 3) + lane;
+    const uint32_t* __restrict__ pq = Q + (sq >> 3) + lane;
+    const uint32_t shr = (sr & 7u) * 4u, shq = (sq & 7u) * 4u;
+    int S_prev = 0, best = 0, bpos = -1;
+    uint32_t o = 0, r0 = 0, r1 = 0, q0 = 0, q1 = 0;
+    auto fetch = [&](uint32_t at) {  // the lane's words of the step at offset `at`
+        if (at + 8u * lane < avail) {
+            r0 = __ldg(pr);
+            r1 = __ldg(pr + 1);
+            q0 = __ldg(pq);
+            q1 = __ldg(pq + 1);
+        }
+        pr += 32;
+        pq += 32;
+    };
+    fetch(0);
     while (true) {
         const uint32_t loff = o + 8u * lane;
-        const int cnt_in = (avail > loff) ? (int)min(avail - loff, 8u) : 0;
-        uint32_t rw = 0, qw = 0;
-        if (cnt_in > 0) {
-            if (dir == 0) {
-                rw = sa_load8(ref, (int64_t)rl + loff);
-                qw = sa_load8(qp, (int64_t)ql + loff);
-            } else {
-                rw = sa_rev_nibbles(sa_load8(ref, (int64_t)rl - loff - 8));
-                qw = sa_rev_nibbles(sa_load8(qp, (int64_t)ql - loff - 8));
-            }
-        }
-        int ps[8];
-        int p = 0, lmax = INT_MIN, lmax_k = 0, lmin = INT_MAX;
+        const uint32_t in = avail > loff ? min(avail - loff, 8u) : 0u;
+        uint32_t lo, hi;
+        sa_merge8(__funnelshift_r(r0, r1, shr), __funnelshift_r(q0, q1, shq), lo, hi);
+        fetch(o + 256);
+        // prefix sums; (largest << 3) | (7 - its first base) in lmax
+        int ps[8], p = 0, lmax = INT_MIN, lmin = INT_MAX;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            int s = (kk < cnt_in) ? sub[(((rw >> (4 * kk)) & 7u) << 3) | ((qw >> (4 * kk)) & 7u)] : 0;
-            p += s;
-            ps[kk] = p;
-            if (kk < cnt_in) {
-                if (p > lmax) {
-                    lmax = p;
-                    lmax_k = kk;
-                }
-                lmin = min(lmin, p);
-            }
+        for (int k = 0; k < 8; ++k) {
+            p += (uint32_t)k < in ? sa_tbl(tblb, lo, hi, k) : -(xdrop + 1);
+            ps[k] = p;
+            lmax = max(lmax, p * 8 + 7 - k);
+            lmin = min(lmin, p);
         }
         const int incl = sa_warp_incl_sum(p);
-        const int pre = incl - p;
-        const int step_total = __shfl_sync(SA_FULL, incl, 31);
-        const int base = S_prev + pre;
-        const int amax = cnt_in > 0 ? base + lmax : INT_MIN;
+        const int base = S_prev + incl - p;
+        const int amax = base + (lmax >> 3);
         const int im = sa_warp_incl_max(amax);
-        int excl = __shfl_up_sync(SA_FULL, im, 1);
-        if (lane == 0) excl = INT_MIN;
-        const int Mbefore = max(best, excl);
-        int stop_k = -1, bmax = INT_MIN, bmax_k = 0;
-        const bool possible = (cnt_in < 8) || (max(Mbefore, amax) - (base + lmin) > xdrop);
-        if (possible) {
-            int M = Mbefore;
+        int before = __shfl_up_sync(SA_FULL, im, 1);
+        before = lane ? max(best, before) : best;
+        const bool possible = max(before, amax) - (base + lmin) > xdrop;
+        if (__any_sync(SA_FULL, possible)) {
+            // exact test of the lanes where a stop is possible
+            int stop_k = -1, bmax = INT_MIN, bmax_k = 0;
+            if (possible) {
+                int M = before;
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                if (stop_k < 0) {
-                    if (kk >= cnt_in) {
-                        stop_k = kk;
-                    } else {
-                        const int Sv = base + ps[kk];
+                for (int k = 0; k < 8; ++k)
+                    if (stop_k < 0) {
+                        const int Sv = base + ps[k];
                         M = max(M, Sv);
-                        if (M - Sv > xdrop) stop_k = kk;
-                        else if (Sv > bmax) {
+                        if (M - Sv > xdrop) {
+                            stop_k = k;
+                        } else if (Sv > bmax) {
                             bmax = Sv;
-                            bmax_k = kk;
+                            bmax_k = k;
                         }
                     }
+            }
+            const uint32_t sm = __ballot_sync(SA_FULL, stop_k >= 0);
+            if (sm) {
+                const int f = __ffs(sm) - 1;
+                // best of the lanes before the stop, and of the stopping one up to it
+                const int cv = lane < f ? amax : lane == f ? bmax : INT_MIN;
+                const int top = __reduce_max_sync(SA_FULL, cv);
+                if (top > best) {
+                    const int src = __ffs(__ballot_sync(SA_FULL, cv == top)) - 1;
+                    bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)(lane == f ? bmax_k : 7 - (lmax & 7)), src);
+                    best = top;
                 }
+                return {best, bpos, __shfl_sync(SA_FULL, loff + (uint32_t)stop_k, f)};
             }
         }
-        const uint32_t sm = __ballot_sync(SA_FULL, stop_k >= 0);
-        int cv;
-        uint32_t ci;
-        if (sm) {
-            const int f = __ffs(sm) - 1;
-            if (lane < f) {
-                cv = amax;
-                ci = loff + lmax_k;
-            } else if (lane == f) {
-                cv = bmax;
-                ci = loff + bmax_k;
-            } else {
-                cv = INT_MIN;
-                ci = 0xffffffffu;
-            }
-            sa_warp_argmax(cv, ci);
-            if (cv > best) {
-                best = cv;
-                bpos = (int)ci + dir;
-            }
-            const uint32_t stop_idx = __shfl_sync(SA_FULL, loff + (uint32_t)stop_k, f);
-            res.stop = stop_idx;
-            break;
+        const int top = __shfl_sync(SA_FULL, im, 31);
+        if (top > best) {
+            const int src = __ffs(__ballot_sync(SA_FULL, amax == top)) - 1;
+            bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)(7 - (lmax & 7)), src);
+            best = top;
         }
-        cv = amax;
-        ci = loff + lmax_k;
-        sa_warp_argmax(cv, ci);
-        if (cv > best) {
-            best = cv;
-            bpos = (int)ci + dir;
-        }
-        S_prev += step_total;
+        S_prev += __shfl_sync(SA_FULL, incl, 31);
         o += 256;
     }
-    res.best = best;
-    res.pos = bpos;
-    return res;
 }
 
 __global__ void __launch_bounds__(256)
 sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
-    __shared__ int sub[64];
-    if (threadIdx.x < 64) sub[threadIdx.x] = P.sub_mat[threadIdx.x];
+    __shared__ int tbl[64];
+    if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
     __syncthreads();
+    const char* tblb = reinterpret_cast<const char*>(tbl);
     if (a.ctr->error) return;
     const int lane = threadIdx.x & 31;
     const unsigned long long nlong = min(a.ctr->long_count, (unsigned long long)a.long_cap);
     unsigned long long tiles_acc = 0;
+    const uint32_t* const ref_rev = a.ref + sa_rev_words(a.ref_len);
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);
     while (true) {
-        unsigned long long idx = 0;
-        if (lane == 0) idx = atomicAdd(&a.ctr->long_cursor, 1ull);
-        idx = __shfl_sync(SA_FULL, idx, 0);
+        const unsigned long long idx = __shfl_sync(SA_FULL, next, 0);
         if (idx >= nlong) break;
+        if (lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);  // read while this hit is scanned
         const SaLongHit L = a.long_q[idx];
         const SaUnit U = a.units[L.unit & ~SA_CHAIN_NEXT];
         const uint32_t rl = L.ref_loc, ql = L.query_loc;
-        const uint32_t avail_r = (rl < a.ref_len && ql < U.q_len) ? min(a.ref_len - rl, U.q_len - ql) : 0u;
-        const SaDirResult R = sa_warp_xdrop(sub, a.ref, U.q_packed, rl, ql, avail_r, 0, a.xdrop);
-        const SaDirResult Lr = sa_warp_xdrop(sub, a.ref, U.q_packed, rl, ql, min(rl, ql), 1, a.xdrop);
+        const SaDirResult R = sa_warp_xdrop(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql), a.xdrop);
+        SaDirResult Lr = sa_warp_xdrop(tblb, ref_rev, U.q_packed + sa_rev_words(U.q_len), a.ref_len - rl, U.q_len - ql,
+                                       min(rl, ql), a.xdrop);
+        ++Lr.pos;  // left offsets are 1-based, 0 when best is 0
         tiles_acc += (R.stop >> 5) + (Lr.stop >> 5) + 2;
         const int total = R.best + Lr.best;
         const int ext = R.pos + Lr.pos;
