@@ -24,21 +24,23 @@
 // the most significant key throughout.
 //
 // A record becomes five words whose lexicographic order is the wanted one (and
-// which give the record back), and the sort is a merge sort of them: tiles of
-// SA_SORT_TILE records sorted in shared memory, straight out of the set, then
-// passes that merge pairs of runs.  The host has read the record count by then,
-// so a call launches what its size needs: one kernel up to one tile.  An LSD
-// radix sort of every key byte, planned on the device, took 46 launches for any
-// size and a one-CTA histogram scan per pass.  Measured (one B200, records ->
-// order, ms): 37 records 0.21 -> 0.025, 26 K 0.28 -> 0.10, 458 K 1.18 -> 0.25, 4.7 M
-// 2.90 -> 2.03; a repeat-masker call's 3.7 K, three sorts before and two now, 0.67 ->
-// 0.14.
+// which give the record back).  The sort: tiles of SA_SORT_TILE records, straight
+// out of the set; then, up to SA_RANK_TILES tiles, one kernel in which a warp per
+// record finds its rank in every tile at once; for more, passes that merge
+// pairs of runs.  The host has read the record count by then, so a call launches
+// what its size needs: one kernel up to one tile.  An LSD radix sort of every
+// key byte, planned on the device, took 46 launches for any size and a one-CTA
+// histogram scan per pass.  Measured (one B200, dedup phase, ms, radix sort and
+// this): 36 records 0.21 and 0.026, 26 K 0.28 and 0.064, 458 K 1.18 and 0.22, 4.7 M 2.90
+// and 2.23; a repeat-masker call's 3.7 K, three sorts and two, 0.67 and 0.083.
 #include <algorithm>
 
 #include "sa_launch.h"
 #include "sa_radix.cuh"
 
-#define SA_SORT_TILE 2048
+#define SA_SORT_TILE 1024
+#define SA_RANK_TILES 32  // a lane per tile
+#define SA_MERGE_OUT 2048
 
 enum SaOrder { kOrderPlain, kOrderDiag, kOrderFinal };
 
@@ -103,46 +105,63 @@ __device__ __forceinline__ void sa_store_key(SaRec* rec, uint32_t* scope, uint64
     }
 }
 
-struct SaTileSmem {
-    ulonglong2 ab[SA_SORT_TILE];
-    uint32_t c[SA_SORT_TILE];
-    unsigned long long ws[33];
+// Key i of a merge CTA lies at i + i / 8: a thread's 8 keys start 9 places after
+// its neighbour's, so that the threads' reads spread over the banks.
+#define SA_MERGE_PER 8
+#define SA_MERGE_THREADS (SA_MERGE_OUT / SA_MERGE_PER)
+struct SaMergeSmem {
+    ulonglong2 ab[SA_MERGE_OUT + SA_MERGE_THREADS];
+    uint32_t c[SA_MERGE_OUT + SA_MERGE_THREADS];
 };
 
-// Bitonic sort of the tile's first n2 (a power of two, <= SA_SORT_TILE) keys by
-// SA_SORT_TILE / 2 threads, one pair per thread and stage.  A warp's pairs at
-// distance <= 32 lie in its own 64 keys, so those stages need no block barrier.
-__device__ __forceinline__ void sa_tile_sort(SaTileSmem& s, uint32_t n2) {
-    const uint32_t t = threadIdx.x;
-    __syncthreads();
-    for (uint32_t k = 2; k <= n2; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (j >= 32) __syncthreads();
-            else __syncwarp();
-            if (t < n2 / 2) {
-                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), p = i + j;
-                const ulonglong2 x = s.ab[i], y = s.ab[p];
-                const uint32_t xc = s.c[i], yc = s.c[p];
-                const bool less = sa_key_less({y.x, y.y, yc}, {x.x, x.y, xc});
-                if (less == ((i & k) == 0)) {
-                    s.ab[i] = y;
-                    s.ab[p] = x;
-                    s.c[i] = yc;
-                    s.c[p] = xc;
-                }
-            }
-        }
-    __syncthreads();
-}
-
-__device__ __forceinline__ uint32_t sa_pow2_at_least(uint32_t n) { return n <= 64 ? 64u : 1u << (32 - __clz(n - 1)); }
-
-__device__ __forceinline__ void sa_tile_put(SaTileSmem& s, uint32_t i, const SaKey& k) {
+__device__ __forceinline__ void sa_merge_put(SaMergeSmem& s, uint32_t i, const SaKey& k) {
+    i += i / SA_MERGE_PER;
     s.ab[i] = make_ulonglong2(k.a, k.b);
     s.c[i] = k.c;
 }
 
-__device__ __forceinline__ SaKey sa_tile_get(const SaTileSmem& s, uint32_t i) { return {s.ab[i].x, s.ab[i].y, s.c[i]}; }
+__device__ __forceinline__ SaKey sa_merge_get(const SaMergeSmem& s, uint32_t i) {
+    i += i / SA_MERGE_PER;
+    const ulonglong2 v = s.ab[i];
+    return {v.x, v.y, s.c[i]};
+}
+
+// One tile: SA_SORT_TILE threads, a key each.
+struct SaTileSmem {
+    ulonglong2 ab[2][SA_SORT_TILE];
+    uint32_t c[2][SA_SORT_TILE];
+};
+
+__device__ __forceinline__ uint32_t sa_pow2_at_least(uint32_t n) { return n <= 32 ? 32u : 1u << (32 - __clz(n - 1)); }
+
+// Bitonic sort of the keys of threads 0 .. n2 - 1 (a power of two, at least 32;
+// keys that are no records hold all ones).  Partners up to 16 lanes away are
+// read by shuffles, the others through shared memory, two buffers in turn:
+// 15 of 55 stages have a barrier.  (With the keys in shared memory throughout,
+// or merged there, a tile took 35-40 us.)
+__device__ __forceinline__ SaKey sa_tile_sort(SaTileSmem& s, SaKey mine, uint32_t n2) {
+    const uint32_t t = threadIdx.x;
+    uint32_t buf = 0;
+    for (uint32_t k = 2; k <= n2; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            SaKey other;
+            if (j >= 32) {
+                s.ab[buf][t] = make_ulonglong2(mine.a, mine.b);
+                s.c[buf][t] = mine.c;
+                __syncthreads();
+                const ulonglong2 v = s.ab[buf][t ^ j];
+                other = {v.x, v.y, s.c[buf][t ^ j]};
+                buf ^= 1;
+            } else {
+                other.a = __shfl_xor_sync(0xffffffffu, mine.a, j);
+                other.b = __shfl_xor_sync(0xffffffffu, mine.b, j);
+                other.c = __shfl_xor_sync(0xffffffffu, mine.c, j);
+            }
+            const bool want_less = ((t & j) == 0) == ((t & k) == 0);
+            if (sa_key_less(other, mine) == want_less) mine = other;
+        }
+    return mine;
+}
 
 // Distinct HSP i of the set, in claim order; its slot is emptied, so that the set
 // is left empty for the next call.
@@ -150,10 +169,10 @@ __device__ __forceinline__ SaRec sa_take_from_set(const SaHashSet& hs, uint64_t 
     const unsigned long long h = hs.used[i];
     const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(hs.keys + 2 * h);
     SaRec r;
+    r.score = hs.score[h];
     r.ref_start = (uint32_t)k.x;
     r.query_start = (uint32_t)(k.y >> 32);
     r.len = (uint32_t)k.y;
-    r.score = hs.score[h];
     scope = (uint32_t)(k.x >> 32);
     *reinterpret_cast<ulonglong2*>(hs.keys + 2 * h) = make_ulonglong2(~0ull, ~0ull);
     return r;
@@ -176,100 +195,114 @@ __device__ __forceinline__ bool sa_diag_keep(const SaRec& r, uint32_t scope, boo
 }
 
 // Sorts one tile of the n records: out of the set (SET) or out of src/src_scope
-// (records), into dst.  last: dst gets records, else keys.  Bound by the
-// latency of the scattered set reads and of the 66 stages; 2048 records of 20
-// bytes leave 4 CTAs per SM their shared memory.
+// (records), into dst.  last: dst gets records, else keys.
 template <int ORDER, bool SET>
-__global__ void __launch_bounds__(SA_SORT_TILE / 2)
+__global__ void __launch_bounds__(SA_SORT_TILE)
 sa_k_tile_sort(SaHashSet hs, const SaRec* src, const uint32_t* src_scope, SaRec* dst, uint32_t* dst_scope, uint64_t n,
                const unsigned long long* d_n, bool last) {
     __shared__ SaTileSmem s;
     if (d_n) n = *d_n;
-    const uint64_t base = (uint64_t)blockIdx.x * SA_SORT_TILE;
+    const uint64_t base = (uint64_t)blockIdx.x * SA_SORT_TILE, i = base + threadIdx.x;
     if (base >= n) return;
-    const uint32_t cnt = (uint32_t)min((uint64_t)SA_SORT_TILE, n - base), n2 = sa_pow2_at_least(cnt);
-    for (uint32_t i = threadIdx.x; i < n2; i += SA_SORT_TILE / 2) {
-        SaKey k{~0ull, ~0ull, ~0u};
-        if (i < cnt) {
-            uint32_t scope;
-            SaRec r;
-            if (SET) {
-                r = sa_take_from_set(hs, base + i, scope);
-            } else {
-                r = src[base + i];
-                scope = src_scope[base + i];
-            }
-            k = sa_key_of<ORDER>(r, scope);
+    SaKey k{~0ull, ~0ull, ~0u};
+    if (i < n) {
+        uint32_t scope;
+        SaRec r;
+        if (SET) {
+            r = sa_take_from_set(hs, i, scope);
+        } else {
+            r = src[i];
+            scope = src_scope[i];
         }
-        sa_tile_put(s, i, k);
+        k = sa_key_of<ORDER>(r, scope);
     }
-    sa_tile_sort(s, n2);
-    for (uint32_t i = threadIdx.x; i < cnt; i += SA_SORT_TILE / 2)
-        sa_store_key<ORDER>(dst, dst_scope, base + i, sa_tile_get(s, i), last);
+    k = sa_tile_sort(s, k, sa_pow2_at_least((uint32_t)min((uint64_t)SA_SORT_TILE, n - base)));
+    if (i < n) sa_store_key<ORDER>(dst, dst_scope, i, k, last);
 }
 
 // A repeat-masker call of at most one tile: diagonal order, unique, final order.
-__global__ void __launch_bounds__(SA_SORT_TILE / 2)
+__global__ void __launch_bounds__(SA_SORT_TILE)
 sa_k_tile_rm(SaHashSet hs, SaRec* dst, uint32_t n, bool exclude, unsigned long long* n_out) {
     __shared__ SaTileSmem s;
-    constexpr int T = SA_SORT_TILE / 2;
-    const uint32_t t = threadIdx.x, n2 = sa_pow2_at_least(n);
-    for (uint32_t i = t; i < n2; i += T) {
-        SaKey k{~0ull, ~0ull, ~0u};
-        if (i < n) {
-            uint32_t scope;
-            const SaRec r = sa_take_from_set(hs, i, scope);
-            k = sa_key_of<kOrderDiag>(r, scope);
-        }
-        sa_tile_put(s, i, k);
+    __shared__ uint32_t ws[SA_SORT_TILE / 32 + 1];
+    const uint32_t t = threadIdx.x;
+    SaKey k{~0ull, ~0ull, ~0u};
+    if (t < n) {
+        uint32_t scope;
+        const SaRec r = sa_take_from_set(hs, t, scope);
+        k = sa_key_of<kOrderDiag>(r, scope);
     }
-    sa_tile_sort(s, n2);
-    // records 2t and 2t + 1 of this thread, and the one before
-    SaRec r[3];
-    uint32_t sc[3];
-    bool keep[2];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const uint32_t i = 2 * t + j;  // record i - 1
-        if (i >= 1 && i <= n) {
-            const SaKey k = sa_tile_get(s, i - 1);
-            r[j] = sa_rec_of<kOrderDiag>(k);
-            sc[j] = (uint32_t)(k.a >> 32);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-        keep[j] = 2 * t + j < n && sa_diag_keep(r[j + 1], sc[j + 1], 2 * t + j == 0, r[j], sc[j], exclude);
-    unsigned long long m;
-    const uint32_t at = (uint32_t)sa_block_excl_sum<unsigned long long, T>((unsigned long long)keep[0] + keep[1], s.ws, &m);
-    const uint32_t m2 = sa_pow2_at_least((uint32_t)m);
-    if (keep[0]) sa_tile_put(s, at, sa_key_of<kOrderFinal>(r[1], sc[1]));
-    if (keep[1]) sa_tile_put(s, at + keep[0], sa_key_of<kOrderFinal>(r[2], sc[2]));
-    for (uint32_t i = (uint32_t)m + t; i < m2; i += T) sa_tile_put(s, i, {~0ull, ~0ull, ~0u});
+    k = sa_tile_sort(s, k, sa_pow2_at_least(n));
     __syncthreads();
-    sa_tile_sort(s, m2);
-    for (uint32_t i = t; i < (uint32_t)m; i += T) dst[i] = sa_rec_of<kOrderFinal>(sa_tile_get(s, i));
+    s.ab[0][t] = make_ulonglong2(k.a, k.b);
+    s.c[0][t] = k.c;
+    __syncthreads();
+    bool keep = false;
+    if (t < n) {
+        const uint32_t scope = (uint32_t)(k.a >> 32);
+        SaKey b = k;
+        if (t) b = {s.ab[0][t - 1].x, s.ab[0][t - 1].y, s.c[0][t - 1]};
+        const SaRec r = sa_rec_of<kOrderDiag>(k);
+        keep = sa_diag_keep(r, scope, t == 0, sa_rec_of<kOrderDiag>(b), (uint32_t)(b.a >> 32), exclude);
+        k = sa_key_of<kOrderFinal>(r, scope);
+    }
+    uint32_t m;
+    const uint32_t at = sa_block_excl_sum<uint32_t, SA_SORT_TILE>(keep, ws, &m);
+    if (keep) {
+        s.ab[1][at] = make_ulonglong2(k.a, k.b);
+        s.c[1][at] = k.c;
+    }
+    __syncthreads();
+    k = {~0ull, ~0ull, ~0u};
+    if (t < m) k = {s.ab[1][t].x, s.ab[1][t].y, s.c[1][t]};
+    __syncthreads();
+    k = sa_tile_sort(s, k, sa_pow2_at_least(m));
+    if (t < m) dst[t] = sa_rec_of<kOrderFinal>(k);
     if (t == 0) *n_out = m;
 }
 
-// One merge pass: runs of `run` sorted keys, pair by pair.  A CTA writes
-// SA_SORT_TILE consecutive outputs: two warps find where its first and last
-// output cut the two runs (merge path, a 32-way search: each probe is a
-// scattered read), the inputs between go to shared memory, and each thread
-// merges 8 outputs.  Bound by memory traffic (40 bytes per record and pass) for
-// large n, by latency for small.
+// All tiles to the output at once (at most SA_RANK_TILES): a warp per record,
+// lane l counts tile l's keys below the record's; the sum is its place.  One
+// kernel in place of five merge passes (13 us each, mostly latency) for 26 K
+// records.
 template <int ORDER>
 __global__ void __launch_bounds__(256)
+sa_k_rank(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope, SaRec* __restrict__ dst,
+          uint32_t* __restrict__ dst_scope, uint64_t n_max, const unsigned long long* d_n, bool last) {
+    const uint32_t n = (uint32_t)(d_n ? *d_n : n_max);
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * 8;
+    const uint32_t base = lane * SA_SORT_TILE, size = base < n ? min((uint32_t)SA_SORT_TILE, n - base) : 0u;
+    for (uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += warps) {
+        const SaKey k = sa_load_key(src, src_scope, i);
+        uint32_t lo = 0, hi = size;
+        if (lane == i / SA_SORT_TILE) lo = hi = i % SA_SORT_TILE;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (sa_key_less(sa_load_key(src, src_scope, base + mid), k)) lo = mid + 1;
+            else hi = mid;
+        }
+        const uint32_t rank = __reduce_add_sync(0xffffffffu, lo);
+        if (lane == 0) sa_store_key<ORDER>(dst, dst_scope, rank, k, last);
+    }
+}
+
+// One merge pass: runs of `run` sorted keys, pair by pair.  A CTA writes
+// SA_MERGE_OUT consecutive outputs: two warps find where its first and last
+// output cut the two runs (merge path, a 32-way search: each probe is a
+// scattered read), the inputs between go to shared memory, and each thread
+// merges 8 outputs.  Moves 40 bytes per record and pass.
+template <int ORDER>
+__global__ void __launch_bounds__(SA_MERGE_THREADS)
 sa_k_merge(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope, SaRec* __restrict__ dst,
            uint32_t* __restrict__ dst_scope, uint64_t n, const unsigned long long* d_n, uint64_t run, bool last) {
-    __shared__ SaTileSmem s;
+    __shared__ SaMergeSmem s;
     __shared__ uint64_t cut[2];
     if (d_n) n = *d_n;
-    const uint64_t o0 = (uint64_t)blockIdx.x * SA_SORT_TILE;
+    const uint64_t o0 = (uint64_t)blockIdx.x * SA_MERGE_OUT;
     if (o0 >= n) return;
-    const uint64_t pair = o0 / (2 * run) * (2 * run);  // runs are multiples of the tile
+    const uint64_t pair = o0 / (2 * run) * (2 * run);  // pairs of runs are multiples of SA_MERGE_OUT
     const uint64_t la = min(run, n - pair), b0 = pair + la, lb = min(run, n - b0);
-    const uint64_t d0 = o0 - pair, d1 = min(d0 + SA_SORT_TILE, la + lb);
+    const uint64_t d0 = o0 - pair, d1 = min(d0 + SA_MERGE_OUT, la + lb);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp < 2) {
         const uint64_t d = warp ? d1 : d0;
@@ -289,34 +322,43 @@ sa_k_merge(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope
     __syncthreads();
     const uint32_t na = (uint32_t)(cut[1] - cut[0]), m = (uint32_t)(d1 - d0), nb = m - na;
     const uint64_t a0 = pair + cut[0], bb = b0 + (d0 - cut[0]);
-    for (uint32_t i = threadIdx.x; i < m; i += 256)
-        sa_tile_put(s, i, sa_load_key(src, src_scope, i < na ? a0 + i : bb + (i - na)));
-    __syncthreads();
-    constexpr uint32_t PER = SA_SORT_TILE / 256;
-    const uint32_t d = min(threadIdx.x * PER, m);
-    uint32_t lo = d > nb ? d - nb : 0, hi = min(d, na);
-    while (lo < hi) {
-        const uint32_t i = (lo + hi) >> 1;
-        if (sa_key_less(sa_tile_get(s, i), sa_tile_get(s, na + d - 1 - i))) lo = i + 1;
-        else hi = i;
-    }
-    uint32_t ia = lo, ib = na + d - lo;
-    SaKey out[PER];
 #pragma unroll
-    for (uint32_t k = 0; k < PER; ++k) {
-        if (d + k < m) {
-            const bool take_a = ib >= m || (ia < na && sa_key_less(sa_tile_get(s, ia), sa_tile_get(s, ib)));
-            out[k] = sa_tile_get(s, take_a ? ia : ib);
-            ia += take_a;
-            ib += !take_a;
+    for (int j = 0; j < SA_MERGE_PER; ++j) {
+        const uint32_t i = j * SA_MERGE_THREADS + threadIdx.x;
+        if (i < m) sa_merge_put(s, i, sa_load_key(src, src_scope, i < na ? a0 + i : bb + (i - na)));
+    }
+    __syncthreads();
+    const uint32_t d = threadIdx.x * SA_MERGE_PER;
+    SaKey out[SA_MERGE_PER];
+    if (d < m) {
+        uint32_t lo = d > nb ? d - nb : 0, hi = min(d, na);
+        while (lo < hi) {
+            const uint32_t i = (lo + hi) >> 1;
+            if (sa_key_less(sa_merge_get(s, i), sa_merge_get(s, na + d - 1 - i))) lo = i + 1;
+            else hi = i;
+        }
+        uint32_t ia = lo, ib = d - lo;
+        SaKey ka{~0ull, ~0ull, ~0u}, kb = ka;
+        if (ia < na) ka = sa_merge_get(s, ia);
+        if (ib < nb) kb = sa_merge_get(s, na + ib);
+#pragma unroll
+        for (int k = 0; k < SA_MERGE_PER; ++k) {
+            const bool take_a = ib >= nb || (ia < na && sa_key_less(ka, kb));
+            out[k] = take_a ? ka : kb;
+            if (take_a) {
+                if (++ia < na) ka = sa_merge_get(s, ia);
+            } else {
+                if (++ib < nb) kb = sa_merge_get(s, na + ib);
+            }
         }
     }
     __syncthreads();
 #pragma unroll
-    for (uint32_t k = 0; k < PER; ++k)
-        if (d + k < m) sa_tile_put(s, d + k, out[k]);
+    for (int k = 0; k < SA_MERGE_PER; ++k)
+        if (d + k < m) sa_merge_put(s, d + k, out[k]);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < m; i += 256) sa_store_key<ORDER>(dst, dst_scope, o0 + i, sa_tile_get(s, i), last);
+    for (uint32_t i = threadIdx.x; i < m; i += SA_MERGE_THREADS)
+        sa_store_key<ORDER>(dst, dst_scope, o0 + i, sa_merge_get(s, i), last);
 }
 
 // unique_copy(hspDiagEqual) over records in diagonal order (keys of
@@ -423,14 +465,22 @@ int sa_check_set(const SaWork& w, const SaCounters& c) {
     return c.hash_overflow || c.hash_used > w.surv_cap || c.hash_used > w.hset.used_cap ? SA_DERR_SURV_OVERFLOW : 0;
 }
 
-// Merge passes over n keys in buffer b; the last one writes records.  Returns
-// the buffer they end in.
+// From sorted tiles of n keys in buffer b to one order, of records (of keys for
+// kOrderDiag).  Returns the buffer they end in.
 template <int ORDER>
-static int sa_merge_passes(SaWork& w, int b, uint64_t n, const unsigned long long* d_n, cudaStream_t st) {
-    const unsigned tiles = (unsigned)((n + SA_SORT_TILE - 1) / SA_SORT_TILE);
+static int sa_merge_tiles(SaWork& w, int b, uint64_t n, const unsigned long long* d_n, cudaStream_t st) {
+    const bool records = ORDER != kOrderDiag;
+    if (n <= SA_SORT_TILE) return b;
+    if (n <= (uint64_t)SA_RANK_TILES * SA_SORT_TILE) {
+        const int g = (int)std::min<uint64_t>((n + 7) / 8, 148 * 8);
+        sa_k_rank<ORDER><<<g, 256, 0, st>>>(w.rec[b], w.scope[b], w.rec[b ^ 1], w.scope[b ^ 1], n, d_n, records);
+        sa_note_launch();
+        return b ^ 1;
+    }
+    const unsigned g = (unsigned)((n + SA_MERGE_OUT - 1) / SA_MERGE_OUT);
     for (uint64_t run = SA_SORT_TILE; run < n; run *= 2, b ^= 1) {
-        sa_k_merge<ORDER><<<tiles, 256, 0, st>>>(w.rec[b], w.scope[b], w.rec[b ^ 1], w.scope[b ^ 1], n, d_n, run,
-                                                 2 * run >= n && ORDER != kOrderDiag);
+        sa_k_merge<ORDER><<<g, SA_MERGE_THREADS, 0, st>>>(w.rec[b], w.scope[b], w.rec[b ^ 1], w.scope[b ^ 1], n, d_n, run,
+                                                          2 * run >= n && records);
         sa_note_launch();
     }
     return b;
@@ -439,10 +489,10 @@ static int sa_merge_passes(SaWork& w, int b, uint64_t n, const unsigned long lon
 int sa_launch_sort(SaWork& w, uint64_t n, cudaStream_t st) {
     if (n == 0) return 0;
     const unsigned tiles = (unsigned)((n + SA_SORT_TILE - 1) / SA_SORT_TILE);
-    sa_k_tile_sort<kOrderPlain, true><<<tiles, SA_SORT_TILE / 2, 0, st>>>(w.hset, nullptr, nullptr, w.rec[0], w.scope[0], n,
+    sa_k_tile_sort<kOrderPlain, true><<<tiles, SA_SORT_TILE, 0, st>>>(w.hset, nullptr, nullptr, w.rec[0], w.scope[0], n,
                                                                     nullptr, tiles == 1);
     sa_note_launch();
-    return sa_merge_passes<kOrderPlain>(w, 0, n, nullptr, st);
+    return sa_merge_tiles<kOrderPlain>(w, 0, n, nullptr, st);
 }
 
 void sa_launch_unit_counts(SaWork& w, int buf, uint64_t n, uint32_t units, cudaStream_t st) {
@@ -453,16 +503,16 @@ void sa_launch_unit_counts(SaWork& w, int buf, uint64_t n, uint32_t units, cudaS
 int sa_launch_sort_rm(SaWork& w, uint64_t n, bool exclude, cudaStream_t st) {
     if (n == 0) return 0;
     if (n <= SA_SORT_TILE) {
-        sa_k_tile_rm<<<1, SA_SORT_TILE / 2, 0, st>>>(w.hset, w.rec[0], (uint32_t)n, exclude, &w.ctr->uniq_count);
+        sa_k_tile_rm<<<1, SA_SORT_TILE, 0, st>>>(w.hset, w.rec[0], (uint32_t)n, exclude, &w.ctr->uniq_count);
         sa_note_launch();
         return 0;
     }
     const unsigned tiles = (unsigned)((n + SA_SORT_TILE - 1) / SA_SORT_TILE);
     const int G = (int)std::min<uint64_t>(tiles, SA_MAX_CTAS);
-    sa_k_tile_sort<kOrderDiag, true><<<tiles, SA_SORT_TILE / 2, 0, st>>>(w.hset, nullptr, nullptr, w.rec[0], w.scope[0], n,
+    sa_k_tile_sort<kOrderDiag, true><<<tiles, SA_SORT_TILE, 0, st>>>(w.hset, nullptr, nullptr, w.rec[0], w.scope[0], n,
                                                                    nullptr, false);
     sa_note_launch();
-    const int b = sa_merge_passes<kOrderDiag>(w, 0, n, nullptr, st);
+    const int b = sa_merge_tiles<kOrderDiag>(w, 0, n, nullptr, st);
     sa_k_diag_count<<<G, 256, 0, st>>>(w.rec[b], w.scope[b], n, exclude, w.cta_a);
     sa_note_launch();
     sa_k_scan_partials<<<1, 1024, 0, st>>>(w.cta_a, w.cta_b, G, &w.ctr->uniq_count, nullptr);
@@ -470,8 +520,8 @@ int sa_launch_sort_rm(SaWork& w, uint64_t n, bool exclude, cudaStream_t st) {
     sa_k_diag_emit<<<G, 256, 0, st>>>(w.rec[b], w.scope[b], n, exclude, w.cta_a, w.rec[b ^ 1], w.scope[b ^ 1]);
     sa_note_launch();
     // the count after unique stays on the device: n bounds it, and passes past it copy
-    sa_k_tile_sort<kOrderFinal, false><<<tiles, SA_SORT_TILE / 2, 0, st>>>(w.hset, w.rec[b ^ 1], w.scope[b ^ 1], w.rec[b],
+    sa_k_tile_sort<kOrderFinal, false><<<tiles, SA_SORT_TILE, 0, st>>>(w.hset, w.rec[b ^ 1], w.scope[b ^ 1], w.rec[b],
                                                                      w.scope[b], n, &w.ctr->uniq_count, false);
     sa_note_launch();
-    return sa_merge_passes<kOrderFinal>(w, b, n, &w.ctr->uniq_count, st);
+    return sa_merge_tiles<kOrderFinal>(w, b, n, &w.ctr->uniq_count, st);
 }

@@ -11,13 +11,13 @@ from tests.helpers import compare_segments, random_text
 
 pytestmark = pytest.mark.gpu
 
-SIZES = (1, 2, 63, 65, 2047, 2048, 2049, 4096, 4097, 6145, 10_241)
+SIZES = (1, 2, 31, 33, 1023, 1024, 1025, 2049, 4097, 32_768, 32_769)
 
 
 @pytest.fixture(scope="module")
 def setup(built):
     rng = np.random.default_rng(21)
-    T, Q = random_text(rng, 700_000, gc=0.5), random_text(rng, 300_000, gc=0.5)
+    T, Q = random_text(rng, 2_200_000, gc=0.5), random_text(rng, 400_000, gc=0.5)
     p = oracle.params(hspthresh=600, noentropy=True)
     idx, pos = oracle.build_table(T, p)
     sf = SeedFilter()
