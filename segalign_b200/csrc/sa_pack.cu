@@ -30,44 +30,24 @@ sa_k_scan_partials(unsigned long long* a, unsigned long long* b, int G, unsigned
     }
 }
 
-__global__ void __launch_bounds__(1024)
-sa_k_radix_scan(unsigned int* hist, int G, const int* in_buf, int pass, const unsigned long long* d_n) {
-    if (in_buf && in_buf[pass] < 0) return;
-    constexpr int PER = 8, TILE = 1024 * PER;
-    __shared__ unsigned int tile[TILE];
-    __shared__ unsigned int ws[33];
-    const int t = threadIdx.x;
-    const uint32_t n = 256u * sa_radix_active(*d_n, (uint32_t)G);
+// One CTA per digit: its row of the bin-major histogram [256][A] becomes
+// exclusive prefixes within the digit; the row's sum goes to hist[256 * A + digit].
+// (One CTA for the whole histogram took 78 us at 592 active CTAs.)
+__global__ void __launch_bounds__(256)
+sa_k_radix_scan(unsigned int* hist, int G, const unsigned long long* d_n) {
+    __shared__ unsigned int ws[9];
+    const uint32_t A = sa_radix_active(*d_n, (uint32_t)G);
+    unsigned int* const row = hist + (uint64_t)blockIdx.x * A;
     unsigned int carry = 0;
-    for (uint32_t base = 0; base < n; base += TILE) {
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            const uint32_t i = base + k * 1024 + t;
-            tile[k * 1024 + t] = i < n ? hist[i] : 0u;
-        }
-        __syncthreads();
-        unsigned int v[PER], s = 0;
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            v[k] = tile[t * PER + k];
-            s += v[k];
-        }
+    for (uint32_t i0 = 0; i0 < A; i0 += 256) {
+        const uint32_t i = i0 + threadIdx.x;
+        const unsigned int v = i < A ? row[i] : 0u;
         unsigned int tot;
-        unsigned int run = sa_block_excl_sum<unsigned int, 1024>(s, ws, &tot) + carry;
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            tile[t * PER + k] = run;
-            run += v[k];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            const uint32_t i = base + k * 1024 + t;
-            if (i < n) hist[i] = tile[k * 1024 + t];
-        }
+        const unsigned int e = sa_block_excl_sum<unsigned int, 256>(v, ws, &tot);
+        if (i < A) row[i] = carry + e;
         carry += tot;
-        __syncthreads();
     }
+    if (threadIdx.x == 0) hist[256ull * A + blockIdx.x] = carry;
 }
 
 // ---------------------------------------------------------------------------
@@ -167,35 +147,9 @@ void sa_launch_pad_fill(uint32_t* base, uint64_t n, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// Spaced-seed key of the window starting at base p (common/ntcoding.cpp:43-61):
-// invalid unless all seed_size codes are 0..3 (uppercase ACGT); the key folds
-// the shape positions in order, first position most significant.
+// Table keys of target positions p = start + i * step (sa_window_key), in order
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t sa_key_at(const uint32_t* __restrict__ packed, int64_t p,
-                                              const SaParams& P) {
-    uint32_t w[4];
-    w[0] = sa_load8(packed, p);
-    w[1] = sa_load8(packed, p + 8);
-    w[2] = sa_load8(packed, p + 16);
-    w[3] = sa_load8(packed, p + 24);
-    uint32_t bad = 0;
-    const int ss = P.seed_size;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int n = ss - 8 * i;
-        uint32_t m = n >= 8 ? 0x44444444u : (n <= 0 ? 0u : (0x44444444u & ((1u << (4 * n)) - 1u)));
-        bad |= w[i] & m;
-    }
-    if (bad) return SA_INVALID_KEY;
-    uint32_t key = 0;
-    for (int i = 0; i < P.kmer_size; ++i) {
-        int sp = P.shape_pos[i];
-        key = (key << 2) | ((w[sp >> 3] >> (4 * (sp & 7))) & 3u);
-    }
-    return key;
-}
-
-// Table keys, pass 1: per-CTA count of valid positions p = start + i*step.
+// Any step, pass 1: per-CTA count of the valid positions.
 __global__ void __launch_bounds__(256)
 sa_k_table_count(const uint32_t* __restrict__ ref, uint32_t start, uint64_t n, uint32_t step, SaParams P,
                  unsigned long long* cta_a) {
@@ -203,14 +157,14 @@ sa_k_table_count(const uint32_t* __restrict__ ref, uint32_t start, uint64_t n, u
     sa_cta_range(n, a, b);
     unsigned long long c = 0;
     for (uint64_t i = a + threadIdx.x; i < b; i += 256)
-        c += sa_key_at(ref, (int64_t)start + (int64_t)i * step, P) != SA_INVALID_KEY;
+        c += sa_window_key(ref, (uint32_t)(start + i * step), P) != SA_INVALID_KEY;
     __shared__ unsigned long long ws[9];
     unsigned long long tot;
     sa_block_excl_sum<unsigned long long, 256>(c, ws, &tot);
     if (threadIdx.x == 0) cta_a[blockIdx.x] = tot;
 }
 
-// Table keys, pass 2: ordered compaction of (key, position) pairs.
+// Any step, pass 2: ordered compaction of (key, position) pairs.
 __global__ void __launch_bounds__(256)
 sa_k_table_emit(const uint32_t* __restrict__ ref, uint32_t start, uint64_t n, uint32_t step, SaParams P,
                 const unsigned long long* cta_a, uint32_t* keys, uint32_t* vals) {
@@ -222,7 +176,7 @@ sa_k_table_emit(const uint32_t* __restrict__ ref, uint32_t start, uint64_t n, ui
         uint64_t i = r + threadIdx.x;
         uint32_t key = SA_INVALID_KEY;
         uint32_t pos = start + (uint32_t)(i * step);
-        if (i < b) key = sa_key_at(ref, (int64_t)start + (int64_t)i * step, P);
+        if (i < b) key = sa_window_key(ref, (uint32_t)(start + i * step), P);
         unsigned long long v = key != SA_INVALID_KEY, tot;
         unsigned long long e = sa_block_excl_sum<unsigned long long, 256>(v, ws, &tot);
         if (v) {
@@ -233,14 +187,93 @@ sa_k_table_emit(const uint32_t* __restrict__ ref, uint32_t start, uint64_t n, ui
     }
 }
 
+// Keys of the windows that start at the 8 bases of word pw[0] (not checked for
+// ACGT), from the five words that hold every base they reach (seed_size <= 32).
+// For each shape position s in order (common/ntcoding.cpp:21-37) the word of
+// bases s .. s + 7 gives the next 2-bit code of all 8 keys at once.
+__device__ __forceinline__ void sa_keys8(const uint32_t* __restrict__ pw, const SaParams& P, uint32_t* key) {
+    const uint32_t W0 = __ldg(pw), W1 = __ldg(pw + 1), W2 = __ldg(pw + 2), W3 = __ldg(pw + 3), W4 = __ldg(pw + 4);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) key[k] = 0;
+    for (int i = 0; i < P.kmer_size; ++i) {
+        const uint32_t sp = (uint32_t)P.shape_pos[i], q = sp >> 3;
+        const uint32_t a = q == 0 ? W0 : q == 1 ? W1 : q == 2 ? W2 : W3;
+        const uint32_t b = q == 0 ? W1 : q == 1 ? W2 : q == 2 ? W3 : W4;
+        const uint32_t win = __funnelshift_r(a, b, 4u * (sp & 7u));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) key[k] = (key[k] << 2) | ((win >> (4 * k)) & 3u);
+    }
+}
+
+// Step 1: a thread takes the 8 positions of one packed word.  Pass 1 counts the
+// valid ones (no keys), pass 2 computes the 8 keys together (sa_keys8) and
+// writes those.  20 Mbp: 164 + 248 us with a key per position and pass, each
+// through local memory, 20 + 93 us now.
+__device__ __forceinline__ uint32_t sa_table_valid8(const uint32_t* __restrict__ ref, uint64_t g, uint64_t p0, uint64_t p1,
+                                                    uint32_t seed_size) {
+    uint32_t ok = sa_valid_windows8(ref + g, seed_size);
+    if (8 * g < p0) ok &= 0xffu << (p0 - 8 * g);
+    if (8 * g + 8 > p1) ok &= 0xffu >> (8 * g + 8 - p1);
+    return ok & 0xffu;
+}
+
+__global__ void __launch_bounds__(256)
+sa_k_table_count8(const uint32_t* __restrict__ ref, uint64_t p0, uint64_t p1, uint32_t seed_size,
+                  unsigned long long* cta_a) {
+    uint64_t a, b;
+    sa_cta_range(p1 > p0 ? ((p1 - 1) >> 3) - (p0 >> 3) + 1 : 0, a, b);
+    unsigned long long c = 0;
+    for (uint64_t g = (p0 >> 3) + a + threadIdx.x; g < (p0 >> 3) + b; g += 256)
+        c += __popc(sa_table_valid8(ref, g, p0, p1, seed_size));
+    __shared__ unsigned long long ws[9];
+    unsigned long long tot;
+    sa_block_excl_sum<unsigned long long, 256>(c, ws, &tot);
+    if (threadIdx.x == 0) cta_a[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(256)
+sa_k_table_emit8(const uint32_t* __restrict__ ref, uint64_t p0, uint64_t p1, SaParams P,
+                 const unsigned long long* cta_a, uint32_t* keys, uint32_t* vals) {
+    uint64_t a, b;
+    sa_cta_range(p1 > p0 ? ((p1 - 1) >> 3) - (p0 >> 3) + 1 : 0, a, b);
+    unsigned long long base = cta_a[blockIdx.x];
+    __shared__ uint32_t ws[9];
+    __shared__ uint32_t s_key[2048], s_pos[2048];  // a round's valid positions, to be written in whole lines
+    for (uint64_t g0 = (p0 >> 3) + a; g0 < (p0 >> 3) + b; g0 += 256) {
+        const uint64_t g = g0 + threadIdx.x;
+        const uint32_t ok = g < (p0 >> 3) + b ? sa_table_valid8(ref, g, p0, p1, (uint32_t)P.seed_size) : 0u;
+        uint32_t tot;
+        uint32_t at = sa_block_excl_sum<uint32_t, 256>(__popc(ok), ws, &tot);
+        if (ok) {
+            uint32_t key[8];
+            sa_keys8(ref + g, P, key);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (ok >> k & 1u) {
+                    s_key[at] = key[k];
+                    s_pos[at++] = (uint32_t)(8 * g + k);
+                }
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < tot; i += 256) {
+            keys[base + i] = s_key[i];
+            vals[base + i] = s_pos[i];
+        }
+        base += tot;
+        __syncthreads();
+    }
+}
+
 void sa_launch_table_keys(const uint32_t* ref, uint32_t start, uint64_t num_steps, uint32_t step,
                           const SaParams& p, uint32_t* keys, uint32_t* vals, unsigned long long* cta_a,
                           unsigned long long* cta_b, unsigned long long* d_total, int G, cudaStream_t st) {
-    sa_k_table_count<<<G, 256, 0, st>>>(ref, start, num_steps, step, p, cta_a);
+    if (step == 1) sa_k_table_count8<<<G, 256, 0, st>>>(ref, start, start + num_steps, (uint32_t)p.seed_size, cta_a);
+    else sa_k_table_count<<<G, 256, 0, st>>>(ref, start, num_steps, step, p, cta_a);
     sa_note_launch();
     sa_k_scan_partials<<<1, 1024, 0, st>>>(cta_a, cta_b, G, d_total, nullptr);
     sa_note_launch();
-    sa_k_table_emit<<<G, 256, 0, st>>>(ref, start, num_steps, step, p, cta_a, keys, vals);
+    if (step == 1) sa_k_table_emit8<<<G, 256, 0, st>>>(ref, start, start + num_steps, p, cta_a, keys, vals);
+    else sa_k_table_emit<<<G, 256, 0, st>>>(ref, start, num_steps, step, p, cta_a, keys, vals);
     sa_note_launch();
 }
 
@@ -273,44 +306,40 @@ struct SaKvOps {
         uint32_t* v[2];
     };
     struct Pass {
+        const uint32_t *k, *v;
+        uint32_t *k_out, *v_out;
         uint32_t shift;
     };
-    static __device__ __forceinline__ Pass pass_of(const Ctx&, int pass) { return {8u * (uint32_t)pass}; }
+    static __device__ __forceinline__ Pass pass_of(const Ctx& c, int pass) {
+        if (pass & 1) return {c.k[1], c.v[1], c.k[0], c.v[0], 8u * (uint32_t)pass};
+        return {c.k[0], c.v[0], c.k[1], c.v[1], 8u * (uint32_t)pass};
+    }
     struct Item {
         uint32_t k, v;
     };
-    static __device__ __forceinline__ Item load(const Ctx& c, int buf, uint64_t i) { return {c.k[buf][i], c.v[buf][i]}; }
+    static __device__ __forceinline__ Item load(const Pass& p, uint64_t i) { return {p.k[i], p.v[i]}; }
     static __device__ __forceinline__ uint32_t digit_of(const Pass& p, const Item& x) { return (x.k >> p.shift) & 0xffu; }
-    static __device__ __forceinline__ void store(const Ctx& c, int buf, const Item& x, uint32_t dst) {
-        c.k[buf ^ 1][dst] = x.k;
-        c.v[buf ^ 1][dst] = x.v;
+    static __device__ __forceinline__ void store(const Pass& p, const Item& x, uint32_t dst) {
+        p.k_out[dst] = x.k;
+        p.v_out[dst] = x.v;
     }
 };
-
-__global__ void sa_k_plan_noskip(int* in_buf, int passes) {
-    for (int p = 0; p <= passes; ++p) in_buf[p] = p & 1;
-}
 
 void sa_launch_sort_kv(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                        const unsigned long long* d_n, int bits, unsigned int* cta_hist, int G,
                        cudaStream_t st, int* result_in_tmp) {
     int passes = (bits + 7) / 8;
-    // in_buf lives right after the histogram workspace
-    int* in_buf = reinterpret_cast<int*>(cta_hist + 256 * (uint64_t)SA_MAX_CTAS);
-    sa_k_plan_noskip<<<1, 1, 0, st>>>(in_buf, passes);
-    sa_note_launch();
     SaKvOps::Ctx c;
     c.k[0] = keys;
     c.k[1] = keys_tmp;
     c.v[0] = vals;
     c.v[1] = vals_tmp;
-    SaRadixCtl ctl{d_n, in_buf};
     for (int p = 0; p < passes; ++p) {
-        sa_k_radix_up<SaKvOps><<<G, SA_RADIX_BLOCK, 0, st>>>(c, p, ctl, cta_hist);
+        sa_k_radix_up<SaKvOps><<<G, SA_RADIX_BLOCK, 0, st>>>(c, p, d_n, cta_hist);
         sa_note_launch();
-        sa_k_radix_scan<<<1, 1024, 0, st>>>(cta_hist, G, in_buf, p, d_n);
+        sa_k_radix_scan<<<256, 256, 0, st>>>(cta_hist, G, d_n);
         sa_note_launch();
-        sa_k_radix_down<SaKvOps><<<G, SA_RADIX_BLOCK, 0, st>>>(c, p, ctl, cta_hist);
+        sa_k_radix_down<SaKvOps><<<G, SA_RADIX_BLOCK, 0, st>>>(c, p, d_n, cta_hist);
         sa_note_launch();
     }
     *result_in_tmp = passes & 1;
@@ -322,45 +351,20 @@ void sa_launch_sort_kv(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint3
 // j, SA_INVALID_KEY unless all seed_size bases are uppercase ACGT.
 // ---------------------------------------------------------------------------
 //
-// One thread takes the 8 positions of one packed word, p0 = 8g .. 8g + 7, and
-// the five words from word g on, which hold every base their windows reach
-// (seed_size <= 32 bases, padding after the last word).  Validity: a 40-bit
-// mask of the windows' non-ACGT bases (code bit 2), tested against the
-// seed_size bits from each position.  Keys: for each shape position s in
-// increasing order (the shape's order, common/ntcoding.cpp:21-37), the word
-// of bases p0 + s .. p0 + s + 7 gives the next 2-bit code of all 8 keys at once.
+// One thread takes the 8 positions of one packed word.
 __global__ void __launch_bounds__(256)
 sa_k_query_keys(const uint32_t* __restrict__ packed, uint64_t len, SaParams P, uint32_t* __restrict__ keys) {
-    uint64_t smask = 0;  // bit s set: shape position s is a care position
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-        if (i < P.kmer_size) smask |= 1ull << P.shape_pos[i];
-    const uint32_t ss = (uint32_t)P.seed_size;
-    const uint64_t wmask = ss >= 64 ? ~0ull : (1ull << ss) - 1;
     const uint64_t ngroups = (len + 7) / 8;
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < ngroups;
          g += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t* pw = packed + g;
-        const uint32_t W0 = __ldg(pw), W1 = __ldg(pw + 1), W2 = __ldg(pw + 2), W3 = __ldg(pw + 3), W4 = __ldg(pw + 4);
-        const uint64_t bad = (uint64_t)sa_nonacgt8(W0) | ((uint64_t)sa_nonacgt8(W1) << 8) |
-                             ((uint64_t)sa_nonacgt8(W2) << 16) | ((uint64_t)sa_nonacgt8(W3) << 24) |
-                             ((uint64_t)sa_nonacgt8(W4) << 32);
+        const uint32_t ok = sa_valid_windows8(pw, (uint32_t)P.seed_size);
         uint32_t key[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) key[k] = 0;
-        for (uint64_t m = smask; m; m &= m - 1) {
-            const uint32_t sp = (uint32_t)(__ffsll((long long)m) - 1);
-            const uint32_t q = sp >> 3;
-            const uint32_t a = q == 0 ? W0 : q == 1 ? W1 : q == 2 ? W2 : W3;
-            const uint32_t b = q == 0 ? W1 : q == 1 ? W2 : q == 2 ? W3 : W4;
-            const uint32_t win = __funnelshift_r(a, b, 4u * (sp & 7u));
-#pragma unroll
-            for (int k = 0; k < 8; ++k) key[k] = (key[k] << 2) | ((win >> (4 * k)) & 3u);
-        }
+        sa_keys8(pw, P, key);
         const uint64_t p0 = 8 * g;
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (p0 + k < len) keys[p0 + k] = ((bad >> k) & wmask) ? SA_INVALID_KEY : key[k];
+            if (p0 + k < len) keys[p0 + k] = (ok >> k & 1u) ? key[k] : SA_INVALID_KEY;
     }
 }
 

@@ -6,13 +6,11 @@
 // [n*c/G, n*(c+1)/G), with n read from device memory, so a whole call can be
 // launched without host round trips.  The sort passes use only the first
 // A = min(G, ceil(n / SA_RADIX_MIN_ITEMS)) CTAs, so small sorts scan small
-// histograms.  One pass = up-sweep (per-CTA digit histogram), a single-CTA
-// exclusive scan of the bin-major histogram [256][A], and a stable down-sweep
-// scatter that ranks equal digits inside a warp with __match_any_sync and
-// across warps with a per-round shared-memory prefix.
-// A pass whose input buffer is recorded as -1 is skipped (all items share
-// that digit), which is how the fixed-layout HSP keys avoid scattering
-// constant bytes.
+// histograms.  One pass = up-sweep (per-CTA digit histogram), an exclusive scan
+// of each digit's row of the bin-major histogram [256][A] (a CTA per digit), and a
+// stable down-sweep scatter that ranks equal digits inside a warp with
+// ballots and across warps with a per-round shared-memory prefix.
+// Pass p reads buffer p & 1.
 #pragma once
 #include <cstdint>
 #include "sa_internal.cuh"
@@ -82,29 +80,21 @@ __device__ __forceinline__ T sa_block_excl_sum(T v, T* ws, T* total) {
 __global__ void sa_k_scan_partials(unsigned long long* a, unsigned long long* b, int G,
                                    unsigned long long* ta, unsigned long long* tb);
 
-// Exclusive scan of the bin-major histogram [256][A] in place (one CTA of
-// 1024), A = sa_radix_active(*d_n, G).
-__global__ void sa_k_radix_scan(unsigned int* hist, int G, const int* in_buf, int pass,
-                                const unsigned long long* d_n);
-
-struct SaRadixCtl {
-    const unsigned long long* d_n;  // item count
-    const int* in_buf;              // [passes]: input buffer of each pass, -1 = skip
-};
+// Exclusive scan of every digit's row of the histogram [256][A], A =
+// sa_radix_active(*d_n, G), by 256 CTAs; the rows' sums follow the histogram.
+__global__ void sa_k_radix_scan(unsigned int* hist, int G, const unsigned long long* d_n);
 
 // Ops must provide:
 //   struct Ctx;  struct Item;  (one item: its key and payload)
 //   struct Pass;  (what selects the digit of one pass, resolved once per kernel)
 //   static __device__ Pass pass_of(const Ctx&, int pass);
-//   static __device__ Item load(const Ctx&, int buf, uint64_t i);
+//   static __device__ Item load(const Pass&, uint64_t i);
 //   static __device__ uint32_t digit_of(const Pass&, const Item&);
-//   static __device__ void store(const Ctx&, int buf, const Item&, uint32_t dst);  (into buffer buf ^ 1)
+//   static __device__ void store(const Pass&, const Item&, uint32_t dst);
 template <class Ops>
 __global__ void __launch_bounds__(SA_RADIX_BLOCK)
-sa_k_radix_up(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, unsigned int* hist) {
-    const int buf = ctl.in_buf[pass];
-    if (buf < 0) return;
-    const uint64_t n = *ctl.d_n;
+sa_k_radix_up(typename Ops::Ctx ctx, int pass, const unsigned long long* d_n, unsigned int* hist) {
+    const uint64_t n = *d_n;
     const uint32_t A = sa_radix_active(n, gridDim.x);
     if (blockIdx.x >= A) return;
     __shared__ unsigned int h[256];
@@ -114,33 +104,57 @@ sa_k_radix_up(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, unsigned int* his
     uint64_t a, b;
     sa_radix_range(n, A, a, b);
     const typename Ops::Pass P = Ops::pass_of(ctx, pass);
-    for (uint64_t i = a + t; i < b; i += SA_RADIX_BLOCK) atomicAdd(&h[Ops::digit_of(P, Ops::load(ctx, buf, i))], 1u);
+    // eight loads in flight per thread: one at a time left the pass at load latency
+    constexpr int J = 8;
+    for (uint64_t i0 = a + t; i0 < b; i0 += J * SA_RADIX_BLOCK) {
+        uint32_t d[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const uint64_t i = i0 + j * SA_RADIX_BLOCK;
+            d[j] = i < b ? Ops::digit_of(P, Ops::load(P, i)) : 256u;
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (d[j] < 256u) atomicAdd(&h[d[j]], 1u);
+    }
     __syncthreads();
     hist[(uint64_t)t * A + blockIdx.x] = h[t];
 }
 
 // Down-sweep: tiles of SA_RADIX_TILE = 256 x SA_RADIX_ITEMS items.  Warp w
 // ranks the tile's items [w * 32 * ITEMS, (w + 1) * 32 * ITEMS) row by row
-// (coalesced loads, __match_any_sync within a row, a per-warp digit count
+// (coalesced loads, ballots within a row, a per-warp digit count
 // carried across rows); per-digit warp prefixes and the tile's digit starts
 // then place every item in digit order in shared memory, and the tile is
 // written back in that order, so items of one digit leave as runs of
 // consecutive addresses.  Items keep their input order within a digit
 // (stable).
+// 20 M pairs, a pass, us: 4 items 221, 8 items 168, 16 items 231 (with __match_any_sync 240,
+// 374 and 310)
 #ifndef SA_RADIX_ITEMS
-#define SA_RADIX_ITEMS 4
+#define SA_RADIX_ITEMS 8
 #endif
 #define SA_RADIX_TILE (SA_RADIX_BLOCK * SA_RADIX_ITEMS)
 
+// Lanes whose 9-bit digit equals this lane's (__match_any_sync goes through the
+// distinct values one by one, which is most of 32 here).
+__device__ __forceinline__ uint32_t sa_digit_peers(uint32_t d) {
+    uint32_t peers = ~0u;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? m : ~m;
+    }
+    return peers;
+}
+
 template <class Ops>
 __global__ void __launch_bounds__(SA_RADIX_BLOCK)
-sa_k_radix_down(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, const unsigned int* hist) {
+sa_k_radix_down(typename Ops::Ctx ctx, int pass, const unsigned long long* d_n, const unsigned int* hist) {
     constexpr int NWARP = SA_RADIX_BLOCK / 32;
     constexpr int K = SA_RADIX_ITEMS;
     using Item = typename Ops::Item;
-    const int buf = ctl.in_buf[pass];
-    if (buf < 0) return;
-    const uint64_t n = *ctl.d_n;
+    const uint64_t n = *d_n;
     const uint32_t A = sa_radix_active(n, gridDim.x);
     if (blockIdx.x >= A) return;
     __shared__ unsigned int offs[256];           // next output index of each digit (this CTA)
@@ -149,11 +163,25 @@ sa_k_radix_down(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, const unsigned 
     __shared__ unsigned int ws[NWARP + 1];
     __shared__ Item stage[SA_RADIX_TILE];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    offs[t] = hist[(uint64_t)t * A + blockIdx.x];
+    {   // digit t starts after the items of smaller digits
+        unsigned int all;
+        const unsigned int first = sa_block_excl_sum<unsigned int, SA_RADIX_BLOCK>(hist[256ull * A + t], ws, &all);
+        offs[t] = first + hist[(uint64_t)t * A + blockIdx.x];
+    }
     uint64_t a, b;
     sa_radix_range(n, A, a, b);
     const uint32_t lt = sa_lanemask_lt();
     const typename Ops::Pass P = Ops::pass_of(ctx, pass);
+    // a tile's items are loaded while the tile before is placed
+    Item ahead[K];
+    auto fetch = [&](uint64_t base) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint64_t i = base + (uint64_t)warp * 32 * K + (uint64_t)k * 32 + lane;
+            if (i < b) ahead[k] = Ops::load(P, i);
+        }
+    };
+    fetch(a);
     for (uint64_t base = a; base < b; base += SA_RADIX_TILE) {
 #pragma unroll
         for (int w = 0; w < NWARP; ++w) wcnt[w][t] = 0;
@@ -162,14 +190,13 @@ sa_k_radix_down(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, const unsigned 
         uint32_t d[K], r[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const uint64_t i = base + (uint64_t)warp * 32 * K + (uint64_t)k * 32 + lane;
-            const bool valid = i < b;
-            if (valid) it[k] = Ops::load(ctx, buf, i);
-            d[k] = valid ? Ops::digit_of(P, it[k]) : 256u;
+            it[k] = ahead[k];
+            d[k] = base + (uint64_t)warp * 32 * K + (uint64_t)k * 32 + lane < b ? Ops::digit_of(P, it[k]) : 256u;
         }
+        fetch(base + SA_RADIX_TILE);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const uint32_t peers = __match_any_sync(0xffffffffu, d[k]);
+            const uint32_t peers = sa_digit_peers(d[k]);
             const uint32_t rank = __popc(peers & lt);
             const bool valid = d[k] < 256u;
             r[k] = valid ? wcnt[warp][d[k]] + rank : 0u;
@@ -200,7 +227,7 @@ sa_k_radix_down(typename Ops::Ctx ctx, int pass, SaRadixCtl ctl, const unsigned 
             if (s < tile_n) {
                 const Item x = stage[s];
                 const uint32_t dd = Ops::digit_of(P, x);
-                Ops::store(ctx, buf, x, offs[dd] + (s - tstart[dd]));
+                Ops::store(P, x, offs[dd] + (s - tstart[dd]));
             }
         }
         __syncthreads();
