@@ -91,6 +91,9 @@ struct DevState {
     uint64_t nbuckets = 0;
     uint32_t* pos = nullptr;
     uint64_t num_index = 0;
+    uint64_t index_cap = 0, pos_cap = 0;   // entries allocated
+    void* table_ws = nullptr;              // workspace of the last table build (at most kTableWsKeep bytes)
+    uint64_t table_ws_cap = 0;
     // shape of a table that holds every seed window of the resident target
     // (built here at step 1), else 0
     uint64_t table_full = 0;
@@ -250,6 +253,37 @@ void finish_packed(Packed& pk) { sa_launch_reverse_packed(pk.data, pk.len, pk.da
 void make_rc_packed(const Packed& pk, Packed& rc) {
     sa_launch_reverse_packed(pk.data, pk.len, rc.data, true, 0);
     finish_packed(rc);
+}
+
+// A block stream rebuilds the table for every target block: its arrays are
+// rewritten where they fit, and the build's workspace (16 bytes per position,
+// up to kTableWsKeep) stays until sa_clear_ref.  Allocating and freeing them
+// took 4 of the 5 ms of a 20 Mbp build.
+constexpr uint64_t kTableWsKeep = 2ull << 30;
+
+void release_table(DevState& d) {
+    if (d.index) cudaFree(d.index);
+    if (d.pos) cudaFree(d.pos);
+    if (d.table_ws) cudaFree(d.table_ws);
+    d.index = d.pos = nullptr;
+    d.table_ws = nullptr;
+    d.index_cap = d.pos_cap = d.table_ws_cap = 0;
+    d.nbuckets = d.num_index = 0;
+    d.table_full = 0;
+}
+
+// An array of at least `need` entries: the one there if it fits and is not
+// many times larger.  The caller has synchronized the device, so no call still
+// reads the table.
+int table_array(uint32_t** p, uint64_t* cap, uint64_t need) {
+    if (need == 0) need = 1;
+    if (*p && *cap >= need && *cap / 4 <= need + (1ull << 22)) return SA_OK;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    SA_CUDA_OK(cudaMalloc(p, 4 * need));
+    *cap = need;
+    return SA_OK;
 }
 
 // Uploads text[0, len) and packs it into pk (and its reverse complement into rc if given).
@@ -642,7 +676,7 @@ int check_ready(bool need_query) {
         return SA_ERR_STATE;
     }
     for (auto& d : g.devs) {
-        if (!d.ref.data || !d.index || !d.pos) {
+        if (!d.ref.data || !d.nbuckets || !d.pos) {
             sa_set_error(SA_ERR_STATE, "no resident target and seed table");
             return SA_ERR_STATE;
         }
@@ -1440,11 +1474,7 @@ int sa_clear_ref(void) {
         cudaSetDevice(d.dev);
         d.ref.release();
         d.ref_rc.release();
-        if (d.index) cudaFree(d.index);
-        if (d.pos) cudaFree(d.pos);
-        d.index = d.pos = nullptr;
-        d.nbuckets = d.num_index = 0;
-        d.table_full = 0;
+        release_table(d);
     }
     g.last_ref_ptr = nullptr;
     return SA_OK;
@@ -1461,56 +1491,48 @@ static int build_table_on(DevState& d, const Packed& ref, uint32_t step) {
     int64_t span = (int64_t)ref.len - p.seed_size + offset;
     uint64_t num_steps = span > 0 ? (uint64_t)span / step : 0;
     uint64_t nb = 1ull << (2 * p.kmer_size);
-    uint64_t cap = num_steps ? num_steps : 1;
-    uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr;
-    unsigned long long* scratch = nullptr;
-    unsigned int* hist = nullptr;
-    auto cleanup = [&]() {
-        if (keys) cudaFree(keys);
-        if (vals) cudaFree(vals);
-        if (keys2) cudaFree(keys2);
-        if (vals2) cudaFree(vals2);
-        if (scratch) cudaFree(scratch);
-        if (hist) cudaFree(hist);
-    };
-    cudaError_t e = cudaSuccess;
-    if ((e = cudaMalloc(&keys, 4 * cap)) != cudaSuccess || (e = cudaMalloc(&vals, 4 * cap)) != cudaSuccess ||
-        (e = cudaMalloc(&keys2, 4 * cap)) != cudaSuccess || (e = cudaMalloc(&vals2, 4 * cap)) != cudaSuccess ||
-        (e = cudaMalloc(&scratch, 8 * (2 * SA_MAX_CTAS + 4))) != cudaSuccess ||
-        (e = cudaMalloc(&hist, 4 * (256 * (uint64_t)SA_MAX_CTAS + 64))) != cudaSuccess) {
-        cleanup();
-        return sa_cuda_fail(e, "cudaMalloc(table build)", __FILE__, __LINE__);
+    const uint64_t cap = num_steps ? num_steps : 1;
+    d.nbuckets = d.num_index = 0;  // no table until this one is complete
+    SA_CUDA_OK(cudaDeviceSynchronize());
+    // keys and positions, twice (the sort's two buffers), one of the position
+    // arrays being the table's own; per-CTA counts and digit histograms
+    const uint64_t arr = (4 * cap + 255) & ~255ull, counts = 8 * (2 * SA_MAX_CTAS + 32),
+                   hists = 4 * (256 * (uint64_t)SA_MAX_CTAS + 256), need = 3 * arr + counts + hists;
+    if (d.table_ws_cap < need) {
+        if (d.table_ws) cudaFree(d.table_ws);
+        d.table_ws = nullptr;
+        d.table_ws_cap = 0;
+        SA_CUDA_OK(cudaMalloc(&d.table_ws, need));
+        d.table_ws_cap = need;
     }
-    const int Gr = std::min(g.tuning.range_ctas, SA_MAX_CTAS);
-    unsigned long long* cta_a = scratch;
-    unsigned long long* cta_b = scratch + SA_MAX_CTAS;
-    unsigned long long* d_total = scratch + 2 * SA_MAX_CTAS;
+    SA_TRY(table_array(&d.index, &d.index_cap, nb));
+    SA_TRY(table_array(&d.pos, &d.pos_cap, cap));
+    char* ws = (char*)d.table_ws;
+    uint32_t* const key0 = (uint32_t*)ws;
+    uint32_t* const key1 = (uint32_t*)(ws + arr);
+    uint32_t* const other = (uint32_t*)(ws + 2 * arr);
+    unsigned long long* const cta_a = (unsigned long long*)(ws + 3 * arr);
+    unsigned long long* const cta_b = cta_a + SA_MAX_CTAS;
+    unsigned long long* const d_total = cta_a + 2 * SA_MAX_CTAS;
+    unsigned int* const hist = (unsigned int*)(ws + 3 * arr + counts);
+    const bool odd = ((2 * p.kmer_size + 7) / 8) & 1;  // sort passes: the last one writes buffer 1 if odd
+    uint32_t* const val0 = odd ? other : d.pos;
+    uint32_t* const val1 = odd ? d.pos : other;
+    // 6-7 CTAs per SM in flight (20 Mbp: a sort's counting pass 25 us on 592 CTAs, 21 on 1024)
+    const int Gr = SA_MAX_CTAS;
     cudaMemset(d_total, 0, 8);
-    sa_launch_table_keys(ref.data, start, num_steps, step, p, keys, vals, cta_a, cta_b, d_total, Gr, 0);
+    sa_launch_table_keys(ref.data, start, num_steps, step, p, key0, val0, cta_a, cta_b, d_total, Gr, 0);
     int in_tmp = 0;
-    sa_launch_sort_kv(keys, vals, keys2, vals2, d_total, 2 * p.kmer_size, hist, Gr, 0, &in_tmp);
+    sa_launch_sort_kv(key0, val0, key1, val1, d_total, 2 * p.kmer_size, hist, Gr, 0, &in_tmp);
+    sa_launch_table_index(in_tmp ? key1 : key0, d_total, d.index, nb, 0);
     unsigned long long n_valid = 0;
-    e = cudaMemcpy(&n_valid, d_total, 8, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-        cleanup();
-        return sa_cuda_fail(e, "table build", __FILE__, __LINE__);
+    cudaError_t e = cudaMemcpy(&n_valid, d_total, 8, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (d.table_ws_cap > kTableWsKeep) {
+        cudaFree(d.table_ws);
+        d.table_ws = nullptr;
+        d.table_ws_cap = 0;
     }
-    if (d.index) cudaFree(d.index);
-    if (d.pos) cudaFree(d.pos);
-    d.index = d.pos = nullptr;
-    if ((e = cudaMalloc(&d.index, 4 * nb)) != cudaSuccess) {
-        cleanup();
-        return sa_cuda_fail(e, "cudaMalloc(index table)", __FILE__, __LINE__);
-    }
-    uint32_t* sk = in_tmp ? keys2 : keys;
-    uint32_t* sv = in_tmp ? vals2 : vals;
-    sa_launch_table_index(sk, d_total, d.index, nb, 0);
-    // keep the sorted positions as the position table; free the rest
-    d.pos = sv;
-    if (sv == vals) vals = nullptr;
-    else vals2 = nullptr;
-    e = cudaDeviceSynchronize();
-    cleanup();
     if (e != cudaSuccess) return sa_cuda_fail(e, "table build", __FILE__, __LINE__);
     d.nbuckets = nb;
     d.num_index = n_valid;
@@ -1567,15 +1589,15 @@ int sa_send_seed_pos_table(const uint32_t* index_table, uint32_t index_table_siz
             sa_set_error(SA_ERR_ARG, "position %u of the table lies past the target end", pos_table[i]);
             return SA_ERR_ARG;
         }
+    std::unique_lock<std::shared_mutex> dev_wide(g_capture_mu);
     for (auto& d : g.devs) {
         SA_CUDA_OK(cudaSetDevice(d.dev));
         d.table_full = 0;
-        if (d.index) cudaFree(d.index);
-        if (d.pos) cudaFree(d.pos);
-        d.index = d.pos = nullptr;
-        SA_CUDA_OK(cudaMalloc(&d.index, 4ull * index_table_size));
+        d.nbuckets = d.num_index = 0;
+        SA_CUDA_OK(cudaDeviceSynchronize());
+        SA_TRY(table_array(&d.index, &d.index_cap, index_table_size));
+        SA_TRY(table_array(&d.pos, &d.pos_cap, num_index));
         SA_CUDA_OK(cudaMemcpy(d.index, index_table, 4ull * index_table_size, cudaMemcpyHostToDevice));
-        SA_CUDA_OK(cudaMalloc(&d.pos, 4ull * (num_index ? num_index : 1)));
         if (num_index) SA_CUDA_OK(cudaMemcpy(d.pos, pos_table, 4ull * num_index, cudaMemcpyHostToDevice));
         d.nbuckets = index_table_size;
         d.num_index = num_index;
@@ -1586,7 +1608,7 @@ int sa_send_seed_pos_table(const uint32_t* index_table, uint32_t index_table_siz
 int sa_get_seed_pos_table(uint32_t* index_table, uint64_t index_cap, uint32_t* pos_table, uint64_t pos_cap,
                           uint64_t* index_table_size, uint64_t* num_index) {
     Global& g = G();
-    if (g.devs.empty() || !g.devs[0].index) return SA_ERR_STATE;
+    if (g.devs.empty() || !g.devs[0].nbuckets) return SA_ERR_STATE;
     DevState& d = g.devs[0];
     if (index_table_size) *index_table_size = d.nbuckets;
     if (num_index) *num_index = d.num_index;
