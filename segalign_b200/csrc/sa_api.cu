@@ -355,7 +355,7 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
     w.surv_cap = surv_cap;
     w.long_cap = long_cap;
     // the list is two records of `out` per hit
-    w.list_cap = std::min<uint64_t>(surv_cap / 2, env_u64("SA_LIST_CAP", ~0ull)) & ~31ull;
+    w.list_cap = std::min<uint64_t>(std::min<uint64_t>(surv_cap / 2, 1ull << 31), env_u64("SA_LIST_CAP", ~0ull)) & ~31ull;
     const uint64_t nunits = batch ? std::max<uint64_t>(64, std::min<uint64_t>(units, SA_MAX_UNITS)) : 64;
     s->max_units = (uint32_t)nunits;
     std::vector<Part> parts = {

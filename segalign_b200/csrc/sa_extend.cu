@@ -30,6 +30,7 @@
 #include "sa_radix.cuh"
 
 #define SA_FULL 0xffffffffu
+#define SA_LANE_TABLES 256  // lane kernel: the 64-entry score table
 
 struct SaExtK {
     const uint32_t* ref;
@@ -54,13 +55,11 @@ struct SaExtK {
     int32_t match, swing; // smallest match score, and that minus the lowest mismatch score
     uint32_t mismatches;  // as many mismatches in a row cannot stop a scan
     uint32_t shift[16];   // shape positions, the first one again in the unused places
-    uint4* list;          // hits the sweep leaves to the lane kernel, two words of 16 bytes each:
+    uint4* list;          // hits the sweep leaves to the scans, two words of 16 bytes each:
                           // {rl, ql, scope, unit | SA_CHAIN_NEXT}, {SaSwept}
     uint64_t list_cap;    // 0: no sweep
-    // scanned hits that others may follow [list_cap]: {rl, ql, unit, bases left of
-    // the hit}, position of the right end, stop words right and left
-    uint4* lead;
-    uint32_t *lead_right, *lead_stop_r, *lead_stop_l;
+    uint4* scanned;       // per list record and side (right, left): {best, its offset (-1: best is 0), start and
+                          // depth of the step that stops}
 };
 
 // Largest compacted seed c in [0, nnz) with E[c] <= h (E strictly increasing,
@@ -254,7 +253,6 @@ __device__ __forceinline__ void sa_window_exact(const char* tblb, uint32_t lo, u
 #define SA_CHAIN_BLOCK 1024u
 #define SA_CHAIN_NEXT 0x80000000u  // unit bit: a hit follows on the diagonal within `gap` bases
 #define SA_CHAIN_DROP 0x40000000u  // unit bit, inside the sweep: what it saw of the hit allows dropping it
-#define SA_CHAIN_HIGH 0x40000000u  // unit bit, in `lead`: the hit's total is at least hspthresh
 #define SA_CHAIN_GAP 13u           // largest `gap`
 #define SA_SWEEP_RIGHT 32u         // bases the sweep scores right and left of a hit
 #define SA_SWEEP_LEFT 64u
@@ -371,7 +369,7 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // is done: it adds its tiles and leaves nothing else.  These are the chance
 // hits, four of five on the genome workload.  The others gather in a buffer
 // per warp; full batches of them take the chain test, and those it does not
-// drop go to `list`, which the lane kernel scans.
+// drop go to `list`, for the scans (sa_k_scan).
 //
 // Why apart from the lane kernel: a chance hit's work there was the hand-out,
 // two direction set-ups and the bookkeeping of an iteration, most of it run
@@ -383,13 +381,12 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // Bound by the L1 data pipe (83%: 96 table lookups and 128 wavefronts of target
 // loads in about 250 per round), with the ALU pipe and issue at 70%.  On a 2.5 Mbp query
 // against the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in
-// the lane kernel 5.65 ms; sweep 2.00, lane kernel 1.46, chain walk 0.33: 3.75 ms (4.79
-// with the sweep and no chains).  The chain test on all hits as they were
+// the lane kernel 5.65 ms; sweep 2.00, scans 0.81, finish 0.70: 3.33 ms, its launches
+// included (without chains 4.4).  The chain test on all hits as they were
 // scored, with the rounds split evenly over the warps, made the sweep 2.33 ms.
-// Lane phase of 24 Mbp: 55.0 -> 34.5 ms; of a repeat-masker call, 0.80 -> 0.40 ms,
-// and its warp kernel 0.78 -> 0.14.
+// Lane phase of 24 Mbp: 55.0 -> 30.8 ms.
 // ---------------------------------------------------------------------------
-// What the sweep leaves of a hit, for the lane kernel to go on from: per
+// What the sweep leaves of a hit, for the scans to go on from: per
 // direction the best score (low half) and best - score (high half) after the
 // direction's sweep, and in `rest` the offsets of the first bases reaching the
 // bests (a byte each) and these flags.  A direction that has stopped leaves its
@@ -398,6 +395,7 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 #define SA_SWEPT_STOP_R 0x20000u
 #define SA_SWEPT_STOP_L 0x40000u
 #define SA_SWEPT_TILE_2 0x80000u   // the left scan stopped in its second 32-base tile
+#define SA_SWEPT_LONG 0x100000u    // the hit went to the long queue (set by sa_k_scan)
 
 // One 8-base window of a scan, from its first base on (REV: from base 7
 // down), in the lane kernel's packed form with SA_SWEEP_LEFT in place of STEP
@@ -567,7 +565,7 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                         if (i == 4) tl = stop_l ? 2 : 3;  // tiles of both scans, if they stop
                     }
                     x.y = sa_swept_word(p, at);
-                    // a window that reaches past an end scans it to the end: the lane kernel does that
+                    // where a window reaches past a sequence end, the scans start anew
                     const bool inside = min(rl, ql) >= SA_SWEEP_LEFT && (uint64_t)rl + SA_SWEEP_RIGHT <= a.ref_len &&
                                         (uint64_t)ql + SA_SWEEP_RIGHT <= U.q_len;
                     left = !inside || !stop_r || !stop_l || (int)(float)(best_r + (at >> SA_SWEEP_SH)) >= a.hspthresh;
@@ -601,13 +599,19 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
     }
 }
 
-// Match, transition and non-ACGT bits of 32 bases.
-__device__ __forceinline__ void sa_masks32(const uint32_t* __restrict__ R, const uint32_t* __restrict__ Q, uint32_t rl,
-                                           uint32_t ql, int off, uint32_t& m, uint32_t& t, uint32_t& bad) {
+// Match, transition and non-ACGT bits of 32 bases from word pr[0] and pq[0]
+// (shifted by sr, sq bits); the words after the 32 bases' first four are left in
+// rl, ql, which hold those first words on entry.
+__device__ __forceinline__ void sa_masks32(const uint32_t* __restrict__ pr, const uint32_t* __restrict__ pq, uint32_t sr,
+                                           uint32_t sq, uint32_t& rl, uint32_t& ql, uint32_t& m, uint32_t& t,
+                                           uint32_t& bad) {
     uint32_t mm[4], tt[4], bb[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const uint32_t rw = sa_load8(R, (int64_t)rl + off + 8 * k), qw = sa_load8(Q, (int64_t)ql + off + 8 * k);
+        const uint32_t rn = __ldg(pr + k + 1), qn = __ldg(pq + k + 1);
+        const uint32_t rw = __funnelshift_r(rl, rn, sr), qw = __funnelshift_r(ql, qn, sq);
+        rl = rn;
+        ql = qn;
         sa_match_bits<true>(rw, qw, mm[k], tt[k]);
         bb[k] = sa_nibble_bits(((rw | qw) >> 2) & 0x11111111u);
     }
@@ -617,9 +621,9 @@ __device__ __forceinline__ void sa_masks32(const uint32_t* __restrict__ R, const
 }
 
 // The dropped hits that follow the scanned hit (rl, ql) of `unit` (high: its
-// total is at least hspthresh): their number and the tiles of their scans.  stop_r, stop_l: offsets at which the hit's
-// right and left scans stop; a hit d bases on stops at stop_r - d and
-// stop_l + d.
+// total is at least hspthresh): their number and the tiles of their scans.
+// stop_r, stop_l: offsets at which the hit's right and left scans stop; a hit d
+// bases on stops at stop_r - d and stop_l + d.
 struct SaChain {
     unsigned long long tiles;
     uint32_t n;
@@ -632,11 +636,16 @@ __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaPar
     const uint32_t S = a.seed_size, j = ql - S;
     uint32_t ahead = U.j_hi - 1 - j;
     if (U.flags & 1u) ahead = min(ahead, U.rm_hi - rl);
-    uint32_t n = 0, last = 0, m0, t0, b0;
-    sa_masks32(a.ref, U.q_packed, rl, ql, -32, m0, t0, b0);
+    const uint32_t* __restrict__ pr = a.ref + (int)(rl >> 3) - 4;
+    const uint32_t* __restrict__ pq = U.q_packed + (int)(ql >> 3) - 4;
+    const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
+    uint32_t n = 0, last = 0, m0, t0, b0, wr = __ldg(pr), wq = __ldg(pq);
+    sa_masks32(pr, pq, sr, sq, wr, wq, m0, t0, b0);
     for (uint32_t c = 0; c + 1 - last <= a.gap; c += 32) {
         uint32_t m1, t1, b1;
-        sa_masks32(a.ref, U.q_packed, rl, ql, (int)c, m1, t1, b1);
+        pr += 4;
+        pq += 4;
+        sa_masks32(pr, pq, sr, sq, wr, wq, m1, t1, b1);
         if ((m0 & m1) == ~0u && !(b0 | b1) && last == c && c + 32 <= ahead && stop_r >= c + 64 &&
             ((j + c) & (SA_CHAIN_BLOCK - 1)) + 32 < SA_CHAIN_BLOCK && sa_sweep_margin(a, U, rl + c + 1, ql + c + 1) &&
             sa_sweep_margin(a, U, rl + c + 32, ql + c + 32)) {
@@ -667,22 +676,22 @@ __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaPar
     return {tiles, n};
 }
 
-// Where a scan of the fast form stops, to the base: w = (step start / 8) << 16
-// | (best - score there), from the stopping step (sa_stop_word).  sr, sq: the
-// scan's first bases in R and Q; SH: log2 of the table's score scale.
-__device__ __forceinline__ uint32_t sa_stop_word(uint32_t o, int depth) {
-    return (min(o >> 3, 0xffffu) << 16) | (uint32_t)depth;
-}
-
+// Where a scan of the fast form stops, to the base, from offset o where best -
+// score is `depth` on.  sr, sq: the scan's first bases in R and Q; SH: log2 of the
+// table's score scale.
 template <int SH>
 __device__ __forceinline__ uint32_t sa_stop_offset(const char* tblb, const uint32_t* __restrict__ R,
                                                 const uint32_t* __restrict__ Q, uint32_t sr, uint32_t sq,
-                                                uint32_t avail, int xdrop, uint32_t w) {
-    // a step that starts past the word's range: from the scan's start
-    uint32_t o = (w >> 16) == 0xffffu ? 0u : (w >> 16) * 8;
-    int S = (w >> 16) == 0xffffu ? 0 : -(int)(w & 0xffffu), best = 0;
+                                                uint32_t avail, int xdrop, uint32_t o, uint32_t depth) {
+    int S = -(int)depth, best = 0;
+    const uint32_t* __restrict__ pr = R + (sr >> 3) + (o >> 3);  // o is a multiple of 8
+    const uint32_t* __restrict__ pq = Q + (sq >> 3) + (o >> 3);
+    uint32_t r0 = __ldg(pr), q0 = __ldg(pq);
     while (true) {
-        const uint32_t rw = sa_load8(R, (int64_t)sr + o), qw = sa_load8(Q, (int64_t)sq + o);
+        const uint32_t r1 = __ldg(++pr), q1 = __ldg(++pq);
+        const uint32_t rw = __funnelshift_r(r0, r1, (sr & 7u) * 4u), qw = __funnelshift_r(q0, q1, (sq & 7u) * 4u);
+        r0 = r1;
+        q0 = q1;
         uint32_t lo, hi;
         sa_merge8(rw, qw, lo, hi);
 #pragma unroll
@@ -696,23 +705,43 @@ __device__ __forceinline__ uint32_t sa_stop_offset(const char* tblb, const uint3
     }
 }
 
-// Shared memory of the lane kernel: score table, the 8 warps' rings of
-// candidate HSPs, per thread the stop words of its current hit, then per warp
-// `tile` hit records and the tile's E window (relative to the tile's first hit).
-struct SaLaneSmem {
-    int tbl[64];
-    uint4 em[8][64];       // {ref_start, query_start (before the rm flip), len, scope}
-    uint2 ex[8][64];       // {total, unit}
-    uint32_t stop[2][256];
-    uint32_t left[2][256]; // list hits: what the sweep left of the left direction
-};
-
-// A tile of the list holds half as many hits, of two 16-byte words each.
-__host__ __device__ __forceinline__ uint32_t sa_list_tile(uint32_t tile) { return tile / 2 < 32 ? 32 : tile / 2; }
-
-static size_t sa_lane_smem(uint32_t tile, bool list) {
-    return sizeof(SaLaneSmem) + 8 * (size_t)(list ? sa_list_tile(tile) * 2 * sizeof(uint4)
-                                                  : tile * (sizeof(uint4) + sizeof(uint32_t)));
+// Keep test of one candidate HSP per lane (total >= hspthresh): entropy factor
+// from the per-base match counts over the HSP when the total is in the entropy
+// range (src/seed_filter.cu:580-621), then insertion of the kept ones into the
+// call's set of distinct HSPs (rm: query start flipped on the reverse strand,
+// repeat_masker_src/seed_filter.cu:704-707).  r: {ref_start, query_start (before
+// the rm flip), len, scope}; the candidate counts as `hits` survivors.  Called
+// by the whole warp.
+__device__ __forceinline__ void sa_keep_candidates(const SaExtK& a, bool on, uint4 r, int total, uint32_t unit,
+                                                   uint32_t hits) {
+    const int lane = threadIdx.x & 31;
+    int keep = 0, score = 0;
+    bool known = false;
+    uint32_t qs = 0;
+    if (on) {
+        const SaUnit U = a.units[unit];
+        const int ext = (int)r.z;
+        qs = r.y;
+        if (U.flags & 2u) qs = a.ref_len - 1 - (qs + r.z);
+        // A candidate whose key the set already holds was kept with this same
+        // key (the scope fixes the unit, so the same bases): it is a survivor,
+        // and its match counts, logs and insertion are skipped.
+        known = sa_hash_contains(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z);
+        if (known) {
+            keep = 1;
+        } else {
+            int cnt[4] = {0, 0, 0, 0};
+            const bool eb = sa_entropy_branch(a, total);
+            if (eb) sa_count_matches_span(a.ref, r.x, U.q_packed, r.y, (int64_t)ext + 1, cnt);
+            sa_keep_score(total, ext, cnt, eb, a.hspthresh, &keep, &score);
+        }
+    }
+    const uint32_t kept = __reduce_add_sync(SA_FULL, keep ? hits : 0u);
+    if (lane == 0 && kept) atomicAdd(&a.ctr->surv_count, (unsigned long long)kept);
+    unsigned long long claimed = ~0ull;
+    if (keep && !known)
+        claimed = sa_hash_insert(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z, score, &a.ctr->hash_overflow);
+    sa_hash_note_used(a.hset, &a.ctr->hash_used, claimed);
 }
 
 // Keep test of `n` (<= 32) ring candidates from slot `head` on, one per lane:
@@ -733,45 +762,15 @@ __device__ __forceinline__ void sa_flush_candidates(const SaExtK& a, const uint4
         x = s_ex[slot];
     }
     __syncwarp();  // slots are rewritten by later appends
-    int keep = 0, score = 0;
-    bool known = false;
-    uint32_t qs = 0;
-    if (on) {
-        const SaUnit U = a.units[x.y];
-        const int total = (int)x.x, ext = (int)r.z;
-        qs = r.y;
-        if (U.flags & 2u) qs = a.ref_len - 1 - (qs + r.z);
-        // A candidate whose key the set already holds was kept with this same
-        // key (the scope fixes the unit, so the same bases): it is a survivor,
-        // and its match counts, logs and insertion are skipped.
-        known = sa_hash_contains(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z);
-        if (known) {
-            keep = 1;
-        } else {
-            int cnt[4] = {0, 0, 0, 0};
-            const bool eb = sa_entropy_branch(a, total);
-            if (eb) sa_count_matches_span(a.ref, r.x, U.q_packed, r.y, (int64_t)ext + 1, cnt);
-            sa_keep_score(total, ext, cnt, eb, a.hspthresh, &keep, &score);
-        }
-    }
-    const uint32_t km = __ballot_sync(SA_FULL, keep != 0);
-    if (lane == 0 && km) atomicAdd(&a.ctr->surv_count, (unsigned long long)__popc(km));
-    unsigned long long claimed = ~0ull;
-    if (keep && !known)
-        claimed = sa_hash_insert(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z, score, &a.ctr->hash_overflow);
-    sa_hash_note_used(a.hset, &a.ctr->hash_used, claimed);
+    sa_keep_candidates(a, on, r, (int)x.x, x.y, 1);
 }
 
-// A list this short leaves most lanes without a hit, and a long scan's lane
-// steps are the call's critical path: hits past SA_FEW_CAP bases go to the warp
-// kernel, whose warps would idle too (lane + warp kernel at caps of 8192 and 128,
-// ms: 11 long hits 0.083 and 0.049, 785 0.152 and 0.082, 12 K 0.455 and 0.209).
-// A call with more keeps the tuning's cap: a warp per hit of a few hundred bases
-// costs more than a lane (120 K long hits: 0.35 and 0.74 ms).
-#define SA_FEW_HITS 32768u
-#define SA_FEW_CAP 128u
-// LIST: the hits come from the sweep's list; else from the compacted seeds.
-template <int MIN_CTAS, int STEP, bool EXACT, bool LIST>
+// Dynamic shared memory of the lane kernel for `tile` hits per warp tile.
+static size_t sa_lane_smem(uint32_t tile) {
+    return SA_LANE_TABLES + 8 * (size_t)tile * 16 + 8 * (size_t)(tile + 1) * 8 + 8 * 64 * 16 + 8 * 64 * 8;
+}
+
+template <int MIN_CTAS, int STEP, bool EXACT>
 __global__ void __launch_bounds__(256, MIN_CTAS)
 sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
     constexpr int NW = STEP / 8;                  // 8-base windows per step
@@ -784,25 +783,26 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     // tile E window, and a 64-entry ring of candidate HSPs awaiting the keep
     // test and insertion.
     extern __shared__ __align__(16) unsigned char sa_smem[];
-    SaLaneSmem& L = *reinterpret_cast<SaLaneSmem*>(sa_smem);
-    const uint32_t TILE = LIST ? sa_list_tile(a.tile_hits) : a.tile_hits;
+    const uint32_t TILE = a.tile_hits;
     // entry (q << 3) | r: target code r vs query code q.  Codes 0..3 use
     // entries 0..27 only, one per bank: lookups of A/C/G/T pairs never conflict.
-    int* const tbl = L.tbl;
+    int* tbl = reinterpret_cast<int*>(sa_smem);
     if (threadIdx.x < 64) {
         const int sc = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
         tbl[threadIdx.x] = EXACT ? sc : sc * SCALE - 1;
     }
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
-    if (a.ctr->error || (LIST && a.ctr->list_count > a.list_cap)) return;
+    if (a.ctr->error) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t lt = sa_lanemask_lt();
-    const uint32_t lane_cap = LIST && a.ctr->list_count <= SA_FEW_HITS ? min(a.lane_cap, SA_FEW_CAP) : a.lane_cap;
-    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + sizeof(SaLaneSmem)) + wid * (LIST ? 2 * TILE : TILE);
-    uint32_t* const s_E = reinterpret_cast<uint32_t*>(sa_smem + sizeof(SaLaneSmem) + 128 * (size_t)TILE) + wid * TILE;
-    uint4* const s_em = L.em[wid];
-    uint2* const s_ex = L.ex[wid];
+    uint4* const s_hits = reinterpret_cast<uint4*>(sa_smem + SA_LANE_TABLES) + wid * TILE;
+    unsigned long long* const s_E =
+        reinterpret_cast<unsigned long long*>(sa_smem + SA_LANE_TABLES + 128 * (size_t)TILE) + wid * (TILE + 1);
+    unsigned char* const em_base = sa_smem + SA_LANE_TABLES + 128 * (size_t)TILE + 64 * (size_t)(TILE + 1);
+    uint4* const s_em = reinterpret_cast<uint4*>(em_base) + wid * 64;
+    uint2* const s_ex = reinterpret_cast<uint2*>(em_base + 8 * 64 * 16) + wid * 64;
+
     // H, nnz, ref_len, seed_size and xdrop are read where used (registers
     // are the lane kernel's limit)
     const uint32_t* __restrict__ ref = a.ref;
@@ -830,15 +830,14 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     // Start of a direction of the current hit (dir 0: right of the hit; 1:
     // left, read rightwards in the reversed copies): offsets, bases
     // available, word shifts and the first NW + 1 words of both sequences.
-    // LIST: from where the sweep left off (w: its word, first: offset of best).
-    auto begin_dir = [&](const uint32_t* __restrict__ qp, uint32_t qlen, uint32_t from, uint32_t w, uint32_t first) {
+    auto begin_dir = [&](const uint32_t* __restrict__ qp, uint32_t qlen) {
         const uint32_t ref_len = a.ref_len;
         const uint32_t sr = dir ? ref_len - rl : rl, sq = dir ? qlen - ql : ql;
         avail = min(ref_len - sr, qlen - sq);
         sh_r = (sr & 7u) * 4u;
         sh_q = (sq & 7u) * 4u;
-        pr = (dir ? ref + sa_rev_words(ref_len) : ref) + (sr >> 3) + (from >> 3);
-        pq = (dir ? qp + sa_rev_words(qlen) : qp) + (sq >> 3) + (from >> 3);
+        pr = (dir ? ref + sa_rev_words(ref_len) : ref) + (sr >> 3);
+        pq = (dir ? qp + sa_rev_words(qlen) : qp) + (sq >> 3);
 #pragma unroll
         for (int j = 0; j <= NW; ++j) {
             w_r[j] = __ldg(pr + j);
@@ -846,25 +845,16 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         }
         pr += NW + 1;
         pq += NW + 1;
-        o = from;
-        best = (int)(w & 0xffffu);
-        S = best - (int)(w >> 16);
-        bpos = (int)first;
-    };
-    // The left direction of the current hit, as begin_dir takes it.
-    auto begin_left = [&](const uint32_t* __restrict__ qp, uint32_t qlen) {
-        if (!LIST) return begin_dir(qp, qlen, 0, 0, 0);
-        const uint32_t w = L.left[0][threadIdx.x], rest = L.left[1][threadIdx.x];
-        const bool anew = !(rest & SA_SWEPT_SEEN);
-        begin_dir(qp, qlen, anew ? 0u : SA_SWEEP_LEFT, anew ? 0u : w, anew ? 0u : (rest >> 8) & 0xffu);
+        o = 0;
+        S = 0;
+        best = 0;
+        bpos = 0;
     };
 
     while (true) {
         // ---- idle lanes take the next hits of the warp tile, in order ----
         const uint32_t idle = __ballot_sync(SA_FULL, !has);
         bool fresh = false;
-        bool finished = false, to_long = false;
-        uint4 swept = make_uint4(0, 0, 0, 0);
         if (idle && !(exhausted && tile_pos >= tile_n)) {
             if (tile_pos >= tile_n) {
                 // Take the next tile of hits and expand it: the hits of the
@@ -874,34 +864,28 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 unsigned long long t0 = 0;
                 if (lane == 0) t0 = atomicAdd(&a.ctr->hit_cursor, (unsigned long long)TILE);
                 t0 = __shfl_sync(SA_FULL, t0, 0);
-                const uint64_t H = LIST ? a.ctr->list_count : a.ctr->num_hits, nnz = a.ctr->nnz;
+                const uint64_t H = a.ctr->num_hits, nnz = a.ctr->nnz;
                 if (t0 >= H) {
                     exhausted = true;
                     tile_n = tile_pos = 0;
-                } else if (LIST) {
-                    tile_n = (uint32_t)min((unsigned long long)TILE, H - t0);
-                    tile_pos = 0;
-                    for (uint32_t i = lane; i < 2 * tile_n; i += 32) s_hits[i] = __ldcs(a.list + 2 * t0 + i);
-                    __syncwarp();
                 } else {
                     uint32_t n = (uint32_t)min((unsigned long long)TILE, H - t0);
                     const uint64_t c0 = sa_warp_find_seed(a.cs.E, nnz, t0);
                     const uint32_t nw = (uint32_t)min((uint64_t)n, nnz - c0);  // seeds of the window
-                    const uint32_t skip0 = (uint32_t)(t0 - a.cs.E[c0]);  // hits of the first seed before the tile
-                    for (uint32_t i = lane; i < nw; i += 32)
-                        s_E[i] = i ? (uint32_t)min(a.cs.E[c0 + i] - t0, 0xffffffffull) : 0u;
+                    for (uint32_t i = lane; i <= nw; i += 32) s_E[i] = a.cs.E[c0 + i];  // E[nnz] == H
                     __syncwarp();
                     // record of hit t0 + i: its seed by binary search in the E window
                     auto record = [&](uint32_t i) {
-                        uint32_t lo = 0, hi = nw;  // last k in [0, nw) with E[c0+k] <= t0 + i
+                        const unsigned long long h = t0 + i;
+                        uint32_t lo = 0, hi = nw;  // last k in [0, nw) with E[c0+k] <= h
                         while (hi - lo > 1) {
                             const uint32_t mid = (lo + hi) >> 1;
-                            if (s_E[mid] <= i) lo = mid;
+                            if (s_E[mid] <= h) lo = mid;
                             else hi = mid;
                         }
                         const uint64_t c = c0 + lo;
                         uint4 r;
-                        r.x = __ldg(a.pos_table + a.cs.lo[c] + (lo ? i - s_E[lo] : i + skip0)) + a.seed_size;  // find_hits :192
+                        r.x = __ldg(a.pos_table + a.cs.lo[c] + (uint32_t)(h - s_E[lo])) + a.seed_size;  // find_hits :192
                         r.y = a.cs.qpos[c] + a.seed_size;                                                 // find_hits :176
                         r.z = a.cs.scope[c];
                         r.w = a.cs.unit[c];
@@ -940,8 +924,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 const uint32_t m = min((uint32_t)__popc(idle), tile_n - tile_pos);
                 const uint32_t rank = __popc(idle & lt);
                 if (!has && rank < m) {
-                    const uint4 r = s_hits[(tile_pos + rank) * (LIST ? 2 : 1)];
-                    if (LIST) swept = s_hits[2 * (tile_pos + rank) + 1];
+                    const uint4 r = s_hits[tile_pos + rank];
                     rl = r.x;
                     ql = r.y;
                     scope = r.z;
@@ -955,45 +938,29 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         // ---- start of a direction: a fresh hit (right), or the left side of
         // the current hit after its right end ----
         if (fresh || setup) {
-            const SaUnit U = a.units[unit_id & ~SA_CHAIN_NEXT];
+            const SaUnit U = a.units[unit_id];
             if (fresh) {
+                // rm: hits outside [ref_start, ref_end] are never extended
+                // (repeat_masker_src/seed_filter.cu:237-243, 304-333).
+                bool skip = (U.flags & 1u) && !(rl >= U.rm_lo && rl <= U.rm_hi);
                 // Coordinates past either sequence end (a caller-supplied table or
                 // seed beyond the sequences) are rejected, not read.
                 if (rl > a.ref_len || ql > U.q_len) {
                     atomicCAS(&a.ctr->error, 0ull, 5ull);
-                } else {
+                    skip = true;
+                }
+                if (!skip) {
                     has = true;
                     nocap = false;
                     setup = true;
                     dir = 0;
                     tiles = 0;
-                    if (!LIST) ++ext_acc;  // else counted by the sweep
-                    if (LIST) {
-                        if (!(swept.z & SA_SWEPT_SEEN)) swept.x = swept.z = 0;
-                        L.left[0][threadIdx.x] = swept.y;
-                        L.left[1][threadIdx.x] = swept.z;
-                        if (swept.z) {
-                            if (swept.z & SA_SWEPT_STOP_L) tiles = (swept.z & SA_SWEPT_TILE_2) ? 2 : 1;
-                            L.stop[0][threadIdx.x] = L.stop[1][threadIdx.x] = 0;  // stops the sweep saw: from the scan's start
-                            if (swept.z & SA_SWEPT_STOP_R) {
-                                ++tiles;
-                                Rbest = (int)(swept.x & 0xffffu);
-                                Rpos = Rbest > 0 ? (int)(swept.z & 0xffu) : -1;
-                                dir = 1;
-                                if (swept.z & SA_SWEPT_STOP_L) {  // a candidate as it is
-                                    setup = false;
-                                    finished = true;
-                                }
-                            }
-                        }
-                    }
+                    ++ext_acc;
                 }
             }
             if (setup) {
                 setup = false;
-                if (dir) begin_left(U.q_packed, U.q_len);
-                else begin_dir(U.q_packed, U.q_len, LIST && swept.z ? SA_SWEEP_RIGHT : 0u, LIST ? swept.x : 0u,
-                               LIST ? swept.z & 0xffu : 0u);
+                begin_dir(U.q_packed, U.q_len);
             }
         }
         const bool done = !__any_sync(SA_FULL, has) && exhausted && tile_pos >= tile_n;
@@ -1001,18 +968,8 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         // ---- up to `substeps` STEP-base steps per busy lane: the lanes still
         // scanning go on while any lane of the warp does; a lane stops for
         // this iteration when its direction ends or it goes to the long queue ----
+        bool finished = false, to_long = false;
         int Lpos = 0, total = 0;
-        auto finish_hit = [&]() {
-            if (LIST && (L.left[1][threadIdx.x] & SA_SWEPT_STOP_L)) {  // the sweep saw the left scan stop
-                best = (int)(L.left[0][threadIdx.x] & 0xffffu);
-                bpos = (int)((L.left[1][threadIdx.x] >> 8) & 0xffu);
-            }
-            Lpos = best > 0 ? bpos + 1 : 0;  // left offsets are 1-based
-            total = Rbest + best;
-            tiles_acc += tiles;
-            has = false;
-        };
-        if (LIST && finished) finish_hit();
         bool scanning = has;
 #pragma unroll 1
         for (uint32_t sub = 0; sub < a.substeps; ++sub) {
@@ -1035,7 +992,6 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 pq += NW;
                 const bool edge = o + STEP > avail;
                 bool stop = false;
-                int depth = 0;
                 uint32_t lo, hi;
                 if (EXACT) {
                     bool alive = true;
@@ -1060,8 +1016,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                     // B - min > SCALE * xdrop + STEP  <=>  (B >> SH) - (min >> SH) > xdrop, because
                     // the low parts of B (0..STEP) and min (0..STEP-1) differ by less than SCALE
                     const uint32_t T = (uint32_t)a.xdrop * SCALE + STEP;
-                    depth = best - S;
-                    int Pk = STEP - (depth << SH), B = STEP, at = 0;
+                    int Pk = ((S - best) << SH) + STEP, B = STEP, at = 0;
                     if (!edge) {
     #pragma unroll
                         for (int j = 0; j < NW; ++j) {
@@ -1087,25 +1042,28 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                     // Steps start at multiples of STEP (8, 16 or 32), so the stop offset
                     // lies in 32-base tile o >> 5 whichever base of the step it is.
                     tiles += (o >> 5) + 1;
-                    if (LIST) L.stop[dir][threadIdx.x] = sa_stop_word(o, depth);
                     if (dir == 0) {
                         Rbest = best;
                         Rpos = best > 0 ? bpos : -1;  // -1 when no positive score
                         dir = 1;
-                        if (LIST && (L.left[1][threadIdx.x] & SA_SWEPT_STOP_L)) finished = true;
-                        else setup = true;
+                        setup = true;
                     } else {
                         finished = true;
                     }
                     scanning = false;
                 } else {
                     o += STEP;
-                    if (o >= lane_cap && !nocap) {
+                    if (o >= a.lane_cap && !nocap) {
                         to_long = true;
                         scanning = false;
                     }
                 }
-                if (finished) finish_hit();
+                if (finished) {
+                    Lpos = best > 0 ? bpos + 1 : 0;  // left offsets are 1-based
+                    total = Rbest + best;
+                    tiles_acc += tiles;
+                    has = false;
+                }
             }
             // switch_now: a lane whose right side ended in this step starts
             // its left side at once and scans in the iteration's remaining
@@ -1113,8 +1071,8 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
             if (a.switch_now && sub + 1 < a.substeps && __any_sync(SA_FULL, setup)) {
                 if (setup) {
                     setup = false;
-                    const SaUnit U = a.units[unit_id & ~SA_CHAIN_NEXT];
-                    begin_left(U.q_packed, U.q_len);
+                    const SaUnit U = a.units[unit_id];
+                    begin_dir(U.q_packed, U.q_len);
                     scanning = true;
                 }
             }
@@ -1154,7 +1112,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 const uint32_t slot = (em_tail + __popc(em & lt)) & 63u;
                 // {ref_start, query_start (before the rm flip), len, scope}, {total, unit} (:606-608)
                 s_em[slot] = make_uint4(rl - (uint32_t)Lpos, ql - (uint32_t)Lpos, (uint32_t)(Rpos + Lpos), scope);
-                s_ex[slot] = make_uint2((uint32_t)total, unit_id & ~SA_CHAIN_NEXT);
+                s_ex[slot] = make_uint2((uint32_t)total, unit_id);
             }
             em_tail += __popc(em);
             // full batches of 32; at the end, whatever is left
@@ -1163,24 +1121,6 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 __syncwarp();
                 sa_flush_candidates(a, s_em, s_ex, em_head, n);
                 em_head += n;
-            }
-        }
-        // ---- hits that may stand for the dropped ones after them ----
-        if (LIST) {
-            const bool leads = finished && (unit_id & SA_CHAIN_NEXT);
-            const uint32_t cm = __ballot_sync(SA_FULL, leads);
-            if (cm) {
-                const int leader = __ffs(cm) - 1;
-                unsigned long long at = 0;
-                if (lane == leader) at = atomicAdd(&a.ctr->chain_count, (unsigned long long)__popc(cm));
-                at = __shfl_sync(SA_FULL, at, leader) + __popc(cm & lt);
-                if (leads) {  // at most one per list record
-                    const uint32_t high = (int)(float)total >= a.hspthresh ? SA_CHAIN_HIGH : 0u;
-                    a.lead[at] = make_uint4(rl, ql, (unit_id & ~SA_CHAIN_NEXT) | high, (uint32_t)Lpos);
-                    a.lead_right[at] = (uint32_t)Rpos;
-                    a.lead_stop_r[at] = L.stop[0][threadIdx.x];
-                    a.lead_stop_l[at] = L.stop[1][threadIdx.x];
-                }
             }
         }
         if (done) break;
@@ -1198,58 +1138,327 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     }
 }
 
-// Chains, second half: one thread per scanned hit that others may follow
-// counts the dropped ones after it.  They are survivors if its HSP was kept,
-// that is, if the set holds it (the lane kernel has filled the set).
-// SH: log2 of the lane kernel's score scale (sa_stop_offset's table).
-template <int SH>
-__global__ void __launch_bounds__(256)
-sa_k_chain_walk(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
+// ---------------------------------------------------------------------------
+// The scans of listed hits, from where the sweep left off; left sides are read
+// rightwards in the reversed copies.  A warp takes a batch of records and one of
+// their sides; a lane scans one hit's side, STEP bases per step in the fast form,
+// writes the result for sa_k_finish and takes the next of the batch.
+//
+// Bound by instruction issue.  With one side and no keep test a lane's state fits
+// 64 registers (4 CTAs per SM), and a hand-out is the only thing between steps:
+// the lane kernel, which took both sides and the keep test, spent half of its
+// instructions around the steps.  Scans, chains and keep tests of 2.5 Mbp at
+// 1-in-500 differences, us: lane kernel and a kernel for the chains 1674, now
+// 1510 (scans 807); of a 1 Mbp call 203 -> 175.  A launch per side left two tails (248 -> 353 us
+// where scans are long).  Batches shrink on short lists so that all warps have some.
+// ---------------------------------------------------------------------------
+#define SA_SCAN_BATCH 64
+#define SA_LONG_NONE 0xffffffffu  // unit of a queue entry for a hit that is in the queue already
+
+// A list this short leaves most lanes without a hit, and a long scan's lane
+// steps are the call's critical path: hits past SA_FEW_CAP bases go to the warp
+// kernel, whose warps would idle too (lane + warp kernel at caps of 8192 and 128,
+// ms: 11 long hits 0.083 and 0.049, 785 0.152 and 0.082, 12 K 0.455 and 0.209).
+// A call with more keeps the tuning's cap: a warp per hit of a few hundred bases
+// costs more than a lane (120 K long hits: 0.35 and 0.74 ms).
+#define SA_FEW_HITS 32768u
+#define SA_FEW_CAP 128u
+
+template <int STEP>
+__global__ void __launch_bounds__(256, 4)
+sa_k_scan(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
+    constexpr int NW = STEP / 8, SCALE = 2 * STEP, SH = STEP == 8 ? 4 : STEP == 16 ? 5 : 6;
     __shared__ int tbl[64];
+    __shared__ uint4 s_hit[8][SA_SCAN_BATCH];   // {rl, ql, unit, swept word}
+    __shared__ uint2 s_rest[8][SA_SCAN_BATCH];  // {swept rest, list index}
+    if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] * SCALE - 1;
+    __syncthreads();
+    const char* tblb = reinterpret_cast<const char*>(tbl);
+    SaCounters* const ctr = a.ctr;
+    const unsigned long long n_list = ctr->list_count;
+    if (ctr->error || n_list > a.list_cap) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t lt = sa_lanemask_lt();
+    const uint32_t lane_cap = n_list <= SA_FEW_HITS ? min(a.lane_cap, SA_FEW_CAP) : a.lane_cap;
+    const unsigned long long warps = gridDim.x * 8ull;
+    const uint32_t q = (uint32_t)min((unsigned long long)SA_SCAN_BATCH, max(8ull, (2 * n_list + warps - 1) / warps));
+    uint32_t batch_pos = 0, batch_n = 0;
+    bool exhausted = false;
+    // the lane's scan: place in `scanned`, offset, bases available, word shifts, words of the coming step, next addresses
+    bool has = false, nocap = false;
+    uint32_t idx = 0, o = 0, avail = 0, sh_r = 0, sh_q = 0, w_r[NW + 1], w_q[NW + 1];
+#pragma unroll
+    for (int j = 0; j <= NW; ++j) w_r[j] = w_q[j] = 0;
+    const uint32_t* __restrict__ pr = a.ref;
+    const uint32_t* __restrict__ pq = a.ref;
+    int S = 0, best = 0, bpos = -1;
+    while (true) {
+        const uint32_t idle = __ballot_sync(SA_FULL, !has);
+        if (idle) {
+            while (batch_pos >= batch_n && !exhausted) {
+                // the next q list records' hits that need this side
+                unsigned long long t0 = 0;
+                if (lane == 0) t0 = atomicAdd(&ctr->scan_cursor, 1ull);
+                t0 = __shfl_sync(SA_FULL, t0, 0);
+                const uint32_t side = t0 & 1u;
+                t0 = (t0 >> 1) * q;
+                batch_pos = batch_n = 0;
+                if (t0 >= n_list) {
+                    exhausted = true;
+                    break;
+                }
+#pragma unroll
+                for (int k = 0; k < SA_SCAN_BATCH / 32; ++k) {
+                    const unsigned long long i = t0 + 32 * k + lane;
+                    uint4 h = make_uint4(0, 0, 0, 0), x = h;
+                    bool need = false;
+                    if (32 * k + lane < q && i < n_list) {
+                        h = a.list[2 * i];
+                        x = a.list[2 * i + 1];
+                        need = !(x.z & (side ? SA_SWEPT_STOP_L | SA_SWEPT_LONG : SA_SWEPT_STOP_R | SA_SWEPT_LONG));
+                    }
+                    const uint32_t m = __ballot_sync(SA_FULL, need);
+                    if (need) {
+                        const uint32_t at = batch_n + __popc(m & lt);
+                        s_hit[wid][at] = make_uint4(h.x, h.y, h.w & ~SA_CHAIN_NEXT, side ? x.y : x.x);
+                        s_rest[wid][at] = make_uint2(x.z, 2 * (uint32_t)i + side);
+                    }
+                    batch_n += __popc(m);
+                }
+                __syncwarp();
+            }
+            const uint32_t m = min((uint32_t)__popc(idle), batch_n - batch_pos), rank = __popc(idle & lt);
+            if (!has && rank < m) {
+                const uint4 h = s_hit[wid][batch_pos + rank];
+                const uint2 x = s_rest[wid][batch_pos + rank];
+                const SaUnit U = a.units[h.z];
+                const uint32_t ref_len = a.ref_len;
+                const bool seen = x.x & SA_SWEPT_SEEN;
+                idx = x.y;
+                const uint32_t side = x.y & 1u;
+                const uint32_t sr = side ? ref_len - h.x : h.x, sq = side ? U.q_len - h.y : h.y;
+                o = seen ? (side ? SA_SWEEP_LEFT : SA_SWEEP_RIGHT) : 0u;
+                best = seen ? (int)(h.w & 0xffffu) : 0;
+                S = seen ? best - (int)(h.w >> 16) : 0;
+                bpos = best ? (int)((x.x >> (side ? 8 : 0)) & 0xffu) : -1;
+                avail = min(ref_len - sr, U.q_len - sq);
+                sh_r = (sr & 7u) * 4u;
+                sh_q = (sq & 7u) * 4u;
+                pr = (side ? a.ref + sa_rev_words(ref_len) : a.ref) + (sr >> 3) + (o >> 3);
+                pq = (side ? U.q_packed + sa_rev_words(U.q_len) : U.q_packed) + (sq >> 3) + (o >> 3);
+#pragma unroll
+                for (int j = 0; j <= NW; ++j) {
+                    w_r[j] = __ldg(pr + j);
+                    w_q[j] = __ldg(pq + j);
+                }
+                pr += NW + 1;
+                pq += NW + 1;
+                has = true;
+                nocap = false;
+            }
+            batch_pos += m;
+        }
+        if (!__any_sync(SA_FULL, has)) break;
+        bool to_long = false;
+#pragma unroll 1
+        for (uint32_t sub = 0; sub < a.substeps; ++sub) {
+            if (has && !to_long) {
+                uint32_t rwin[NW], qwin[NW];
+#pragma unroll
+                for (int j = 0; j < NW; ++j) {
+                    rwin[j] = __funnelshift_r(w_r[j], w_r[j + 1], sh_r);
+                    qwin[j] = __funnelshift_r(w_q[j], w_q[j + 1], sh_q);
+                }
+                w_r[0] = w_r[NW];
+                w_q[0] = w_q[NW];
+#pragma unroll
+                for (int j = 1; j <= NW; ++j) {
+                    w_r[j] = __ldg(pr + j - 1);
+                    w_q[j] = __ldg(pq + j - 1);
+                }
+                pr += NW;
+                pq += NW;
+                // the lane kernel's fast form
+                const uint32_t T = (uint32_t)a.xdrop * SCALE + STEP;
+                const int depth = best - S;
+                int Pk = STEP - (depth << SH), B = STEP, at = 0;
+                bool stop = false;
+                uint32_t lo, hi;
+                if (o + STEP <= avail) {
+#pragma unroll
+                    for (int j = 0; j < NW; ++j) {
+                        sa_merge8(rwin[j], qwin[j], lo, hi);
+                        sa_window_fast<false>(tblb, lo, hi, o + 8 * j, avail, 0, T, Pk, B, at, stop);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < NW; ++j) {
+                        sa_merge8(rwin[j], qwin[j], lo, hi);
+                        sa_window_fast<true>(tblb, lo, hi, o + 8 * j, avail, -(a.xdrop + 1) * SCALE - 1, T, Pk, B, at,
+                                             stop);
+                    }
+                }
+                const int low = at & (SCALE - 1);
+                if (low != STEP) bpos = (int)o + (STEP - 1 - low);
+                S = best + (Pk >> SH);  // exact after a full step without a stop
+                best += at >> SH;
+                if (stop) {
+                    a.scanned[idx] = make_uint4((uint32_t)best, (uint32_t)bpos, o, (uint32_t)depth);
+                    has = false;
+                } else {
+                    o += STEP;
+                    to_long = o >= lane_cap && !nocap;
+                }
+            }
+            if (sub + 1 < a.substeps && !__any_sync(SA_FULL, has && !to_long)) break;
+        }
+        const uint32_t lm = __ballot_sync(SA_FULL, to_long);
+        if (lm) {
+            unsigned long long base = 0;
+            const int leader = __ffs(lm) - 1;
+            if (lane == leader) base = atomicAdd(&ctr->long_count, (unsigned long long)__popc(lm));
+            base = __shfl_sync(SA_FULL, base, leader) + __popc(lm & lt);
+            if (to_long) {
+                if (base < a.long_cap) {
+                    uint4* const rec = a.list + (idx & ~1u);
+                    const uint4 h = rec[0];
+                    SaLongHit e;
+                    e.ref_loc = h.x;
+                    e.query_loc = h.y;
+                    e.unit = atomicOr(&rec[1].z, SA_SWEPT_LONG) & SA_SWEPT_LONG ? SA_LONG_NONE : h.w;  // once per hit
+                    e.scope = h.z;
+                    a.long_q[base] = e;
+                    has = false;
+                } else {
+                    nocap = true;  // queue full: finish this hit in the lane
+                    atomicAdd(&ctr->long_overflow, 1ull);
+                }
+            }
+        }
+    }
+}
+
+// Listed hit i as the sweep and the scans left it.  All loads are issued at once
+// (`scanned` is stale for a side that the sweep finished, or never written).
+struct SaListed {
+    uint4 h, x, r, l;
+};
+
+__device__ __forceinline__ SaListed sa_listed(const SaExtK& a, unsigned long long i) {
+    return {a.list[2 * i], a.list[2 * i + 1], a.scanned[2 * i], a.scanned[2 * i + 1]};
+}
+
+// Its sides in e.r and e.l, also where the sweep stopped (told from offset 0 on), and their tiles.
+__device__ __forceinline__ uint32_t sa_listed_sides(SaListed& e) {
+    if (e.x.z & SA_SWEPT_STOP_R) e.r = make_uint4(e.x.x & 0xffffu, e.x.x & 0xffffu ? e.x.z & 0xffu : ~0u, 0, 0);
+    uint32_t tiles = (e.r.z >> 5) + 2;
+    if (e.x.z & SA_SWEPT_STOP_L) {
+        e.l = make_uint4(e.x.y & 0xffffu, e.x.y & 0xffffu ? (e.x.z >> 8) & 0xffu : ~0u, 0, 0);
+        return tiles + ((e.x.z & SA_SWEPT_TILE_2) ? 1 : 0);
+    }
+    return tiles + (e.l.z >> 5);
+}
+
+// Listed hits to HSPs: tiles; for a hit that others may follow the dropped ones
+// after it (sa_chain_members), which survive if its HSP is kept; and the keep
+// test.  A warp sorts its records into those that start chains and candidates,
+// and takes either 32 at a time: with a record per lane throughout the kernel
+// took 1.27 ms where this takes 0.70.  Of that the keep tests are 0.2, the chains
+// 0.2, and the rest is the pass over the records.
+#define SA_FINISH_RING 128
+__global__ void __launch_bounds__(256, 4)
+sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
+    constexpr int SH = 4;  // log2 of the score scale of sa_stop_offset's table
+    __shared__ int tbl[64];
+    __shared__ uint32_t s_lead[8][SA_FINISH_RING];
+    __shared__ uint2 s_cand[8][SA_FINISH_RING];  // {list index, survivors it stands for}
     if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SH) - 1;
     __syncthreads();
-    const SaCounters* __restrict__ ctr = a.ctr;
-    const unsigned long long n = ctr->chain_count;
-    if (ctr->error) return;
-    unsigned long long tiles = 0, kept = 0;
-    for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull) {
-        const uint4 h = a.lead[i];
-        const uint32_t unit = h.z & ~SA_CHAIN_HIGH;
-        const SaUnit U = a.units[unit];
-        const uint32_t rl = h.x, ql = h.y;
-        const char* tblb = reinterpret_cast<const char*>(tbl);
-        const uint32_t stop_r = sa_stop_offset<SH>(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql),
-                                                   a.xdrop, a.lead_stop_r[i]);
-        const uint32_t stop_l = sa_stop_offset<SH>(tblb, a.ref + sa_rev_words(a.ref_len), U.q_packed + sa_rev_words(U.q_len),
-                                                   a.ref_len - rl, U.q_len - ql, min(rl, ql), a.xdrop,
-                                                   a.lead_stop_l[i]);
-        const SaChain c = sa_chain_members(a, P, unit, rl, ql, stop_r, stop_l, h.z & SA_CHAIN_HIGH);
-        if (!c.n) continue;
-        tiles += c.tiles;
-        const uint32_t len = a.lead_right[i] + h.w;
-        uint32_t qs = ql - h.w;
-        if (U.flags & 2u) qs = a.ref_len - 1 - (qs + len);
-        // chains are of calls and units with one MAX_HITS iteration: scope (unit << 4) | 0, unit 0 in a call
-        if ((h.z & SA_CHAIN_HIGH) && sa_hash_holds(a.hset, ctr->hash_mask, unit << 4, rl - h.w, qs, len)) kept += c.n;
+    const char* tblb = reinterpret_cast<const char*>(tbl);
+    SaCounters* const ctr = a.ctr;
+    const unsigned long long n = ctr->list_count;
+    if (ctr->error || n > a.list_cap) return;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = sa_lanemask_lt();
+    uint32_t* const lead = s_lead[threadIdx.x >> 5];
+    uint2* const cand = s_cand[threadIdx.x >> 5];
+    uint32_t l0 = 0, l1 = 0, c0 = 0, c1 = 0;  // ring cursors
+    unsigned long long tiles = 0;
+    for (unsigned long long i0 = (blockIdx.x * 8ull + (threadIdx.x >> 5)) * 32;; i0 += gridDim.x * 256ull) {
+        const bool done = i0 >= n;
+        const unsigned long long i = i0 + lane;
+        bool leads = false, high = false;
+        if (i < n) {
+            SaListed e = sa_listed(a, i);
+            if (!(e.x.z & SA_SWEPT_LONG)) {
+                tiles += sa_listed_sides(e);
+                leads = e.h.w & SA_CHAIN_NEXT;
+                high = !leads && (int)(float)((int)e.r.x + (int)e.l.x) >= a.hspthresh;
+            }
+        }
+        const uint32_t lm = __ballot_sync(SA_FULL, leads), cm = __ballot_sync(SA_FULL, high);
+        if (leads) lead[(l1 + __popc(lm & lt)) % SA_FINISH_RING] = (uint32_t)i;
+        if (high) cand[(c1 + __popc(cm & lt)) % SA_FINISH_RING] = make_uint2((uint32_t)i, 1);
+        l1 += __popc(lm);
+        c1 += __popc(cm);
+        __syncwarp();
+        while (l1 - l0 >= 32 || (done && l1 != l0)) {
+            const bool on = lane < (int)(l1 - l0);
+            uint32_t k = 0, hits = 1;
+            high = false;
+            if (on) {
+                k = lead[(l0 + lane) % SA_FINISH_RING];
+                SaListed e = sa_listed(a, k);
+                sa_listed_sides(e);
+                const uint32_t rl = e.h.x, ql = e.h.y, unit = e.h.w & ~SA_CHAIN_NEXT;
+                const SaUnit U = a.units[unit];
+                const uint32_t stop_r = sa_stop_offset<SH>(tblb, a.ref, U.q_packed, rl, ql,
+                                                           min(a.ref_len - rl, U.q_len - ql), a.xdrop, e.r.z, e.r.w);
+                const uint32_t stop_l = sa_stop_offset<SH>(
+                    tblb, a.ref + sa_rev_words(a.ref_len), U.q_packed + sa_rev_words(U.q_len), a.ref_len - rl,
+                    U.q_len - ql, min(rl, ql), a.xdrop, e.l.z, e.l.w);
+                high = (int)(float)((int)e.r.x + (int)e.l.x) >= a.hspthresh;
+                const SaChain c = sa_chain_members(a, P, unit, rl, ql, stop_r, stop_l, high);
+                hits += c.n;
+                tiles += c.tiles;
+            }
+            l0 += min(l1 - l0, 32u);
+            const uint32_t m = __ballot_sync(SA_FULL, high);
+            if (high) cand[(c1 + __popc(m & lt)) % SA_FINISH_RING] = make_uint2(k, hits);
+            c1 += __popc(m);
+            __syncwarp();
+        }
+        while (c1 - c0 >= 32 || (done && c1 != c0)) {
+            const bool on = lane < (int)(c1 - c0);
+            uint4 seg = make_uint4(0, 0, 0, 0);
+            uint32_t unit = 0, hits = 0;
+            int total = 0;
+            if (on) {
+                const uint2 x = cand[(c0 + lane) % SA_FINISH_RING];
+                SaListed e = sa_listed(a, x.x);
+                sa_listed_sides(e);
+                const uint32_t left = e.l.y + 1;  // left offsets are 1-based, 0 when best is 0
+                seg = make_uint4(e.h.x - left, e.h.y - left, e.r.y + left, e.h.z);
+                total = (int)e.r.x + (int)e.l.x;
+                unit = e.h.w & ~SA_CHAIN_NEXT;
+                hits = x.y;
+            }
+            c0 += min(c1 - c0, 32u);
+            __syncwarp();
+            sa_keep_candidates(a, on, seg, total, unit, hits);
+        }
+        if (done) break;
     }
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        tiles += __shfl_xor_sync(SA_FULL, tiles, s);
-        kept += __shfl_xor_sync(SA_FULL, kept, s);
-    }
-    if ((threadIdx.x & 31) == 0 && tiles) {
-        atomicAdd(&a.ctr->base_steps, tiles);
-        if (kept) atomicAdd(&a.ctr->surv_count, kept);
-    }
+    for (int s = 16; s >= 1; s >>= 1) tiles += __shfl_xor_sync(SA_FULL, tiles, s);
+    if (lane == 0 && tiles) atomicAdd(&ctr->base_steps, tiles);
 }
 
 // Between the segments of a large batch: the list and the queue start again
 // (an overflow stays to be seen).
 __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
     if (ctr->list_count <= list_cap) ctr->list_count = 0;
-    ctr->hit_cursor = 0;
-    ctr->sweep_cursor = 0;
-    ctr->chain_count = 0;
+    ctr->sweep_cursor = ctr->scan_cursor = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1379,6 +1588,7 @@ sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
         if (idx >= nlong) break;
         if (lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);  // read while this hit is scanned
         const SaLongHit L = a.long_q[idx];
+        if (L.unit == SA_LONG_NONE) continue;
         const SaUnit U = a.units[L.unit & ~SA_CHAIN_NEXT];
         const uint32_t rl = L.ref_loc, ql = L.query_loc;
         const SaDirResult R = sa_warp_xdrop(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql), a.xdrop);
@@ -1444,7 +1654,7 @@ static bool sa_lane_fast_form(const SaParams& p, int step) {
     return x >= 0 && 7 * mx <= x && x * scale - low * step < (1ll << 31) && mx * scale * step < (1ll << 31);
 }
 
-// The sweep and the lane kernel after it use the fast form, and what passes
+// The sweep and the scans after it use the fast form, and what passes
 // between them fits its 16-bit fields.
 static bool sa_sweep_params(const SaParams& p, const SaTuning& t) {
     int mx = 0;
@@ -1475,10 +1685,7 @@ static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaParams& p, c
     // buffers of the dedup that are free until then
     a.list = reinterpret_cast<uint4*>(w.out);
     a.list_cap = x.sweep && sa_sweep_params(p, t) ? w.list_cap : 0;
-    a.lead = reinterpret_cast<uint4*>(w.rec[0]);
-    a.lead_right = w.scope[0];
-    a.lead_stop_r = w.scope[1];
-    a.lead_stop_l = w.out_scope;
+    a.scanned = reinterpret_cast<uint4*>(w.rec[0]);
     // the 48-base window of sa_chain_test holds the seeds of hits up to `gap` either way
     a.gap = (uint32_t)std::max(0, std::min({(int)SA_CHAIN_GAP, p.seed_size - 1, 32 - p.seed_size}));
     a.ref = x.ref;
@@ -1502,28 +1709,25 @@ static SaExtK sa_ext_args(SaWork& w, const SaExtendArgs& x, const SaParams& p, c
     return a;
 }
 
-template <int C, int STEP, bool EXACT, bool LIST>
+template <int C, int STEP, bool EXACT>
 static void sa_lane_launch(const SaExtK& a, const SaParams& p, int grid, size_t smem, cudaStream_t st) {
-    if (grid > 0) sa_k_extend_lane<C, STEP, EXACT, LIST><<<grid, 256, smem, st>>>(a, p);
-    else cudaFuncSetAttribute(sa_k_extend_lane<C, STEP, EXACT, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
-enum SaLaneForm { kLaneFast, kLaneExact, kLaneList };
-
-template <int C, int STEP>
-static void sa_lane_dispatch_form(const SaExtK& a, const SaParams& p, SaLaneForm form, int grid, size_t smem,
-                                  cudaStream_t st) {
-    if (form == kLaneList) sa_lane_launch<C, STEP, false, true>(a, p, grid, smem, st);
-    else if (form == kLaneExact) sa_lane_launch<C, STEP, true, false>(a, p, grid, smem, st);
-    else sa_lane_launch<C, STEP, false, false>(a, p, grid, smem, st);
+    if (grid > 0) sa_k_extend_lane<C, STEP, EXACT><<<grid, 256, smem, st>>>(a, p);
+    else cudaFuncSetAttribute(sa_k_extend_lane<C, STEP, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 template <int C>
-static void sa_lane_dispatch(const SaExtK& a, const SaParams& p, int step, SaLaneForm form, int grid, size_t smem,
+static void sa_lane_dispatch(const SaExtK& a, const SaParams& p, int step, bool exact, int grid, size_t smem,
                              cudaStream_t st) {
-    if (step == 32) sa_lane_dispatch_form<C, 32>(a, p, form, grid, smem, st);
-    else if (step == 16) sa_lane_dispatch_form<C, 16>(a, p, form, grid, smem, st);
-    else sa_lane_dispatch_form<C, 8>(a, p, form, grid, smem, st);
+    if (step == 32) {
+        if (exact) sa_lane_launch<C, 32, true>(a, p, grid, smem, st);
+        else sa_lane_launch<C, 32, false>(a, p, grid, smem, st);
+    } else if (step == 16) {
+        if (exact) sa_lane_launch<C, 16, true>(a, p, grid, smem, st);
+        else sa_lane_launch<C, 16, false>(a, p, grid, smem, st);
+    } else {
+        if (exact) sa_lane_launch<C, 8, true>(a, p, grid, smem, st);
+        else sa_lane_launch<C, 8, false>(a, p, grid, smem, st);
+    }
 }
 
 // Allows every lane-kernel instance the largest tile's shared memory, once
@@ -1536,49 +1740,55 @@ void sa_prepare_extend_lane(const SaParams& p, const SaTuning& t) {
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
     if (dev < 0 || dev >= 64 || done[dev]) return;
-    const size_t smem = sa_lane_smem(1024, false);
+    const size_t smem = sa_lane_smem(1024);
     SaExtK none{};
     for (int step : {8, 16, 32})
-        for (SaLaneForm form : {kLaneFast, kLaneExact, kLaneList}) {
-            sa_lane_dispatch<2>(none, p, step, form, 0, smem, 0);
-            sa_lane_dispatch<3>(none, p, step, form, 0, smem, 0);
-            sa_lane_dispatch<4>(none, p, step, form, 0, smem, 0);
+        for (bool exact : {false, true}) {
+            sa_lane_dispatch<2>(none, p, step, exact, 0, smem, 0);
+            sa_lane_dispatch<3>(none, p, step, exact, 0, smem, 0);
+            sa_lane_dispatch<4>(none, p, step, exact, 0, smem, 0);
         }
     done[dev] = true;
+}
+
+template <int STEP>
+static void sa_scan_launch(const SaExtK& a, const SaParams& p, int grid, cudaStream_t st) {
+    sa_k_scan<STEP><<<grid, 256, 0, st>>>(a, p);
+    sa_note_launch();
 }
 
 void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, const SaTuning& t, int num_sms,
                            cudaStream_t st, int grid_ctas) {
     sa_prepare_extend_lane(p, t);
-    // Register budget follows the CTAs per SM: 4 -> <= 64 registers, 3 -> <= 85, 2 -> <= 128.
     const SaExtK a = sa_ext_args(w, x, p, t);
-    const int grid = grid_ctas > 0 ? grid_ctas : num_sms * t.ext_ctas_per_sm;
-    const SaLaneForm form = a.list_cap ? kLaneList : sa_lane_fast_form(p, t.step_bases) ? kLaneFast : kLaneExact;
-    const size_t smem = sa_lane_smem(a.tile_hits, form == kLaneList);
+    if (!a.list_cap) {
+        // Register budget follows the CTAs per SM: 4 -> <= 64 registers, 3 -> <= 85, 2 -> <= 128.
+        const int grid = grid_ctas > 0 ? grid_ctas : num_sms * t.ext_ctas_per_sm;
+        const size_t smem = sa_lane_smem(a.tile_hits);
+        const bool exact = !sa_lane_fast_form(p, t.step_bases);
+        if (t.ext_ctas_per_sm >= 4) sa_lane_dispatch<4>(a, p, t.step_bases, exact, grid, smem, st);
+        else if (t.ext_ctas_per_sm == 3) sa_lane_dispatch<3>(a, p, t.step_bases, exact, grid, smem, st);
+        else sa_lane_dispatch<2>(a, p, t.step_bases, exact, grid, smem, st);
+        sa_note_launch();
+        return;
+    }
     // Segments of hits whose list is sure to fit in practice; one unless the
     // caller knows of more hits (x.hits).  A list that overflows all the same is
     // seen by the host (list_count), which runs the call again without the sweep.
-    const uint64_t seg = form == kLaneList ? 4 * a.list_cap & ~31ull : 0;
+    const uint64_t seg = 4 * a.list_cap & ~31ull;
+    const int grid = num_sms * 4;
     uint64_t h0 = 0;
     do {
-        const uint64_t h1 = form == kLaneList && x.hits > h0 + seg ? h0 + seg : ~0ull;
-        if (form == kLaneList) {
-            if (h0) sa_k_next_segment<<<1, 1, 0, st>>>(w.ctr, a.list_cap);
-            const int g = num_sms * 4;
-            if (p.transition) sa_k_sweep<true><<<g, 256, 0, st>>>(a, p, h0, h1);
-            else sa_k_sweep<false><<<g, 256, 0, st>>>(a, p, h0, h1);
-            sa_note_launch();
-        }
-        if (t.ext_ctas_per_sm >= 4) sa_lane_dispatch<4>(a, p, t.step_bases, form, grid, smem, st);
-        else if (t.ext_ctas_per_sm == 3) sa_lane_dispatch<3>(a, p, t.step_bases, form, grid, smem, st);
-        else sa_lane_dispatch<2>(a, p, t.step_bases, form, grid, smem, st);
+        const uint64_t h1 = x.hits > h0 + seg ? h0 + seg : ~0ull;
+        if (h0) sa_k_next_segment<<<1, 1, 0, st>>>(w.ctr, a.list_cap);
+        if (p.transition) sa_k_sweep<true><<<grid, 256, 0, st>>>(a, p, h0, h1);
+        else sa_k_sweep<false><<<grid, 256, 0, st>>>(a, p, h0, h1);
         sa_note_launch();
-        if (form == kLaneList && a.chain) {
-            if (t.step_bases == 32) sa_k_chain_walk<6><<<num_sms * 4, 256, 0, st>>>(a, p);
-            else if (t.step_bases == 16) sa_k_chain_walk<5><<<num_sms * 4, 256, 0, st>>>(a, p);
-            else sa_k_chain_walk<4><<<num_sms * 4, 256, 0, st>>>(a, p);
-            sa_note_launch();
-        }
+        if (t.step_bases == 32) sa_scan_launch<32>(a, p, grid, st);
+        else if (t.step_bases == 16) sa_scan_launch<16>(a, p, grid, st);
+        else sa_scan_launch<8>(a, p, grid, st);
+        sa_k_finish<<<grid, 256, 0, st>>>(a, p);
+        sa_note_launch();
         h0 = h1;
     } while (h0 != ~0ull);
 }

@@ -104,9 +104,9 @@ struct SaCounters {
     unsigned long long hash_used;      // slots claimed in the HSP set (entries of its used list)
     unsigned long long chain_bad;      // nonzero: the call's hits are not known to be every seed match of its windows
     unsigned long long windows;        // plain call: valid seed windows in [j_lo, j_hi)
-    unsigned long long list_count;     // hits the sweep left to the lane kernel (past the list's capacity: the call is run again without it)
-    unsigned long long chain_count;    // scanned hits that others may follow
+    unsigned long long list_count;     // hits the sweep left to the scans (past the list's capacity: the call is run again without it)
     unsigned long long sweep_cursor;   // sweep work counter
+    unsigned long long scan_cursor;    // scan work counter
 };
 
 // Open-addressing set of distinct HSPs of one call: slot = 16-byte key
@@ -189,22 +189,6 @@ __device__ __forceinline__ bool sa_hash_contains(const SaHashSet& hs, unsigned l
         asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(s0), "=l"(s1) : "l"(hs.keys + 2 * h));
         if (s0 == k0 && s1 == k1) return true;
         if (s0 == ~0ull || s1 == ~0ull) return false;
-        h = (h + 1) & mask;
-    }
-    return false;
-}
-
-// Whether the set holds the key, after the kernel that fills it: the search
-// goes as far as an insertion would.
-__device__ __forceinline__ bool sa_hash_holds(const SaHashSet& hs, unsigned long long mask, uint32_t scope,
-                                              uint32_t rs, uint32_t qs, uint32_t len) {
-    const unsigned long long k0 = ((unsigned long long)scope << 32) | rs;
-    const unsigned long long k1 = ((unsigned long long)qs << 32) | len;
-    unsigned long long h = sa_hash_mix(k0, k1) & mask;
-    for (int probe = 0; probe < SA_HASH_MAX_PROBES; ++probe) {
-        const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(hs.keys + 2 * h);
-        if (s.x == k0 && s.y == k1) return true;
-        if (s.x == ~0ull && s.y == ~0ull) return false;
         h = (h + 1) & mask;
     }
     return false;

@@ -101,7 +101,7 @@ struct SaWork {
     // survivors (ping-pong) and dedup output
     SaRec* rec[2];
     uint32_t* scope[2];
-    uint64_t list_cap;      // hits the sweep may leave to the lane kernel (a list in `out`), 0: no sweep
+    uint64_t list_cap;      // hits the sweep may leave to the scans (a list in `out`), 0: no sweep
     uint64_t surv_cap;
     SaHashSet hset;         // [2 * surv_cap] slots: distinct HSPs of the call; used list aliases rec[1]
     bool hash_clean;        // host: every slot of hset is empty (no full clear needed)
