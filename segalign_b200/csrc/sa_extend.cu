@@ -11,13 +11,17 @@
 //   best = max over o < stop, pos = first o reaching best (right: -1 if
 //   best == 0; left: 0).
 // This file computes the same quantities in two phases:
-//   phase A (sa_k_extend_lane): one hit per lane.  A warp keeps its 32 lanes
+//   phase A, for scores and steps that sa_sweep_params admits: sa_k_sweep scores
+//     the bases near every hit, which finishes the chance hits, and drops hits
+//     whose HSP another hit of the diagonal gives; sa_k_scan goes on with the
+//     others' sides; sa_k_finish counts and keeps.
+//   phase A, general form (sa_k_extend_lane): one hit per lane.  A warp keeps its 32 lanes
 //     busy by handing out the next hits of its tile, in order, to lanes that
 //     finish.  Hits are expanded on the fly from the compacted seed
 //     list.  The short random-hit extensions that dominate the hit count
 //     finish here in a few steps.
 //   phase B (sa_k_extend_warp): hits whose extension passes `lane_cap` bases in
-//     one direction move to a queue and are redone by one warp per hit,
+//     one direction move to a queue and are redone by a warp per side,
 //     256 bases per step.  Each lane scans 8 bases; warp scans carry the
 //     running sum and maximum.
 // Kept HSPs, with their dedup scope, go into the call's set of distinct HSPs
@@ -382,7 +386,7 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // loads in about 250 per round), with the ALU pipe and issue at 70%.  On a 2.5 Mbp query
 // against the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in
 // the lane kernel 5.65 ms; sweep 2.00, scans 0.81, finish 0.70: 3.33 ms, its launches
-// included (without chains 4.4).  The chain test on all hits as they were
+// included (with the lane kernel after the sweep 3.75, and 4.79 without chains).  The chain test on all hits as they were
 // scored, with the rounds split evenly over the warps, made the sweep 2.33 ms.
 // Lane phase of 24 Mbp: 55.0 -> 30.8 ms.
 // ---------------------------------------------------------------------------
@@ -673,6 +677,56 @@ __device__ __forceinline__ SaChain sa_chain_members(const SaExtK& a, const SaPar
         t0 = t1;
         b0 = b1;
     }
+    return {tiles, n};
+}
+
+// sa_chain_members by a warp, 32 bases per lane: whether a hit goes on with the
+// chain depends on the hit before it, at most a.gap (< 32) bases back, so a lane
+// needs the last one of the lane below only; and a chain ends with its block of
+// SA_CHAIN_BLOCK positions.  All lanes get the result.
+__device__ __forceinline__ SaChain sa_warp_chain_members(const SaExtK& a, const SaParams& P, uint32_t unit, uint32_t rl,
+                                                         uint32_t ql, uint32_t stop_r, uint32_t stop_l, bool high) {
+    static_assert(SA_CHAIN_BLOCK <= 32 * 32, "a chain fits the warp");
+    const SaUnit U = a.units[unit];
+    const int lane = threadIdx.x & 31;
+    const uint32_t S = a.seed_size, j = ql - S, c = 32 * lane;
+    uint32_t ahead = U.j_hi - 1 - j;
+    if (U.flags & 1u) ahead = min(ahead, U.rm_hi - rl);
+    uint32_t hits = 0, m0 = 0, m1 = 0, b0 = 0, b1 = 0;  // hits bit i - 1: a match ends c + i bases on
+    // a block that starts past either sequence's end holds no hit of the chain and is not read
+    if (c <= ahead && c <= a.ref_len - rl) {
+        const uint32_t sr = (rl & 7u) * 4u, sq = (ql & 7u) * 4u;
+        const uint32_t* __restrict__ pr = a.ref + (int)(rl >> 3) - 4 + (c >> 3);
+        const uint32_t* __restrict__ pq = U.q_packed + (int)(ql >> 3) - 4 + (c >> 3);
+        uint32_t t0, t1, wr = __ldg(pr), wq = __ldg(pq);
+        sa_masks32(pr, pq, sr, sq, wr, wq, m0, t0, b0);
+        sa_masks32(pr + 4, pq + 4, sr, sq, wr, wq, m1, t1, b1);
+        hits = P.transition ? sa_seed_bits<true>(a, P.kmer_size, m0, m1, t0, t1, 33 - S)
+                            : sa_seed_bits<false>(a, P.kmer_size, m0, m1, t0, t1, 33 - S);
+    }
+    const uint32_t below = __shfl_up_sync(SA_FULL, hits, 1);
+    uint32_t last = lane ? c - __clz(below) : 0, n = 0;
+    unsigned long long tiles = 0;
+    bool ended = (lane && !below) || !hits;
+    if (!ended)
+        for (uint32_t h = hits; h; h &= h - 1) {
+            const uint32_t i = __ffs(h), d = c + i, delta = d - last;
+            if (d > ahead || delta > a.gap || delta > ((j + d) & (SA_CHAIN_BLOCK - 1)) ||
+                (stop_r - d < SA_SWEEP_RIGHT && (!high || stop_l + d >= SA_SWEEP_LEFT)) ||
+                !sa_sweep_margin(a, U, rl + d, ql + d) || __funnelshift_rc(b0, b1, i) ||
+                !sa_chain_joined(a, ~__funnelshift_rc(m0, m1, i), delta)) {
+                ended = true;
+                break;
+            }
+            ++n;
+            tiles += ((stop_r - d) >> 5) + ((stop_l + d) >> 5) + 2;
+            last = d;
+        }
+    const uint32_t em = __ballot_sync(SA_FULL, ended);
+    if (em && lane > __ffs(em) - 1) n = tiles = 0;  // the chain ends below
+    n = __reduce_add_sync(SA_FULL, n);
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) tiles += __shfl_xor_sync(SA_FULL, tiles, s);
     return {tiles, n};
 }
 
@@ -1462,10 +1516,13 @@ __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
 }
 
 // ---------------------------------------------------------------------------
-// Phase B: one warp per long hit, 256 bases per step, 8 per lane.
+// Phase B: two warps per long hit, one per side, 256 bases per step, 8 per lane;
+// then the right side's warp runs the keep test and the other follows the chain.
 //
 // Bound by the latency of a step: its loads are issued a step ahead, and the
-// warp's part of it is one scan of sums and one of maxima (10 shuffles).
+// warp's part of it is one scan of sums and one of maxima (10 shuffles).  One warp
+// for both sides, and a chain followed by one lane, made it 22 us for a call
+// of 881 positions (15 now), 29 (22) for 250,000 against 1 Mbp, 95 (84) for a repeat-masker call.
 // ---------------------------------------------------------------------------
 struct SaDirResult {
     int best;
@@ -1573,31 +1630,56 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
 __global__ void __launch_bounds__(256)
 sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
     __shared__ int tbl[64];
+    __shared__ unsigned long long s_idx[4];
+    __shared__ SaDirResult s_dir[4][2];
+    __shared__ uint32_t s_follow[4];
     if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
     if (a.ctr->error) return;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, pair = threadIdx.x >> 6;
+    const bool left = threadIdx.x & 32u;
     const unsigned long long nlong = min(a.ctr->long_count, (unsigned long long)a.long_cap);
-    unsigned long long tiles_acc = 0;
-    const uint32_t* const ref_rev = a.ref + sa_rev_words(a.ref_len);
-    unsigned long long next = 0;
-    if (lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);
+    unsigned long long tiles_acc = 0, next = 0;
+    bool kept = false;  // the right warp's last hit
+    auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
+    if (!left && lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);
     while (true) {
-        const unsigned long long idx = __shfl_sync(SA_FULL, next, 0);
+        if (!left && lane == 0) s_idx[pair] = next;
+        meet();
+        const unsigned long long idx = s_idx[pair];
+        if (kept && lane == 0) atomicAdd(&a.ctr->surv_count, 1ull + s_follow[pair]);
+        kept = false;
         if (idx >= nlong) break;
-        if (lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);  // read while this hit is scanned
+        if (!left && lane == 0) next = atomicAdd(&a.ctr->long_cursor, 1ull);  // read while this hit is scanned
         const SaLongHit L = a.long_q[idx];
-        if (L.unit == SA_LONG_NONE) continue;
-        const SaUnit U = a.units[L.unit & ~SA_CHAIN_NEXT];
+        const bool on = L.unit != SA_LONG_NONE;
+        const uint32_t unit = L.unit & ~SA_CHAIN_NEXT;
+        const SaUnit U = a.units[on ? unit : 0];
         const uint32_t rl = L.ref_loc, ql = L.query_loc;
-        const SaDirResult R = sa_warp_xdrop(tblb, a.ref, U.q_packed, rl, ql, min(a.ref_len - rl, U.q_len - ql), a.xdrop);
-        SaDirResult Lr = sa_warp_xdrop(tblb, ref_rev, U.q_packed + sa_rev_words(U.q_len), a.ref_len - rl, U.q_len - ql,
-                                       min(rl, ql), a.xdrop);
+        if (on) {
+            const SaDirResult d = left ? sa_warp_xdrop(tblb, a.ref + sa_rev_words(a.ref_len),
+                                                       U.q_packed + sa_rev_words(U.q_len), a.ref_len - rl,
+                                                       U.q_len - ql, min(rl, ql), a.xdrop)
+                                       : sa_warp_xdrop(tblb, a.ref, U.q_packed, rl, ql,
+                                                       min(a.ref_len - rl, U.q_len - ql), a.xdrop);
+            if (lane == 0) s_dir[pair][left] = d;
+        }
+        meet();
+        if (!on) continue;
+        const SaDirResult R = s_dir[pair][0];
+        SaDirResult Lr = s_dir[pair][1];
         ++Lr.pos;  // left offsets are 1-based, 0 when best is 0
-        tiles_acc += (R.stop >> 5) + (Lr.stop >> 5) + 2;
         const int total = R.best + Lr.best;
         const int ext = R.pos + Lr.pos;
+        if (left) {  // the dropped hits that follow, while the right warp runs the keep test
+            SaChain ch = {0, 0};
+            if (L.unit & SA_CHAIN_NEXT)
+                ch = sa_warp_chain_members(a, P, unit, rl, ql, R.stop, Lr.stop, (int)(float)total >= a.hspthresh);
+            if (lane == 0) s_follow[pair] = ch.n;
+            tiles_acc += (R.stop >> 5) + (Lr.stop >> 5) + 2 + ch.tiles;
+            continue;
+        }
         int cnt[4] = {0, 0, 0, 0};
         const bool eb = sa_entropy_branch(a, total);
         if (eb) {
@@ -1612,17 +1694,10 @@ sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
                 for (int s = 16; s >= 1; s >>= 1) cnt[b] += __shfl_xor_sync(SA_FULL, cnt[b], s);
         }
         if (lane == 0) {
-            uint32_t stands_for = 1;
-            if (L.unit & SA_CHAIN_NEXT) {
-                const SaChain ch = sa_chain_members(a, P, L.unit & ~SA_CHAIN_NEXT, rl, ql, R.stop, Lr.stop,
-                                                    (int)(float)total >= a.hspthresh);
-                stands_for += ch.n;
-                tiles_acc += ch.tiles;
-            }
             int keep, score;
             sa_keep_score(total, ext, cnt, eb, a.hspthresh, &keep, &score);
+            kept = keep;
             if (keep) {
-                atomicAdd(&a.ctr->surv_count, (unsigned long long)stands_for);
                 const uint32_t rs = rl - (uint32_t)Lr.pos;
                 uint32_t qs = ql - (uint32_t)Lr.pos;
                 const uint32_t len = (uint32_t)ext;
@@ -1636,7 +1711,7 @@ sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
             }
         }
     }
-    if (lane == 0) atomicAdd(&a.ctr->base_steps, tiles_acc);
+    if (left && lane == 0 && tiles_acc) atomicAdd(&a.ctr->base_steps, tiles_acc);
 }
 
 // The fast scoring form holds when 7 * max(0, max_sub) <= xdrop (see the
