@@ -114,6 +114,7 @@ struct Slot {
     SaWork w{};
     void* arena = nullptr;  // one device allocation carved into the workspace
     SaCounters* h_ctr = nullptr;
+    char* h_up = nullptr;  // pinned: zeros for the counters, then the descriptor and the units
     SaCallDesc* h_desc = nullptr;
     SaUnit* h_units = nullptr;
     SaRec* h_out = nullptr;
@@ -323,8 +324,7 @@ void free_slot(Slot* s) {
     if (s->arena) cudaFree(s->arena);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->h_ctr) cudaFreeHost(s->h_ctr);
-    if (s->h_desc) cudaFreeHost(s->h_desc);
-    if (s->h_units) cudaFreeHost(s->h_units);
+    if (s->h_up) cudaFreeHost(s->h_up);
     if (s->h_out) cudaFreeHost(s->h_out);
     for (auto& e : s->ev)
         if (e) cudaEventDestroy(e);
@@ -337,6 +337,11 @@ void free_slot(Slot* s) {
 // Workspace kinds: plain calls (host seed words), batched passes (device
 // seeding over query windows), or both (passes of coalesced plain calls, and
 // plain calls one at a time), with at most `units` units per pass.
+// Offsets in a slot's block of counters, descriptor and units, on the device (consecutive parts
+// of the arena) and in h_up.
+constexpr size_t kUpDesc = 256, kUpUnits = 512;
+static_assert(sizeof(SaCounters) <= kUpDesc && sizeof(SaCallDesc) <= kUpUnits - kUpDesc, "a part of 256 bytes each");
+
 enum SlotKind { kSlotPlain = 0, kSlotBatch = 1, kSlotBoth = 2 };
 
 int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_cap, Slot** out,
@@ -370,7 +375,6 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         {(void**)&w.cs.unit, 4 * (seed_cap + 1)},
         {(void**)&w.cta_a, 8 * SA_MAX_CTAS},
         {(void**)&w.cta_b, 8 * SA_MAX_CTAS},
-        {(void**)&w.limits, 8 * SA_MAX_ITERS},
         {(void**)&w.long_q, sizeof(SaLongHit) * long_cap},
         {(void**)&w.rec[0], sizeof(SaRec) * surv_cap},
         {(void**)&w.rec[1], sizeof(SaRec) * surv_cap},
@@ -408,8 +412,7 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
     w.hash_clean = false;
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMallocHost(&s->h_ctr, sizeof(SaCounters)) != cudaSuccess ||
-        cudaMallocHost(&s->h_desc, sizeof(SaCallDesc)) != cudaSuccess ||
-        cudaMallocHost(&s->h_units, sizeof(SaUnit) * nunits) != cudaSuccess ||
+        cudaMallocHost(&s->h_up, kUpUnits + sizeof(SaUnit) * nunits) != cudaSuccess ||
         cudaEventCreate(&s->ev[0]) != cudaSuccess || cudaEventCreate(&s->ev[1]) != cudaSuccess ||
         cudaEventCreate(&s->ev[2]) != cudaSuccess || cudaEventCreate(&s->ev[3]) != cudaSuccess ||
         cudaEventCreate(&s->ev[4]) != cudaSuccess || cudaEventCreate(&s->ev[5]) != cudaSuccess) {
@@ -417,6 +420,9 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         sa_set_error(SA_ERR_NOMEM, "pinned host allocation failed");
         return SA_ERR_NOMEM;
     }
+    std::memset(s->h_up, 0, kUpUnits);
+    s->h_desc = reinterpret_cast<SaCallDesc*>(s->h_up + kUpDesc);
+    s->h_units = reinterpret_cast<SaUnit*>(s->h_up + kUpUnits);
     *out = s;
     return SA_OK;
 }
@@ -505,12 +511,10 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     cudaStream_t st = s->stream;
     const SaCallGrids cg = sa_call_grids(g.tuning, d.num_sms, mode);
     const int Gr = cg.range_ctas;
-    SA_CUDA_OK(cudaMemcpyAsync(w.desc, s->h_desc, sizeof(SaCallDesc), cudaMemcpyHostToDevice, st));
-    SA_CUDA_OK(cudaMemcpyAsync(w.units, s->h_units, sizeof(SaUnit), cudaMemcpyHostToDevice, st));
-    SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
+    // zeroed counters, descriptor and unit lie in one block on both sides
+    SA_CUDA_OK(cudaMemcpyAsync(w.ctr, s->h_up, kUpUnits + sizeof(SaUnit), cudaMemcpyHostToDevice, st));
     const bool chain = chains_allowed(d) && !s->no_sweep;
     sa_launch_lookup_seeds(w, d.index, (uint32_t)d.nbuckets, g.params, Gr, st, chain);
-    sa_launch_hash_init(w, st);
     tm.mark(1);
     SaExtendArgs xa;
     xa.chain = chain ? 1 : 0;

@@ -107,6 +107,7 @@ struct SaCounters {
     unsigned long long list_count;     // hits the sweep left to the scans (past the list's capacity: the call is run again without it)
     unsigned long long sweep_cursor;   // sweep work counter
     unsigned long long scan_cursor;    // scan work counter
+    unsigned long long lookup_done;    // CTAs of sa_k_lookup_count that have written their sums
 };
 
 // Open-addressing set of distinct HSPs of one call: slot = 16-byte key
@@ -192,6 +193,16 @@ __device__ __forceinline__ bool sa_hash_contains(const SaHashSet& hs, unsigned l
         h = (h + 1) & mask;
     }
     return false;
+}
+
+// Slots of a call's HSP set: the smallest power of two >= 2 * hits (at least
+// 1024), at most `max_slots` (a power of two, the whole table).  The table is
+// known to be empty (the previous call's output emptied the slots it used).
+__device__ __forceinline__ unsigned long long sa_hash_slots(unsigned long long hits, unsigned long long max_slots) {
+    const unsigned long long want = hits < 512 ? 1024 : 2 * hits;
+    unsigned long long slots = 1;
+    while (slots < want && slots < max_slots) slots <<= 1;
+    return slots;
 }
 
 __device__ __forceinline__ uint32_t sa_lanemask_lt();

@@ -87,14 +87,12 @@ struct SaWork {
     uint64_t* seeds;        // [seed_cap]
     uint32_t* s_lo;         // [seed_cap] bucket start per seed
     uint32_t* s_cnt;        // [seed_cap] bucket size per seed
-    uint64_t* s_P;          // [seed_cap] inclusive hit prefix per seed
+    uint64_t* s_P;          // [seed_cap] inclusive hit prefix per seed (calls of several MAX_HITS iterations)
     SaSeedList cs;          // compacted seeds [seed_cap + 1]
     uint64_t seed_cap;
     // per-CTA partials (range-partitioned kernels)
     unsigned long long* cta_a;  // [SA_MAX_CTAS]
     unsigned long long* cta_b;  // [SA_MAX_CTAS]
-    // MAX_HITS iteration limits (seed indices) [SA_MAX_ITERS]
-    uint64_t* limits;
     // long queue
     SaLongHit* long_q;
     uint64_t long_cap;
@@ -199,6 +197,7 @@ bool sa_chain_params(const SaParams& p, const SaTuning& t);
 // ---- sa_sort.cu ----
 // Sizes the call's HSP set (device side, from the hit count); sa_launch_hash_clear
 // empties every slot.
+unsigned long long sa_hash_max_slots(const SaWork& w);
 void sa_launch_hash_init(SaWork& w, cudaStream_t st);
 void sa_launch_hash_clear(SaWork& w, cudaStream_t st);
 // Kernel attributes of the lane kernel, set once per device outside stream capture.

@@ -16,27 +16,51 @@
 #define SA_DERR_MAX_HITS 2       // one seed holds >= MAX_HITS hits (reference UB)
 #define SA_DERR_ITERS 3          // more MAX_HITS iterations than supported
 
+// A call's words are split over the CTAs at multiples of 4 (16-byte loads).
+__device__ __forceinline__ void sa_seed_range(uint64_t n, uint64_t& a, uint64_t& b) {
+    sa_cta_range((n + 3) / 4, a, b);
+    a *= 4;
+    b = min(n, 4 * b);
+}
+
+// Bucket bounds of every word, and per CTA its hits and its words with hits; the
+// CTA that finishes last turns these into prefixes and sets what depends on the
+// totals: the number of MAX_HITS iterations (src/seed_filter.cu:686) and the
+// size of the HSP set.  (A launch each for the prefixes, the iterations, the
+// scopes and the set took 13 us of a call's 76.)
+//
+// Bound by latency: word, bucket bounds and, with `chain`, the query window are
+// loads that wait for one another, so a thread takes SA_WORDS words at a time and
+// a CTA has 512 threads (1.3 M words with transitions: 58 us with one word at a time and 256
+// threads, 56 with four, 38 with both; the next kernel 64, 30 and 22 us).
+//
 // With `chain`, also checks that the call's words are every seed word of the
 // query window [j_lo, j_hi), in seeder order (src/seeder.cpp:57-74): word i is
 // the one that its position and its place i % S in the position's group of S
 // words call for, positions increase, and there are as many of them as valid
-// windows (counted into ctr->windows, compared by sa_k_groups).  Only then may
-// the extension tell a call's hits from the sequences alone.  A word out of
-// place sets ctr->chain_bad; nothing else depends on the check.
-__global__ void __launch_bounds__(256)
+// windows (counted into ctr->windows).  Only then may the extension tell a call's
+// hits from the sequences alone.  A word out of place sets ctr->chain_bad; nothing
+// else depends on the check.  Hits of different iterations are deduplicated
+// apart, so chains need one iteration too.
+#define SA_WORDS 4
+#define SA_CALL_BLOCK 512
+__global__ void __launch_bounds__(SA_CALL_BLOCK)
 sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restrict__ desc,
                   const uint32_t* __restrict__ index, uint32_t nbuckets, uint32_t* __restrict__ s_lo,
                   uint32_t* __restrict__ s_cnt, unsigned long long* cta_a, unsigned long long* cta_b,
-                  SaCounters* ctr, const SaUnit* __restrict__ units, SaParams P, int chain) {
+                  SaCounters* ctr, const SaUnit* __restrict__ units, SaParams P, int chain,
+                  unsigned long long max_slots) {
+    constexpr int J = SA_WORDS;
+    const uint64_t n = desc->num_seeds;
     uint64_t a, b;
-    sa_cta_range(desc->num_seeds, a, b);
+    sa_seed_range(n, a, b);
     unsigned long long hits = 0, nz = 0;
     const uint32_t S = P.transition ? 1u + (uint32_t)P.kmer_size : 1u;
     SaUnit U{};
     bool bad = false;
     if (chain) {
         U = units[0];
-        const uint64_t n = desc->num_seeds, span = U.j_hi > U.j_lo ? U.j_hi - U.j_lo : 0;
+        const uint64_t span = U.j_hi > U.j_lo ? U.j_hi - U.j_lo : 0;
         // few words over a wide window are no seeder's chunk, and counting its windows would cost more than the call
         if (n % S || U.j_hi > U.q_len || span > (1u << 20) + 2 * n) {
             bad = true;
@@ -45,7 +69,7 @@ sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restri
             uint64_t ga, gb;  // words of 8 positions
             sa_cta_range(span ? ((U.j_hi - 1) >> 3) - (U.j_lo >> 3) + 1 : 0, ga, gb);
             unsigned long long windows = 0;
-            for (uint64_t g = (U.j_lo >> 3) + ga + threadIdx.x; g < (U.j_lo >> 3) + gb; g += 256) {
+            for (uint64_t g = (U.j_lo >> 3) + ga + threadIdx.x; g < (U.j_lo >> 3) + gb; g += SA_CALL_BLOCK) {
                 uint32_t ok = sa_valid_windows8(U.q_packed + g, (uint32_t)P.seed_size);
                 if (8 * g < U.j_lo) ok &= 0xffu << (U.j_lo - 8 * g);
                 if (8 * g + 8 > U.j_hi) ok &= 0xffu >> (8 * g + 8 - U.j_hi);
@@ -56,131 +80,203 @@ sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restri
             if ((threadIdx.x & 31) == 0 && windows) atomicAdd(&ctr->windows, windows);
         }
     }
-    for (uint64_t i = a + threadIdx.x; i < b; i += 256) {
-        const uint64_t word = seeds[i];
-        uint32_t key = (uint32_t)(word >> 32);
-        if (chain) {
-            const uint32_t j = (uint32_t)word, v = (uint32_t)(i % S);
-            const uint32_t before = i ? (uint32_t)seeds[i - 1] : 0u;
-            bool ok = j >= U.j_lo && j < U.j_hi && (v ? before == j : (i == 0 || before < j));
-            if (ok) {
-                const uint32_t k0 = sa_window_key(U.q_packed, j, P);
-                ok = k0 != SA_INVALID_KEY && key == (v ? k0 ^ (2u << (2 * (v - 1))) : k0);
+    for (uint64_t i0 = a + threadIdx.x; i0 < b; i0 += SA_CALL_BLOCK * J) {
+        uint64_t word[J];
+        uint32_t lo[J], hi[J];
+#pragma unroll
+        for (int k = 0; k < J; ++k) word[k] = i0 + SA_CALL_BLOCK * k < b ? seeds[i0 + SA_CALL_BLOCK * k] : 0;
+#pragma unroll
+        for (int k = 0; k < J; ++k) {
+            const uint32_t key = (uint32_t)(word[k] >> 32);
+            lo[k] = hi[k] = 0;
+            if (i0 + SA_CALL_BLOCK * k < b) {
+                if (key < nbuckets) {
+                    hi[k] = __ldg(index + key);
+                    lo[k] = key ? __ldg(index + key - 1) : 0u;
+                } else {
+                    atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_BAD_KEY);
+                }
             }
-            bad |= !ok;
         }
-        uint32_t lo = 0, cnt = 0;
-        if (key < nbuckets) {
-            uint32_t hi = __ldg(index + key);
-            lo = key ? __ldg(index + key - 1) : 0u;
-            cnt = hi - lo;
-        } else {
-            atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_BAD_KEY);
+        if (chain) {
+#pragma unroll
+            for (int k = 0; k < J; ++k) {
+                const uint64_t i = i0 + SA_CALL_BLOCK * k;
+                if (i >= b) break;
+                const uint32_t key = (uint32_t)(word[k] >> 32), j = (uint32_t)word[k], v = (uint32_t)i % S;
+                const uint32_t before = i ? (uint32_t)seeds[i - 1] : 0u;
+                bool ok = j >= U.j_lo && j < U.j_hi && (v ? before == j : (i == 0 || before < j));
+                if (ok) {
+                    // the position's first word is checked against its window, the others against that word
+                    const uint32_t k0 = v ? (uint32_t)(seeds[i - v] >> 32) : sa_window_key(U.q_packed, j, P);
+                    ok = k0 != SA_INVALID_KEY && key == (v ? k0 ^ (2u << (2 * (v - 1))) : k0);
+                }
+                bad |= !ok;
+            }
         }
-        s_lo[i] = lo;
-        s_cnt[i] = cnt;
-        hits += cnt;
-        nz += cnt != 0;
+#pragma unroll
+        for (int k = 0; k < J; ++k) {
+            const uint64_t i = i0 + SA_CALL_BLOCK * k;
+            if (i < b) {
+                s_lo[i] = lo[k];
+                s_cnt[i] = hi[k] - lo[k];
+                hits += hi[k] - lo[k];
+                nz += hi[k] != lo[k];
+            }
+        }
     }
     if (bad) ctr->chain_bad = 1;
-    __shared__ unsigned long long ws[9];
-    unsigned long long tot;
-    sa_block_excl_sum<unsigned long long, 256>(hits, ws, &tot);
-    if (threadIdx.x == 0) cta_a[blockIdx.x] = tot;
-    sa_block_excl_sum<unsigned long long, 256>(nz, ws, &tot);
-    if (threadIdx.x == 0) cta_b[blockIdx.x] = tot;
+    __shared__ unsigned long long ws[SA_CALL_BLOCK / 32 + 1];
+    __shared__ bool last;
+    unsigned long long th, tz;
+    sa_block_excl_sum<unsigned long long, SA_CALL_BLOCK>(hits, ws, &th);
+    sa_block_excl_sum<unsigned long long, SA_CALL_BLOCK>(nz, ws, &tz);
+    if (threadIdx.x == 0) {
+        cta_a[blockIdx.x] = th;
+        cta_b[blockIdx.x] = tz;
+    }
+    __threadfence();  // this CTA's sums and counters before its ticket
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&ctr->lookup_done, 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr int PER = SA_MAX_CTAS / SA_CALL_BLOCK;  // sums per thread
+    unsigned long long va[PER], vb[PER], sa = 0, sb = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const uint32_t c = PER * threadIdx.x + k;
+        va[k] = c < gridDim.x ? __ldcg(cta_a + c) : 0;
+        vb[k] = c < gridDim.x ? __ldcg(cta_b + c) : 0;
+        sa += va[k];
+        sb += vb[k];
+    }
+    unsigned long long ea = sa_block_excl_sum<unsigned long long, SA_CALL_BLOCK>(sa, ws, &th);
+    unsigned long long eb = sa_block_excl_sum<unsigned long long, SA_CALL_BLOCK>(sb, ws, &tz);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const uint32_t c = PER * threadIdx.x + k;
+        if (c < gridDim.x) {
+            cta_a[c] = ea;
+            cta_b[c] = eb;
+        }
+        ea += va[k];
+        eb += vb[k];
+    }
+    if (threadIdx.x == 0) {
+        ctr->num_hits = th;
+        ctr->nnz = tz;
+        ctr->hash_mask = sa_hash_slots(th, max_slots) - 1;
+        const uint64_t MH = desc->max_hits;
+        uint64_t num_iter = MH ? th / MH + 1 : 1;
+        if (num_iter > 1 || __ldcg(&ctr->windows) * S != n) ctr->chain_bad = 1;
+        if (num_iter > SA_MAX_ITERS) {
+            atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_ITERS);
+            num_iter = 1;
+        }
+        ctr->num_iter = num_iter;
+    }
 }
 
-__global__ void __launch_bounds__(256)
+// The words with hits, compacted.  A thread takes four consecutive words, and
+// both prefixes come from one scan: a round's hits above the low 12 bits, its
+// words with hits in them.  With more than one iteration the scope is the
+// word's index until sa_k_iterations, which also needs the hit prefix of every word.
+__global__ void __launch_bounds__(SA_CALL_BLOCK)
 sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restrict__ desc,
                  const uint32_t* __restrict__ s_lo, const uint32_t* __restrict__ s_cnt,
                  uint64_t* __restrict__ s_P, SaSeedList cs, const unsigned long long* cta_a,
                  const unsigned long long* cta_b, SaCounters* ctr) {
     const uint64_t n = desc->num_seeds;
     uint64_t a, b;
-    sa_cta_range(n, a, b);
+    sa_seed_range(n, a, b);
+    const bool split = ctr->num_iter > 1;
     unsigned long long hbase = cta_a[blockIdx.x], cbase = cta_b[blockIdx.x];
-    __shared__ unsigned long long ws[9];
-    for (uint64_t r = a; r < b; r += 256) {
-        uint64_t i = r + threadIdx.x;
-        uint32_t cnt = i < b ? s_cnt[i] : 0u;
-        unsigned long long th, tc;
-        unsigned long long eh = sa_block_excl_sum<unsigned long long, 256>(cnt, ws, &th);
-        unsigned long long ec = sa_block_excl_sum<unsigned long long, 256>(cnt != 0, ws, &tc);
-        if (i < b) {
-            s_P[i] = hbase + eh + cnt;  // inclusive prefix (thrust::inclusive_scan, :682)
-            if (cnt) {
-                uint64_t c = cbase + ec;
-                cs.E[c] = hbase + eh;
-                cs.lo[c] = s_lo[i];
-                cs.qpos[c] = (uint32_t)(seeds[i] & 0xffffffffu);
-                cs.scope[c] = (uint32_t)i;  // seed index; turned into the iteration by sa_k_scope
-                cs.unit[c] = 0;
-            }
+    __shared__ unsigned long long ws[SA_CALL_BLOCK / 32 + 1];
+    for (uint64_t r = a; r < b; r += 4 * SA_CALL_BLOCK) {
+        const uint64_t i0 = r + 4 * threadIdx.x;
+        uint32_t cnt[4] = {0, 0, 0, 0};
+        if (i0 + 4 <= b) {
+            const uint4 v = *reinterpret_cast<const uint4*>(s_cnt + i0);
+            cnt[0] = v.x, cnt[1] = v.y, cnt[2] = v.z, cnt[3] = v.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i0 + k < b) cnt[k] = s_cnt[i0 + k];
         }
-        hbase += th;
-        cbase += tc;
+        unsigned long long sum = 0, total;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sum += ((unsigned long long)cnt[k] << 12) + (cnt[k] != 0);
+        const unsigned long long e = sa_block_excl_sum<unsigned long long, SA_CALL_BLOCK>(sum, ws, &total);
+        uint64_t h = hbase + (e >> 12), c = cbase + (e & 4095);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (cnt[k]) {
+                cs.E[c] = h;
+                cs.lo[c] = s_lo[i0 + k];
+                cs.qpos[c] = (uint32_t)seeds[i0 + k];
+                cs.scope[c] = split ? (uint32_t)(i0 + k) : 0u;
+                cs.unit[c] = 0;
+                ++c;
+                h += cnt[k];
+            }
+            if (split && i0 + k < b) s_P[i0 + k] = h;  // inclusive prefix (thrust::inclusive_scan, :682)
+        }
+        hbase += total >> 12;
+        cbase += total & 4095;
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) cs.E[ctr->nnz] = ctr->num_hits;
 }
 
-// MAX_HITS iterations (src/seed_filter.cu:686-697): num_iter = num_hits/MAX_HITS + 1;
-// limit[i] = lower_bound(P, lim) - 1, lim = P[limit[i]] + MAX_HITS, last limit = n-1.
-// Hits of different iterations are deduplicated apart, so chains need one.
-__global__ void sa_k_groups(const uint64_t* __restrict__ P, const SaCallDesc* desc, uint64_t* limits,
-                            SaCounters* ctr, uint32_t words_per_window) {
-    const uint64_t n = desc->num_seeds, MH = desc->max_hits, H = ctr->num_hits;
-    uint64_t num_iter = MH ? H / MH + 1 : 1;
-    if (num_iter > 1 || ctr->windows * words_per_window != n) ctr->chain_bad = 1;
-    if (num_iter > SA_MAX_ITERS) {
-        atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_ITERS);
-        num_iter = 1;
-    }
-    ctr->num_iter = num_iter;
-    uint64_t lim = MH;
-    int64_t prev = -1;
-    for (uint64_t it = 0; it + 1 < num_iter; ++it) {
-        uint64_t lo = 0, hi = n;  // first index with P >= lim
-        while (lo < hi) {
-            uint64_t mid = (lo + hi) >> 1;
-            if (P[mid] < lim) lo = mid + 1;
-            else hi = mid;
+// MAX_HITS iterations (src/seed_filter.cu:686-697), for calls with more than one:
+// limit[i] = lower_bound(P, lim) - 1, lim = P[limit[i]] + MAX_HITS, last limit =
+// n - 1; a word's scope is the first iteration whose limit is at least its index.
+// Every CTA finds the limits for itself.
+__global__ void __launch_bounds__(256)
+sa_k_iterations(const uint64_t* __restrict__ P, const SaCallDesc* desc, SaSeedList cs, SaCounters* ctr) {
+    const uint64_t num_iter = ctr->num_iter;
+    if (num_iter <= 1) return;
+    __shared__ uint64_t limits[SA_MAX_ITERS];
+    if (threadIdx.x == 0) {
+        const uint64_t n = desc->num_seeds, MH = desc->max_hits;
+        uint64_t lim = MH;
+        int64_t prev = -1;
+        for (uint64_t it = 0; it + 1 < num_iter; ++it) {
+            uint64_t lo = 0, hi = n;  // first index with P >= lim
+            while (lo < hi) {
+                uint64_t mid = (lo + hi) >> 1;
+                if (P[mid] < lim) lo = mid + 1;
+                else hi = mid;
+            }
+            int64_t pos = (int64_t)lo - 1;
+            if (pos <= prev) {
+                atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_MAX_HITS);
+                pos = prev + 1;
+            }
+            limits[it] = (uint64_t)pos;
+            lim = P[pos] + MH;
+            prev = pos;
         }
-        int64_t pos = (int64_t)lo - 1;
-        if (pos <= prev) {
-            atomicCAS(&ctr->error, 0ull, (unsigned long long)SA_DERR_MAX_HITS);
-            pos = prev + 1;
-        }
-        limits[it] = (uint64_t)pos;
-        lim = P[pos] + MH;
-        prev = pos;
+        limits[num_iter - 1] = n ? n - 1 : 0;
     }
-    limits[num_iter - 1] = n ? n - 1 : 0;
-}
-
-// Seed index -> iteration: the first iteration whose limit is >= the seed index.
-__global__ void sa_k_scope(SaSeedList cs, const uint64_t* __restrict__ limits, SaCounters* ctr) {
-    const uint64_t nnz = ctr->nnz, it = ctr->num_iter;
-    for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < nnz; c += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = cs.scope[c];
+    __syncthreads();
+    const uint64_t nnz = ctr->nnz;
+    for (uint64_t c = blockIdx.x * 256ull + threadIdx.x; c < nnz; c += gridDim.x * 256ull) {
+        const uint32_t s = cs.scope[c];
         uint32_t g = 0;
-        while (g + 1 < it && (uint64_t)s > limits[g]) ++g;
+        while (g + 1 < num_iter && (uint64_t)s > limits[g]) ++g;
         cs.scope[c] = g;
     }
 }
 
 void sa_launch_lookup_seeds(SaWork& w, const uint32_t* index, uint32_t nbuckets, const SaParams& p, int G,
                             cudaStream_t st, bool chain) {
-    sa_k_lookup_count<<<G, 256, 0, st>>>(w.seeds, w.desc, index, nbuckets, w.s_lo, w.s_cnt, w.cta_a, w.cta_b, w.ctr,
-                                         w.units, p, chain ? 1 : 0);
+    sa_k_lookup_count<<<G, SA_CALL_BLOCK, 0, st>>>(w.seeds, w.desc, index, nbuckets, w.s_lo, w.s_cnt, w.cta_a, w.cta_b, w.ctr,
+                                         w.units, p, chain ? 1 : 0, sa_hash_max_slots(w));
     sa_note_launch();
-    sa_k_scan_partials<<<1, 1024, 0, st>>>(w.cta_a, w.cta_b, G, &w.ctr->num_hits, &w.ctr->nnz);
+    sa_k_lookup_emit<<<G, SA_CALL_BLOCK, 0, st>>>(w.seeds, w.desc, w.s_lo, w.s_cnt, w.s_P, w.cs, w.cta_a, w.cta_b, w.ctr);
     sa_note_launch();
-    sa_k_lookup_emit<<<G, 256, 0, st>>>(w.seeds, w.desc, w.s_lo, w.s_cnt, w.s_P, w.cs, w.cta_a, w.cta_b, w.ctr);
-    sa_note_launch();
-    sa_k_groups<<<1, 1, 0, st>>>(w.s_P, w.desc, w.limits, w.ctr, p.transition ? 1u + (uint32_t)p.kmer_size : 1u);
-    sa_note_launch();
-    sa_k_scope<<<148 * 4, 256, 0, st>>>(w.cs, w.limits, w.ctr);
+    sa_k_iterations<<<148, 256, 0, st>>>(w.s_P, w.desc, w.cs, w.ctr);
     sa_note_launch();
 }
 

@@ -41,7 +41,7 @@ constexpr uint64_t kParts[] = {
     8 * kSeeds,                                          // seeds
     4 * kSeeds, 4 * kSeeds, 8 * kSeeds,                  // s_lo, s_cnt, s_P
     8 * (kSeeds + 1), 4 * (kSeeds + 1), 4 * (kSeeds + 1), 4 * (kSeeds + 1), 4 * (kSeeds + 1),  // cs
-    8 * SA_MAX_CTAS, 8 * SA_MAX_CTAS, 8 * SA_MAX_ITERS,  // cta_a, cta_b, limits
+    8 * SA_MAX_CTAS, 8 * SA_MAX_CTAS,                    // cta_a, cta_b
     sizeof(SaLongHit) * SA_NOALLOC_LONG_CAP,             // long queue
     sizeof(SaRec) * kSurv, sizeof(SaRec) * kSurv, 4 * kSurv, 4 * kSurv,  // rec[2], scope[2]
     16 * 2 * kSurv, 4 * 2 * kSurv,                       // HSP set: keys, scores
@@ -102,7 +102,6 @@ void carve(void* base, SaWork& w) {
     take((void**)&w.cs.unit);
     take((void**)&w.cta_a);
     take((void**)&w.cta_b);
-    take((void**)&w.limits);
     take((void**)&w.long_q);
     take((void**)&w.rec[0]);
     take((void**)&w.rec[1]);
@@ -191,7 +190,6 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
         sa_launch_lookup_seeds(w, v.index, (uint32_t)v.nbuckets, v.params, cg.range_ctas, st, xa.chain != 0);
         if (!w.hash_clean) sa_launch_hash_clear(w, st);
         w.hash_clean = false;
-        sa_launch_hash_init(w, st);
         sa_launch_extend_lane(w, xa, v.params, cg.lane_tuning, v.num_sms, st, cg.lane_ctas);
         sa_launch_extend_warp(w, xa, v.params, v.tuning, v.num_sms, st);
         SA_CUDA_OK(cudaGetLastError());

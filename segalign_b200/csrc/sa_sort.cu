@@ -427,18 +427,12 @@ __global__ void sa_k_unit_counts(const uint32_t* __restrict__ scope, uint64_t n,
     }
 }
 
-// Sizes the call's HSP set: the smallest power of two >= 2 * hits (at least
-// 1024), at most `max_slots` (a power of two, the whole table).  The table is
-// known to be empty (the previous call's output emptied the slots it used).
+// Sizes a batch's HSP set (sa_hash_slots).
 __global__ void sa_k_hash_init(SaCounters* ctr, unsigned long long max_slots) {
-    unsigned long long want = 2 * ctr->num_hits;
-    if (want < 1024) want = 1024;
-    unsigned long long slots = 1;
-    while (slots < want && slots < max_slots) slots <<= 1;
-    ctr->hash_mask = slots - 1;
+    ctr->hash_mask = sa_hash_slots(ctr->num_hits, max_slots) - 1;
 }
 
-static unsigned long long sa_hash_max_slots(const SaWork& w) {
+unsigned long long sa_hash_max_slots(const SaWork& w) {
     unsigned long long max_slots = 1;
     while (max_slots * 2 <= 2 * w.surv_cap) max_slots <<= 1;
     return max_slots;
