@@ -444,6 +444,7 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
     if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SA_SWEEP_SH) - 1;
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
+    sa_wait_prior();
     SaCounters* const ctr = a.ctr;
     const uint64_t H = min((uint64_t)ctr->num_hits, h_end), nnz = ctr->nnz;
     if (ctr->error || h_begin >= H) return;
@@ -1228,6 +1229,7 @@ sa_k_scan(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) 
     if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] * SCALE - 1;
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
+    sa_wait_prior();
     SaCounters* const ctr = a.ctr;
     const unsigned long long n_list = ctr->list_count;
     if (ctr->error || n_list > a.list_cap) return;
@@ -1429,6 +1431,7 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
     if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SH) - 1;
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
+    sa_wait_prior();
     SaCounters* const ctr = a.ctr;
     const unsigned long long n = ctr->list_count;
     if (ctr->error || n > a.list_cap) return;
@@ -1636,6 +1639,7 @@ sa_k_extend_warp(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
     if (threadIdx.x < 64) tbl[threadIdx.x] = P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)];
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
+    sa_wait_prior();
     if (a.ctr->error) return;
     const int lane = threadIdx.x & 31, pair = threadIdx.x >> 6;
     const bool left = threadIdx.x & 32u;
@@ -1828,7 +1832,7 @@ void sa_prepare_extend_lane(const SaParams& p, const SaTuning& t) {
 
 template <int STEP>
 static void sa_scan_launch(const SaExtK& a, const SaParams& p, int grid, cudaStream_t st) {
-    sa_k_scan<STEP><<<grid, 256, 0, st>>>(a, p);
+    sa_launch_next(sa_k_scan<STEP>, grid, 256, st, a, p);
     sa_note_launch();
 }
 
@@ -1856,13 +1860,12 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
     do {
         const uint64_t h1 = x.hits > h0 + seg ? h0 + seg : ~0ull;
         if (h0) sa_k_next_segment<<<1, 1, 0, st>>>(w.ctr, a.list_cap);
-        if (p.transition) sa_k_sweep<true><<<grid, 256, 0, st>>>(a, p, h0, h1);
-        else sa_k_sweep<false><<<grid, 256, 0, st>>>(a, p, h0, h1);
+        sa_launch_next(p.transition ? sa_k_sweep<true> : sa_k_sweep<false>, grid, 256, st, a, p, h0, h1);
         sa_note_launch();
         if (t.step_bases == 32) sa_scan_launch<32>(a, p, grid, st);
         else if (t.step_bases == 16) sa_scan_launch<16>(a, p, grid, st);
         else sa_scan_launch<8>(a, p, grid, st);
-        sa_k_finish<<<grid, 256, 0, st>>>(a, p);
+        sa_launch_next(sa_k_finish, grid, 256, st, a, p);
         sa_note_launch();
         h0 = h1;
     } while (h0 != ~0ull);
@@ -1870,6 +1873,6 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
 
 void sa_launch_extend_warp(SaWork& w, const SaExtendArgs& x, const SaParams& p, const SaTuning& t, int num_sms,
                            cudaStream_t st) {
-    sa_k_extend_warp<<<num_sms * 4, t.long_block, 0, st>>>(sa_ext_args(w, x, p, t), p);
+    sa_launch_next(sa_k_extend_warp, num_sms * 4, t.long_block, st, sa_ext_args(w, x, p, t), p);
     sa_note_launch();
 }

@@ -110,6 +110,13 @@ struct SaCounters {
     unsigned long long lookup_done;    // CTAs of sa_k_lookup_count that have written their sums
 };
 
+// Waits until the kernels before this one in the stream are done and their
+// writes are seen; a no-op in a kernel launched the plain way.
+__device__ __forceinline__ void sa_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel's CTAs take free places on the chip already.
+__device__ __forceinline__ void sa_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Open-addressing set of distinct HSPs of one call: slot = 16-byte key
 // {(scope << 32) | ref_start, (query_start << 32) | len} claimed with a
 // 128-bit compare-and-swap (all ones = empty), plus the score.  Within one

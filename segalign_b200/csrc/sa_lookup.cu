@@ -51,6 +51,7 @@ sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restri
                   SaCounters* ctr, const SaUnit* __restrict__ units, SaParams P, int chain,
                   unsigned long long max_slots) {
     constexpr int J = SA_WORDS;
+    sa_allow_next();
     const uint64_t n = desc->num_seeds;
     uint64_t a, b;
     sa_seed_range(n, a, b);
@@ -187,6 +188,8 @@ sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restric
                  const uint32_t* __restrict__ s_lo, const uint32_t* __restrict__ s_cnt,
                  uint64_t* __restrict__ s_P, SaSeedList cs, const unsigned long long* cta_a,
                  const unsigned long long* cta_b, SaCounters* ctr) {
+    sa_wait_prior();
+    sa_allow_next();
     const uint64_t n = desc->num_seeds;
     uint64_t a, b;
     sa_seed_range(n, a, b);
@@ -234,6 +237,8 @@ sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restric
 // Every CTA finds the limits for itself.
 __global__ void __launch_bounds__(256)
 sa_k_iterations(const uint64_t* __restrict__ P, const SaCallDesc* desc, SaSeedList cs, SaCounters* ctr) {
+    sa_wait_prior();
+    sa_allow_next();
     const uint64_t num_iter = ctr->num_iter;
     if (num_iter <= 1) return;
     __shared__ uint64_t limits[SA_MAX_ITERS];
@@ -274,9 +279,10 @@ void sa_launch_lookup_seeds(SaWork& w, const uint32_t* index, uint32_t nbuckets,
     sa_k_lookup_count<<<G, SA_CALL_BLOCK, 0, st>>>(w.seeds, w.desc, index, nbuckets, w.s_lo, w.s_cnt, w.cta_a, w.cta_b, w.ctr,
                                          w.units, p, chain ? 1 : 0, sa_hash_max_slots(w));
     sa_note_launch();
-    sa_k_lookup_emit<<<G, SA_CALL_BLOCK, 0, st>>>(w.seeds, w.desc, w.s_lo, w.s_cnt, w.s_P, w.cs, w.cta_a, w.cta_b, w.ctr);
+    sa_launch_next(sa_k_lookup_emit, G, SA_CALL_BLOCK, st, w.seeds, w.desc, w.s_lo, w.s_cnt, w.s_P, w.cs, w.cta_a,
+                   w.cta_b, w.ctr);
     sa_note_launch();
-    sa_k_iterations<<<148, 256, 0, st>>>(w.s_P, w.desc, w.cs, w.ctr);
+    sa_launch_next(sa_k_iterations, 148, 256, st, w.s_P, w.desc, w.cs, w.ctr);
     sa_note_launch();
 }
 
