@@ -25,13 +25,12 @@
 //
 // A record becomes five words whose lexicographic order is the wanted one (and
 // which give the record back).  The sort: tiles of SA_SORT_TILE records, straight
-// out of the set; then, up to SA_RANK_TILES tiles, one kernel in which a warp per
-// record finds its rank in every tile at once; for more, passes that merge
-// pairs of runs.  The host has read the record count by then, so a call launches
+// out of the set; then, up to SA_RANK_MAX records, passes in which 8 lanes find a
+// record's rank in 8 runs at once; for more, passes that merge pairs of runs.  The host has read the record count by then, so a call launches
 // what its size needs: one kernel up to one tile.  An LSD radix sort of every
 // key byte, planned on the device, took 46 launches for any size and a one-CTA
 // histogram scan per pass.  Measured (one B200, dedup phase, ms, radix sort and
-// this): 36 records 0.21 and 0.026, 26 K 0.28 and 0.064, 458 K 1.18 and 0.22, 4.7 M 2.90
+// this): 36 records 0.21 and 0.023, 26 K 0.28 and 0.052, 458 K 1.18 and 0.22, 4.7 M 2.90
 // and 2.23; a repeat-masker call's 3.7 K, three sorts and two, 0.67 and 0.083.
 #include <algorithm>
 
@@ -39,7 +38,9 @@
 #include "sa_radix.cuh"
 
 #define SA_SORT_TILE 1024
-#define SA_RANK_TILES 32  // a lane per tile
+// Records up to which rank passes are used.  They and merge passes, us: 26 K records 21 and 62, 57 K
+// 26 and 84, 106 K 75 and 100; at 458 K 424 and 143 (each probe is a scattered read).
+#define SA_RANK_MAX 131072u
 #define SA_MERGE_OUT 2048
 
 enum SaOrder { kOrderPlain, kOrderDiag, kOrderFinal };
@@ -261,28 +262,40 @@ sa_k_tile_rm(SaHashSet hs, SaRec* dst, uint32_t n, bool exclude, unsigned long l
     if (t == 0) *n_out = m;
 }
 
-// All tiles to the output at once (at most SA_RANK_TILES): a warp per record,
-// lane l counts tile l's keys below the record's; the sum is its place.  One
-// kernel in place of five merge passes (13 us each, mostly latency) for 26 K
-// records.
+// One pass over groups of 8 runs of `run` sorted keys: 8 lanes per record, lane l
+// counts the keys of its group's run l below the record's, and the sum is its
+// place in the group.  Distinct keys.  Each count is a chain of dependent reads, but
+// one pass replaces three merge passes of 14 us, which are latency too.  (A lane per
+// tile and a warp per record, all of up to 32 tiles in one pass, took 28 us for 26 K; two
+// passes of 8 take 21, and go on past 32 tiles.)
 template <int ORDER>
 __global__ void __launch_bounds__(256)
-sa_k_rank(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope, SaRec* __restrict__ dst,
-          uint32_t* __restrict__ dst_scope, uint64_t n_max, const unsigned long long* d_n, bool last) {
+sa_k_rank8(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope, SaRec* __restrict__ dst,
+           uint32_t* __restrict__ dst_scope, uint64_t n_max, const unsigned long long* d_n, uint32_t run, bool last) {
+    sa_wait_prior();
     const uint32_t n = (uint32_t)(d_n ? *d_n : n_max);
-    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * 8;
-    const uint32_t base = lane * SA_SORT_TILE, size = base < n ? min((uint32_t)SA_SORT_TILE, n - base) : 0u;
-    for (uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += warps) {
-        const SaKey k = sa_load_key(src, src_scope, i);
-        uint32_t lo = 0, hi = size;
-        if (lane == i / SA_SORT_TILE) lo = hi = i % SA_SORT_TILE;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (sa_key_less(sa_load_key(src, src_scope, base + mid), k)) lo = mid + 1;
-            else hi = mid;
+    const uint32_t lane = threadIdx.x & 7;
+    // a warp's four records stay together: i0 is the first
+    for (uint32_t i0 = blockIdx.x * 32 + (threadIdx.x >> 5) * 4; i0 < n; i0 += gridDim.x * 32) {
+        const uint32_t i = i0 + (threadIdx.x >> 3) % 4;
+        SaKey k = {0, 0, 0};
+        uint32_t lo = 0, hi = 0, group = 0;
+        if (i < n) {
+            k = sa_load_key(src, src_scope, i);
+            group = i / (8 * run) * (8 * run);
+            const uint32_t base = group + lane * run;
+            hi = base < n ? min(run, n - base) : 0u;
+            if (lane == i % (8 * run) / run) lo = hi = i % run;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (sa_key_less(sa_load_key(src, src_scope, base + mid), k)) lo = mid + 1;
+                else hi = mid;
+            }
         }
-        const uint32_t rank = __reduce_add_sync(0xffffffffu, lo);
-        if (lane == 0) sa_store_key<ORDER>(dst, dst_scope, rank, k, last);
+        __syncwarp();
+#pragma unroll
+        for (int x = 4; x >= 1; x >>= 1) lo += __shfl_xor_sync(0xffffffffu, lo, x);
+        if (lane == 0 && i < n) sa_store_key<ORDER>(dst, dst_scope, group + lo, k, last);
     }
 }
 
@@ -465,11 +478,14 @@ template <int ORDER>
 static int sa_merge_tiles(SaWork& w, int b, uint64_t n, const unsigned long long* d_n, cudaStream_t st) {
     const bool records = ORDER != kOrderDiag;
     if (n <= SA_SORT_TILE) return b;
-    if (n <= (uint64_t)SA_RANK_TILES * SA_SORT_TILE) {
-        const int g = (int)std::min<uint64_t>((n + 7) / 8, 148 * 8);
-        sa_k_rank<ORDER><<<g, 256, 0, st>>>(w.rec[b], w.scope[b], w.rec[b ^ 1], w.scope[b ^ 1], n, d_n, records);
-        sa_note_launch();
-        return b ^ 1;
+    if (n <= SA_RANK_MAX) {
+        const int g = (int)std::min<uint64_t>((n + 31) / 32, 148 * 8);
+        for (uint32_t run = SA_SORT_TILE; run < n; run *= 8, b ^= 1) {
+            sa_launch_next(sa_k_rank8<ORDER>, g, 256, st, w.rec[b], w.scope[b], w.rec[b ^ 1], w.scope[b ^ 1], n, d_n, run,
+                           8ull * run >= n && records);
+            sa_note_launch();
+        }
+        return b;
     }
     const unsigned g = (unsigned)((n + SA_MERGE_OUT - 1) / SA_MERGE_OUT);
     for (uint64_t run = SA_SORT_TILE; run < n; run *= 2, b ^= 1) {

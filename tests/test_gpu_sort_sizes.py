@@ -78,3 +78,30 @@ def test_repeat_masker(setup, n, rev, exclude):
         compare_segments(sf.rm_seed_and_filter(seeds, rev, lo, hi), run(seeds), f"{n} rm rev={rev} exclude={exclude}")
     finally:
         sf.set_rm_exclude_diagonal(False)
+
+
+@pytest.fixture(scope="module")
+def large(built):
+    rng = np.random.default_rng(22)
+    T, Q = random_text(rng, 2_200_000, gc=0.5), random_text(rng, 1_150_000, gc=0.5)
+    p = oracle.params(hspthresh=600, noentropy=True)
+    idx, pos = oracle.build_table(T, p)
+    sf = SeedFilter()
+    sf.initialize_interface(1)
+    sf.generate_shape_pos("12of19")
+    sf.initialize_processor(False, 1_200_000, 19, build_sub_mat(910), 910, 600, True)
+    sf.send_ref_write_request(T)
+    sf.generate_seed_pos_table(None, 1, 19, 12)
+    sf.send_query_write_request(Q, 0)
+    R, C = oracle.encode(T), oracle.encode(Q)
+    return sf, host_seeds(Q, 0, len(Q) - 19), lambda s: oracle.seed_and_filter(p, R, C, idx, pos, s, False)[0]
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 65_535, 65_536, 65_537, 131_071, 131_072, 131_073])
+def test_limits_of_rank_passes(large, n):
+    """One, two and three passes of eight runs each, and the merge passes above them."""
+    sf, words, run = large
+    seeds = _prefix(words, n, lambda s: len(run(s)) - 1)
+    want = run(seeds)
+    assert len(want) - 1 == n
+    compare_segments(sf.seed_and_filter(seeds, False, 0), want, f"{n} records")
