@@ -185,8 +185,7 @@ sa_k_lookup_count(const uint64_t* __restrict__ seeds, const SaCallDesc* __restri
 // word's index until sa_k_iterations, which also needs the hit prefix of every word.
 __global__ void __launch_bounds__(SA_CALL_BLOCK)
 sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restrict__ desc,
-                 const uint32_t* __restrict__ s_lo, const uint32_t* __restrict__ s_cnt,
-                 uint64_t* __restrict__ s_P, SaSeedList cs, const unsigned long long* cta_a,
+                 const uint32_t* s_lo, const uint32_t* s_cnt, uint64_t* s_P, SaSeedList cs, const unsigned long long* cta_a,
                  const unsigned long long* cta_b, SaCounters* ctr) {
     sa_wait_prior();
     sa_allow_next();
@@ -236,7 +235,7 @@ sa_k_lookup_emit(const uint64_t* __restrict__ seeds, const SaCallDesc* __restric
 // n - 1; a word's scope is the first iteration whose limit is at least its index.
 // Every CTA finds the limits for itself.
 __global__ void __launch_bounds__(256)
-sa_k_iterations(const uint64_t* __restrict__ P, const SaCallDesc* desc, SaSeedList cs, SaCounters* ctr) {
+sa_k_iterations(const uint64_t* P, const SaCallDesc* desc, SaSeedList cs, SaCounters* ctr) {
     sa_wait_prior();
     sa_allow_next();
     const uint64_t num_iter = ctr->num_iter;

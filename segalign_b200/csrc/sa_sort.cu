@@ -270,8 +270,8 @@ sa_k_tile_rm(SaHashSet hs, SaRec* dst, uint32_t n, bool exclude, unsigned long l
 // passes of 8 take 21, and go on past 32 tiles.)
 template <int ORDER>
 __global__ void __launch_bounds__(256)
-sa_k_rank8(const SaRec* __restrict__ src, const uint32_t* __restrict__ src_scope, SaRec* __restrict__ dst,
-           uint32_t* __restrict__ dst_scope, uint64_t n_max, const unsigned long long* d_n, uint32_t run, bool last) {
+sa_k_rank8(const SaRec* src, const uint32_t* src_scope, SaRec* dst, uint32_t* dst_scope, uint64_t n_max,
+           const unsigned long long* d_n, uint32_t run, bool last) {
     sa_wait_prior();
     const uint32_t n = (uint32_t)(d_n ? *d_n : n_max);
     const uint32_t lane = threadIdx.x & 7;
