@@ -385,7 +385,7 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // Bound by the L1 data pipe (83%: 96 table lookups and 128 wavefronts of target
 // loads in about 250 per round), with the ALU pipe and issue at 70%.  On a 2.5 Mbp query
 // against the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in
-// the lane kernel 5.65 ms; sweep 2.00, scans 0.81, finish 0.70: 3.33 ms, its launches
+// the lane kernel 5.65 ms; sweep 2.00, scans 0.81, finish 0.64: 3.31 ms, its launches
 // included (with the lane kernel after the sweep 3.75, and 4.79 without chains).  The chain test on all hits as they were
 // scored, with the rounds split evenly over the warps, made the sweep 2.33 ms.
 // Lane phase of 24 Mbp: 55.0 -> 30.8 ms.
@@ -766,7 +766,13 @@ __device__ __forceinline__ uint32_t sa_stop_offset(const char* tblb, const uint3
 // call's set of distinct HSPs (rm: query start flipped on the reverse strand,
 // repeat_masker_src/seed_filter.cu:704-707).  r: {ref_start, query_start (before
 // the rm flip), len, scope}; the candidate counts as `hits` survivors.  Called
-// by the whole warp.
+// by the whole warp.  LOOKUP: look it up in the set first (sa_set_query: the
+// query start of its key).
+__device__ __forceinline__ uint32_t sa_set_query(const SaExtK& a, uint32_t flags, const uint4& r) {
+    return (flags & 2u) ? a.ref_len - 1 - (r.y + r.z) : r.y;
+}
+
+template <bool LOOKUP>
 __device__ __forceinline__ void sa_keep_candidates(const SaExtK& a, bool on, uint4 r, int total, uint32_t unit,
                                                    uint32_t hits) {
     const int lane = threadIdx.x & 31;
@@ -776,12 +782,11 @@ __device__ __forceinline__ void sa_keep_candidates(const SaExtK& a, bool on, uin
     if (on) {
         const SaUnit U = a.units[unit];
         const int ext = (int)r.z;
-        qs = r.y;
-        if (U.flags & 2u) qs = a.ref_len - 1 - (qs + r.z);
+        qs = sa_set_query(a, U.flags, r);
         // A candidate whose key the set already holds was kept with this same
         // key (the scope fixes the unit, so the same bases): it is a survivor,
         // and its match counts, logs and insertion are skipped.
-        known = sa_hash_contains(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z);
+        known = LOOKUP && sa_hash_contains(a.hset, a.ctr->hash_mask, r.w, r.x, qs, r.z);
         if (known) {
             keep = 1;
         } else {
@@ -817,7 +822,7 @@ __device__ __forceinline__ void sa_flush_candidates(const SaExtK& a, const uint4
         x = s_ex[slot];
     }
     __syncwarp();  // slots are rewritten by later appends
-    sa_keep_candidates(a, on, r, (int)x.x, x.y, 1);
+    sa_keep_candidates<true>(a, on, r, (int)x.x, x.y, 1);
 }
 
 // Dynamic shared memory of the lane kernel for `tile` hits per warp tile.
@@ -1204,7 +1209,7 @@ sa_k_extend_lane(const __grid_constant__ SaExtK a, const __grid_constant__ SaPar
 // the lane kernel, which took both sides and the keep test, spent half of its
 // instructions around the steps.  Scans, chains and keep tests of 2.5 Mbp at
 // 1-in-500 differences, us: lane kernel and a kernel for the chains 1674, now
-// 1510 (scans 807); of a 1 Mbp call 203 -> 175.  A launch per side left two tails (248 -> 353 us
+// 1450 (scans 807); of a call of 250,000 positions 203 -> 175.  A launch per side left two tails (248 -> 353 us
 // where scans are long).  Batches shrink on short lists so that all warps have some.
 // ---------------------------------------------------------------------------
 #define SA_SCAN_BATCH 64
@@ -1419,8 +1424,9 @@ __device__ __forceinline__ uint32_t sa_listed_sides(SaListed& e) {
 // after it (sa_chain_members), which survive if its HSP is kept; and the keep
 // test.  A warp sorts its records into those that start chains and candidates,
 // and takes either 32 at a time: with a record per lane throughout the kernel
-// took 1.27 ms where this takes 0.70.  Of that the keep tests are 0.2, the chains
-// 0.2, and the rest is the pass over the records.
+// took 1.27 ms where this takes 0.64.  Candidates that the set holds already (most)
+// end with that look-up; the others gather again, because a few lanes of nearly every batch
+// counting matches cost 0.07 ms.  The chains are 0.2 ms.
 #define SA_FINISH_RING 128
 __global__ void __launch_bounds__(256, 4)
 sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) {
@@ -1428,6 +1434,7 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
     __shared__ int tbl[64];
     __shared__ uint32_t s_lead[8][SA_FINISH_RING];
     __shared__ uint2 s_cand[8][SA_FINISH_RING];  // {list index, survivors it stands for}
+    __shared__ uint4 s_seg[8][64], s_new[8][64];  // candidates that the set does not hold: segment, {total, unit, survivors}
     if (threadIdx.x < 64) tbl[threadIdx.x] = (P.sub_mat[(threadIdx.x & 7) * 8 + (threadIdx.x >> 3)] << SH) - 1;
     __syncthreads();
     const char* tblb = reinterpret_cast<const char*>(tbl);
@@ -1439,8 +1446,10 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
     const uint32_t lt = sa_lanemask_lt();
     uint32_t* const lead = s_lead[threadIdx.x >> 5];
     uint2* const cand = s_cand[threadIdx.x >> 5];
-    uint32_t l0 = 0, l1 = 0, c0 = 0, c1 = 0;  // ring cursors
-    unsigned long long tiles = 0;
+    uint4* const fresh_seg = s_seg[threadIdx.x >> 5];
+    uint4* const fresh = s_new[threadIdx.x >> 5];
+    uint32_t l0 = 0, l1 = 0, c0 = 0, c1 = 0, f0 = 0, f1 = 0;  // ring cursors
+    unsigned long long tiles = 0, known = 0;
     for (unsigned long long i0 = (blockIdx.x * 8ull + (threadIdx.x >> 5)) * 32;; i0 += gridDim.x * 256ull) {
         const bool done = i0 >= n;
         const unsigned long long i = i0 + lane;
@@ -1487,28 +1496,51 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
         }
         while (c1 - c0 >= 32 || (done && c1 != c0)) {
             const bool on = lane < (int)(c1 - c0);
-            uint4 seg = make_uint4(0, 0, 0, 0);
-            uint32_t unit = 0, hits = 0;
-            int total = 0;
+            uint4 seg = make_uint4(0, 0, 0, 0), x = seg;
+            bool is_new = false;
             if (on) {
-                const uint2 x = cand[(c0 + lane) % SA_FINISH_RING];
-                SaListed e = sa_listed(a, x.x);
+                const uint2 c = cand[(c0 + lane) % SA_FINISH_RING];
+                SaListed e = sa_listed(a, c.x);
                 sa_listed_sides(e);
                 const uint32_t left = e.l.y + 1;  // left offsets are 1-based, 0 when best is 0
                 seg = make_uint4(e.h.x - left, e.h.y - left, e.r.y + left, e.h.z);
-                total = (int)e.r.x + (int)e.l.x;
-                unit = e.h.w & ~SA_CHAIN_NEXT;
-                hits = x.y;
+                x = make_uint4(e.r.x + e.l.x, e.h.w & ~SA_CHAIN_NEXT, c.y, 0);
+                // a key in the set was kept: see sa_keep_candidates
+                is_new = !sa_hash_contains(a.hset, ctr->hash_mask, seg.w, seg.x,
+                                           sa_set_query(a, a.units[x.y].flags, seg), seg.z);
+                if (!is_new) known += c.y;
             }
             c0 += min(c1 - c0, 32u);
+            const uint32_t m = __ballot_sync(SA_FULL, is_new);
+            if (is_new) {
+                fresh_seg[(f1 + __popc(m & lt)) % 64] = seg;
+                fresh[(f1 + __popc(m & lt)) % 64] = x;
+            }
+            f1 += __popc(m);
             __syncwarp();
-            sa_keep_candidates(a, on, seg, total, unit, hits);
+            if (f1 - f0 >= 32) {
+                seg = fresh_seg[(f0 + lane) % 64];
+                x = fresh[(f0 + lane) % 64];
+                f0 += 32;
+                __syncwarp();
+                sa_keep_candidates<false>(a, true, seg, (int)x.x, x.y, x.z);
+            }
+        }
+        if (done && f1 != f0) {
+            const bool on = lane < (int)(f1 - f0);
+            const uint4 seg = fresh_seg[(f0 + lane) % 64], x = fresh[(f0 + lane) % 64];
+            f0 = f1;
+            sa_keep_candidates<false>(a, on, seg, (int)x.x, x.y, x.z);
         }
         if (done) break;
     }
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) tiles += __shfl_xor_sync(SA_FULL, tiles, s);
+    for (int s = 16; s >= 1; s >>= 1) {
+        tiles += __shfl_xor_sync(SA_FULL, tiles, s);
+        known += __shfl_xor_sync(SA_FULL, known, s);
+    }
     if (lane == 0 && tiles) atomicAdd(&ctr->base_steps, tiles);
+    if (lane == 0 && known) atomicAdd(&ctr->surv_count, known);
 }
 
 // Between the segments of a large batch: the list and the queue start again
