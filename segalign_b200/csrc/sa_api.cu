@@ -527,6 +527,7 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     xa.hspthresh = g.params.hspthresh;
     xa.noentropy = g.params.noentropy;
     xa.windowed = mode == 1 ? 1 : 0;
+    xa.ctas = mode == 1 ? g.tuning.rm_lane_ctas : g.tuning.call_lane_ctas;
     sa_launch_extend_lane(w, xa, g.params, cg.lane_tuning, d.num_sms, st, cg.lane_ctas);
     tm.mark(2);
     sa_launch_extend_warp(w, xa, g.params, g.tuning, d.num_sms, st);

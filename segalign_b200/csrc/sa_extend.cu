@@ -1891,7 +1891,7 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
     // and the next of its own (2, 3 and 4 CTAs per SM, ms: 250,000 positions against 100 Mbp 0.323, 0.292, 0.294;
     // against 1 Mbp 0.028, 0.030, 0.033; the 40 calls of a 5 Mbp seeder run on 12 slots
     // 15.4, 15.8, 16.5).
-    const int grid = num_sms * (grid_ctas > 0 ? 3 : 4);
+    const int grid = x.ctas > 0 ? x.ctas : num_sms * (grid_ctas > 0 ? 3 : 4);
     uint64_t h0 = 0;
     do {
         const uint64_t h1 = x.hits > h0 + seg ? h0 + seg : ~0ull;

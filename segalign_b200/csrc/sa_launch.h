@@ -202,6 +202,8 @@ struct SaExtendArgs {
     int32_t chain = 0;
     int32_t sweep = 0;   // 1: the sweep takes the hits first (if the scores allow the fast form)
     uint64_t hits = 0;   // the call's hits, where the caller has read them
+    // CTAs of a call's sweep, scan and finish (call_lane_ctas, rm_lane_ctas); 0: chosen by sa_launch_extend_lane
+    int ctas = 0;
 };
 // Phase A (lane per hit) and phase B (warp per long hit); B must follow A.
 // grid: CTAs of the persistent launch (0: num_sms x ext_ctas_per_sm).

@@ -182,6 +182,7 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
     xa.xdrop = v.params.xdrop;
     xa.hspthresh = v.params.hspthresh;
     xa.noentropy = v.params.noentropy;
+    xa.ctas = v.tuning.call_lane_ctas;
     SaCounters c;
     for (bool sweep = true;; sweep = false) {  // again without the sweep if its list was too small
         xa.sweep = sweep ? 1 : 0;
