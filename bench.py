@@ -109,14 +109,19 @@ def seeder_calls(query_len: int):
     return calls
 
 
+EXTEND_KERNELS = "sa_k_sweep, sa_k_scan and sa_k_finish"  # the "extend_lane" phase of the default parameters
+
+
 def lane_traffic(hits: float, workload: str):
-    """DRAM bytes (read + write) of one lane-kernel launch, scaled by hits from
-    the ncu capture of this workload recorded in profiles/extend_lane_dram.json;
-    (None, why) if there is none."""
+    """DRAM bytes (read + write) of one pass's sweep, scans and finish, scaled by
+    hits from the ncu capture of this workload recorded in
+    profiles/extend_lane_dram.json; (None, why) if there is none."""
     path = os.path.join(ROOT, "profiles", "extend_lane_dram.json")
     try:
         with open(path) as f:
             d = json.load(f)[workload]
+        if d["kernel"] != EXTEND_KERNELS:
+            return None, f"the capture recorded for the {workload} workload is of {d['kernel']}"
         per_hit = float(d["dram_bytes"]) / float(d["hits"])
     except (OSError, KeyError, ValueError, ZeroDivisionError, TypeError):
         return None, f"no ncu capture recorded for the {workload} workload"
@@ -124,8 +129,8 @@ def lane_traffic(hits: float, workload: str):
 
 
 def lane_limit(workload: str):
-    """The lane kernel's measured issue-bound limit (ncu full capture) recorded
-    beside its DRAM traffic in profiles/extend_lane_dram.json, or None."""
+    """The sweep's measured limit (ncu) recorded beside the DRAM traffic in
+    profiles/extend_lane_dram.json, or None."""
     try:
         with open(os.path.join(ROOT, "profiles", "extend_lane_dram.json")) as f:
             return json.load(f)[workload].get("issue")
@@ -597,7 +602,7 @@ def run_ours(args):
     job = job_figures(ms_step, float(hits), float(hsps), dist)
     ms_step_max, hits_all, hsps_all, value = job["ms_per_step"], job["extensions"], job["hsps"], job["value"]
 
-    # roofline of the dominant kernel (lane-per-hit X-drop): algorithmic bytes
+    # roofline of the extension (sweep, scans, finish): algorithmic bytes
     # = 24 B per hit-bearing seed (E, lo, j, scope, unit) + 4 B per hit (pos)
     # + 24 B per 32-base tile scanned (2 sequences x 32 bases x 3 bits)
     # + 16 B per surviving HSP record
@@ -607,7 +612,7 @@ def run_ours(args):
     achieved = alg_bytes / (lane_ms_avg / 1000.0) / 1e9
     traffic, traffic_src = lane_traffic(hits, args.workload)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "traffic_source": traffic_src, "kernel": "sa_k_extend_lane",
+                "traffic": traffic, "traffic_source": traffic_src, "kernel": EXTEND_KERNELS,
                 "peak_source": peak_src, "alg_bytes_per_launch": alg_bytes, "launch_ms": lane_ms_avg,
                 "limit": lane_limit(args.workload)}
 
@@ -844,7 +849,7 @@ def run_large(sf, args, flush, barrier) -> dict:
            "device_ms_per_step": tb["dev_ms"], "extensions_per_step": st["num_hits"], "hsps_per_step": st["num_hsps"],
            "phase_ms": {"lookup": tb["lookup_ms"], "extend_lane": tb["lane_ms"], "extend_warp": tb["warp_ms"],
                         "dedup": tb["dedup_ms"]},
-           "roofline": {"kernel": "sa_k_extend_lane", "achieved": alg / (tb["lane_ms"] / 1000) / 1e9, "peak": peak,
+           "roofline": {"kernel": EXTEND_KERNELS, "achieved": alg / (tb["lane_ms"] / 1000) / 1e9, "peak": peak,
                         "frac": alg / (tb["lane_ms"] / 1000) / 1e9 / peak, "unit": "GB/s",
                         "traffic": lane_traffic(st["num_hits"], "large")[0]}}
     outs = tb["outs"]
