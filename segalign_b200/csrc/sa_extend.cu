@@ -1576,7 +1576,9 @@ __device__ __forceinline__ int sa_warp_incl_max(int v) {
 }
 
 // Rightward scan from base sr of R and sq of Q; `avail` bases until either
-// ends.  A base past the end scores -(xdrop + 1), which stops the scan there.
+// ends.  The end stops the scan by itself, whatever the scores and xdrop (which
+// has no upper limit): a base past it scores 0, and the lane that holds the
+// first of them stops there.
 // tblb: plain scores.
 __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restrict__ R, const uint32_t* __restrict__ Q,
                                      uint32_t sr, uint32_t sq, uint32_t avail, int xdrop) {
@@ -1607,7 +1609,7 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
         int ps[8], p = 0, lmax = INT_MIN, lmin = INT_MAX;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            p += (uint32_t)k < in ? sa_tbl(tblb, lo, hi, k) : -(xdrop + 1);
+            p += (uint32_t)k < in ? sa_tbl(tblb, lo, hi, k) : 0;
             ps[k] = p;
             lmax = max(lmax, p * 8 + 7 - k);
             lmin = min(lmin, p);
@@ -1618,7 +1620,7 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
         const int im = sa_warp_incl_max(amax);
         int before = __shfl_up_sync(SA_FULL, im, 1);
         before = lane ? max(best, before) : best;
-        const bool possible = max(before, amax) - (base + lmin) > xdrop;
+        const bool possible = in < 8 || max(before, amax) - (base + lmin) > xdrop;
         if (__any_sync(SA_FULL, possible)) {
             // exact test of the lanes where a stop is possible
             int stop_k = -1, bmax = INT_MIN, bmax_k = 0;
@@ -1629,7 +1631,7 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
                     if (stop_k < 0) {
                         const int Sv = base + ps[k];
                         M = max(M, Sv);
-                        if (M - Sv > xdrop) {
+                        if ((uint32_t)k >= in || M - Sv > xdrop) {
                             stop_k = k;
                         } else if (Sv > bmax) {
                             bmax = Sv;

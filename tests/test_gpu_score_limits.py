@@ -1,0 +1,74 @@
+"""GPU tests of scans with scores and X-drops far from the default table's: the
+end of a sequence ends every scan whatever these are.  HSP lists and the
+statistics of every hit equal the oracle's."""
+import numpy as np
+import pytest
+
+import oracle
+from segalign_b200 import SeedFilter, build_sub_mat, host_revcomp, host_seeds
+from tests.helpers import compare_segments, random_text
+
+pytestmark = pytest.mark.gpu
+
+
+def _filter(p, sub, xdrop, hspthresh):
+    """A filter with these scores, and the oracle's parameters set alike."""
+    sf = SeedFilter()
+    sf.initialize_interface(1)
+    sf.generate_shape_pos("12of19")
+    sf.initialize_processor(False, 20_000, 19, sub, xdrop, hspthresh, bool(p.noentropy))
+    p.sub_mat[:] = [int(x) for x in sub]
+    p.xdrop, p.hspthresh = xdrop, hspthresh
+    return sf
+
+
+def _pair(rng, n):
+    """A target and a query of its pieces, from like to unlike."""
+    t = np.frombuffer(random_text(rng, n), dtype=np.uint8).copy()
+    q = t.copy()
+    for k in range(0, n, 300):
+        m = rng.random(len(q[k:k + 300])) < 0.3 * k / n
+        q[k:k + 300][m] = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(0, 4, int(m.sum()))]
+    return t.tobytes(), q.tobytes()
+
+
+def _check_calls(sf, p, T, Q, calls, what):
+    """Plain calls and one batched call on the windows `calls` of both strands."""
+    idx, pos = oracle.build_table(T, p)
+    sf.send_ref_write_request(T)
+    sf.generate_seed_pos_table(None, 1, 19, 12)
+    sf.send_query_write_request(Q, 0)
+    R, units, wants, total = oracle.encode(T), [], [], 0
+    for rev in (False, True):
+        text = host_revcomp(Q) if rev else Q
+        for a, b in calls:
+            seeds = host_seeds(text, a, b)
+            want, st = oracle.seed_and_filter(p, R, oracle.encode(text), idx, pos, seeds, rev)
+            compare_segments(sf.seed_and_filter(seeds, rev, 0), want, f"{what} {(rev, a, b)}")
+            cs = sf.last_call_stats()
+            assert cs["tiles"] == st["tiles_right"] + st["tiles_left"], (what, rev, a, b)
+            assert cs["survivors"] == st["survivors"] and cs["hits_extended"] == st["hits_extended"], (what, rev, a, b)
+            units.append((0, int(rev), a, b))
+            wants.append(want)
+            total += st["tiles_right"] + st["tiles_left"]
+    for u, got, want in zip(units, sf.seed_and_filter_batch(units), wants):
+        compare_segments(got, want, f"{what} unit {u}")
+    assert sf.last_call_stats()["tiles"] == total, what
+    return wants
+
+
+@pytest.mark.parametrize("xdrop", [1 << 25, 1 << 28, 1 << 30, 2_000_000_000, 2**31 - 1])
+@pytest.mark.parametrize("lane_cap", [64, 8192])
+def test_scans_that_only_a_sequence_end_stops(built, xdrop, lane_cap):
+    """lane_cap 64: the warp kernel ends them; 8192: the lanes do."""
+    T, Q = _pair(np.random.default_rng(31), 3001)
+    p = oracle.params()
+    sf = _filter(p, build_sub_mat(910), xdrop, 3000)
+    saved = sf.get_tuning()
+    sf.set_tuning(lane_cap=lane_cap)
+    try:
+        L = len(Q) - 19
+        wants = _check_calls(sf, p, T, Q, ((0, L), (700, 1200), (L - 40, L)), f"xdrop {xdrop} lane_cap {lane_cap}")
+        assert sum(len(w) - 1 for w in wants) > 0
+    finally:
+        sf.set_tuning(lane_cap=saved["lane_cap"])
