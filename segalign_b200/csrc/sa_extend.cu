@@ -570,12 +570,14 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                         if (i == 4) tl = stop_l ? 2 : 3;  // tiles of both scans, if they stop
                     }
                     x.y = sa_swept_word(p, at);
-                    // where a window reaches past a sequence end, the scans start anew
+                    // where a window reaches past a sequence end, it holds scores of padding: nothing
+                    // of it is passed on, and the scans start anew
                     const bool inside = min(rl, ql) >= SA_SWEEP_LEFT && (uint64_t)rl + SA_SWEEP_RIGHT <= a.ref_len &&
                                         (uint64_t)ql + SA_SWEEP_RIGHT <= U.q_len;
                     left = !inside || !stop_r || !stop_l || (int)(float)(best_r + (at >> SA_SWEEP_SH)) >= a.hspthresh;
-                    x.z |= (sa_swept_pos(at) << 8) | (inside ? SA_SWEPT_SEEN : 0u) | (stop_r ? SA_SWEPT_STOP_R : 0u) |
-                           (stop_l ? SA_SWEPT_STOP_L : 0u) | (tl == 3 ? SA_SWEPT_TILE_2 : 0u);
+                    x.z = inside ? x.z | (sa_swept_pos(at) << 8) | SA_SWEPT_SEEN | (stop_r ? SA_SWEPT_STOP_R : 0u) |
+                                       (stop_l ? SA_SWEPT_STOP_L : 0u) | (tl == 3 ? SA_SWEPT_TILE_2 : 0u)
+                                 : 0u;
                     if (!left) tiles += tl;
                     if (!(stop_r && !stop_l) && sa_sweep_margin(a, U, rl, ql)) rec.w |= SA_CHAIN_DROP;
                 }

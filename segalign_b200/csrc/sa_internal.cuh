@@ -4,8 +4,8 @@
 // ("nibble-packed"), base i in bits [4*(i&7), 4*(i&7)+4) of word i>>3.  Codes
 // are the reference's (common/parameters.h:4-11): A0 C1 G2 T3 L4 N5 X6 E7.
 // Every packed array carries SA_PADW words of padding on both sides (filled
-// with E codes) so that 8-base windows next to either end can be loaded
-// without bounds checks; scoring itself never reads past the sequence.
+// with E codes) so that windows next to either end can be loaded without bounds
+// checks; what they score past the sequence goes into no result.
 // Every packed sequence of the library is followed, in the same allocation,
 // by its reversed copy (base i = base len-1-i of the sequence, with its own
 // padding): word 0 of the copy lies sa_rev_words(len) words after word 0 of

@@ -72,3 +72,19 @@ def test_scans_that_only_a_sequence_end_stops(built, xdrop, lane_cap):
         assert sum(len(w) - 1 for w in wants) > 0
     finally:
         sf.set_tuning(lane_cap=saved["lane_cap"])
+
+
+@pytest.mark.parametrize("end", [-9100, -911, -910, -100, 0, 60])
+@pytest.mark.parametrize("xdrop", [910, 3000])
+def test_scores_of_codes_past_the_ends(built, end, xdrop):
+    """Hits next to both ends of both sequences: what a table gives for the code
+    that fills the padding (E) is never counted, in lists or in tiles."""
+    T, Q = _pair(np.random.default_rng(32), 2011)
+    p = oracle.params()
+    sub = build_sub_mat(910).reshape(8, 8)
+    sub[7, :] = sub[:, 7] = end
+    sf = _filter(p, sub.reshape(-1), xdrop, 2200)
+    for t, q in ((T, Q), (T[:150], Q[:131]), (T[700:], Q[700:1100]), (T[:411], T[303:411]), (T[1900:], T[1900:]),
+                 (T[77:120], T[77:120])):
+        L = len(q) - 19
+        _check_calls(sf, p, t, q, ((0, L), (0, min(L, 70)), (max(0, L - 70), L)), f"E {end} xdrop {xdrop} {len(t)}x{len(q)}")
