@@ -1607,18 +1607,21 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
         uint32_t lo, hi;
         sa_merge8(__funnelshift_r(r0, r1, shr), __funnelshift_r(q0, q1, shq), lo, hi);
         fetch(o + 256);
-        // prefix sums; (largest << 3) | (7 - its first base) in lmax
-        int ps[8], p = 0, lmax = INT_MIN, lmin = INT_MAX;
+        // prefix sums; the largest and its first base
+        int ps[8], p = 0, lmax = INT_MIN, lmax_k = 0, lmin = INT_MAX;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             p += (uint32_t)k < in ? sa_tbl(tblb, lo, hi, k) : 0;
             ps[k] = p;
-            lmax = max(lmax, p * 8 + 7 - k);
+            if (p > lmax) {
+                lmax = p;
+                lmax_k = k;
+            }
             lmin = min(lmin, p);
         }
         const int incl = sa_warp_incl_sum(p);
         const int base = S_prev + incl - p;
-        const int amax = base + (lmax >> 3);
+        const int amax = base + lmax;
         const int im = sa_warp_incl_max(amax);
         int before = __shfl_up_sync(SA_FULL, im, 1);
         before = lane ? max(best, before) : best;
@@ -1649,7 +1652,7 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
                 const int top = __reduce_max_sync(SA_FULL, cv);
                 if (top > best) {
                     const int src = __ffs(__ballot_sync(SA_FULL, cv == top)) - 1;
-                    bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)(lane == f ? bmax_k : 7 - (lmax & 7)), src);
+                    bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)(lane == f ? bmax_k : lmax_k), src);
                     best = top;
                 }
                 return {best, bpos, __shfl_sync(SA_FULL, loff + (uint32_t)stop_k, f)};
@@ -1658,7 +1661,7 @@ __device__ SaDirResult sa_warp_xdrop(const char* tblb, const uint32_t* __restric
         const int top = __shfl_sync(SA_FULL, im, 31);
         if (top > best) {
             const int src = __ffs(__ballot_sync(SA_FULL, amax == top)) - 1;
-            bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)(7 - (lmax & 7)), src);
+            bpos = (int)__shfl_sync(SA_FULL, loff + (uint32_t)lmax_k, src);
             best = top;
         }
         S_prev += __shfl_sync(SA_FULL, incl, 31);

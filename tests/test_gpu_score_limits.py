@@ -88,3 +88,26 @@ def test_scores_of_codes_past_the_ends(built, end, xdrop):
                  (T[77:120], T[77:120])):
         L = len(q) - 19
         _check_calls(sf, p, t, q, ((0, L), (0, min(L, 70)), (max(0, L - 70), L)), f"E {end} xdrop {xdrop} {len(t)}x{len(q)}")
+
+
+@pytest.mark.parametrize("bits", [24, 26])
+def test_large_scores_in_the_warp_kernel(built, bits):
+    """Scores whose sums over 8 bases pass 2^28, totals below 2^31; every hit passes the lane cap."""
+    rng = np.random.default_rng(33)
+    T = np.frombuffer(random_text(rng, 6000, gc=0.5), dtype=np.uint8)
+    Q = np.frombuffer(random_text(rng, 4000, gc=0.5), dtype=np.uint8).copy()
+    for k in range(0, 4000, 40):
+        at = int(rng.integers(0, 5900))
+        Q[k + 9:k + 31] = T[at:at + 22]
+    sub = np.full((8, 8), -(1 << bits), dtype=np.int32)
+    np.fill_diagonal(sub[:4, :4], 1 << bits)
+    p = oracle.params(noentropy=True)
+    sf = _filter(p, sub.reshape(-1), 3 << bits, 14 << bits)
+    saved = sf.get_tuning()
+    sf.set_tuning(lane_cap=8, step_bases=8)
+    try:
+        L = len(Q) - 19
+        wants = _check_calls(sf, p, T.tobytes(), Q.tobytes(), ((0, L), (L // 2, L)), f"scores of 2^{bits}")
+        assert len(wants[0]) - 1 > 50 and max(int(w["score"].max()) for w in wants) < 31 << bits
+    finally:
+        sf.set_tuning(lane_cap=saved["lane_cap"], step_bases=saved["step_bases"])
