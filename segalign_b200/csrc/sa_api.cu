@@ -622,7 +622,7 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     t_stats.hits_extended = c.extended;
     t_stats.seeds_with_hits = c.nnz;
     t_stats.survivors = c.surv_count;
-    t_stats.long_hits = c.long_count;
+    t_stats.long_hits = c.long_count - c.long_again;
     t_stats.tiles = c.base_steps;
     t_stats.num_iter = (uint32_t)c.num_iter;
     t_stats.batch_calls = 1;
@@ -836,7 +836,7 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     res.tot.nnz += c.nnz;
     res.tot.surv_count += c.surv_count;
     res.tot.uniq_count += nh;
-    res.tot.long_count += c.long_count;
+    res.tot.long_count += c.long_count - c.long_again;
     res.tot.base_steps += c.base_steps;
     std::vector<unsigned long long> hb(n), he(n);
     std::vector<uint32_t> cnt(n);

@@ -400,6 +400,7 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 #define SA_SWEPT_STOP_L 0x40000u
 #define SA_SWEPT_TILE_2 0x80000u   // the left scan stopped in its second 32-base tile
 #define SA_SWEPT_LONG 0x100000u    // the hit went to the long queue (set by sa_k_scan)
+#define SA_SWEPT_FULL 0x200000u    // a side passed the cap and found the queue full
 
 // One 8-base window of a scan, from its first base on (REV: from base 7
 // down), in the lane kernel's packed form with SA_SWEEP_LEFT in place of STEP
@@ -1381,22 +1382,27 @@ sa_k_scan(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P) 
             const int leader = __ffs(lm) - 1;
             if (lane == leader) base = atomicAdd(&ctr->long_count, (unsigned long long)__popc(lm));
             base = __shfl_sync(SA_FULL, base, leader) + __popc(lm & lt);
+            bool again = false;
             if (to_long) {
+                uint4* const rec = a.list + (idx & ~1u);
+                const uint32_t was = atomicOr(&rec[1].z, base < a.long_cap ? SA_SWEPT_LONG : SA_SWEPT_FULL);
+                again = was & (SA_SWEPT_LONG | SA_SWEPT_FULL);
                 if (base < a.long_cap) {
-                    uint4* const rec = a.list + (idx & ~1u);
                     const uint4 h = rec[0];
                     SaLongHit e;
                     e.ref_loc = h.x;
                     e.query_loc = h.y;
-                    e.unit = atomicOr(&rec[1].z, SA_SWEPT_LONG) & SA_SWEPT_LONG ? SA_LONG_NONE : h.w;  // once per hit
+                    e.unit = was & SA_SWEPT_LONG ? SA_LONG_NONE : h.w;  // once per hit
                     e.scope = h.z;
                     a.long_q[base] = e;
                     has = false;
                 } else {
-                    nocap = true;  // queue full: finish this hit in the lane
+                    nocap = true;  // queue full: finish this side in the lane
                     atomicAdd(&ctr->long_overflow, 1ull);
                 }
             }
+            const uint32_t am = __ballot_sync(SA_FULL, again);
+            if (lane == 0 && am) atomicAdd(&ctr->long_again, (unsigned long long)__popc(am));
         }
     }
 }

@@ -89,13 +89,13 @@ struct SaCounters {
     unsigned long long num_hits;       // total hits (ungapped extensions)
     unsigned long long nnz;            // seeds with >= 1 hit
     unsigned long long hit_cursor;     // extension work counter
-    unsigned long long long_count;     // hits in the long queue
+    unsigned long long long_count;     // pushes to the long queue (the lane kernel's hits, the scans' sides)
     unsigned long long long_cursor;
     unsigned long long surv_count;     // survivors appended
     unsigned long long extended;       // hits actually extended (rm window)
     unsigned long long base_steps;     // bases scored
     unsigned long long long_overflow;  // long-queue pushes refused (handled in place)
-    unsigned long long surv_overflow;  // survivor appends refused -> error
+    unsigned long long long_again;     // pushes among them by the second side of a hit
     unsigned long long uniq_count;     // records after dedup
     unsigned long long num_iter;       // MAX_HITS iterations
     unsigned long long error;          // nonzero = device-side error code
