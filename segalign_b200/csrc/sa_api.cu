@@ -126,6 +126,7 @@ struct Slot {
     uint64_t graph_key = 0;
     uint64_t graph_kernels = 0;
     bool graph_off = false;  // capture failed once: launch directly
+    bool segments = false;   // the call at hand has more hits than one sweep's list is sure to hold
     bool no_sweep = false;   // the call at hand runs without the sweep (its list was too small)
     uint32_t max_units = 64;  // units per batched pass (batched kinds)
 };
@@ -528,6 +529,10 @@ int launch_call_chain(Slot* s, int mode, PhaseTimer& tm) {
     xa.noentropy = g.params.noentropy;
     xa.windowed = mode == 1 ? 1 : 0;
     xa.ctas = mode == 1 ? g.tuning.rm_lane_ctas : g.tuning.call_lane_ctas;
+    if (s->segments && !s->no_sweep) {
+        SA_CUDA_OK(sa_read_hits(w, s->h_ctr, st));
+        xa.hits = s->h_ctr->num_hits;
+    }
     sa_launch_extend_lane(w, xa, g.params, cg.lane_tuning, d.num_sms, st, cg.lane_ctas);
     tm.mark(2);
     sa_launch_extend_warp(w, xa, g.params, g.tuning, d.num_sms, st);
@@ -545,11 +550,13 @@ bool graphs_enabled() {
 // Runs the call chain: replays the slot's CUDA graph, capturing it first when
 // the chain changed (mode, or anything invalidate_graphs covers).
 int run_chain(Slot* s, int mode, PhaseTimer& tm) {
-    // phase timing (a diagnostic mode) records events between the kernels: direct launches
-    if (!graphs_enabled() || s->graph_off || tm.on) return launch_call_chain(s, mode, tm);
+    // Direct launches: phase timing (a diagnostic mode) records events between the
+    // kernels, and a call in segments or without the sweep has another chain than the
+    // captured one, which stays.
+    if (!graphs_enabled() || s->graph_off || tm.on || s->segments || s->no_sweep) return launch_call_chain(s, mode, tm);
     Global& g = G();
     cudaStream_t st = s->stream;
-    const uint64_t key = (g_graph_gen.load() << 2) | (uint64_t)(s->no_sweep ? 2 : 0) | (uint64_t)mode;
+    const uint64_t key = (g_graph_gen.load() << 1) | (uint64_t)mode;
     if (!s->graph || s->graph_key != key) {
         if (s->graph) cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
@@ -608,13 +615,18 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     tm.mark(0);
     SA_CUDA_OK(cudaMemcpyAsync(w.seeds, seeds, 8ull * n, cudaMemcpyHostToDevice, st));
     SaCounters c;
-    for (s->no_sweep = false;; s->no_sweep = true) {
+    s->no_sweep = false;
+    s->segments = sa_expect_segments(n, d.num_index, d.nbuckets, w.list_cap);
+    while (true) {
         if (!w.hash_clean) sa_launch_hash_clear(w, st);
         w.hash_clean = false;  // until this call is seen to complete
         SA_TRY(run_chain(s, mode, tm));
         SA_CUDA_OK(cudaStreamSynchronize(st));
         c = *s->h_ctr;
         if (c.list_count <= w.list_cap) break;
+        // the list was too small: again
+        if (!s->segments && c.num_hits > sa_sweep_segment(w.list_cap)) s->segments = true;
+        else s->no_sweep = true;
     }
     std::memset(&t_stats, 0, sizeof t_stats);
     t_stats.num_seeds = n;
@@ -750,7 +762,7 @@ struct BatchResult {
 // Runs units [u0, u1) in one device pass.  Returns SA_ERR_CAPACITY when the
 // survivors do not fit (the caller splits the range).
 int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t u0, uint32_t u1, bool want_out,
-                    BatchResult& res, bool sweep = true) {
+                    BatchResult& res, bool sweep = true, bool segments = false) {
     Global& g = G();
     SaWork& w = s->w;
     cudaStream_t st = s->stream;
@@ -808,9 +820,9 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     xa.chain = chain ? 1 : 0;
     xa.sweep = sweep ? 1 : 0;
     // so many seed slots that the hits may need several segments: read their number
-    if ((double)slots * ((double)d.num_index / (double)d.nbuckets + 1.0) > (double)w.list_cap) {
-        SA_CUDA_OK(cudaMemcpyAsync(s->h_ctr, w.ctr, sizeof(SaCounters), cudaMemcpyDeviceToHost, st));
-        SA_CUDA_OK(cudaStreamSynchronize(st));
+    if ((double)slots * ((double)d.num_index / (double)d.nbuckets + 1.0) > (double)w.list_cap) segments = true;
+    if (segments && sweep) {
+        SA_CUDA_OK(sa_read_hits(w, s->h_ctr, st));
         xa.hits = s->h_ctr->num_hits;
     }
     sa_launch_extend_lane(w, xa, g.params, g.tuning, d.num_sms, st);
@@ -823,7 +835,10 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     SaCounters c = *s->h_ctr;
     const int bad = sa_check_set(w, c);
     if (bad == SA_DERR_SURV_OVERFLOW) return SA_ERR_CAPACITY;
-    if (c.list_count > w.list_cap) return run_batch_group(d, s, units, u0, u1, want_out, res, false);
+    if (c.list_count > w.list_cap) {
+        const bool split = !segments && c.num_hits > sa_sweep_segment(w.list_cap);
+        return run_batch_group(d, s, units, u0, u1, want_out, res, split, split);
+    }
     if (bad) return map_device_error(bad);
     const uint64_t nh = c.hash_used;
     const int buf = sa_launch_sort(w, nh, st);
@@ -1962,6 +1977,7 @@ int sa_resident_view(uint32_t buffer, SaResidentView* v) {
     v->ref_len = (uint32_t)d.ref.len;
     v->index = d.index;
     v->nbuckets = d.nbuckets;
+    v->num_index = d.num_index;
     v->pos = d.pos;
     v->q_packed[0] = d.qf[buffer].data;
     v->q_packed[1] = d.qr[buffer].data;

@@ -436,6 +436,7 @@ __device__ __forceinline__ uint32_t sa_swept_pos(int at) {
 }
 
 #define SA_SWEEP_BUF 128  // unfinished hits a warp gathers
+#define SA_SWEEP_END (1ull << 48)  // sweep cursor past every run
 
 template <bool TRANS>
 __global__ void __launch_bounds__(256, 4)
@@ -489,6 +490,8 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)kept);
         at = __shfl_sync(SA_FULL, at, 0);
+        // too small a list: the call runs again, the rest of this sweep is given up
+        if (lane == 0 && at + kept > a.list_cap) atomicMax(&ctr->sweep_cursor, SA_SWEEP_END);
         for (uint32_t i = lane; i < 2 * kept; i += 32)
             if (at + (i >> 1) < a.list_cap) a.list[2 * at + i] = (i & 1) ? swept[i >> 1] : buf[i >> 1];
         __syncwarp();
@@ -1551,11 +1554,12 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
     if (lane == 0 && known) atomicAdd(&ctr->surv_count, known);
 }
 
-// Between the segments of a large batch: the list and the queue start again
-// (an overflow stays to be seen).
+// Between the segments of a call: the list starts again (the queue of long hits goes
+// on, for the warp kernel after the last one).  An overflow stays to be seen, and
+// the sweeps after it have nothing left to do.
 __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
-    if (ctr->list_count <= list_cap) ctr->list_count = 0;
-    ctr->sweep_cursor = ctr->scan_cursor = 0;
+    if (ctr->list_count > list_cap) return;
+    ctr->list_count = ctr->sweep_cursor = ctr->scan_cursor = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1896,10 +1900,10 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& x, const SaParams& p, 
         sa_note_launch();
         return;
     }
-    // Segments of hits whose list is sure to fit in practice; one unless the
-    // caller knows of more hits (x.hits).  A list that overflows all the same is
-    // seen by the host (list_count), which runs the call again without the sweep.
-    const uint64_t seg = 4 * a.list_cap & ~31ull;
+    // One segment unless the caller knows of more hits (x.hits).  A list that
+    // overflows is seen by the host (list_count), which runs the call again: in segments
+    // where one sweep had more hits than that, else without the sweep.
+    const uint64_t seg = sa_sweep_segment(a.list_cap);
     // A batch fills the chip; a call leaves a place per SM to the kernels beside it
     // and the next of its own (2, 3 and 4 CTAs per SM, ms: 250,000 positions against 100 Mbp 0.323, 0.292, 0.294;
     // against 1 Mbp 0.028, 0.030, 0.033; the 40 calls of a 5 Mbp seeder run on 12 slots

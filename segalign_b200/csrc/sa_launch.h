@@ -201,7 +201,7 @@ struct SaExtendArgs {
     // says whether the scores allow chains; the device checks the seeds)
     int32_t chain = 0;
     int32_t sweep = 0;   // 1: the sweep takes the hits first (if the scores allow the fast form)
-    uint64_t hits = 0;   // the call's hits, where the caller has read them
+    uint64_t hits = 0;   // the call's hits, where the caller has read them (sa_read_hits)
     // CTAs of a call's sweep, scan and finish (call_lane_ctas, rm_lane_ctas); 0: chosen by sa_launch_extend_lane
     int ctas = 0;
 };
@@ -211,6 +211,23 @@ void sa_launch_extend_lane(SaWork& w, const SaExtendArgs& a, const SaParams& p, 
                            int num_sms, cudaStream_t st, int grid = 0);
 void sa_launch_extend_warp(SaWork& w, const SaExtendArgs& a, const SaParams& p, const SaTuning& t,
                            int num_sms, cudaStream_t st);
+
+// Hits of one segment: its sweep lists at most a quarter of them in practice (4-8%
+// on genomes).  A list that is too small all the same is seen in list_count.
+inline uint64_t sa_sweep_segment(uint64_t list_cap) { return 4 * list_cap & ~31ull; }
+
+// Whether a call of n seed words is to be expected to have more hits than one
+// segment holds: its caller then reads their number before the sweep (10 us of a call of
+// a millisecond and more; a call run as one segment whose list is too small runs twice).
+inline bool sa_expect_segments(uint64_t n, uint64_t num_index, uint64_t nbuckets, uint64_t list_cap) {
+    return (double)n * (double)num_index > (double)nbuckets * (double)sa_sweep_segment(list_cap);
+}
+
+// Hits of the lookup just launched, into h_ctr (pinned where it matters): synchronizes.
+inline cudaError_t sa_read_hits(const SaWork& w, SaCounters* h_ctr, cudaStream_t st) {
+    const cudaError_t e = cudaMemcpyAsync(h_ctr, w.ctr, sizeof(SaCounters), cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
 
 // Whether the parameters allow chains of hits (SaExtK's chain fields).
 bool sa_chain_params(const SaParams& p, const SaTuning& t);
@@ -246,7 +263,7 @@ struct SaResidentView {
     const uint32_t* ref;
     uint32_t ref_len;
     const uint32_t* index;
-    uint64_t nbuckets;
+    uint64_t nbuckets, num_index;
     const uint32_t* pos;
     const uint32_t* q_packed[2];  // forward, reverse complement of the requested buffer
     uint32_t q_len;

@@ -184,19 +184,27 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
     xa.noentropy = v.params.noentropy;
     xa.ctas = v.tuning.call_lane_ctas;
     SaCounters c;
-    for (bool sweep = true;; sweep = false) {  // again without the sweep if its list was too small
+    bool sweep = true, segments = sa_expect_segments(num_seeds, v.num_index, v.nbuckets, w.list_cap);
+    while (true) {
         xa.sweep = sweep ? 1 : 0;
         xa.chain = sweep && v.chain ? 1 : 0;
         SA_CUDA_OK(cudaMemsetAsync(w.ctr, 0, sizeof(SaCounters), st));
         sa_launch_lookup_seeds(w, v.index, (uint32_t)v.nbuckets, v.params, cg.range_ctas, st, xa.chain != 0);
         if (!w.hash_clean) sa_launch_hash_clear(w, st);
         w.hash_clean = false;
+        if (segments && sweep) {
+            SA_CUDA_OK(sa_read_hits(w, &c, st));
+            xa.hits = c.num_hits;
+        }
         sa_launch_extend_lane(w, xa, v.params, cg.lane_tuning, v.num_sms, st, cg.lane_ctas);
         sa_launch_extend_warp(w, xa, v.params, v.tuning, v.num_sms, st);
         SA_CUDA_OK(cudaGetLastError());
         SA_CUDA_OK(cudaMemcpyAsync(&c, w.ctr, sizeof c, cudaMemcpyDeviceToHost, st));
         SA_CUDA_OK(cudaStreamSynchronize(st));
         if (c.list_count <= w.list_cap) break;
+        // the list was too small: again, in segments where one sweep had more hits than that, else without the sweep
+        if (!segments && c.num_hits > sa_sweep_segment(w.list_cap)) segments = true;
+        else sweep = false;
     }
     const int bad = sa_check_set(w, c);
     if (bad == SA_DERR_SURV_OVERFLOW) {
