@@ -53,7 +53,9 @@ void sa_set_error(int, const char* fmt, ...) {
 
 int sa_cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
     sa_set_error(SA_ERR_CUDA, "%s failed: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
-    return e == cudaErrorMemoryAllocation ? SA_ERR_NOMEM : SA_ERR_CUDA;
+    if (e != cudaErrorMemoryAllocation) return SA_ERR_CUDA;
+    cudaGetLastError();  // reported here: not the next call's
+    return SA_ERR_NOMEM;
 }
 
 #define SA_TRY(expr)                   \
@@ -274,17 +276,31 @@ void release_table(DevState& d) {
     d.table_full = 0;
 }
 
-// An array of at least `need` entries: the one there if it fits and is not
-// many times larger.  The caller has synchronized the device, so no call still
-// reads the table.
-int table_array(uint32_t** p, uint64_t* cap, uint64_t need) {
-    if (need == 0) need = 1;
-    if (*p && *cap >= need && *cap / 4 <= need + (1ull << 22)) return SA_OK;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    *cap = 0;
-    SA_CUDA_OK(cudaMalloc(p, 4 * need));
-    *cap = need;
+// Makes d's arrays hold nb buckets and num positions, each the one there if it
+// fits and is not many times larger.  What is new is allocated before the table
+// there is given up, so a failure leaves that in place.  The caller has
+// synchronized the device, so no call still reads the table.
+int take_table_arrays(DevState& d, uint64_t nb, uint64_t num) {
+    uint32_t** const array[2] = {&d.index, &d.pos};
+    uint64_t* const cap[2] = {&d.index_cap, &d.pos_cap};
+    const uint64_t need[2] = {std::max<uint64_t>(nb, 1), std::max<uint64_t>(num, 1)};
+    uint32_t* fresh[2] = {nullptr, nullptr};
+    for (int i = 0; i < 2; ++i) {
+        if (*array[i] && *cap[i] >= need[i] && *cap[i] / 4 <= need[i] + (1ull << 22)) continue;
+        const cudaError_t e = cudaMalloc(&fresh[i], 4 * need[i]);
+        if (e != cudaSuccess) {
+            if (i) cudaFree(fresh[0]);
+            return sa_cuda_fail(e, "cudaMalloc(seed table)", __FILE__, __LINE__);
+        }
+    }
+    for (int i = 0; i < 2; ++i)
+        if (fresh[i]) {
+            cudaFree(*array[i]);
+            *array[i] = fresh[i];
+            *cap[i] = need[i];
+        }
+    d.nbuckets = d.num_index = 0;  // no table until the new one is complete
+    d.table_full = 0;
     return SA_OK;
 }
 
@@ -1512,7 +1528,6 @@ static int build_table_on(DevState& d, const Packed& ref, uint32_t step) {
     uint64_t num_steps = span > 0 ? (uint64_t)span / step : 0;
     uint64_t nb = 1ull << (2 * p.kmer_size);
     const uint64_t cap = num_steps ? num_steps : 1;
-    d.nbuckets = d.num_index = 0;  // no table until this one is complete
     SA_CUDA_OK(cudaDeviceSynchronize());
     // keys and positions, twice (the sort's two buffers), one of the position
     // arrays being the table's own; per-CTA counts and digit histograms
@@ -1525,8 +1540,7 @@ static int build_table_on(DevState& d, const Packed& ref, uint32_t step) {
         SA_CUDA_OK(cudaMalloc(&d.table_ws, need));
         d.table_ws_cap = need;
     }
-    SA_TRY(table_array(&d.index, &d.index_cap, nb));
-    SA_TRY(table_array(&d.pos, &d.pos_cap, cap));
+    SA_TRY(take_table_arrays(d, nb, cap));
     char* ws = (char*)d.table_ws;
     uint32_t* const key0 = (uint32_t*)ws;
     uint32_t* const key1 = (uint32_t*)(ws + arr);
@@ -1576,7 +1590,6 @@ int sa_generate_seed_pos_table(const char* ref_str, size_t start_addr, uint32_t 
     const bool resident = ref_str == g.last_ref_ptr && start_addr == g.last_ref_start &&
                           ref_length == g.last_ref_len && g.last_ref_ptr;
     for (auto& d : g.devs) {
-        d.table_full = 0;
         if (resident && d.ref.data) {
             SA_TRY(build_table_on(d, d.ref, step));
             if (step == 1) d.table_full = sa_shape_id(g.params);
@@ -1612,11 +1625,8 @@ int sa_send_seed_pos_table(const uint32_t* index_table, uint32_t index_table_siz
     std::unique_lock<std::shared_mutex> dev_wide(g_capture_mu);
     for (auto& d : g.devs) {
         SA_CUDA_OK(cudaSetDevice(d.dev));
-        d.table_full = 0;
-        d.nbuckets = d.num_index = 0;
         SA_CUDA_OK(cudaDeviceSynchronize());
-        SA_TRY(table_array(&d.index, &d.index_cap, index_table_size));
-        SA_TRY(table_array(&d.pos, &d.pos_cap, num_index));
+        SA_TRY(take_table_arrays(d, index_table_size, num_index));
         SA_CUDA_OK(cudaMemcpy(d.index, index_table, 4ull * index_table_size, cudaMemcpyHostToDevice));
         if (num_index) SA_CUDA_OK(cudaMemcpy(d.pos, pos_table, 4ull * num_index, cudaMemcpyHostToDevice));
         d.nbuckets = index_table_size;
