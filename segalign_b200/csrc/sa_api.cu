@@ -400,7 +400,6 @@ int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_c
         {(void**)&w.hset.keys, 16 * 2 * surv_cap},
         {(void**)&w.hset.score, 4 * 2 * surv_cap},
         {(void**)&w.out, sizeof(SaRec) * surv_cap},
-        {(void**)&w.out_scope, 4 * surv_cap},
         {(void**)&w.scope_count, batch ? 4 * nunits : 0},
         {(void**)&w.ctr, sizeof(SaCounters)},
         {(void**)&w.desc, sizeof(SaCallDesc)},
@@ -617,8 +616,6 @@ int run_call(Slot* s, const uint64_t* seeds, uint32_t n, int rev, const Packed& 
     hd->num_seeds = n;
     hd->max_hits = max_hits_now();
     hd->num_units = 1;
-    hd->num_scopes_max = SA_MAX_ITERS;
-    hd->rm_exclude_diag = (uint32_t)g.rm_exclude_diag;
     SaUnit* u = s->h_units;
     u[0].q_packed = q.data;
     u[0].q_len = (uint32_t)q.len;
@@ -811,8 +808,6 @@ int run_batch_group(DevState& d, Slot* s, const SaResolvedUnit* units, uint32_t 
     hd->num_seeds = slots;
     hd->max_hits = max_hits_now();
     hd->num_units = n;
-    hd->num_scopes_max = n;
-    hd->rm_exclude_diag = 0;
     const int Gr = std::min(g.tuning.range_ctas, SA_MAX_CTAS);
     PhaseTimer tm(s);
     tm.mark(0);

@@ -13,8 +13,6 @@ struct SaCallDesc {
     uint64_t num_seeds;     // seed words (plain) or seed slots (batched)
     uint64_t max_hits;      // MAX_HITS (dedup iteration size)
     uint32_t num_units;
-    uint32_t num_scopes_max;
-    uint32_t rm_exclude_diag;
     uint32_t pad;
 };
 
@@ -104,7 +102,6 @@ struct SaWork {
     SaHashSet hset;         // [2 * surv_cap] slots: distinct HSPs of the call; used list aliases rec[1]
     bool hash_clean;        // host: every slot of hset is empty (no full clear needed)
     SaRec* out;             // [surv_cap] the sweep's list
-    uint32_t* out_scope;
     uint32_t* scope_count;  // [SA_MAX_UNITS] records per batch unit
     // counters + descriptor
     SaCounters* ctr;

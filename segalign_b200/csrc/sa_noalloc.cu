@@ -45,7 +45,7 @@ constexpr uint64_t kParts[] = {
     sizeof(SaLongHit) * SA_NOALLOC_LONG_CAP,             // long queue
     sizeof(SaRec) * kSurv, sizeof(SaRec) * kSurv, 4 * kSurv, 4 * kSurv,  // rec[2], scope[2]
     16 * 2 * kSurv, 4 * 2 * kSurv,                       // HSP set: keys, scores
-    sizeof(SaRec) * kSurv, 4 * kSurv,                    // out, out_scope
+    sizeof(SaRec) * kSurv,                               // out
     sizeof(SaCounters), sizeof(SaCallDesc), sizeof(SaUnit) * SA_NOALLOC_UNITS,
 };
 constexpr uint64_t total_bytes() {
@@ -110,7 +110,6 @@ void carve(void* base, SaWork& w) {
     take((void**)&w.hset.keys);
     take((void**)&w.hset.score);
     take((void**)&w.out);
-    take((void**)&w.out_scope);
     take((void**)&w.ctr);
     take((void**)&w.desc);
     take((void**)&w.units);
@@ -163,7 +162,6 @@ int sa_seed_and_filter_noalloc(const uint64_t* seeds, uint32_t num_seeds, int re
     desc.num_seeds = num_seeds;
     desc.max_hits = v.max_hits;
     desc.num_units = 1;
-    desc.num_scopes_max = SA_MAX_ITERS;
     SaUnit unit{};
     unit.q_packed = q;
     unit.q_len = v.q_len;
