@@ -1784,7 +1784,7 @@ static bool sa_lane_fast_form(const SaParams& p, int step) {
 
 // The sweep and the scans after it use the fast form, and what passes
 // between them fits its 16-bit fields.
-static bool sa_sweep_params(const SaParams& p, const SaTuning& t) {
+bool sa_sweep_params(const SaParams& p, const SaTuning& t) {
     int mx = 0;
     for (int i = 0; i < 64; ++i) mx = std::max(mx, p.sub_mat[i]);
     return sa_lane_fast_form(p, t.step_bases) && sa_lane_fast_form(p, SA_SWEEP_LEFT) && p.xdrop <= 0xffff &&

@@ -226,6 +226,9 @@ inline cudaError_t sa_read_hits(const SaWork& w, SaCounters* h_ctr, cudaStream_t
     return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
+// Whether the scores allow the sweep (and the scans and finish kernel after it); else
+// every hit goes to the lane kernel.
+bool sa_sweep_params(const SaParams& p, const SaTuning& t);
 // Whether the parameters allow chains of hits (SaExtK's chain fields).
 bool sa_chain_params(const SaParams& p, const SaTuning& t);
 
