@@ -112,24 +112,8 @@ def seeder_calls(query_len: int):
 EXTEND_KERNELS = "sa_k_sweep, sa_k_scan and sa_k_finish"  # the "extend_lane" phase of the default parameters
 
 
-def lane_traffic(hits: float, workload: str):
-    """DRAM bytes (read + write) of one pass's sweep, scans and finish, scaled by
-    hits from the ncu capture of this workload recorded in
-    profiles/extend_lane_dram.json; (None, why) if there is none."""
-    path = os.path.join(ROOT, "profiles", "extend_lane_dram.json")
-    try:
-        with open(path) as f:
-            d = json.load(f)[workload]
-        if d["kernel"] != EXTEND_KERNELS:
-            return None, f"the capture recorded for the {workload} workload is of {d['kernel']}"
-        per_hit = float(d["dram_bytes"]) / float(d["hits"])
-    except (OSError, KeyError, ValueError, ZeroDivisionError, TypeError):
-        return None, f"no ncu capture recorded for the {workload} workload"
-    return per_hit * hits, f"ncu dram bytes per hit of {d['workload']} x this launch's hits"
-
-
 def lane_limit(workload: str):
-    """The sweep's measured limit (ncu) recorded beside the DRAM traffic in
+    """The sweep's measured limit (ncu) recorded in
     profiles/extend_lane_dram.json, or None."""
     try:
         with open(os.path.join(ROOT, "profiles", "extend_lane_dram.json")) as f:
@@ -610,9 +594,9 @@ def run_ours(args):
     alg_bytes = 24.0 * nnz + 4.0 * hits + 24.0 * tiles + 16.0 * surv
     peak, peak_src = peaks()
     achieved = alg_bytes / (lane_ms_avg / 1000.0) / 1e9
-    traffic, traffic_src = lane_traffic(hits, args.workload)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "traffic_source": traffic_src, "kernel": EXTEND_KERNELS,
+                "traffic": None, "traffic_source": "DRAM counters are captured on small cases only",
+                "kernel": EXTEND_KERNELS,
                 "peak_source": peak_src, "alg_bytes_per_launch": alg_bytes, "launch_ms": lane_ms_avg,
                 "limit": lane_limit(args.workload)}
 
@@ -850,8 +834,7 @@ def run_large(sf, args, flush, barrier) -> dict:
            "phase_ms": {"lookup": tb["lookup_ms"], "extend_lane": tb["lane_ms"], "extend_warp": tb["warp_ms"],
                         "dedup": tb["dedup_ms"]},
            "roofline": {"kernel": EXTEND_KERNELS, "achieved": alg / (tb["lane_ms"] / 1000) / 1e9, "peak": peak,
-                        "frac": alg / (tb["lane_ms"] / 1000) / 1e9 / peak, "unit": "GB/s",
-                        "traffic": lane_traffic(st["num_hits"], "large")[0]}}
+                        "frac": alg / (tb["lane_ms"] / 1000) / 1e9 / peak, "unit": "GB/s", "traffic": None}}
     outs = tb["outs"]
     # plain path with host buffers on the same units (seeds with transitions on the host)
     sf.set_timing(False)
