@@ -112,6 +112,16 @@ def seeder_calls(query_len: int):
 EXTEND_KERNELS = "sa_k_sweep, sa_k_scan and sa_k_finish"  # the "extend_lane" phase of the default parameters
 
 
+def extension_bytes(st: dict, target_bp: int, query_bp: int) -> float:
+    """Bytes that the extension of a pass cannot do without: 24 per hit-bearing
+    seed (E, lo, j, scope, unit), 4 per hit (its target position), either strand's
+    packed query and the packed target once (4 bits per base), 16 per HSP.  The
+    statistic `tiles` is no measure of bytes: it counts the tiles of hits that are not
+    scanned because another hit of their diagonal gives their HSP."""
+    return (24.0 * st["seeds_with_hits"] + 4.0 * st["num_hits"] + 0.5 * target_bp + 2 * 0.5 * query_bp
+            + 16.0 * st["num_hsps"])
+
+
 def lane_limit(workload: str):
     """The sweep's measured limit (ncu) recorded in
     profiles/extend_lane_dram.json, or None."""
@@ -586,12 +596,9 @@ def run_ours(args):
     job = job_figures(ms_step, float(hits), float(hsps), dist)
     ms_step_max, hits_all, hsps_all, value = job["ms_per_step"], job["extensions"], job["hsps"], job["value"]
 
-    # roofline of the extension (sweep, scans, finish): algorithmic bytes
-    # = 24 B per hit-bearing seed (E, lo, j, scope, unit) + 4 B per hit (pos)
-    # + 24 B per 32-base tile scanned (2 sequences x 32 bases x 3 bits)
-    # + 16 B per surviving HSP record
+    # roofline of the extension (sweep, scans, finish)
     lane_ms_avg = tb["lane_ms"]
-    alg_bytes = 24.0 * nnz + 4.0 * hits + 24.0 * tiles + 16.0 * surv
+    alg_bytes = extension_bytes(st, len(w.target), len(w.query))
     peak, peak_src = peaks()
     achieved = alg_bytes / (lane_ms_avg / 1000.0) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -824,7 +831,7 @@ def run_large(sf, args, flush, barrier) -> dict:
     tb = timed_batch_steps(sf, units, 2, flush, barrier)
     st = tb["stats"]
     wall = sum(tb["wall_s"]) / len(tb["wall_s"])
-    alg = 24.0 * st["seeds_with_hits"] + 4.0 * st["num_hits"] + 24.0 * st["tiles"] + 16.0 * st["survivors"]
+    alg = extension_bytes(st, len(w.target), len(q))
     peak, _ = peaks()
     res = {"workload": f"600 Mbp target (12 chr) x the first {len(q) / 1e6:.0f} Mbp of a 600 Mbp query, GC 41%, "
                        "45% repeats, 12of19 with one transition (13 seed words per position), both strands, "
