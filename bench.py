@@ -646,10 +646,10 @@ def run_ours(args):
         e2e_s = (time.perf_counter() - t0) / k_e2e
         e2e_s_max = allreduce(e2e_s, "max")
         e2e_hits = allreduce(float(sst["num_hits"]), "sum")
-        # per call: seed words + call descriptor (32 B) + unit (32 B) + scope flags (1 KiB) up;
-        # counters (128 B) + header and HSP records (16 B each) down
-        h2d = sst["num_seeds"] * 8 + sst["num_calls"] * (32 + 32 + 1024)
-        d2h = (sst["num_hsps"] + sst["num_calls"]) * 16 + sst["num_calls"] * 128
+        # per call: seed words (8 B each) and one block of zeroed counters, descriptor and unit (544 B) up;
+        # counters (176 B) and HSP records (16 B each) down
+        h2d = sst["num_seeds"] * 8 + sst["num_calls"] * 544
+        d2h = sst["num_hsps"] * 16 + sst["num_calls"] * 176
         out["e2e"] = {"value": e2e_hits / e2e_s_max, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                       "d2h_bytes_per_step": int(d2h), "path": f"sa_seed_and_filter per 250 kbp unit from "
                       f"{e2e_threads} host threads (C++ seeder), host wall time", "steps": k_e2e}
