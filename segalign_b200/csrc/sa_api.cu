@@ -350,17 +350,17 @@ void free_slot(Slot* s) {
     delete s;
 }
 
-// Carves one slot workspace out of a single device allocation.
-// Workspace kinds: plain calls (host seed words), batched passes (device
-// seeding over query windows), or both (passes of coalesced plain calls, and
-// plain calls one at a time), with at most `units` units per pass.
 // Offsets in a slot's block of counters, descriptor and units, on the device (consecutive parts
 // of the arena) and in h_up.
 constexpr size_t kUpDesc = 256, kUpUnits = 512;
 static_assert(sizeof(SaCounters) <= kUpDesc && sizeof(SaCallDesc) <= kUpUnits - kUpDesc, "a part of 256 bytes each");
 
+// Workspace kinds: plain calls (host seed words), batched passes (device
+// seeding over query windows), or both (passes of coalesced plain calls, and
+// plain calls one at a time), with at most `units` units per pass.
 enum SlotKind { kSlotPlain = 0, kSlotBatch = 1, kSlotBoth = 2 };
 
+// Carves one slot workspace out of a single device allocation.
 int make_slot(int dev_idx, uint64_t seed_cap, uint64_t surv_cap, uint64_t long_cap, Slot** out,
               SlotKind kind = kSlotPlain, uint64_t units = SA_MAX_UNITS) {
     const bool batch = kind != kSlotPlain, host_seeds = kind != kSlotBatch;
@@ -2052,7 +2052,7 @@ int sa_set_tuning_param(const char* name, int value) {
     }
     if (n == "rm_lane_ctas") {
         if (value < 0 || value > 8 * SA_MAX_CTAS) {
-            sa_set_error(SA_ERR_ARG, "rm_lane_ctas must be 0 (the batched grid) .. %d (got %d)", 8 * SA_MAX_CTAS,
+            sa_set_error(SA_ERR_ARG, "rm_lane_ctas must be 0 (the default grid) .. %d (got %d)", 8 * SA_MAX_CTAS,
                          value);
             return SA_ERR_ARG;
         }
@@ -2061,7 +2061,7 @@ int sa_set_tuning_param(const char* name, int value) {
     }
     if (n == "call_lane_ctas") {
         if (value < 0 || value > 8 * SA_MAX_CTAS) {
-            sa_set_error(SA_ERR_ARG, "call_lane_ctas must be 0 (half the batched grid) .. %d (got %d)",
+            sa_set_error(SA_ERR_ARG, "call_lane_ctas must be 0 (the default grid) .. %d (got %d)",
                          8 * SA_MAX_CTAS, value);
             return SA_ERR_ARG;
         }

@@ -810,11 +810,7 @@ __device__ __forceinline__ void sa_keep_candidates(const SaExtK& a, bool on, uin
     sa_hash_note_used(a.hset, &a.ctr->hash_used, claimed);
 }
 
-// Keep test of `n` (<= 32) ring candidates from slot `head` on, one per lane:
-// entropy factor from the per-base match counts over the HSP when the total
-// is in the entropy range (src/seed_filter.cu:580-621), then insertion of the
-// kept ones into the call's set of distinct HSPs (rm: query start flipped on
-// the reverse strand, repeat_masker_src/seed_filter.cu:704-707).  Called by
+// Keep test of `n` (<= 32) ring candidates from slot `head` on, one per lane, by
 // the whole warp; leaves the slots free for reuse.
 __device__ __forceinline__ void sa_flush_candidates(const SaExtK& a, const uint4* s_em, const uint2* s_ex,
                                                     uint32_t head, uint32_t n) {

@@ -134,11 +134,12 @@ struct SaTuning {
                          // iteration (with substeps > 1) instead of at the next one
     int call_range_ctas; // CTAs of the range-partitioned kernels of a plain or rm call (at most
                          // MAX_SEEDS seed words: fewer CTAs than a batch needs)
-    int call_lane_ctas;  // CTAs of a plain call's lane kernel; 0: half of the batched
-                         // grid, so that concurrent calls' kernels share the SMs and fill
-                         // each other's ramp-up and tail instead of queueing
-    // a repeat-masker call's lane kernel (its hits are windowed and its calls
-    // large): CTAs (0: the batched grid), steps per iteration, switch_now
+    int call_lane_ctas;  // CTAs of a plain call's sweep, scan and finish kernels; 0: 3 per SM,
+                         // so that concurrent calls' kernels share the SMs and fill each
+                         // other's ramp-up and tail instead of queueing.  Of the lane kernel in
+                         // their place: 0: half of a batch's grid
+    // a repeat-masker call's (its hits are windowed and its calls large): CTAs (0: 3 per
+    // SM, of the lane kernel ext_ctas_per_sm), steps per iteration, switch_now
     int rm_lane_ctas, rm_substeps, rm_switch_now;
 };
 
@@ -277,7 +278,7 @@ struct SaResidentView {
 int sa_resident_view(uint32_t buffer, SaResidentView* v);
 
 // Grids and lane-kernel settings of one plain (mode 0) or repeat-masker
-// (mode 1) call: CTAs of the range-partitioned kernels (lookup, dedup), CTAs of
+// (mode 1) call: CTAs of the range-partitioned kernels (lookup), CTAs of
 // the lane kernel, and the tuning the lane kernel runs with.
 struct SaCallGrids {
     int range_ctas;
