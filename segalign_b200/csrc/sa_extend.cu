@@ -436,7 +436,6 @@ __device__ __forceinline__ uint32_t sa_swept_pos(int at) {
 }
 
 #define SA_SWEEP_BUF 128  // unfinished hits a warp gathers
-#define SA_SWEEP_END (1ull << 48)  // sweep cursor past every run
 
 template <bool TRANS>
 __global__ void __launch_bounds__(256, 4)
@@ -490,8 +489,6 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(&ctr->list_count, (unsigned long long)kept);
         at = __shfl_sync(SA_FULL, at, 0);
-        // too small a list: the call runs again, the rest of this sweep is given up
-        if (lane == 0 && at + kept > a.list_cap) atomicMax(&ctr->sweep_cursor, SA_SWEEP_END);
         for (uint32_t i = lane; i < 2 * kept; i += 32)
             if (at + (i >> 1) < a.list_cap) a.list[2 * at + i] = (i & 1) ? swept[i >> 1] : buf[i >> 1];
         __syncwarp();
@@ -574,14 +571,15 @@ sa_k_sweep(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P,
                         if (i == 4) tl = stop_l ? 2 : 3;  // tiles of both scans, if they stop
                     }
                     x.y = sa_swept_word(p, at);
-                    // where a window reaches past a sequence end, it holds scores of padding: nothing
-                    // of it is passed on, and the scans start anew
+                    // where a window reaches past a sequence end, it holds scores of padding: neither scan
+                    // has stopped, and both start anew (what else is passed on is not looked at)
                     const bool inside = min(rl, ql) >= SA_SWEEP_LEFT && (uint64_t)rl + SA_SWEEP_RIGHT <= a.ref_len &&
                                         (uint64_t)ql + SA_SWEEP_RIGHT <= U.q_len;
-                    left = !inside || !stop_r || !stop_l || (int)(float)(best_r + (at >> SA_SWEEP_SH)) >= a.hspthresh;
-                    x.z = inside ? x.z | (sa_swept_pos(at) << 8) | SA_SWEPT_SEEN | (stop_r ? SA_SWEPT_STOP_R : 0u) |
-                                       (stop_l ? SA_SWEPT_STOP_L : 0u) | (tl == 3 ? SA_SWEPT_TILE_2 : 0u)
-                                 : 0u;
+                    stop_r = stop_r && inside;
+                    stop_l = stop_l && inside;
+                    left = !stop_r || !stop_l || (int)(float)(best_r + (at >> SA_SWEEP_SH)) >= a.hspthresh;
+                    x.z |= (sa_swept_pos(at) << 8) | (inside ? SA_SWEPT_SEEN : 0u) | (stop_r ? SA_SWEPT_STOP_R : 0u) |
+                           (stop_l ? SA_SWEPT_STOP_L : 0u) | (tl == 3 ? SA_SWEPT_TILE_2 : 0u);
                     if (!left) tiles += tl;
                     if (!(stop_r && !stop_l) && sa_sweep_margin(a, U, rl, ql)) rec.w |= SA_CHAIN_DROP;
                 }
@@ -1552,10 +1550,11 @@ sa_k_finish(const __grid_constant__ SaExtK a, const __grid_constant__ SaParams P
 
 // Between the segments of a call: the list starts again (the queue of long hits goes
 // on, for the warp kernel after the last one).  An overflow stays to be seen, and
-// the sweeps after it have nothing left to do.
+// the sweeps after it find their cursor past every run.  (To end the sweep that
+// overflows, by a test where it writes or takes runs, cost every sweep 0.6%.)
 __global__ void sa_k_next_segment(SaCounters* ctr, uint64_t list_cap) {
-    if (ctr->list_count > list_cap) return;
-    ctr->list_count = ctr->sweep_cursor = ctr->scan_cursor = 0;
+    if (ctr->list_count > list_cap) ctr->sweep_cursor = 1ull << 48;
+    else ctr->list_count = ctr->sweep_cursor = ctr->scan_cursor = 0;
 }
 
 // ---------------------------------------------------------------------------
