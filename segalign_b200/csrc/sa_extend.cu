@@ -385,8 +385,8 @@ __device__ __forceinline__ uint32_t sa_chain_test(const SaExtK& a, int kmer, con
 // Bound by the L1 data pipe (83%: 96 table lookups and 128 wavefronts of target
 // loads in about 250 per round), with the ALU pipe and issue at 70%.  On a 2.5 Mbp query
 // against the 100 Mbp genome (60.2 M hits, both strands, one B200): every hit in
-// the lane kernel 5.65 ms; sweep 2.00, scans 0.81, finish 0.64: 3.31 ms, its launches
-// included (with the lane kernel after the sweep 3.75, and 4.79 without chains).  The chain test on all hits as they were
+// the lane kernel 5.65 ms; sweep 2.04, scans 0.73, finish 0.51 ms, together 3.29 between events
+// (with the lane kernel after the sweep 3.75, and 4.79 without chains).  The chain test on all hits as they were
 // scored, with the rounds split evenly over the warps, made the sweep 2.33 ms.
 // Lane phase of 24 Mbp: 55.0 -> 30.8 ms.
 // ---------------------------------------------------------------------------
@@ -1429,7 +1429,7 @@ __device__ __forceinline__ uint32_t sa_listed_sides(SaListed& e) {
 // after it (sa_chain_members), which survive if its HSP is kept; and the keep
 // test.  A warp sorts its records into those that start chains and candidates,
 // and takes either 32 at a time: with a record per lane throughout the kernel
-// took 1.27 ms where this takes 0.64.  Candidates that the set holds already (most)
+// took 1.27 ms where this takes 0.51 (60.2 M hits).  Candidates that the set holds already (most)
 // end with that look-up; the others gather again, because a few lanes of nearly every batch
 // counting matches cost 0.07 ms.  The chains are 0.2 ms.
 #define SA_FINISH_RING 128
