@@ -112,7 +112,8 @@ struct SaCounters {
 
 // Waits until the kernels before this one in the stream are done and their
 // writes are seen; a no-op in a kernel launched the plain way.  What those write is
-// not read through const __restrict__ pointers, whose loads need not stay behind it.
+// not read through const __restrict__ pointers, whose loads need not stay behind it, unless
+// the address comes from a plain read after it (the seed search, from the seeds' number).
 __device__ __forceinline__ void sa_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Lets the next kernel's CTAs take free places on the chip already.
